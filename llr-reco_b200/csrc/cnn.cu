@@ -804,10 +804,10 @@ int ensure_workspace(llr_cnn* n, long long vox) {
   int cmax = 0;
   for (int l = 0; l < n->n_layers; ++l) cmax = std::max(cmax, std::max(n->cin[l], n->cout[l]));
   for (int l = 1; l < n->n_layers; ++l)
-    LLR_CUDA_TRY(cudaMalloc((void**)&n->act[l], sizeof(float) * vox * n->cin[l]));
-  LLR_CUDA_TRY(cudaMalloc((void**)&n->d_g0, sizeof(float) * vox * cmax));
-  LLR_CUDA_TRY(cudaMalloc((void**)&n->d_g1, sizeof(float) * vox * cmax));
-  LLR_CUDA_TRY(cudaMalloc((void**)&n->d_out, sizeof(float) * vox * n->cout.back()));
+    LLR_CUDA_TRY(device_alloc((void**)&n->act[l], sizeof(float) * vox * n->cin[l]));
+  LLR_CUDA_TRY(device_alloc((void**)&n->d_g0, sizeof(float) * vox * cmax));
+  LLR_CUDA_TRY(device_alloc((void**)&n->d_g1, sizeof(float) * vox * cmax));
+  LLR_CUDA_TRY(device_alloc((void**)&n->d_out, sizeof(float) * vox * n->cout.back()));
   n->cap_vox = vox;
   return LLR_OK;
 }
@@ -864,19 +864,19 @@ int llr_cnn_create(int32_t n_layers, const int32_t* channels, int32_t device, ui
   n->act.assign(n_layers, nullptr);
   auto fail = [&](int st) { llr_cnn_destroy(n); return st; };
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = cudaMalloc((void**)&n->d_master, sizeof(float) * off);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&n->d_grad, sizeof(float) * off);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&n->d_m, sizeof(float) * off);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&n->d_v, sizeof(float) * off);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&n->d_wb, sizeof(uint16_t) * wtot);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&n->d_wt, sizeof(uint16_t) * wtot);
+  if (e == cudaSuccess) e = device_alloc((void**)&n->d_master, sizeof(float) * off);
+  if (e == cudaSuccess) e = device_alloc((void**)&n->d_grad, sizeof(float) * off);
+  if (e == cudaSuccess) e = device_alloc((void**)&n->d_m, sizeof(float) * off);
+  if (e == cudaSuccess) e = device_alloc((void**)&n->d_v, sizeof(float) * off);
+  if (e == cudaSuccess) e = device_alloc((void**)&n->d_wb, sizeof(uint16_t) * wtot);
+  if (e == cudaSuccess) e = device_alloc((void**)&n->d_wt, sizeof(uint16_t) * wtot);
   n->loss_cap = 148 * 16;
-  if (e == cudaSuccess) e = cudaMalloc((void**)&n->d_loss, sizeof(double) * n->loss_cap);
+  if (e == cudaSuccess) e = device_alloc((void**)&n->d_loss, sizeof(double) * n->loss_cap);
   long long maxw = 0;
   for (int l = 0; l < n_layers; ++l) maxw = std::max(maxw, 27LL * channels[l] * channels[l + 1] + channels[l + 1]);
   n->part_cap = maxw * 2 * 148;
-  if (e == cudaSuccess) e = cudaMalloc((void**)&n->d_part, sizeof(float) * n->part_cap);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&n->d_err, sizeof(int));
+  if (e == cudaSuccess) e = device_alloc((void**)&n->d_part, sizeof(float) * n->part_cap);
+  if (e == cudaSuccess) e = device_alloc((void**)&n->d_err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(n->d_err, 0, sizeof(int));
   if (e != cudaSuccess) return fail(cuda_error(e, "cudaMalloc", __FILE__, __LINE__));
   e = cudaMemset(n->d_master, 0, sizeof(float) * off);
@@ -912,6 +912,7 @@ int llr_cnn_destroy(llr_cnn* n) {
                   (void*)n->d_g0, (void*)n->d_g1, (void*)n->d_out, (void*)n->d_part, (void*)n->d_loss,
                   (void*)n->d_err})
     if (p) cudaFree(p);
+  scratch_trim();
   delete n;
   return LLR_OK;
 }

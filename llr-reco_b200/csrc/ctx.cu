@@ -89,7 +89,7 @@ template <class T>
 int dalloc(T** p, size_t n) {
   *p = nullptr;
   if (n == 0) n = 1;
-  LLR_CUDA_TRY(cudaMalloc((void**)p, n * sizeof(T)));
+  LLR_CUDA_TRY(device_alloc((void**)p, n * sizeof(T)));
   return LLR_OK;
 }
 
@@ -120,7 +120,7 @@ int make_plan(llr_ctx* c) {
   if (ws > c->fft_work_bytes) {
     dfree(c->d_fft_work);
     c->d_fft_work = nullptr;
-    LLR_CUDA_TRY(cudaMalloc(&c->d_fft_work, ws));
+    LLR_CUDA_TRY(device_alloc(&c->d_fft_work, ws));
     c->fft_work_bytes = ws;
   }
   r = cufftSetWorkArea(c->plan_fwd, c->d_fft_work);
@@ -459,6 +459,7 @@ int llr_ctx_destroy(llr_ctx* c) {
   dfree(c->d_obj); dfree(c->d_blk_nuc);
   dfree(c->d_block_stat); dfree(c->d_fb); dfree(c->d_gram); dfree(c->d_blk_ra); dfree(c->d_fft_tw); dfree(c->d_err); dfree(c->d_vwide); dfree(c->d_wavelet_work); dfree(c->d_fft_work);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
+  scratch_trim();
   delete c;
   return LLR_OK;
 }

@@ -151,7 +151,7 @@ int llr_dti_fit_dev(const llr_cf32* d_dwi, int32_t nq, const llr_cf32* d_b0, int
   LLR_TRY(design_pinv(b_vals, b_vecs, nq, pinv));
   cudaStream_t s = (cudaStream_t)stream;
   float* d_pinv = nullptr;
-  LLR_CUDA_TRY(cudaMallocAsync((void**)&d_pinv, sizeof(float) * pinv.size(), s));
+  LLR_CUDA_TRY(scratch_alloc((void**)&d_pinv, sizeof(float) * pinv.size(), s));
   cudaError_t e = cudaMemcpyAsync(d_pinv, pinv.data(), sizeof(float) * pinv.size(), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) {
     const long long blocks = std::min<long long>((n_vox + 255) / 256, 148LL * 32);
@@ -178,9 +178,9 @@ int llr_dti_fit(const llr_cf32* dwi, int32_t nq, const llr_cf32* b0, int32_t nb0
     cudaFree(d_out);
     return code;
   };
-  cudaError_t e = cudaMalloc((void**)&d_dwi, sizeof(float2) * (size_t)n_vox * nq);
-  if (e == cudaSuccess && nb0 > 0) e = cudaMalloc((void**)&d_b0, sizeof(float2) * (size_t)n_vox * nb0);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_out, sizeof(float) * (size_t)n_vox * kDtiOut);
+  cudaError_t e = device_alloc((void**)&d_dwi, sizeof(float2) * (size_t)n_vox * nq);
+  if (e == cudaSuccess && nb0 > 0) e = device_alloc((void**)&d_b0, sizeof(float2) * (size_t)n_vox * nb0);
+  if (e == cudaSuccess) e = device_alloc((void**)&d_out, sizeof(float) * (size_t)n_vox * kDtiOut);
   if (e == cudaSuccess) e = cudaMemcpy(d_dwi, dwi, sizeof(float2) * (size_t)n_vox * nq, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && nb0 > 0)
     e = cudaMemcpy(d_b0, b0, sizeof(float2) * (size_t)n_vox * nb0, cudaMemcpyHostToDevice);

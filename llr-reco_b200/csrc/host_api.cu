@@ -109,12 +109,26 @@ int launch_conj_transpose(const float2* in, float2* out, int m, int n, int batch
 int launch_finalize(const double* partials, int np, double scale, double* hist, long long cap, long long* it,
                     int advance, double* out, cudaStream_t s);
 
+// RAII scratch of one call on one stream.
+struct Scratch {
+  void* p = nullptr;
+  cudaStream_t s;
+  explicit Scratch(cudaStream_t stream) : s(stream) {}
+  ~Scratch() { if (p) cudaFreeAsync(p, s); }
+  int alloc(size_t bytes) {
+    cudaError_t e = scratch_alloc(&p, bytes, s);
+    if (e != cudaSuccess) { p = nullptr; return cuda_error(e, "scratch_alloc", __FILE__, __LINE__); }
+    return LLR_OK;
+  }
+  template <class T> T* as() { return reinterpret_cast<T*>(p); }
+};
+
 // RAII device buffer for host-slice entry points.
 struct DevBuf {
   void* p = nullptr;
   ~DevBuf() { if (p) cudaFree(p); }
   int alloc(size_t bytes) {
-    cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
+    cudaError_t e = device_alloc(&p, bytes);
     if (e != cudaSuccess) { p = nullptr; return cuda_error(e, "cudaMalloc", __FILE__, __LINE__); }
     return LLR_OK;
   }
@@ -377,11 +391,11 @@ static int batch_prox(int m, int n, int mode, int rank, float lam, int batch, ll
   int* fb = nullptr;
   float2* gram = nullptr;
   // fallback list + count, then the per-block kept counts + queue counter
-  LLR_CUDA_TRY(cudaMallocAsync((void**)&fb, sizeof(int) * (2 * (size_t)batch + 2), s));
-  cudaError_t e = cudaMallocAsync((void**)&gram, sizeof(float2) * (size_t)batch * (size_t)prox_gram_stride(n), s);
+  LLR_CUDA_TRY(scratch_alloc((void**)&fb, sizeof(int) * (2 * (size_t)batch + 2), s));
+  cudaError_t e = scratch_alloc((void**)&gram, sizeof(float2) * (size_t)batch * (size_t)prox_gram_stride(n), s);
   if (e != cudaSuccess) {
     cudaFreeAsync(fb, s);
-    return cuda_error(e, "cudaMallocAsync", __FILE__, __LINE__);
+    return cuda_error(e, "scratch_alloc", __FILE__, __LINE__);
   }
   op.fb_list = fb;
   op.fb_count = fb + batch;
@@ -393,11 +407,11 @@ static int batch_prox(int m, int n, int mode, int rank, float lam, int batch, ll
   float2* vwide = nullptr;
   if ((n > 64 && n <= kProxMaxN) || prox_needs_wide_fallback(m, n)) {   // wide Jacobi kernel scratch
     op.vwide_ctas = wide_jacobi_ctas();
-    e = cudaMallocAsync((void**)&vwide, sizeof(float2) * (size_t)op.vwide_ctas * (size_t)wide_v_stride(), s);
+    e = scratch_alloc((void**)&vwide, sizeof(float2) * (size_t)op.vwide_ctas * (size_t)wide_v_stride(), s);
     if (e != cudaSuccess) {
       cudaFreeAsync(fb, s);
       cudaFreeAsync(gram, s);
-      return cuda_error(e, "cudaMallocAsync", __FILE__, __LINE__);
+      return cuda_error(e, "scratch_alloc", __FILE__, __LINE__);
     }
     op.vwide = vwide;
   }
@@ -515,7 +529,7 @@ int llr_wavelet_denoise_dev(llr_cf32* d_vols, const int32_t* vs, int32_t nvol, i
   LLR_TRY(wavelet_plan_init(&p, vs[0], vs[1], vs[2], moments, levels));
   if (p.levels == 0) return set_error(LLR_ERR_UNSUPPORTED, "volume too small for one wavelet level");
   const size_t per = wavelet_workspace_elems(p, 1);
-  DevBuf w;
+  Scratch w((cudaStream_t)stream);
   LLR_TRY(w.alloc(per * sizeof(float2)));
   const long long V = (long long)vs[0] * vs[1] * vs[2];
   for (int v = 0; v < nvol; ++v)
@@ -529,7 +543,7 @@ int llr_hard_project_dev(llr_cf32* d_x, const llr_cf32* d_y, int64_t n, double* 
   if (!d_x || !d_y || n < 0) return set_error(LLR_ERR_INVALID, "bad hard_project arguments");
   cudaStream_t s = (cudaStream_t)stream;
   const int nb = 296;
-  DevBuf part;
+  Scratch part(s);
   LLR_TRY(part.alloc(sizeof(double) * (nb + 1)));
   LLR_TRY(launch_hard_project((float2*)d_x, (const float2*)d_y, n, part.as<double>(), nb, s));
   LLR_TRY(launch_finalize(part.as<double>(), nb, 1.0, nullptr, 0, nullptr, 0, part.as<double>() + nb, s));
@@ -678,7 +692,7 @@ int llr_host_free(void* p) {
 }
 int llr_device_alloc(size_t bytes, void** out) {
   if (!out) return set_error(LLR_ERR_INVALID, "null pointer");
-  LLR_CUDA_TRY(cudaMalloc(out, bytes ? bytes : 16));
+  LLR_CUDA_TRY(device_alloc(out, bytes));
   return LLR_OK;
 }
 int llr_device_free(void* p) {

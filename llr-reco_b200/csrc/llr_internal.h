@@ -127,6 +127,11 @@ size_t wavelet_workspace_elems(const WaveletPlan& p, int nvol);
 int wavelet_denoise_strided(const WaveletPlan& p, float2* data, long long sx, long long sy, long long sz,
                             long long sv, int nvol, float alpha, float2* work, cudaStream_t s);
 
+// Stream-ordered scratch of one call (scratch.cu); release with cudaFreeAsync on the same stream.
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+void scratch_trim();   // unused scratch of the current device back to the driver
+cudaError_t device_alloc(void** p, size_t bytes);   // cudaMalloc, retried once without kept scratch
+
 // plan cache for stand-alone signal-model calls
 int get_c2c_plan(int rank, const long long* n, long long batch, cufftHandle* out);
 int cufft_error(cufftResult r, const char* what);

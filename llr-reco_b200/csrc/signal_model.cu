@@ -533,7 +533,7 @@ int signal_model_dev(float2* d_x, const int dims[3], int batch, const float* lin
   phase_tables_host(dims, batch, lin_ksp, h.data());
   phase_tables_host(dims, batch, lin_img, h.data() + nt);
   float2* d_t = nullptr;
-  LLR_CUDA_TRY(cudaMallocAsync((void**)&d_t, sizeof(float2) * 2 * nt, s));
+  LLR_CUDA_TRY(scratch_alloc((void**)&d_t, sizeof(float2) * 2 * nt, s));
   int st = LLR_OK;
   do {
     cudaError_t e = cudaMemcpyAsync(d_t, h.data(), sizeof(float2) * 2 * nt, cudaMemcpyHostToDevice, s);

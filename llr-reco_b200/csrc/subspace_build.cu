@@ -229,11 +229,11 @@ int llr_dti_subspace(const float* b_vals, const float* b_vecs, int32_t nq, int32
   auto cleanup = [&]() {
     cudaFree(d_bg); cudaFree(d_part); cudaFree(d_gram); cudaFree(d_ev); cudaFree(d_vec);
   };
-  cudaError_t e = cudaMalloc((void**)&d_bg, sizeof(double) * bg.size());
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_part, sizeof(double) * (size_t)nparts * np);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_gram, sizeof(double) * np);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_ev, sizeof(double) * nq);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_vec, sizeof(double) * nq * nq);
+  cudaError_t e = device_alloc((void**)&d_bg, sizeof(double) * bg.size());
+  if (e == cudaSuccess) e = device_alloc((void**)&d_part, sizeof(double) * (size_t)nparts * np);
+  if (e == cudaSuccess) e = device_alloc((void**)&d_gram, sizeof(double) * np);
+  if (e == cudaSuccess) e = device_alloc((void**)&d_ev, sizeof(double) * nq);
+  if (e == cudaSuccess) e = device_alloc((void**)&d_vec, sizeof(double) * nq * nq);
   if (e == cudaSuccess) e = cudaMemcpy(d_bg, bg.data(), sizeof(double) * bg.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
     const size_t smem = sizeof(double) * (4 * (size_t)nq + (size_t)kSimBatch * (nq + 1));
