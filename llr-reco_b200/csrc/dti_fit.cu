@@ -24,11 +24,13 @@ namespace {
 constexpr int kDtiOut = 7;   // b0av, e1, e2, e3, md, rd, fa
 
 __device__ __forceinline__ void jacobi_rot(float& app, float& aqq, float& apq, float& arp, float& arq) {
-  // zero apq; arp / arq: the third row's entries against p and q
-  if (apq == 0.f) return;
-  const float th = (aqq - app) / (2.f * apq);
-  const float t = copysignf(1.f, th) / (fabsf(th) + sqrtf(th * th + 1.f));
-  const float c = 1.f / sqrtf(t * t + 1.f), s = t * c;
+  // zero apq; arp / arq: the third row's entries against p and q.  The tangent is the smaller root of
+  // t^2 + t (aqq - app) / apq - 1 = 0 with one square root and one division; entries are scaled to at most
+  // 1, so the squares neither overflow nor lose an apq that matters.
+  if (fabsf(apq) <= 1e-18f) return;
+  const float d = aqq - app, a2 = 2.f * apq;
+  const float t = __fdividef(d >= 0.f ? a2 : -a2, fabsf(d) + sqrtf(fmaf(d, d, a2 * a2)));
+  const float c = rsqrtf(fmaf(t, t, 1.f)), s = t * c;
   app -= t * apq;
   aqq += t * apq;
   apq = 0.f;
@@ -37,10 +39,16 @@ __device__ __forceinline__ void jacobi_rot(float& app, float& aqq, float& apq, f
   arq = s * rp + c * rq;
 }
 
-// eigenvalues of the symmetric [[a, d, e], [d, b, f], [e, f, c]], descending
+// eigenvalues of the symmetric [[a, d, e], [d, b, f], [e, f, c]], descending.  The matrix is scaled by a
+// power of two (exact) so that its largest entry lies in [1, 2).
 __device__ void sym3_eigenvalues(float a, float b, float c, float d, float e, float f, float* out) {
+  const float mx = fmaxf(fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c)), fmaxf(fmaxf(fabsf(d), fabsf(e)), fabsf(f)));
+  const int ex = min(max((__float_as_int(mx) >> 23) & 0xff, 1), 253);
+  const float up = __int_as_float((254 - ex) << 23), dn = __int_as_float(ex << 23);
+  a *= up; b *= up; c *= up; d *= up; e *= up; f *= up;
   for (int sweep = 0; sweep < 8; ++sweep) {
-    if (fabsf(d) + fabsf(e) + fabsf(f) <= 1e-30f + 1e-9f * (fabsf(a) + fabsf(b) + fabsf(c))) break;
+    // off-diagonal entries this far below the diagonal move no eigenvalue by half an ulp
+    if (fabsf(d) + fabsf(e) + fabsf(f) <= 1e-9f * (fabsf(a) + fabsf(b) + fabsf(c))) break;
     jacobi_rot(a, b, d, e, f);   // (0,1); third index 2: (a02, a12) = (e, f)
     jacobi_rot(a, c, e, d, f);   // (0,2); third index 1: (a01, a21) = (d, f)
     jacobi_rot(b, c, f, d, e);   // (1,2); third index 0: (a10, a20) = (d, e)
@@ -49,43 +57,148 @@ __device__ void sym3_eigenvalues(float a, float b, float c, float d, float e, fl
   if (l[0] < l[1]) { float t = l[0]; l[0] = l[1]; l[1] = t; }
   if (l[1] < l[2]) { float t = l[1]; l[1] = l[2]; l[2] = t; }
   if (l[0] < l[1]) { float t = l[0]; l[0] = l[1]; l[1] = t; }
-  out[0] = l[0]; out[1] = l[1]; out[2] = l[2];
+  out[0] = l[0] * dn; out[1] = l[1] * dn; out[2] = l[2] * dn;
 }
 
-__global__ void dti_fit_kernel(const float2* __restrict__ dwi, const float2* __restrict__ b0, long long V, int nq,
-                               int nb0, const float* __restrict__ pinv, float* __restrict__ out) {
-  extern __shared__ float s_pinv[];   // [6][nq]
-  for (int i = threadIdx.x; i < 6 * nq; i += blockDim.x) s_pinv[i] = pinv[i];
-  __syncthreads();
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
-    float s0 = 0.f;
-    for (int k = 0; k < nb0; ++k) {
-      const float2 z = b0[v + V * k];
-      s0 += sqrtf(z.x * z.x + z.y * z.y);
-    }
-    s0 = nb0 > 0 ? s0 / (float)nb0 : 0.f;
-    const float s0c = fmaxf(s0, FLT_MIN);
-    float dt[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int q = 0; q < nq; ++q) {
-      const float2 z = dwi[v + V * q];
-      const float r = logf(fminf(fmaxf(sqrtf(z.x * z.x + z.y * z.y) / s0c, FLT_MIN), 1.f));
+// ln x of a positive normal x: x = 2^k m with m in [sqrt 1/2, sqrt 2), f = m - 1, and
+// ln(1 + f) = f - f^2 / 2 + f^3 P(f), P the least-maximum-error degree-7 fit of the series' tail over
+// that range (relative error 6e-9 before rounding, Lawson's iteratively weighted least squares).
+// Measured against FP64 over (e^-8, 1): relative error at most 1e-7.
+__device__ __forceinline__ float ln_normal(float x) {
+  const int ix = __float_as_int(x) - 0x3f3504f3;
+  const float k = (float)(ix >> 23);
+  const float f = __int_as_float((ix & 0x7fffff) + 0x3f3504f3) - 1.f;
+  float p = -0.07634474337100983f;
+  p = fmaf(p, f, 0.12761567533016205f);
+  p = fmaf(p, f, -0.13160187005996704f);
+  p = fmaf(p, f, 0.14201758801937103f);
+  p = fmaf(p, f, -0.16623356938362122f);
+  p = fmaf(p, f, 0.20001226663589478f);
+  p = fmaf(p, f, -0.2500081956386566f);
+  p = fmaf(p, f, 0.3333333134651184f);
+  const float q = fmaf(p, f, -0.5f);
+  return fmaf(k, 0.69314718056f, fmaf(f * f, q, f));
+}
+
+// Right-hand sides 2 ln(clamp(|z_q| / s0, FLT_MIN, 1)) of QB samples of two voxels (z[voxel][sample]) into
+// the tensor sums dt (the factor 2 is taken out of the weights; w: eight floats per sample, six used).  The
+// common form is ln(|z|^2 / s0^2): one multiplication by the voxel's 1 / s0^2 in place of a square root
+// and a division per sample.  Where a square could leave the range of normal numbers (s0 outside
+// [1e-15, 1e15], |z| below 1e-15 s0) or z is not a number, the batch forms the ratios themselves.
+template <int QB>
+__device__ __forceinline__ void add_samples(const float2 (&z)[2][QB], const float* w, const float* s0c,
+                                            const float* inv2, const float* lo2, float (&dt)[2][6]) {
+  float r[2][QB];
+  bool fast = true;
 #pragma unroll
-      for (int j = 0; j < 6; ++j) dt[j] = fmaf(s_pinv[j * nq + q], r, dt[j]);
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int u = 0; u < QB; ++u) {
+      r[h][u] = z[h][u].x * z[h][u].x + z[h][u].y * z[h][u].y;
+      fast = fast && r[h][u] >= lo2[h];
     }
-    float l[3];
-    sym3_eigenvalues(dt[0], dt[1], dt[2], dt[3], dt[4], dt[5], l);
-    const float md = (l[0] + l[1] + l[2]) / 3.f;
-    const float rd = 0.5f * (l[1] + l[2]);
-    const float num = sqrtf((l[0] - md) * (l[0] - md) + (l[1] - md) * (l[1] - md) + (l[2] - md) * (l[2] - md));
-    const float den = sqrtf(l[0] * l[0] + l[1] * l[1] + l[2] * l[2]);
-    const float fa = 1.22474487139158904910f * num / den;
-    out[v] = s0;
-    out[V + v] = l[0];
-    out[2 * V + v] = l[1];
-    out[3 * V + v] = l[2];
-    out[4 * V + v] = md;
-    out[5 * V + v] = rd;
-    out[6 * V + v] = fa;
+  if (fast) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int u = 0; u < QB; ++u) r[h][u] = ln_normal(fminf(r[h][u] * inv2[h], 1.f));
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll 1
+      for (int u = 0; u < QB; ++u) r[h][u] = 2.f * logf(fminf(fmaxf(sqrtf(r[h][u]) / s0c[h], FLT_MIN), 1.f));
+  }
+#pragma unroll
+  for (int u = 0; u < QB; ++u) {
+    const float4 pa = *reinterpret_cast<const float4*>(w + 8 * u);
+    const float2 pb = *reinterpret_cast<const float2*>(w + 8 * u + 4);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      dt[h][0] = fmaf(pa.x, r[h][u], dt[h][0]);
+      dt[h][1] = fmaf(pa.y, r[h][u], dt[h][1]);
+      dt[h][2] = fmaf(pa.z, r[h][u], dt[h][2]);
+      dt[h][3] = fmaf(pa.w, r[h][u], dt[h][3]);
+      dt[h][4] = fmaf(pb.x, r[h][u], dt[h][4]);
+      dt[h][5] = fmaf(pb.y, r[h][u], dt[h][5]);
+    }
+  }
+}
+
+// Bound: HBM, 8 (nq + nb0) + 28 bytes per voxel (1.83 GB at 192 x 192 x 96 x (54 + 7): 280 us at the measured
+// copy rate); the instruction issue of the logarithms comes next.  Eight samples of two voxels are in flight
+// per thread before the first logarithm, and a row of the weights (two shared loads) serves both voxels.
+// Calls at that size: 625 us with a square root, a division and a logf per sample, one load at a time and
+// IEEE rotations; 485 us with ln_normal and the one-division rotations; 433 us with one range check per
+// batch instead of per sample; 409 us at four CTAs per SM (64 registers) instead of three.
+__global__ void __launch_bounds__(256, 4) dti_fit_kernel(const float2* __restrict__ dwi, const float2* __restrict__ b0,
+                                                      long long V, int nq, int nb0, const float* __restrict__ pinv,
+                                                      float* __restrict__ out) {
+  constexpr int QB = 8;               // samples in flight per voxel
+  extern __shared__ __align__(16) float s_pinv[];   // [nq][8], six used
+  for (int i = threadIdx.x; i < 8 * nq; i += blockDim.x) s_pinv[i] = pinv[i];
+  __syncthreads();
+  const long long step = (long long)gridDim.x * blockDim.x * 2;
+  for (long long vb = blockIdx.x * (long long)blockDim.x * 2 + threadIdx.x; vb < V; vb += step) {
+    // the thread's two voxels are a CTA width apart; a missing second one repeats the first
+    const long long v[2] = {vb, vb + blockDim.x < V ? vb + blockDim.x : vb};
+    float s0[2] = {0.f, 0.f};
+    for (int k = 0; k < nb0; ++k) {
+      float2 z[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) z[h] = b0[v[h] + V * k];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) s0[h] += sqrtf(z[h].x * z[h].x + z[h].y * z[h].y);
+    }
+    float s0c[2], inv2[2], lo2[2], dt[2][6];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      s0[h] = nb0 > 0 ? s0[h] / (float)nb0 : 0.f;
+      s0c[h] = fmaxf(s0[h], FLT_MIN);
+      const bool in_range = s0c[h] >= 1e-15f && s0c[h] <= 1e15f;
+      inv2[h] = in_range ? 1.f / (s0c[h] * s0c[h]) : 0.f;
+      lo2[h] = in_range ? fmaxf(1e-30f * (s0c[h] * s0c[h]), FLT_MIN) : INFINITY;
+#pragma unroll
+      for (int j = 0; j < 6; ++j) dt[h][j] = 0.f;
+    }
+    const float2* p0 = dwi + v[0];
+    const float2* p1 = dwi + v[1];
+    int q = 0;
+    for (; q + QB <= nq; q += QB) {
+      float2 z[2][QB];
+#pragma unroll
+      for (int u = 0; u < QB; ++u) {
+        z[0][u] = __ldcs(p0);
+        z[1][u] = __ldcs(p1);
+        p0 += V;
+        p1 += V;
+      }
+      add_samples<QB>(z, s_pinv + 8 * q, s0c, inv2, lo2, dt);
+    }
+    for (; q < nq; ++q) {
+      const float2 z[2][1] = {{__ldcs(p0)}, {__ldcs(p1)}};
+      p0 += V;
+      p1 += V;
+      add_samples<1>(z, s_pinv + 8 * q, s0c, inv2, lo2, dt);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h == 1 && vb + blockDim.x >= V) break;
+      float l[3];
+      sym3_eigenvalues(dt[h][0], dt[h][1], dt[h][2], dt[h][3], dt[h][4], dt[h][5], l);
+      const float md = (l[0] + l[1] + l[2]) / 3.f;
+      const float rd = 0.5f * (l[1] + l[2]);
+      const float num = sqrtf((l[0] - md) * (l[0] - md) + (l[1] - md) * (l[1] - md) + (l[2] - md) * (l[2] - md));
+      const float den = sqrtf(l[0] * l[0] + l[1] * l[1] + l[2] * l[2]);
+      const float fa = 1.22474487139158904910f * num / den;
+      float* o = out + v[h];
+      o[0] = s0[h];
+      o[V] = l[0];
+      o[2 * V] = l[1];
+      o[3 * V] = l[2];
+      o[4 * V] = md;
+      o[5 * V] = rd;
+      o[6 * V] = fa;
+    }
   }
 }
 
@@ -124,12 +237,12 @@ int design_pinv(const float* b, const float* g, int nq, std::vector<float>& pinv
         for (int j = 0; j < 12; ++j) M[r][j] -= f * M[c][j];
       }
   }
-  pinv.assign((size_t)6 * nq, 0.f);
+  pinv.assign((size_t)8 * nq, 0.f);   // one sample's six weights per 32-byte row, halved
   for (int j = 0; j < 6; ++j)
     for (int q = 0; q < nq; ++q) {
       double s = 0.0;
       for (int i = 0; i < 6; ++i) s += M[j][6 + i] * A[(size_t)q * 6 + i];
-      pinv[(size_t)j * nq + q] = (float)s;
+      pinv[(size_t)q * 8 + j] = 0.5f * (float)s;
     }
   return LLR_OK;
 }
@@ -153,10 +266,13 @@ int llr_dti_fit_dev(const llr_cf32* d_dwi, int32_t nq, const llr_cf32* d_b0, int
   float* d_pinv = nullptr;
   LLR_CUDA_TRY(scratch_alloc((void**)&d_pinv, sizeof(float) * pinv.size(), s));
   cudaError_t e = cudaMemcpyAsync(d_pinv, pinv.data(), sizeof(float) * pinv.size(), cudaMemcpyHostToDevice, s);
+  const size_t smem = sizeof(float) * 8 * (size_t)nq;
+  if (e == cudaSuccess && smem > 48 * 1024)
+    e = cudaFuncSetAttribute(dti_fit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess) {
-    const long long blocks = std::min<long long>((n_vox + 255) / 256, 148LL * 32);
+    const long long blocks = std::min<long long>((n_vox + 511) / 512, 148LL * 32);
     note_launch();
-    dti_fit_kernel<<<(unsigned)blocks, 256, sizeof(float) * 6 * nq, s>>>(
+    dti_fit_kernel<<<(unsigned)blocks, 256, smem, s>>>(
         (const float2*)d_dwi, (const float2*)d_b0, n_vox, nq, nb0, d_pinv, d_out);
     e = cudaGetLastError();
   }

@@ -76,3 +76,23 @@ def test_dti_scalars_cli(gpu, tmp_path):
         m = read_cfl(str(out / k)).reshape(-1, order="F")
         assert np.all(m.imag == 0)
         np.testing.assert_allclose(m.real, exp[k], rtol=1e-6)   # the b-table went through text
+
+
+@pytest.mark.parametrize("V,nq,scale", [(1, 6, 1.0), (255, 7, 1.0), (513, 8, 1e-18), (1025, 17, 1e18)])
+def test_dti_fit_edges_and_extreme_scales(gpu, V, nq, scale):
+    """Voxel counts around the two-voxel split, sample counts around the eight-sample batch, and signals
+    whose squares leave the FP32 range (the ratio is formed without squares there).  Tolerance: the
+    logarithm's argument carries a few FP32 roundings (5e-7), amplified by the fit's conditioning (the
+    phantom test's 1e-4)."""
+    rng = np.random.default_rng(V)
+    g = rng.standard_normal((nq, 3))
+    g /= np.linalg.norm(g, axis=1, keepdims=True)
+    b = np.full(nq, 1000.0)
+    s0 = rng.uniform(0.5, 1.0, (V, 2))
+    lam = rng.uniform(0.2e-3, 2e-3, (V, nq))
+    dwi = s0[:, :1] * np.exp(-1000.0 * lam) * np.exp(1j * rng.uniform(0, 6, (V, nq))) * scale
+    dwi, b0 = dwi.astype(np.complex64), (s0 * scale).astype(np.complex64)
+    got = _fit(dwi, b0, b, g)
+    exp = O.dti_fit(dwi.astype(np.complex128), b0.astype(np.complex128), b, g)
+    for k in ("b0av", "e1", "e2", "e3", "md", "rd"):
+        assert rel_err(got[k], exp[k]) < 1e-4, k
