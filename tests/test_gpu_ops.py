@@ -39,6 +39,28 @@ def test_fft_round_trip_of_ones(gpu):
     np.testing.assert_allclose(buf, 1.0, atol=2e-6)
 
 
+@pytest.mark.parametrize("vol,bs,nq", [((17, 13, 19), (11, 12, 13), 5), ((17, 13, 19), (1, 1, 1), 3),
+                                       ((33, 20, 2), (16, 16, 1), 7), ((9, 11, 34), (3, 5, 17), 300),
+                                       ((40, 30, 20), (6, 5, 4), 2)])
+def test_lift_unlift_row_chunks_and_volume_slices(gpu, vol, bs, nq):
+    """Block sizes around the lift kernel's 256-thread step and 1024-row chunk, and few blocks with many
+    volumes (the volumes split over CTAs): exact copies both ways, voxels outside the grid untouched."""
+    rng = np.random.default_rng(5)
+    x = np.asfortranarray((rng.standard_normal(vol + (nq,)) + 1j * rng.standard_normal(vol + (nq,))).astype(np.complex64))
+    shift = [v // 2 + 1 for v in vol]
+    nb = int(np.prod([v // b for v, b in zip(vol, bs)]))
+    m = int(np.prod(bs))
+    mats = np.zeros(m * nq * nb, np.complex64)
+    llr_b200.lift_data_set(x.reshape(-1, order="F"), nq, mats, vol, bs, shift, 0, nb)
+    exp = O.lift_data_set(x, bs, shift, 0, nb)
+    np.testing.assert_array_equal(mats, exp.reshape(-1, order="F"))
+    out = np.full(x.size, 7, np.complex64)
+    llr_b200.un_lift_data_set(out, nq, mats, vol, bs, shift, 0, nb)
+    ref = np.full(x.shape, 7, np.complex64, order="F")
+    O.un_lift_data_set(ref, exp, bs, shift, 0, nb)
+    np.testing.assert_array_equal(out, ref.reshape(-1, order="F"))
+
+
 @pytest.mark.parametrize("vol,bs,shift", [((40, 30, 20), (8, 6, 4), (28, 14, 6)), ((17, 13, 9), (4, 5, 3), (3, 12, 8))])
 def test_lift_unlift_match_oracle_exactly(gpu, vol, bs, shift):
     rng = np.random.default_rng(11)
