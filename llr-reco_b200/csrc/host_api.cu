@@ -525,17 +525,32 @@ int idwt3_axis(llr_cf32* vol_data, llr_cf32* decomp, unsigned int* vol_size, uns
 int llr_wavelet_denoise_dev(llr_cf32* d_vols, const int32_t* vs, int32_t nvol, int32_t moments, int32_t levels,
                             float alpha, void* stream) {
   if (!d_vols || !vs || nvol < 1) return set_error(LLR_ERR_INVALID, "bad wavelet arguments");
+  // The kernels walk their x axis and keep y fastest: the reference layout (x fastest) is their
+  // (z, x, y), so every warp reads runs along x.  The transform is separable and its level count
+  // depends on the smallest extent alone, so the axis names do not matter.
   WaveletPlan p;
-  LLR_TRY(wavelet_plan_init(&p, vs[0], vs[1], vs[2], moments, levels));
+  LLR_TRY(wavelet_plan_init(&p, vs[2], vs[0], vs[1], moments, levels));
   if (p.levels == 0) return set_error(LLR_ERR_UNSUPPORTED, "volume too small for one wavelet level");
   const size_t per = wavelet_workspace_elems(p, 1);
-  Scratch w((cudaStream_t)stream);
-  LLR_TRY(w.alloc(per * sizeof(float2)));
   const long long V = (long long)vs[0] * vs[1] * vs[2];
-  for (int v = 0; v < nvol; ++v)
-    LLR_TRY(wavelet_denoise_strided(p, (float2*)d_vols + V * v, 1, vs[0], (long long)vs[0] * vs[1], V, 1, alpha,
-                                    w.as<float2>(), (cudaStream_t)stream));
-  LLR_CUDA_TRY(cudaStreamSynchronize((cudaStream_t)stream));
+  // Volumes go through each level together, up to 1 GB of workspace (a launch serves at most 65535
+  // (volume, x chunk) pairs, and there is at most one chunk per plane); one at a time when that much
+  // cannot be had.
+  int nb = (int)std::min<long long>(nvol, std::max<long long>(1, (long long)((1ull << 30) / (per * sizeof(float2)))));
+  nb = std::max(1, std::min(nb, 65535 / (vs[2] + 16)));
+  cudaStream_t s = (cudaStream_t)stream;
+  Scratch w(s);
+  int st = w.alloc(per * nb * sizeof(float2));
+  if (st == LLR_ERR_NOMEM && nb > 1) {
+    cudaGetLastError();
+    nb = 1;
+    st = w.alloc(per * sizeof(float2));
+  }
+  LLR_TRY(st);
+  for (int v = 0; v < nvol; v += nb)
+    LLR_TRY(wavelet_denoise_strided(p, (float2*)d_vols + V * v, (long long)vs[0] * vs[1], 1, vs[0], V,
+                                    std::min(nb, nvol - v), alpha, w.as<float2>(), s));
+  LLR_CUDA_TRY(cudaStreamSynchronize(s));
   return LLR_OK;
 }
 
