@@ -557,7 +557,7 @@ int llr_wavelet_denoise_dev(llr_cf32* d_vols, const int32_t* vs, int32_t nvol, i
 int llr_hard_project_dev(llr_cf32* d_x, const llr_cf32* d_y, int64_t n, double* out, void* stream) {
   if (!d_x || !d_y || n < 0) return set_error(LLR_ERR_INVALID, "bad hard_project arguments");
   cudaStream_t s = (cudaStream_t)stream;
-  const int nb = 296;
+  const int nb = (int)std::max<long long>(1, std::min<long long>((n + 1023) / 1024, 148 * 8));
   Scratch part(s);
   LLR_TRY(part.alloc(sizeof(double) * (nb + 1)));
   LLR_TRY(launch_hard_project((float2*)d_x, (const float2*)d_y, n, part.as<double>(), nb, s));

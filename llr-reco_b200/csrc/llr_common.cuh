@@ -129,6 +129,25 @@ __device__ __forceinline__ float2 phase_at(const PhaseTab& t, const Geom& g, int
   return p;
 }
 
+// Division of 0 <= x < 2^31 by a fixed d >= 1 as a multiplication and a shift: with 2^(s-1) < d <= 2^s
+// and mul = ceil(2^(31+s) / d), floor(x mul / 2^(31+s)) is the quotient (Granlund and Montgomery
+// 1994: mul d - 2^(31+s) < d <= 2^s); mul < 2^32.
+struct FastDiv {
+  unsigned d, mul, sh;
+  FastDiv() = default;
+  explicit FastDiv(int div) {
+    d = (unsigned)div;
+    sh = 0;
+    while ((1ull << sh) < d) ++sh;
+    const unsigned long long p = 1ull << (31 + sh);
+    mul = (unsigned)((p + d - 1) / d);
+  }
+  __host__ __device__ __forceinline__ unsigned div(unsigned x) const {
+    return (unsigned)(((unsigned long long)x * mul) >> (31 + sh));
+  }
+  __host__ __device__ __forceinline__ unsigned mod(unsigned x, unsigned q) const { return x - q * d; }
+};
+
 // Planar (plane-major) internal layout: element (ix, iy, iz, q) at
 // iy + ny * (iz + nz * (ix + nx * q)); every (x, q) plane of ny*nz samples is contiguous.
 __device__ __forceinline__ long long planar_index(const Geom& g, int ix, int iy, int iz, int q) {

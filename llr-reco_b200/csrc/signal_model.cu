@@ -63,52 +63,106 @@ __device__ __forceinline__ float2 apply_phase(float2 v, float2 p, int sign) {
   return v;
 }
 
-// (nyz x nx) row-major per volume  <->  (nx x nyz) row-major per volume.
-__global__ void transpose_kernel(const float2* __restrict__ in, float2* __restrict__ out, Geom g, int to_planar,
-                                 float scale, PhaseTab ph, int sign) {
-  __shared__ float2 tile[32][33];
-  const int q = blockIdx.z;
+// (nyz x nx) row-major per volume  <->  (nx x nyz) row-major per volume, with the planar side's phase and
+// scale.  Bound: HBM, one read and one write per element (3.45 GB at 192 x 192 x 96 x 61: 530 us at the
+// measured copy rate).  A 64 x 64 tile per CTA keeps eight 256-byte rows in flight per warp (a 32 x 32
+// one with its row loop kept in order had one to four); (iy, iz) come from one multiply-shift division.
+// 1071 us -> 662 us at that size.
+constexpr int kTrTile = 64;
+
+template <int XF>   // 1: phase and scale, 0: copy
+__global__ void __launch_bounds__(512) transpose_kernel(const float2* __restrict__ in, float2* __restrict__ out,
+                                                        Geom g, int to_planar, float scale, PhaseTab ph, int sign,
+                                                        FastDiv dy, long long tiles_x) {
+  __shared__ float2 tile[kTrTile][kTrTile + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;   // 16 warps, four rows of 64 each
+  const int q = blockIdx.y;
   const long long base = (long long)q * g.V;
   // to_planar: input rows j (nyz) x cols ix (nx); output rows ix x cols j.
   const long long rows_in = to_planar ? g.nyz : g.nx;
   const long long cols_in = to_planar ? g.nx : g.nyz;
-  const long long c0 = (long long)blockIdx.x * 32, r0 = (long long)blockIdx.y * 32;
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const long long r = r0 + k, c = c0 + threadIdx.x;
-    if (r < rows_in && c < cols_in) tile[k][threadIdx.x] = in[base + r * cols_in + c];
-  }
+  const long long tr = blockIdx.x / tiles_x, tc = blockIdx.x - tr * tiles_x;
+  const long long c0 = tc * kTrTile, r0 = tr * kTrTile;
+  float2 v[8];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long long r = r0 + warp + 16 * k, c = c0 + lane + 32 * h;
+      if (r < rows_in && c < cols_in) v[2 * k + h] = in[base + r * cols_in + c];
+    }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) tile[warp + 16 * k][lane + 32 * h] = v[2 * k + h];
   __syncthreads();
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const long long orow = c0 + k, ocol = r0 + threadIdx.x;  // output row = input col
-    if (orow < cols_in && ocol < rows_in) {
-      float2 v = tile[threadIdx.x][k];
-      long long ix, j;
-      if (to_planar) { ix = orow; j = ocol; } else { ix = ocol; j = orow; }
-      if (sign != 0 || scale != 1.f) {
-        const int iy = (int)(j % g.ny), iz = (int)(j / g.ny);
-        if (sign != 0) v = apply_phase(v, phase_at(ph, g, q, (int)ix, iy, iz), sign);
-        v = cscale(v, scale);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long long orow = c0 + warp + 16 * k, ocol = r0 + lane + 32 * h;   // output row = input col
+      if (orow < cols_in && ocol < rows_in) {
+        float2 w = tile[lane + 32 * h][warp + 16 * k];
+        if (XF) {
+          const int ix = (int)(to_planar ? orow : ocol);
+          const unsigned j = (unsigned)(to_planar ? ocol : orow);
+          if (sign != 0) {
+            const unsigned iz = dy.div(j);
+            w = apply_phase(w, phase_at(ph, g, q, ix, (int)dy.mod(j, iz), (int)iz), sign);
+          }
+          w = cscale(w, scale);
+        }
+        out[base + orow * rows_in + ocol] = w;
       }
-      out[base + orow * rows_in + ocol] = v;
+    }
+}
+
+// x *= scale * exp(sign * i * (theta_x + theta_y + theta_z)) on a reference-layout batch.  qs: volume
+// stride of the tables (0: every volume shares the first one's, 1: one row per volume).
+// Bound: HBM, one read and one write per element (0.37 GB at 144 x 120 x 90 x 15: 57 us at the
+// measured copy rate).  One CTA per run of a (volume, z) plane, four elements in flight per thread, one
+// multiply-shift division per element; three 64-bit divisions per element took 124 us, now 55 us.
+constexpr int kPhaseRun = 1024;
+
+__global__ void __launch_bounds__(256) phase_ref_kernel(float2* x, Geom g, long long planes, FastDiv dx, int qs,
+                                                        const float2* __restrict__ tx, const float2* __restrict__ ty,
+                                                        const float2* __restrict__ tz, int sign, float scale) {
+  const unsigned n = (unsigned)g.nx * (unsigned)g.ny;
+  const unsigned i0 = blockIdx.x * kPhaseRun + threadIdx.x;
+  for (long long p = blockIdx.y; p < planes; p += gridDim.y) {
+    const int q = (int)(p / g.nz), iz = (int)(p - (long long)q * g.nz);
+    const long long qt = (long long)q * qs;
+    const float2 pz = tz[qt * g.nz + iz];
+    float2* xp = x + p * n;
+    float2 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + 256 * u < n) v[u] = xp[i0 + 256 * u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const unsigned i = i0 + 256 * u;
+      if (i < n) {
+        const unsigned iy = dx.div(i), ix = dx.mod(i, iy);
+        const float2 ph = cmul(cmul(tx[qt * g.nx + ix], ty[qt * g.ny + iy]), pz);
+        xp[i] = cscale(sign > 0 ? cmul(v[u], ph) : cmul_bc(v[u], ph), scale);
+      }
     }
   }
 }
 
-// x *= scale * exp(sign * i * (theta_x + theta_y + theta_z)) on a reference-layout batch.
-__global__ void phase_ref_kernel(float2* x, Geom g, int nvol, const float2* tx, const float2* ty, const float2* tz,
-                                 int sign, float scale) {
+// The same for planes of 2^31 samples and more.
+__global__ void phase_ref_big_kernel(float2* x, Geom g, int nvol, int qs, const float2* tx, const float2* ty,
+                                     const float2* tz, int sign, float scale) {
   const long long tot = g.V * nvol;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
-    const int q = (int)(i / g.V);
-    long long r = i - (long long)q * g.V;
+    const long long q = i / g.V;
+    long long r = i - q * g.V;
     const int ix = (int)(r % g.nx);
     r /= g.nx;
     const int iy = (int)(r % g.ny);
     const int iz = (int)(r / g.ny);
-    float2 p = cmul(cmul(tx[(long long)q * g.nx + ix], ty[(long long)q * g.ny + iy]), tz[(long long)q * g.nz + iz]);
-    float2 v = x[i];
-    v = (sign > 0) ? cmul(v, p) : cmul_bc(v, p);
-    x[i] = cscale(v, scale);
+    const float2 p = cmul(cmul(tx[q * qs * g.nx + ix], ty[q * qs * g.ny + iy]), tz[q * qs * g.nz + iz]);
+    x[i] = cscale(sign > 0 ? cmul(x[i], p) : cmul_bc(x[i], p), scale);
   }
 }
 
@@ -185,17 +239,37 @@ __global__ void __launch_bounds__(256) dc_full_kernel(float2* __restrict__ u, co
 }
 
 // Reference hard_project on reference-layout buffers (lib.rs:392-406).
-__global__ void __launch_bounds__(256) hard_project_kernel(float2* __restrict__ x, const float2* __restrict__ y,
-                                                           long long n, double* partials) {
+// Bound: HBM, a read of y, and a read and a write of x where y != 0 (0.28 GB at 144 x 120 x 90 x 15 with 4x
+// line sampling: 43 us).  Every load is unconditional, so that a thread has U of them in flight: where
+// y = 0 the second one reads y again (an L1 hit) and the difference is 0; conditional loads were issued
+// one by one.  One sample in flight and two CTAs per SM took 368 us, now 151 us.
+__global__ void __launch_bounds__(256) hard_project_kernel(float2* x, const float2* __restrict__ y, long long n,
+                                                           double* partials) {
+  constexpr int U = 4;
   __shared__ double sh[8];
   double err = 0.0;
-  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
-    const float2 yv = y[i];
-    if (yv.x != 0.f || yv.y != 0.f) {
-      const float2 xv = x[i];
-      const float dx = xv.x - yv.x, dy = xv.y - yv.y;
-      err += (double)(dx * dx + dy * dy);
-      x[i] = yv;
+  const long long step = (long long)gridDim.x * 256 * U;
+  for (long long i0 = (long long)blockIdx.x * 256 * U + threadIdx.x; i0 < n; i0 += step) {
+    long long at[U];
+    float2 yv[U], xv[U];
+    bool on[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) at[u] = min(i0 + 256 * u, n - 1);
+#pragma unroll
+    for (int u = 0; u < U; ++u) yv[u] = y[at[u]];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      on[u] = i0 + 256 * u < n && (yv[u].x != 0.f || yv[u].y != 0.f);
+      const float2* src = on[u] ? x : y;
+      xv[u] = src[at[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float dx = xv[u].x - yv[u].x, dy = xv[u].y - yv[u].y;
+      if (on[u]) {
+        err += (double)(dx * dx + dy * dy);
+        x[at[u]] = yv[u];
+      }
     }
   }
   const double s = block_reduce_d<256>(err, sh);
@@ -361,22 +435,26 @@ inline unsigned grid_for(long long n, int bs = 256, long long cap = 148LL * 32) 
 // ---------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------
-int launch_ref_to_planar(const float2* ref, float2* planar, const Geom& g, float scale, PhaseTab ph, int phase_sign,
-                         cudaStream_t s) {
-  dim3 grid((unsigned)((g.nx + 31) / 32), (unsigned)((g.nyz + 31) / 32), (unsigned)g.nq);
+static int launch_transpose(const float2* in, float2* out, const Geom& g, int to_planar, float scale, PhaseTab ph,
+                            int sign, cudaStream_t s) {
+  const long long rows = to_planar ? g.nyz : g.nx, cols = to_planar ? g.nx : g.nyz;
+  const long long tx = (cols + kTrTile - 1) / kTrTile, ty = (rows + kTrTile - 1) / kTrTile;
+  dim3 grid((unsigned)(tx * ty), (unsigned)g.nq);
   note_launch();
-  transpose_kernel<<<grid, dim3(32, 8), 0, s>>>(ref, planar, g, 1, scale, ph, phase_sign);
+  (sign != 0 || scale != 1.f ? transpose_kernel<1> : transpose_kernel<0>)<<<grid, 512, 0, s>>>(
+      in, out, g, to_planar, scale, ph, sign, FastDiv(g.ny), tx);
   LLR_CUDA_TRY(cudaGetLastError());
   return LLR_OK;
 }
 
+int launch_ref_to_planar(const float2* ref, float2* planar, const Geom& g, float scale, PhaseTab ph, int phase_sign,
+                         cudaStream_t s) {
+  return launch_transpose(ref, planar, g, 1, scale, ph, phase_sign, s);
+}
+
 int launch_planar_to_ref(const float2* planar, float2* ref, const Geom& g, float scale, PhaseTab ph, int phase_sign,
                          cudaStream_t s) {
-  dim3 grid((unsigned)((g.nyz + 31) / 32), (unsigned)((g.nx + 31) / 32), (unsigned)g.nq);
-  note_launch();
-  transpose_kernel<<<grid, dim3(32, 8), 0, s>>>(planar, ref, g, 0, scale, ph, phase_sign);
-  LLR_CUDA_TRY(cudaGetLastError());
-  return LLR_OK;
+  return launch_transpose(planar, ref, g, 0, scale, ph, phase_sign, s);
 }
 
 int launch_scale_uncovered(float2* data, const Geom& g, const int* cover, const long long* it_ptr,
@@ -464,10 +542,17 @@ int launch_prep_full(float2* y, const Geom& g, PhaseTab ph_img, float scale, cud
   return LLR_OK;
 }
 
-int launch_phase_ref(float2* x, const Geom& g, int nvol, const float2* tx, const float2* ty, const float2* tz, int sign,
-                     float scale, cudaStream_t s) {
+int launch_phase_ref(float2* x, const Geom& g, int nvol, int qs, const float2* tx, const float2* ty, const float2* tz,
+                     int sign, float scale, cudaStream_t s) {
   note_launch();
-  phase_ref_kernel<<<grid_for(g.V * nvol), 256, 0, s>>>(x, g, nvol, tx, ty, tz, sign, scale);
+  const long long plane = (long long)g.nx * g.ny;
+  if (plane >= (1LL << 31) - kPhaseRun) {
+    phase_ref_big_kernel<<<grid_for(g.V * nvol), 256, 0, s>>>(x, g, nvol, qs, tx, ty, tz, sign, scale);
+  } else {
+    const long long planes = (long long)g.nz * nvol;
+    dim3 grid((unsigned)((plane + kPhaseRun - 1) / kPhaseRun), (unsigned)std::min<long long>(planes, 65535));
+    phase_ref_kernel<<<grid, 256, 0, s>>>(x, g, planes, FastDiv(g.nx), qs, tx, ty, tz, sign, scale);
+  }
   LLR_CUDA_TRY(cudaGetLastError());
   return LLR_OK;
 }
@@ -528,10 +613,13 @@ int signal_model_dev(float2* d_x, const int dims[3], int batch, const float* lin
   g.nx = dims[0]; g.ny = dims[1]; g.nz = dims[2]; g.nq = batch;
   g.nyz = (long long)g.ny * g.nz;
   g.V = (long long)g.nx * g.nyz;
-  const size_t nt = (size_t)batch * (dims[0] + dims[1] + dims[2]);
+  // without corrections every volume shares one set of ramps
+  const int qs = (lin_ksp || lin_img) ? 1 : 0;
+  const int nt_vol = qs ? batch : 1;
+  const size_t nt = (size_t)nt_vol * (dims[0] + dims[1] + dims[2]);
   std::vector<float2> h(2 * nt);
-  phase_tables_host(dims, batch, lin_ksp, h.data());
-  phase_tables_host(dims, batch, lin_img, h.data() + nt);
+  phase_tables_host(dims, nt_vol, lin_ksp, h.data());
+  phase_tables_host(dims, nt_vol, lin_img, h.data() + nt);
   float2* d_t = nullptr;
   LLR_CUDA_TRY(scratch_alloc((void**)&d_t, sizeof(float2) * 2 * nt, s));
   int st = LLR_OK;
@@ -539,14 +627,14 @@ int signal_model_dev(float2* d_x, const int dims[3], int batch, const float* lin
     cudaError_t e = cudaMemcpyAsync(d_t, h.data(), sizeof(float2) * 2 * nt, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) { st = cuda_error(e, "cudaMemcpyAsync", __FILE__, __LINE__); break; }
     const float2* ksp_x = d_t;
-    const float2* ksp_y = ksp_x + (size_t)batch * dims[0];
-    const float2* ksp_z = ksp_y + (size_t)batch * dims[1];
+    const float2* ksp_y = ksp_x + (size_t)nt_vol * dims[0];
+    const float2* ksp_z = ksp_y + (size_t)nt_vol * dims[1];
     const float2* img_x = d_t + nt;
-    const float2* img_y = img_x + (size_t)batch * dims[0];
-    const float2* img_z = img_y + (size_t)batch * dims[1];
+    const float2* img_y = img_x + (size_t)nt_vol * dims[0];
+    const float2* img_z = img_y + (size_t)nt_vol * dims[1];
     const bool fwd = direction == LLR_FORWARD;
     // pre: Forward uses the k-space correction, Inverse the image correction; sign +1
-    st = launch_phase_ref(d_x, g, batch, fwd ? ksp_x : img_x, fwd ? ksp_y : img_y, fwd ? ksp_z : img_z, +1, 1.f, s);
+    st = launch_phase_ref(d_x, g, batch, qs, fwd ? ksp_x : img_x, fwd ? ksp_y : img_y, fwd ? ksp_z : img_z, +1, 1.f, s);
     if (st) break;
     cufftHandle plan;
     long long n[3] = {dims[2], dims[1], dims[0]};  // reversed: x fastest (cufft.rs:86)
@@ -558,7 +646,7 @@ int signal_model_dev(float2* d_x, const int dims[3], int batch, const float* lin
     if (r != CUFFT_SUCCESS) { st = cufft_error(r, "cufftExecC2C"); break; }
     // post: sign -1 with the other correction, and the unitary 1/sqrt(N) (cufft.rs:161-163)
     const float sc = (float)(1.0 / std::sqrt((double)g.V));
-    st = launch_phase_ref(d_x, g, batch, fwd ? img_x : ksp_x, fwd ? img_y : ksp_y, fwd ? img_z : ksp_z, -1, sc, s);
+    st = launch_phase_ref(d_x, g, batch, qs, fwd ? img_x : ksp_x, fwd ? img_y : ksp_y, fwd ? img_z : ksp_z, -1, sc, s);
   } while (0);
   cudaError_t e = cudaFreeAsync(d_t, s);
   if (st == LLR_OK && e != cudaSuccess) st = cuda_error(e, "cudaFreeAsync", __FILE__, __LINE__);
