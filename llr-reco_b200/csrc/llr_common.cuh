@@ -82,6 +82,20 @@ __device__ __forceinline__ void cfma_cb(float2& acc, float2 a, float2 b) {
   acc.y = fmaf(-a.x, b.y, acc.y);
 }
 
+// Two FP32 FMAs in one instruction (a * b + c per component, each rounded as fmaf).
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  union U { float2 f; unsigned long long u; };
+  U x, y, z, d;
+  x.f = a; y.f = b; z.f = c;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.u) : "l"(x.u), "l"(y.u), "l"(z.u));
+  return d.f;
+}
+// acc += a * b as two packed FMAs, with b and i b = (-b.y, b.x) given: the same roundings as cfma
+__device__ __forceinline__ void cfma2(float2& acc, float2 a, float2 b, float2 ib) {
+  acc = ffma2(make_float2(a.x, a.x), b, acc);
+  acc = ffma2(make_float2(a.y, a.y), ib, acc);
+}
+
 // ---------------------------------------------------------------------------------------
 // counter-based RNG: SplitMix64 finaliser keyed by (seed, stream, index).  Identical on
 // host and device so that shifts drawn inside a CUDA graph match the host/oracle draw.

@@ -236,10 +236,250 @@ __global__ void __launch_bounds__(kLlrThreads) llr_subspace_kernel(BlockSource s
   }
 }
 
-// Coefficient output: the same gather and low-rank step, storing Z' = LR(X S) as srank
-// planar coefficient volumes (image space) for a shrink in the coefficient domain.
-template <int NPMAX, int KM>
-__global__ void __launch_bounds__(kLlrThreads) llr_subspace_coef_kernel(BlockSource src, SubspaceOp op, SmemLayout L) {
+// Coefficient path (wavelet shrink in the coefficient domain), two kernels.
+//
+// The first forms Z = X S for every voxel, as srank planar coefficient volumes in image space: a stream over
+// the iterate that needs no block structure.  Bound: HBM, 8 nq + 8 srank bytes per voxel (4.6 GB at
+// 128 x 256 x 256 x 61, rank 7: 0.70 ms at the measured copy rate).  Four volumes of two voxels are in flight
+// per thread, a row of S (shared memory, broadcast) serves both voxels, and a phase shared by every
+// volume is taken out of the sum.  The second kernel makes the blocks low rank in place on those volumes
+// (7 / 61 of the data).  One kernel doing both per block waited on its 7 x 7 eigenproblem with the
+// gather's loads idle: 3.52 ms, now 0.89 ms + 0.58 ms.
+template <int KM, bool UNI>   // UNI: every volume has the same phase
+__global__ void __launch_bounds__(256, KM <= 8 && UNI ? 3 : KM <= 8 ? 2 : 1) subspace_project_kernel(const float2* __restrict__ x, float2* __restrict__ z,
+                                                               const float2* __restrict__ S, int srank, Geom g,
+                                                               PhaseTab ph, float scale) {
+  constexpr int QB = 4;
+  extern __shared__ __align__(16) float4 Sq[];   // [nq][KM] (S, i S), zero beyond srank
+  for (int i = threadIdx.x; i < g.nq * KM; i += 256) {
+    const int q = i / KM, k = i - q * KM;
+    const float2 c = k < srank ? S[q + (long long)g.nq * k] : make_float2(0.f, 0.f);
+    Sq[i] = make_float4(c.x, c.y, -c.y, c.x);
+  }
+  __syncthreads();
+  for (long long v0 = blockIdx.x * 512LL + threadIdx.x; v0 < g.V; v0 += gridDim.x * 512LL) {
+    const bool two = v0 + 256 < g.V;              // a missing second voxel repeats the first
+    const long long v[2] = {v0, two ? v0 + 256 : v0};
+    int ix[2], iy[2], iz[2];
+    float2 acc[2][KM];
+    auto coords = [&](int h) {
+      const long long r = v[h] / g.ny;
+      iy[h] = (int)(v[h] - r * g.ny);
+      ix[h] = (int)(r / g.nz);
+      iz[h] = (int)(r - (long long)ix[h] * g.nz);
+    };
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (!UNI) coords(h);
+#pragma unroll
+      for (int k = 0; k < KM; ++k) acc[h][k] = make_float2(0.f, 0.f);
+    }
+    auto add = [&](int q, float2 xv, int h) {
+      if (!UNI) xv = cscale(cmul_bc(xv, phase_at(ph, g, q, ix[h], iy[h], iz[h])), scale);
+#pragma unroll
+      for (int k = 0; k < KM; ++k) {
+        const float4 c = Sq[q * KM + k];
+        cfma2(acc[h][k], xv, make_float2(c.x, c.y), make_float2(c.z, c.w));
+      }
+    };
+    const float2* xa = x + v[0];
+    const float2* xb = x + v[1];
+    int q = 0;
+    for (; q + QB <= g.nq; q += QB) {
+      float2 a[QB], b[QB];
+#pragma unroll
+      for (int u = 0; u < QB; ++u) {
+        a[u] = __ldcs(xa);
+        b[u] = __ldcs(xb);
+        xa += g.V;
+        xb += g.V;
+      }
+#pragma unroll
+      for (int u = 0; u < QB; ++u) {
+        add(q + u, a[u], 0);
+        add(q + u, b[u], 1);
+      }
+    }
+    for (; q < g.nq; ++q) {
+      add(q, __ldcs(xa), 0);
+      add(q, __ldcs(xb), 1);
+      xa += g.V;
+      xb += g.V;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h == 1 && !two) break;
+      float2 p0 = make_float2(1.f, 0.f);
+      if (UNI) {
+        coords(h);
+        p0 = cscale(phase_at(ph, g, 0, ix[h], iy[h], iz[h]), scale);
+      }
+#pragma unroll
+      for (int k = 0; k < KM; ++k)
+        if (k < srank) z[v[h] + g.V * k] = UNI ? cmul_bc(acc[h][k], p0) : acc[h][k];
+    }
+  }
+}
+
+// Low rank of every block of the coefficient volumes, in place, rank at most 8: one warp per block.  Bound:
+// latency (the eigenproblem is a chain of rotations); a warp's chain of gather, Gram sums in
+// registers, rotations and apply needs no CTA barrier, and 24 of them run per SM.  The second read of
+// the block comes from L2.  One CTA per block, 256 threads waiting on one warp's rotations, took 2.47 ms
+// at 128 x 256 x 256 in 8^3 blocks of rank 7, now 0.58 ms.
+constexpr int kCoefK = 8, kCoefWarps = 4;
+
+struct CoefWarp {
+  float2 A[kCoefK * (kCoefK + 1)], V[kCoefK * (kCoefK + 1)];
+  float4 W[kCoefK * kCoefK];   // (W, i W)
+  float4 rot[kCoefK / 2];
+  int2 pairs[kCoefK / 2];
+  float ev[kCoefK], g[kCoefK];
+  Misc misc;
+};
+
+__global__ void __launch_bounds__(32 * kCoefWarps, 5) llr_coef_warp_kernel(BlockSource src, SubspaceOp op) {
+  constexpr int K = kCoefK, lda = K + 1;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, m = op.m, sr = op.srank;
+  CoefWarp* C = reinterpret_cast<CoefWarp*>(smem) + (threadIdx.x >> 5);
+  unsigned short* rowt = reinterpret_cast<unsigned short*>(smem + sizeof(CoefWarp) * kCoefWarps);   // [m][4]: rx ry rz
+  for (int r = threadIdx.x; r < m; r += blockDim.x) {
+    rowt[4 * r] = (unsigned short)(r / (src.by * src.bz));
+    rowt[4 * r + 1] = (unsigned short)(r % src.by);
+    rowt[4 * r + 2] = (unsigned short)((r / src.by) % src.bz);
+  }
+  __syncthreads();
+  int sh[3];
+  block_shift(src, sh);
+  const Geom& g = src.g;
+  const long long nwarps = (long long)gridDim.x * kCoefWarps;
+  for (long long blk = blockIdx.x * (long long)kCoefWarps + (threadIdx.x >> 5); blk < src.nblocks; blk += nwarps) {
+    const int gyi = (int)(blk % src.gy);
+    const long long t = blk / src.gy;
+    const int gzi = (int)(t % src.gz), gxi = (int)(t / src.gz);
+    const int cx = (gxi * src.bx + sh[0]) % g.nx, cy = (gyi * src.by + sh[1]) % g.ny, cz = (gzi * src.bz + sh[2]) % g.nz;
+    auto row = [&](int r) {
+      const ushort4 q = *reinterpret_cast<const ushort4*>(rowt + 4 * r);
+      int ix = cx + q.x, iy = cy + q.y, iz = cz + q.z;
+      if (ix >= g.nx) ix -= g.nx;
+      if (iy >= g.ny) iy -= g.ny;
+      if (iz >= g.nz) iz -= g.nz;
+      return op.coef_out + planar_index(g, ix, iy, iz, 0);
+    };
+    // Gram sums: the diagonal (real), then the pairs i > j
+    float s[K * K];
+#pragma unroll
+    for (int e = 0; e < K * K; ++e) s[e] = 0.f;
+#pragma unroll 2
+    for (int r = lane; r < m; r += 32) {
+      const float2* c = row(r);
+      float2 z[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) z[k] = k < sr ? c[g.V * k] : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < K; ++i) {
+        s[i] = fmaf(z[i].x, z[i].x, fmaf(z[i].y, z[i].y, s[i]));
+#pragma unroll
+        for (int j = 0; j < i; ++j) {   // conj(z_i) z_j
+          float2 a = make_float2(s[K + i * (i - 1) + 2 * j], s[K + i * (i - 1) + 2 * j + 1]);
+          cfma_ca(a, z[i], z[j]);
+          s[K + i * (i - 1) + 2 * j] = a.x;
+          s[K + i * (i - 1) + 2 * j + 1] = a.y;
+        }
+      }
+    }
+    // recursive halving over the warp: lane l ends with the sums of elements 2 l and 2 l + 1
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int i = 0; i < 2 * o; ++i) {
+        const float send = up ? s[i] : s[i + 2 * o], keep = up ? s[i + 2 * o] : s[i];
+        s[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+    if (lane < K / 2) {
+      C->A[(2 * lane) * lda + 2 * lane] = make_float2(s[0], 0.f);
+      C->A[(2 * lane + 1) * lda + 2 * lane + 1] = make_float2(s[1], 0.f);
+    } else {
+      const int p = lane - K / 2;       // pair index i (i - 1) / 2 + j
+      int i = 1;
+      while (i * (i + 1) / 2 <= p) ++i;
+      const int j = p - i * (i - 1) / 2;
+      C->A[i * lda + j] = make_float2(s[0], s[1]);
+      C->A[j * lda + i] = make_float2(s[0], -s[1]);
+    }
+    __syncwarp();
+    jacobi_warp<K>(C->A, C->V, sr, C->rot, C->pairs, &C->misc, 16);
+    __syncwarp();
+    if (lane < sr) C->ev[lane] = C->A[lane * lda + lane].x;
+    __syncwarp();
+    if (lane < sr) {
+      const float e = C->ev[lane];
+      float gv;
+      if (op.mode == LLR_PROX_HARD_RANK) {
+        int pos = 0;
+        for (int j = 0; j < sr; ++j) pos += (C->ev[j] > e) || (C->ev[j] == e && j < lane);
+        gv = pos < op.rank ? 1.f : 0.f;
+      } else {
+        const float sv = sqrtf(fmaxf(e, 0.f));
+        gv = sv > op.lambda ? 1.f - op.lambda / sv : 0.f;
+      }
+      C->g[lane] = gv;
+    }
+    __syncwarp();
+    for (int e = lane; e < K * K; e += 32) {   // W = V diag(g) V^H
+      const int i = e / K, j = e - i * K;
+      float2 w = make_float2(0.f, 0.f);
+      if (i < sr && j < sr)
+        for (int k = 0; k < sr; ++k) {
+          const float2 p = cmul_bc(C->V[i * lda + k], C->V[j * lda + k]);
+          w.x = fmaf(C->g[k], p.x, w.x);
+          w.y = fmaf(C->g[k], p.y, w.y);
+        }
+      C->W[e] = make_float4(w.x, w.y, -w.y, w.x);
+    }
+    __syncwarp();
+#pragma unroll 2
+    for (int r = lane; r < m; r += 32) {   // z <- z W
+      float2* c = const_cast<float2*>(row(r));
+      float2 z[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) z[k] = k < sr ? c[g.V * k] : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        if (j < sr) {
+          float2 a = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int k = 0; k < K; ++k) {
+            const float4 w = C->W[k * K + j];
+            cfma2(a, z[k], make_float2(w.x, w.y), make_float2(w.z, w.w));
+          }
+          c[g.V * j] = a;
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
+int launch_coef_warp(const BlockSource& src, const SubspaceOp& op, cudaStream_t stream) {
+  const size_t sm = sizeof(CoefWarp) * kCoefWarps + sizeof(unsigned short) * 4 * (size_t)op.m;
+  LLR_CUDA_TRY(cudaFuncSetAttribute(llr_coef_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  int occ = 0;
+  LLR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, llr_coef_warp_kernel, 32 * kCoefWarps, sm));
+  if (occ < 1) return set_error(LLR_ERR_UNSUPPORTED, "coefficient kernel cannot be resident (smem %zu B)", sm);
+  const long long want = (src.nblocks + kCoefWarps - 1) / kCoefWarps;
+  note_launch();
+  llr_coef_warp_kernel<<<(unsigned)std::min<long long>(want, 148LL * occ), 32 * kCoefWarps, sm, stream>>>(src, op);
+  LLR_CUDA_TRY(cudaGetLastError());
+  return LLR_OK;
+}
+
+// The same for ranks 9 to 16, whose Gram sums do not fit a lane's registers: one CTA per block, the small
+// eigenproblem by one warp.
+template <int NPMAX>
+__global__ void __launch_bounds__(kLlrThreads) llr_coef_low_rank_kernel(BlockSource src, SubspaceOp op, SmemLayout L) {
   extern __shared__ __align__(16) unsigned char smem[];
   Misc* misc = reinterpret_cast<Misc*>(smem);
   float4* rot = reinterpret_cast<float4*>(smem + L.off_rot);
@@ -251,36 +491,17 @@ __global__ void __launch_bounds__(kLlrThreads) llr_subspace_coef_kernel(BlockSou
   float2* V = reinterpret_cast<float2*>(smem + L.off_V);
   float2* scr = reinterpret_cast<float2*>(smem + L.off_scr);
   float2* Z = reinterpret_cast<float2*>(smem + L.off_C);
-  float2* Ss = Z + (size_t)op.srank * L.ldc;
-  const int m = op.m, nq = op.nq, sr = op.srank;
-  for (int i = threadIdx.x; i < nq * sr; i += blockDim.x) {
-    const int q = i / sr, k = i - q * sr;
-    Ss[i] = op.S[q + (long long)nq * k];
-  }
+  const int m = op.m, sr = op.srank;
   if (threadIdx.x == 0) block_shift(src, misc->shift);
   __syncthreads();
   int sh[3] = {misc->shift[0], misc->shift[1], misc->shift[2]};
-  Geom gc = src.g;
-  gc.nq = sr;
   for (long long blk = blockIdx.x; blk < src.nblocks; blk += gridDim.x) {
     for (int r = threadIdx.x; r < m; r += blockDim.x) {
-      float2 z[KM];
-#pragma unroll
-      for (int k = 0; k < KM; ++k) z[k] = make_float2(0.f, 0.f);
       int ix = 0, iy = 0, iz = 0;
       block_row_coord(src, blk, sh, r, ix, iy, iz);
-      const float2 p0 = phase_at(src.ph, src.g, 0, ix, iy, iz);   // every volume's, when uniform
-#pragma unroll 4
-      for (int q = 0; q < nq; ++q) {
-        float2 v = src.data[planar_index(src.g, ix, iy, iz, q)];
-        v = cscale(cmul_bc(v, src.ph_uniform ? p0 : phase_at(src.ph, src.g, q, ix, iy, iz)), src.load_scale);
-#pragma unroll
-        for (int k = 0; k < KM; ++k)
-          if (k < sr) cfma(z[k], v, Ss[q * sr + k]);
-      }
-#pragma unroll
-      for (int k = 0; k < KM; ++k)
-        if (k < sr) Z[k * L.ldc + r] = z[k];
+      const float2* c = op.coef_out + planar_index(src.g, ix, iy, iz, 0);
+#pragma unroll 8
+      for (int k = 0; k < sr; ++k) Z[k * L.ldc + r] = c[src.g.V * k];
     }
     __syncthreads();
     gram<NPMAX, 2>(Z, L.ldc, m, sr, A, scr, L.ksplit);
@@ -292,10 +513,26 @@ __global__ void __launch_bounds__(kLlrThreads) llr_subspace_coef_kernel(BlockSou
     for (int r = threadIdx.x; r < m; r += blockDim.x) {
       int ix = 0, iy = 0, iz = 0;
       block_row_coord(src, blk, sh, r, ix, iy, iz);
-      for (int k = 0; k < sr; ++k) op.coef_out[planar_index(gc, ix, iy, iz, k)] = Z[k * L.ldc + r];
+      float2* c = op.coef_out + planar_index(src.g, ix, iy, iz, 0);
+      for (int k = 0; k < sr; ++k) c[src.g.V * k] = Z[k * L.ldc + r];
     }
     __syncthreads();
   }
+}
+
+template <int KM>
+int launch_subspace_project(const BlockSource& src, const SubspaceOp& op, cudaStream_t stream) {
+  const size_t sm = sizeof(float4) * (size_t)op.nq * KM;
+  auto kern = src.ph_uniform ? subspace_project_kernel<KM, true> : subspace_project_kernel<KM, false>;
+  if (sm > 48 * 1024) LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  int occ = 0;
+  LLR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, sm));
+  if (occ < 1) return set_error(LLR_ERR_UNSUPPORTED, "subspace projection needs %zu B smem", sm);
+  const long long blocks = std::min<long long>((src.g.V + 511) / 512, 148LL * occ * 4);
+  note_launch();
+  kern<<<(unsigned)blocks, 256, sm, stream>>>(src.data, op.coef_out, op.S, op.srank, src.g, src.ph, src.load_scale);
+  LLR_CUDA_TRY(cudaGetLastError());
+  return LLR_OK;
 }
 
 template <int KM>
@@ -337,8 +574,18 @@ int launch_llr_prox_subspace(const BlockSource& src, const SubspaceOp& op, cudaS
   L.total = align16(L.total + sizeof(float2) * (size_t)op.nq * op.srank);
   if (L.total > 227 * 1024) return set_error(LLR_ERR_UNSUPPORTED, "subspace prox needs %zu B smem", L.total);
   if (op.coef_out && src.kind != 1) return set_error(LLR_ERR_INVALID, "coefficient output needs volume blocks");
+  if (op.coef_out) {   // accumulators sized to the rank (two voxels per thread)
+    if (op.srank <= 4) LLR_TRY(launch_subspace_project<4>(src, op, stream));
+    else if (op.srank <= 6) LLR_TRY(launch_subspace_project<6>(src, op, stream));
+    else if (op.srank == 7) LLR_TRY(launch_subspace_project<7>(src, op, stream));
+    else if (op.srank == 8) LLR_TRY(launch_subspace_project<8>(src, op, stream));
+    else if (op.srank <= 12) LLR_TRY(launch_subspace_project<12>(src, op, stream));
+    else LLR_TRY(launch_subspace_project<16>(src, op, stream));
+    // a row table of more than 8000 rows would leave the warps of the rank-8 kernel too few
+    if (op.srank <= kCoefK && op.m <= 8000) return launch_coef_warp(src, op, stream);
+  }
   // per-thread coefficient registers sized to the rank class (fewer registers, more CTAs per SM)
-  auto kern = op.coef_out ? (op.srank <= 8 ? llr_subspace_coef_kernel<16, 8> : llr_subspace_coef_kernel<16, 16>)
+  auto kern = op.coef_out ? llr_coef_low_rank_kernel<16>
                           : (op.srank <= 8 ? llr_subspace_kernel<16, 8> : llr_subspace_kernel<16, 16>);
   LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
     LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));

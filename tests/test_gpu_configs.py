@@ -107,6 +107,39 @@ def test_c3_coefficient_wavelet(gpu):
     np.testing.assert_allclose(hist, oh, rtol=TOL)
 
 
+@pytest.mark.parametrize("srank,mode,corr", [(1, "soft", False), (7, "hard", True), (8, "soft", True), (9, "soft", False),
+                                             (16, "hard", False)])
+def test_coefficient_path_ranks(gpu, srank, mode, corr):
+    """Coefficient-domain iteration around the rank classes of its kernels (one warp per block to rank 8, one
+    CTA above), with shared and per-volume phases; 21 volumes (not a multiple of the load batch) on
+    24 x 20 x 16 in 8 x 4 x 4 blocks, two iterations against the oracle."""
+    vol, bs, nq, n_iter = (24, 20, 16), (8, 4, 4), 21, 2
+    rng = np.random.default_rng(srank)
+    d = make_dataset(vol, [(0, 1), (1000, nq - 1)], 3.0, srank, centre=6, mask_fn=O.vd_mask)
+    S = np.asfortranarray(np.linalg.qr(rng.standard_normal((nq, srank)) + 1j * rng.standard_normal((nq, srank)))[0]
+                          .astype(np.complex64))
+    lk = rng.integers(-2, 3, (nq, 3)).astype(np.float32) if corr else None
+    ocfg = O.ReconConfig(block_size=bs, mode=mode, rank=min(3, srank), seed=5, wavelet_alpha=0.003, wavelet_moments=2,
+                         wavelet_levels=1, wavelet_space="coeffs", lin_ksp=lk)
+    ocfg.subspace = S.astype(np.complex128)
+    x0 = O.zero_filled(d.y.astype(np.complex128), ocfg)
+    ocfg.lam = 0.02 * O.sigma_max(x0, bs)
+    p = ReconParams(vol_size=vol, nq=nq, block_size=bs, rank=min(3, srank), lam=ocfg.lam, seed=5, subspace_rank=srank,
+                    prox_mode=L.LLR_PROX_SOFT_THRESH if mode == "soft" else L.LLR_PROX_HARD_RANK, wavelet_space=1)
+    p.wavelet_alpha, p.wavelet_moments, p.wavelet_levels = 0.003, 2, 1
+    with ReconContext(p) as ctx:
+        if corr:
+            ctx.set_linear_corrections(lk, None)
+        ctx.upload_kspace(d.y)
+        ctx.upload_subspace(S)
+        ctx.init_zero_filled()
+        hist = ctx.iterate(n_iter)
+        gx = ctx.download_image()
+    ox, oh = O.recon(d.y.astype(np.complex128), ocfg, n_iter, x0=x0)
+    assert rel_err(gx, ox) < TOL, rel_err(gx, ox)
+    np.testing.assert_allclose(hist, oh, rtol=TOL)
+
+
 def test_c5_shape_class_overlapping_blocks(gpu):
     """Config-5 shape class: 106 volumes (6 b0 + 100 over b = 1000 / 2000 / 3000), 12x sampling,
     8^3 blocks at stride 4 (Casorati 512 x 106, each voxel the mean of its 8 block outputs),
