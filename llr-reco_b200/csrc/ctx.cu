@@ -193,6 +193,12 @@ static bool coef_mode(const llr_ctx* c) {
   return c->cfg.subspace_rank > 0 && c->wavelet_on && c->cfg.wavelet_space == 1;
 }
 
+// In coefficient mode with one phase for all volumes, the row and column kernels transform the coefficient
+// volumes and expand in k-space (fft_rows.cu); no expanded image is stored in between.
+static bool expand_in_kspace(const llr_ctx* c) {
+  return coef_mode(c) && c->rows_fft && c->ph_uniform && fft_rows_expand_supported(c->g.ny, c->g.nq, c->cfg.subspace_rank);
+}
+
 // One prox pass on d_x.  standalone == true keeps the raw convention (used by single-step
 // entry points); otherwise the output is the FFT input (or the image, if the wavelet runs).
 static int prox_pass(llr_ctx* c, cudaStream_t s, const int* explicit_shift, bool standalone, float* block_stat) {
@@ -274,6 +280,7 @@ static int wavelet_pass(llr_ctx* c, cudaStream_t s, float store_scale, bool in_i
       LLR_TRY(wavelet_denoise_strided_xf(c->wplan, c->d_work + (size_t)k0 * c->g.V, sx, sy, sz, sv,
                                          std::min(nb, sr - k0), c->cfg.wavelet_alpha, c->d_wavelet_work, none,
                                          nullptr, 0, 1.f, s));
+    if (expand_in_kspace(c)) return LLR_OK;
     return launch_subspace_expand(c->d_work, c->d_x, c->d_S, sr, c->g, ctx_phase(c, c->d_ph_ksp, !c->hybrid), 1,
                                   c->ph_uniform, store_scale, s);
   }
@@ -316,10 +323,30 @@ static int fused_dc_pass(llr_ctx* c, cudaStream_t s, double* out) {
   return launch_finalize(c->d_partials, c->fft_grid, (double)c->load_scale, nullptr, 0, nullptr, 0, out, s);
 }
 
+// The same through the row and column kernels, for planes that do not fit shared memory.
+static int rows_dc_pass(llr_ctx* c, cudaStream_t s) {
+  const float2 *tw_y = c->d_rows_tw, *tw_z = c->d_rows_tw + c->g.ny;
+  const long long planes = (long long)c->g.nx * c->g.nq;
+  int np = 0;
+  if (expand_in_kspace(c)) {
+    const PhaseTab ph = ctx_phase(c, c->d_ph_ksp, false);
+    LLR_TRY(launch_fft_cols(c->d_work, c->d_work, tw_z, c->g, (long long)c->g.nx * c->cfg.subspace_rank, 1, &ph, 1.f, s));
+    LLR_TRY(launch_fft_rows(2, c->d_x, c->d_work, c->d_S, c->cfg.subspace_rank, tw_y, c->d_rows_ptr, c->d_samp_pos, c->d_yhat,
+                            c->d_samp_off, c->g, c->d_partials, &np, s));
+  } else {
+    LLR_TRY(launch_fft_cols(c->d_x, c->d_x, tw_z, c->g, planes, 1, nullptr, 1.f, s));
+    LLR_TRY(launch_fft_rows(0, c->d_x, nullptr, nullptr, 0, tw_y, c->d_rows_ptr, c->d_samp_pos, c->d_yhat, c->d_samp_off, c->g,
+                            c->d_partials, &np, s));
+  }
+  LLR_TRY(launch_fft_cols(c->d_x, c->d_x, tw_z, c->g, planes, -1, nullptr, 1.f, s));
+  return finalize_iteration(c, np, s);
+}
+
 int ctx_enqueue_iteration(llr_ctx* c, cudaStream_t s) {
   LLR_TRY(prox_pass(c, s, nullptr, false, nullptr));
   if (c->wavelet_on) LLR_TRY(wavelet_pass(c, s, 1.f, true));
   if (c->fused_fft) return fused_dc_pass(c, s, nullptr);
+  if (c->rows_fft) return rows_dc_pass(c, s);
   LLR_TRY(exec_fft(c, c->d_x, CUFFT_FORWARD, s));
   LLR_TRY(dc_pass(c, s, 0));
   LLR_TRY(finalize_iteration(c, n_partials(c), s));
@@ -422,6 +449,12 @@ int llr_ctx_create(const llr_config* cfg, llr_ctx** out) {
       if (e != cudaSuccess) return fail(cuda_error(e, "cudaMemcpy", __FILE__, __LINE__));
     }
   }
+  if (cfg->fft_mode == 0 && !c->d_fft_tw && fft_rows_supported(c->g.ny, c->g.nz)) {
+    const std::vector<float2> tw = fft_rows_twiddles(c->g.ny, c->g.nz);
+    if ((st = dalloc(&c->d_rows_tw, tw.size()))) return fail(st);
+    e = cudaMemcpy(c->d_rows_tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return fail(cuda_error(e, "cudaMemcpy", __FILE__, __LINE__));
+  }
   c->wavelet_on = false;
   if (cfg->wavelet_alpha > 0.f) {
     if ((st = wavelet_plan_init(&c->wplan, c->g.nx, c->g.ny, c->g.nz, cfg->wavelet_moments, cfg->wavelet_levels)))
@@ -457,7 +490,7 @@ int llr_ctx_destroy(llr_ctx* c) {
   dfree(c->d_x); dfree(c->d_work); dfree(c->d_yhat); dfree(c->d_samp_pos); dfree(c->d_samp_off);
   dfree(c->d_ph_ksp); dfree(c->d_ph_img); dfree(c->d_S); dfree(c->d_partials); dfree(c->d_hist); dfree(c->d_iter);
   dfree(c->d_obj); dfree(c->d_blk_nuc);
-  dfree(c->d_block_stat); dfree(c->d_fb); dfree(c->d_gram); dfree(c->d_blk_ra); dfree(c->d_fft_tw); dfree(c->d_err); dfree(c->d_vwide); dfree(c->d_wavelet_work); dfree(c->d_fft_work);
+  dfree(c->d_block_stat); dfree(c->d_fb); dfree(c->d_gram); dfree(c->d_blk_ra); dfree(c->d_fft_tw); dfree(c->d_rows_tw); dfree(c->d_rows_ptr); dfree(c->d_err); dfree(c->d_vwide); dfree(c->d_wavelet_work); dfree(c->d_fft_work);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   scratch_trim();
   delete c;
@@ -531,6 +564,8 @@ static int upload_kspace_device(llr_ctx* c) {
   dfree(c->d_samp_off); c->d_samp_off = nullptr;
   c->hybrid = structured;
   c->fused_fft = structured && c->cfg.fft_mode == 0 && c->d_fft_tw != nullptr;
+  c->rows_fft = structured && c->d_rows_tw != nullptr;
+  dfree(c->d_rows_ptr); c->d_rows_ptr = nullptr;
   PhaseTab ph_img_full = ctx_phase(c, c->d_ph_img, true);
   if (structured) {
     // sampled (ky + ny*kz) per volume
@@ -549,6 +584,12 @@ static int upload_kspace_device(llr_ctx* c) {
     LLR_CUDA_TRY(cudaMemcpyAsync(c->d_samp_pos, pos.data(), sizeof(int) * pos.size(), cudaMemcpyHostToDevice, s));
     LLR_CUDA_TRY(cudaMemcpyAsync(c->d_samp_off, c->h_samp_off.data(), sizeof(long long) * (g.nq + 1),
                                  cudaMemcpyHostToDevice, s));
+    if (c->rows_fft) {
+      const std::vector<int> rp = fft_rows_ptr(pos, c->h_samp_off, g.ny, g.nz);
+      LLR_TRY(dalloc(&c->d_rows_ptr, rp.size()));
+      LLR_CUDA_TRY(cudaMemcpyAsync(c->d_rows_ptr, rp.data(), sizeof(int) * rp.size(), cudaMemcpyHostToDevice, s));
+      LLR_CUDA_TRY(cudaStreamSynchronize(s));   // the host copy goes out of scope
+    }
     // y_h = A_x^H y along x: e^{+i theta_img,x} -> IFFT_x -> e^{-i theta_ksp,x} / sqrt(nx)
     LLR_TRY(launch_phase_x(c->d_work, g, g.nq, c->d_ph_img, +1, 1.f, s));
     cufftHandle px;
@@ -612,9 +653,16 @@ int llr_init_zero_filled(llr_ctx* c) {
   if (!c->have_kspace) return set_error(LLR_ERR_STATE, "upload k-space first");
   LLR_CUDA_TRY(cudaSetDevice(c->device));
   cudaStream_t s = c->stream;
-  if (c->hybrid) LLR_CUDA_TRY(cudaMemsetAsync(c->d_x, 0, sizeof(float2) * (size_t)c->g.V * c->g.nq, s));
-  LLR_TRY(dc_pass(c, s, 1));
-  LLR_TRY(exec_fft(c, c->d_x, CUFFT_INVERSE, s));
+  if (c->rows_fft) {   // the measured rows along y, then the columns
+    LLR_TRY(launch_fft_rows(1, c->d_x, nullptr, nullptr, 0, c->d_rows_tw, c->d_rows_ptr, c->d_samp_pos, c->d_yhat, c->d_samp_off,
+                            c->g, c->d_partials, nullptr, s));
+    LLR_TRY(launch_fft_cols(c->d_x, c->d_x, c->d_rows_tw + c->g.ny, c->g, (long long)c->g.nx * c->g.nq, -1, nullptr,
+                            1.f, s));
+  } else {
+    if (c->hybrid) LLR_CUDA_TRY(cudaMemsetAsync(c->d_x, 0, sizeof(float2) * (size_t)c->g.V * c->g.nq, s));
+    LLR_TRY(dc_pass(c, s, 1));
+    LLR_TRY(exec_fft(c, c->d_x, CUFFT_INVERSE, s));
+  }
   LLR_CUDA_TRY(cudaMemsetAsync(c->d_iter, 0, sizeof(long long), s));
   LLR_CUDA_TRY(cudaStreamSynchronize(s));
   c->h_iter = 0;
@@ -702,13 +750,16 @@ static int capture_stage(llr_ctx* c, int stage, cudaGraphExec_t* out) {
   switch (stage) {
     case 0: st = prox_pass(c, s, nullptr, false, nullptr); break;
     case 1: if (c->wavelet_on) st = wavelet_pass(c, s, 1.f, true); break;
-    case 2: st = c->fused_fft ? fused_dc_pass(c, s, nullptr) : exec_fft(c, c->d_x, CUFFT_FORWARD, s); break;
+    case 2:
+      st = c->fused_fft ? fused_dc_pass(c, s, nullptr)
+           : c->rows_fft ? rows_dc_pass(c, s) : exec_fft(c, c->d_x, CUFFT_FORWARD, s);
+      break;
     case 3:
-      if (c->fused_fft) break;
+      if (c->fused_fft || c->rows_fft) break;
       st = dc_pass(c, s, 0);
       if (st == LLR_OK) st = finalize_iteration(c, n_partials(c), s);
       break;
-    case 4: if (!c->fused_fft) st = exec_fft(c, c->d_x, CUFFT_INVERSE, s); break;
+    case 4: if (!c->fused_fft && !c->rows_fft) st = exec_fft(c, c->d_x, CUFFT_INVERSE, s); break;
   }
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(s, &graph);
@@ -1013,6 +1064,7 @@ int llr_ctx_device_bytes(const llr_ctx* c, size_t* bytes) {
   b += c->hybrid ? (size_t)c->n_samp_lines * c->g.nx * sizeof(float2) : (c->have_kspace ? E * sizeof(float2) : 0);
   b += c->fft_work_bytes + c->wavelet_work_elems * sizeof(float2);
   if (c->d_gram) b += (size_t)std::max<long long>(1, c->nblocks) * (size_t)prox_gram_stride(c->g.nq) * sizeof(float2);
+  if (c->d_rows_ptr) b += (size_t)c->g.nq * (c->g.nz + 1) * sizeof(int);
   if (c->d_vwide) b += (size_t)c->vwide_ctas * (size_t)wide_v_stride() * sizeof(float2);
   *bytes = b;
   return LLR_OK;

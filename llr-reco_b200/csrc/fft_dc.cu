@@ -7,8 +7,8 @@
 // Each axis of length N = N1 * N2 is a four-step transform in place: N2 register DFTs of
 // length N1 (stride N2) with twiddles W_N^{n2 k1}, then N1 register DFTs of length N2; the
 // spectrum is left in the permuted order p = N2 (k mod N1) + k / N1, which the DC indexes
-// directly and the inverse (the same steps mirrored) consumes.  Register DFTs of length
-// 2, 3, 4, 6, 8, 12, 16 are nested Cooley-Tukey with FP64-computed twiddle tables.
+// directly and the inverse (the same steps mirrored) consumes.  Register DFTs have lengths 1 to 16
+// (fft_codelets.cuh); a length whose factors do not fit that (a prime above 16, say) goes to cuFFT.
 // Forward and inverse are unnormalised like cuFFT's; the residual sum |F x - yhat|^2 is
 // accumulated in FP64 per CTA (fixed plane order) for the deterministic finalize kernel.
 #include <cmath>
@@ -19,6 +19,7 @@
 #include "llr_common.cuh"
 #include "llr_internal.h"
 #include "llr_prox_common.cuh"
+#include "fft_codelets.cuh"
 
 namespace llr {
 
@@ -28,169 +29,19 @@ constexpr int kFftThreads = 512;
 
 __host__ __device__ inline size_t align16b(size_t x) { return (x + 15) & ~size_t(15); }
 
-// Twiddle-table layout in shared memory (float2 entries): W_ny^j, W_nz^j, then W_R^j for the
-// register sizes 16, 12, 8, 6 (W_4, W_3, W_2 are exact constants).
+// Twiddle-table layout in shared memory (float2 entries): W_ny^j, then W_nz^j.
 struct FftTab {
-  int off_y, off_z, off_16, off_12, off_8, off_6, total;
+  int off_y, off_z, total;
 };
 
-__host__ __device__ inline FftTab fft_tab(int ny, int nz) {
-  FftTab t;
-  t.off_y = 0;
-  t.off_z = ny;
-  t.off_16 = ny + nz;
-  t.off_12 = t.off_16 + 16;
-  t.off_8 = t.off_12 + 12;
-  t.off_6 = t.off_8 + 8;
-  t.total = t.off_6 + 6;
-  return t;
-}
-
-// x * W where W = tw (forward) or conj(tw) (inverse)
-template <int DIR>
-__device__ __forceinline__ float2 twmul(float2 x, float2 tw) {
-  return DIR > 0 ? cmul(x, tw) : cmul_bc(x, tw);
-}
-
-// -i * x (forward) / +i * x (inverse)
-template <int DIR>
-__device__ __forceinline__ float2 rot(float2 x) {
-  return DIR > 0 ? make_float2(x.y, -x.x) : make_float2(-x.y, x.x);
-}
-
-template <int R, int DIR>
-struct Dft;
-
-template <int DIR>
-struct Dft<1, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2*) {}
-};
-
-template <int DIR>
-struct Dft<2, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2*) {
-    const float2 a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
-  }
-};
-
-template <int DIR>
-struct Dft<3, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2*) {
-    const float s = 0.86602540378443864676f;   // sin(2 pi / 3)
-    const float2 a = v[0], b = v[1], c = v[2];
-    const float2 t1 = cadd(b, c);
-    const float2 t2 = make_float2(a.x - 0.5f * t1.x, a.y - 0.5f * t1.y);
-    const float2 t3 = cscale(csub(b, c), s);
-    const float2 r = rot<DIR>(t3);   // -i s (b - c) forward
-    v[0] = cadd(a, t1);
-    v[1] = cadd(t2, r);
-    v[2] = csub(t2, r);
-  }
-};
-
-template <int DIR>
-struct Dft<4, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2*) {
-    const float2 a = v[0], b = v[1], c = v[2], d = v[3];
-    const float2 s0 = cadd(a, c), s1 = csub(a, c), s2 = cadd(b, d), s3 = rot<DIR>(csub(b, d));
-    v[0] = cadd(s0, s2);
-    v[2] = csub(s0, s2);
-    v[1] = cadd(s1, s3);
-    v[3] = csub(s1, s3);
-  }
-};
-
-// W_R^m = e^{-2 pi i m / R} for the register DFTs, evaluated at compile time from the Taylor
-// series of cos and sin in double precision (|x| <= 2 pi, 30 terms).
-constexpr double kTwoPi = 6.283185307179586476925286766559;
-constexpr double taylor_cos(double x) {
-  double t = 1.0, s = 1.0;
-  for (int k = 1; k < 30; ++k) { t *= -x * x / ((2.0 * k - 1.0) * (2.0 * k)); s += t; }
-  return s;
-}
-constexpr double taylor_sin(double x) {
-  double t = x, s = x;
-  for (int k = 1; k < 30; ++k) { t *= -x * x / ((2.0 * k) * (2.0 * k + 1.0)); s += t; }
-  return s;
-}
-template <int R>
-struct TwTab {
-  float re[R], im[R];
-  constexpr TwTab() : re(), im() {
-    for (int m = 0; m < R; ++m) {
-      re[m] = (float)taylor_cos(kTwoPi * m / R);
-      im[m] = (float)-taylor_sin(kTwoPi * m / R);
-    }
-  }
-};
-template <int R>
-__device__ constexpr TwTab<R> kTw = TwTab<R>();
-
-// R = R1 * R2 Cooley-Tukey in registers: input natural order n = R2 n1 + n2, output natural
-// order k = k1 + R1 k2; twiddles W_R^{n2 k1} are compile-time constants.
-template <int R1, int R2, int DIR>
-__device__ __forceinline__ void dft_ct(float2* v, const float2*, const float2* w1, const float2* w2) {
-  constexpr int R = R1 * R2;
-  float2 a[R];
-#pragma unroll
-  for (int n2 = 0; n2 < R2; ++n2) {
-    float2 t[R1];
-#pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1) t[n1] = v[R2 * n1 + n2];
-    Dft<R1, DIR>::run(t, w1);
-#pragma unroll
-    for (int k1 = 0; k1 < R1; ++k1) {
-      const int m = (n2 * k1) % R;
-      a[k1 * R2 + n2] = m == 0 ? t[k1] : twmul<DIR>(t[k1], make_float2(kTw<R>.re[m], kTw<R>.im[m]));
-    }
-  }
-#pragma unroll
-  for (int k1 = 0; k1 < R1; ++k1) {
-    float2 t[R2];
-#pragma unroll
-    for (int n2 = 0; n2 < R2; ++n2) t[n2] = a[k1 * R2 + n2];
-    Dft<R2, DIR>::run(t, w2);
-#pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) v[k1 + R1 * k2] = t[k2];
-  }
-}
-
-template <int DIR>
-struct Dft<6, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2* w) { dft_ct<3, 2, DIR>(v, w, nullptr, nullptr); }
-};
-template <int DIR>
-struct Dft<8, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2* w) { dft_ct<4, 2, DIR>(v, w, nullptr, nullptr); }
-};
-template <int DIR>
-struct Dft<12, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2* w) { dft_ct<4, 3, DIR>(v, w, nullptr, nullptr); }
-};
-template <int DIR>
-struct Dft<16, DIR> {
-  __device__ __forceinline__ static void run(float2* v, const float2* w) { dft_ct<4, 4, DIR>(v, w, nullptr, nullptr); }
-};
-
-__device__ __forceinline__ const float2* small_tab(const float2* tw, const FftTab& T, int R) {
-  switch (R) {
-    case 16: return tw + T.off_16;
-    case 12: return tw + T.off_12;
-    case 8: return tw + T.off_8;
-    case 6: return tw + T.off_6;
-    default: return tw;
-  }
-}
+__host__ __device__ inline FftTab fft_tab(int ny, int nz) { return FftTab{0, ny, ny + nz}; }
 
 // One pass over every transform of an axis: B transforms (batch stride bs), each of length
 // N = N1 N2 with element stride es.  STEP 0: DFTs of length R = N1 over n1 (stride N2), then
 // twiddles; STEP 1: DFTs of length R = N2 over contiguous positions.  Forward order: 0 then 1;
 // inverse: 1 then 0 (twiddles before the DFT).
 template <int R, int DIR, int STEP>
-__device__ __forceinline__ void axis_pass(float2* s, int B, int bs, int es, int N1, int N2, const float2* wN, int N,
-                                          const float2* wR) {
+__device__ __forceinline__ void axis_pass(float2* s, int B, int bs, int es, int N1, int N2, const float2* wN, int N) {
   const int J = STEP == 0 ? N2 : N1;   // transforms of length R per batch entry
   const int tasks = B * J;
   for (int t = threadIdx.x; t < tasks; t += blockDim.x) {
@@ -205,7 +56,7 @@ __device__ __forceinline__ void axis_pass(float2* s, int B, int bs, int es, int 
 #pragma unroll
         for (int i = 1; i < R; ++i) v[i] = twmul<DIR>(v[i], wN[j * i]);
       }
-      Dft<R, DIR>::run(v, wR);
+      Dft<R, DIR>::run(v, nullptr);
       if (DIR > 0) {
 #pragma unroll
         for (int i = 1; i < R; ++i) v[i] = twmul<DIR>(v[i], wN[j * i]);
@@ -215,7 +66,7 @@ __device__ __forceinline__ void axis_pass(float2* s, int B, int bs, int es, int 
     } else {           // j = k1; elements at N2 k1 + n2
 #pragma unroll
       for (int i = 0; i < R; ++i) v[i] = base[(N2 * j + i) * es];
-      Dft<R, DIR>::run(v, wR);
+      Dft<R, DIR>::run(v, nullptr);
 #pragma unroll
       for (int i = 0; i < R; ++i) base[(N2 * j + i) * es] = v[i];
     }
@@ -223,20 +74,10 @@ __device__ __forceinline__ void axis_pass(float2* s, int B, int bs, int es, int 
 }
 
 template <int DIR, int STEP>
-__device__ void axis_dispatch(float2* s, int B, int bs, int es, int N1, int N2, const float2* wN, int N,
-                              const float2* tw, const FftTab& T) {
-  const int R = STEP == 0 ? N1 : N2;
-  const float2* wR = small_tab(tw, T, R);
-  switch (R) {
-    case 2: axis_pass<2, DIR, STEP>(s, B, bs, es, N1, N2, wN, N, wR); break;
-    case 3: axis_pass<3, DIR, STEP>(s, B, bs, es, N1, N2, wN, N, wR); break;
-    case 4: axis_pass<4, DIR, STEP>(s, B, bs, es, N1, N2, wN, N, wR); break;
-    case 6: axis_pass<6, DIR, STEP>(s, B, bs, es, N1, N2, wN, N, wR); break;
-    case 8: axis_pass<8, DIR, STEP>(s, B, bs, es, N1, N2, wN, N, wR); break;
-    case 12: axis_pass<12, DIR, STEP>(s, B, bs, es, N1, N2, wN, N, wR); break;
-    case 16: axis_pass<16, DIR, STEP>(s, B, bs, es, N1, N2, wN, N, wR); break;
-    default: break;
-  }
+__device__ void axis_dispatch(float2* s, int B, int bs, int es, int N1, int N2, const float2* wN, int N) {
+  with_radix(STEP == 0 ? N1 : N2, [&](auto rc) {
+    axis_pass<decltype(rc)::value, DIR, STEP>(s, B, bs, es, N1, N2, wN, N);
+  });
 }
 
 __device__ __forceinline__ int perm_pos(int k, int N1, int N2) { return N2 * (k % N1) + k / N1; }
@@ -319,27 +160,27 @@ __device__ __forceinline__ void z_pass_hbm(float2* s, float2* g, const float2* w
   }
 }
 
-// Plane geometry with run-time sizes (any shape split_len accepts).
+// Plane geometry with run-time sizes (any shape radix_split accepts).
 struct GeoRt {
   static constexpr bool kHbmPasses = false;
   int ny, nz, y1, y2, z1, z2, P;
   __device__ void forward(float2* s, const float2* tw, const FftTab& T) const {
-    axis_dispatch<1, 0>(s, nz, P, 1, y1, y2, tw + T.off_y, ny, tw, T);
+    axis_dispatch<1, 0>(s, nz, P, 1, y1, y2, tw + T.off_y, ny);
     __syncthreads();
-    axis_dispatch<1, 1>(s, nz, P, 1, y1, y2, tw + T.off_y, ny, tw, T);
+    axis_dispatch<1, 1>(s, nz, P, 1, y1, y2, tw + T.off_y, ny);
     __syncthreads();
-    axis_dispatch<1, 0>(s, ny, 1, P, z1, z2, tw + T.off_z, nz, tw, T);
+    axis_dispatch<1, 0>(s, ny, 1, P, z1, z2, tw + T.off_z, nz);
     __syncthreads();
-    axis_dispatch<1, 1>(s, ny, 1, P, z1, z2, tw + T.off_z, nz, tw, T);
+    axis_dispatch<1, 1>(s, ny, 1, P, z1, z2, tw + T.off_z, nz);
   }
   __device__ void inverse(float2* s, const float2* tw, const FftTab& T) const {
-    axis_dispatch<-1, 1>(s, ny, 1, P, z1, z2, tw + T.off_z, nz, tw, T);
+    axis_dispatch<-1, 1>(s, ny, 1, P, z1, z2, tw + T.off_z, nz);
     __syncthreads();
-    axis_dispatch<-1, 0>(s, ny, 1, P, z1, z2, tw + T.off_z, nz, tw, T);
+    axis_dispatch<-1, 0>(s, ny, 1, P, z1, z2, tw + T.off_z, nz);
     __syncthreads();
-    axis_dispatch<-1, 1>(s, nz, P, 1, y1, y2, tw + T.off_y, ny, tw, T);
+    axis_dispatch<-1, 1>(s, nz, P, 1, y1, y2, tw + T.off_y, ny);
     __syncthreads();
-    axis_dispatch<-1, 0>(s, nz, P, 1, y1, y2, tw + T.off_y, ny, tw, T);
+    axis_dispatch<-1, 0>(s, nz, P, 1, y1, y2, tw + T.off_y, ny);
   }
 };
 
@@ -515,18 +356,6 @@ __global__ void __launch_bounds__(NT, 1) fft_dc_fixed_kernel(FftDcArgs a) {
   fft_dc_body(a, GeoFixed<Y1, Y2, Z1, Z2, NT>());
 }
 
-bool split_len(int n, int& n1, int& n2) {
-  static const int R[] = {16, 12, 8, 6, 4, 3, 2};
-  int best = -1;
-  for (int a : R)
-    for (int b : R)
-      if (a * b == n) {
-        const int bal = std::abs(a - b);
-        if (best < 0 || bal < best) { best = bal; n1 = a; n2 = b; }
-      }
-  return best >= 0;
-}
-
 size_t fft_dc_smem(int ny, int nz, int pitch) {
   const FftTab T = fft_tab(ny, nz);
   return align16b(sizeof(float2) * T.total) + 32 * sizeof(double) + sizeof(float2) * (size_t)pitch * nz +
@@ -537,7 +366,7 @@ size_t fft_dc_smem(int ny, int nz, int pitch) {
 
 bool fft_dc_supported(int ny, int nz) {
   int a, b, c, d;
-  if (!split_len(ny, a, b) || !split_len(nz, c, d)) return false;
+  if (!radix_split(ny, a, b) || !radix_split(nz, c, d)) return false;
   return fft_dc_smem(ny, nz, ny | 1) <= 227 * 1024;
 }
 
@@ -553,10 +382,6 @@ std::vector<float2> fft_dc_twiddles(int ny, int nz) {
   };
   fill(T.off_y, ny);
   fill(T.off_z, nz);
-  fill(T.off_16, 16);
-  fill(T.off_12, 12);
-  fill(T.off_8, 8);
-  fill(T.off_6, 6);
   return h;
 }
 
@@ -579,8 +404,8 @@ FftKernelChoice choose_fft(int ny, int nz) {
   else {
     c.kern = fft_dc_kernel;
     c.nt = kFftThreads;
-    split_len(ny, c.y1, c.y2);
-    split_len(nz, c.z1, c.z2);
+    radix_split(ny, c.y1, c.y2);
+    radix_split(nz, c.z1, c.z2);
   }
   return c;
 }

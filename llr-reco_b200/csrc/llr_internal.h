@@ -81,6 +81,16 @@ int fft_dc_grid(int ny, int nz);
 int launch_fft_dc(float2* u, const float2* yhat, const int* pos, const long long* off, const float2* twiddle,
                   const Geom& g, double* partials, int grid, const int* zero_ra, const BlockSource* zsrc,
                   cudaStream_t s);
+// planes that do not fit shared memory (fft_rows.cu)
+bool fft_rows_supported(int ny, int nz);
+bool fft_rows_expand_supported(int ny, int nq, int srank);
+std::vector<float2> fft_rows_twiddles(int ny, int nz);
+std::vector<int> fft_rows_ptr(const std::vector<int>& pos, const std::vector<long long>& off, int ny, int nz);
+int launch_fft_cols(const float2* src, float2* dst, const float2* tw_z, const Geom& g, long long planes, int dir,
+                    const PhaseTab* ph, float scale, cudaStream_t s);
+int launch_fft_rows(int mode, float2* u, const float2* coef, const float2* S, int srank, const float2* tw_y,
+                    const int* rowptr, const int* pos, const float2* yhat, const long long* off, const Geom& g,
+                    double* partials, int* np, cudaStream_t s);
 int launch_diff_norm(const float2* a, const float2* b, long long n, double* part_d, double* part_b, int nblocks,
                      cudaStream_t s);
 int launch_llr_eig_warp(const ProxOp& op, long long nblocks, cudaStream_t stream);
@@ -157,6 +167,9 @@ struct llr_ctx {
   bool fused_fft;           // hybrid and the (y, z) plane fits fft_dc_kernel
   int fft_grid;             // fft_dc_kernel CTAs (= residual partials)
   float2* d_fft_tw;         // fft_dc_kernel twiddle table
+  bool rows_fft;            // hybrid, the plane does not fit fft_dc_kernel: row and column kernels
+  float2* d_rows_tw;        // their twiddles (W_ny, W_nz; null where the lengths do not factor)
+  int* d_rows_ptr;          // first sampled line per (volume, kz)
   float load_scale;         // 1 / N_t
   // device buffers
   float2* d_x;              // iterate (planar, raw convention)

@@ -206,6 +206,34 @@ def test_fused_fft_dc_c2_plane(gpu, nx, nq):
     np.testing.assert_allclose(out[0][1], out[1][1], rtol=2e-6)
 
 
+@pytest.mark.parametrize("ny,nz", [(75, 52), (33, 9), (13, 11), (14, 10), (225, 15), (1, 7), (5, 1), (256, 130), (130, 256),
+                                   (35, 77)])
+def test_row_column_fft_dc(gpu, ny, nz):
+    """Plane sizes of the row and column kernels (every register length 1 to 16, line counts that leave a
+    ragged last tile, planes beyond shared memory), fused against cuFFT passes on the same data with
+    random block shifts; the zero-filled start too.  FP32 transforms of up to 256 x 256: relative 2e-6 each."""
+    nx, nq = 3, 5
+    bs = (3, min(4, ny), min(4, nz))
+    rng = np.random.default_rng(ny)
+    x = np.asfortranarray((rng.standard_normal((nx, ny, nz, nq)) + 1j * rng.standard_normal((nx, ny, nz, nq)))
+                          .astype(np.complex64))
+    y = x * (rng.random((1, ny, nz, nq)) < 0.4)
+    y[..., 0] = 0        # a volume without samples
+    out = {}
+    for mode in (0, 1):
+        p = ReconParams(vol_size=(nx, ny, nz), nq=nq, block_size=bs, prox_mode=L.LLR_PROX_SOFT_THRESH, lam=0.3, seed=3,
+                        fft_mode=mode)
+        with ReconContext(p) as ctx:
+            ctx.upload_kspace(np.asfortranarray(y.astype(np.complex64)))
+            ctx.init_zero_filled()
+            x0 = ctx.download_image()
+            h = ctx.iterate(3)
+            out[mode] = (x0, ctx.download_image(), np.asarray(h))
+    assert rel_err(out[0][0], out[1][0]) < 2e-6
+    assert rel_err(out[0][1], out[1][1]) < 6e-6
+    np.testing.assert_allclose(out[0][2], out[1][2], rtol=6e-6)
+
+
 def test_element_wise_sampling_path(gpu):
     """A sampling set that is not whole x-lines takes the element-wise (3-D FFT) path."""
     d = dataset((16, 12, 8), 5)
