@@ -199,6 +199,16 @@ static bool expand_in_kspace(const llr_ctx* c) {
   return coef_mode(c) && c->rows_fft && c->ph_uniform && fft_rows_expand_supported(c->g.ny, c->g.nq, c->cfg.subspace_rank);
 }
 
+// Voxels outside the shifted block grid are left raw by the prox; where the fused plane kernel follows
+// directly, it scales them as it loads its planes.
+static bool uncovered(const llr_ctx* c) {
+  return c->gx * c->cfg.block_size[0] < c->g.nx || c->gy * c->cfg.block_size[1] < c->g.ny ||
+         c->gz * c->cfg.block_size[2] < c->g.nz;
+}
+static bool uncovered_in_fft(const llr_ctx* c) {
+  return uncovered(c) && c->fused_fft && !c->wavelet_on && fft_dc_scales_uncovered(c->g.ny, c->g.nz);
+}
+
 // One prox pass on d_x.  standalone == true keeps the raw convention (used by single-step
 // entry points); otherwise the output is the FFT input (or the image, if the wavelet runs).
 static int prox_pass(llr_ctx* c, cudaStream_t s, const int* explicit_shift, bool standalone, float* block_stat) {
@@ -259,7 +269,7 @@ static int prox_pass(llr_ctx* c, cudaStream_t s, const int* explicit_shift, bool
   }
   if (block_stat || standalone) return LLR_OK;
   const int cover[3] = {c->gx * c->cfg.block_size[0], c->gy * c->cfg.block_size[1], c->gz * c->cfg.block_size[2]};
-  if (cover[0] < c->g.nx || cover[1] < c->g.ny || cover[2] < c->g.nz) {
+  if (uncovered(c) && !(uncovered_in_fft(c) && !explicit_shift)) {
     const int maxs[3] = {src.mx, src.my, src.mz};
     LLR_TRY(launch_scale_uncovered(c->d_x, c->g, cover, explicit_shift ? nullptr : c->d_iter, c->cfg.seed,
                                    explicit_shift, maxs, c->load_scale, src.ph, c->wavelet_on ? 1 : 0, s));
@@ -318,7 +328,7 @@ static int fused_dc_pass(llr_ctx* c, cudaStream_t s, double* out) {
   const bool zf = defer_zero_blocks(c);
   const BlockSource zsrc = make_source(c, nullptr, 1.f);
   LLR_TRY(launch_fft_dc(c->d_x, c->d_yhat, c->d_samp_pos, c->d_samp_off, c->d_fft_tw, c->g, c->d_partials,
-                        c->fft_grid, zf ? c->d_blk_ra : nullptr, zf ? &zsrc : nullptr, s));
+                        c->fft_grid, zf ? c->d_blk_ra : nullptr, &zsrc, uncovered_in_fft(c) ? c->load_scale : 0.f, s));
   if (!out) return finalize_iteration(c, c->fft_grid, s);
   return launch_finalize(c->d_partials, c->fft_grid, (double)c->load_scale, nullptr, 0, nullptr, 0, out, s);
 }

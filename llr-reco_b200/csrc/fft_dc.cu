@@ -25,8 +25,6 @@ namespace llr {
 
 namespace {
 
-constexpr int kFftThreads = 512;
-
 __host__ __device__ inline size_t align16b(size_t x) { return (x + 15) & ~size_t(15); }
 
 // Twiddle-table layout in shared memory (float2 entries): W_ny^j, then W_nz^j.
@@ -41,16 +39,17 @@ __host__ __device__ inline FftTab fft_tab(int ny, int nz) { return FftTab{0, ny,
 // twiddles; STEP 1: DFTs of length R = N2 over contiguous positions.  Forward order: 0 then 1;
 // inverse: 1 then 0 (twiddles before the DFT).
 template <int R, int DIR, int STEP>
-__device__ __forceinline__ void axis_pass(float2* s, int B, int bs, int es, int N1, int N2, const float2* wN, int N) {
+__device__ __forceinline__ void axis_pass(float2* s, FastDiv dB, int bs, int es, int N1, int N2, const float2* wN) {
   const int J = STEP == 0 ? N2 : N1;   // transforms of length R per batch entry
-  const int tasks = B * J;
+  const int tasks = (int)dB.d * J;
+  const int st = STEP == 0 ? N2 * es : es;
   for (int t = threadIdx.x; t < tasks; t += blockDim.x) {
-    const int b = t % B, j = t / B;
-    float2* base = s + (long long)b * bs;
+    const int j = (int)dB.div(t), b = t - j * (int)dB.d;
+    float2* base = s + b * bs + (STEP == 0 ? j * es : N2 * j * es);
     float2 v[R];
     if (STEP == 0) {   // j = n2; elements at N2 n1 + n2
 #pragma unroll
-      for (int i = 0; i < R; ++i) v[i] = base[(N2 * i + j) * es];
+      for (int i = 0; i < R; ++i) v[i] = base[i * st];
       // twiddle W_N^{n2 k1}, n2 k1 < N (before the inverse DFT, after the forward one)
       if (DIR < 0) {
 #pragma unroll
@@ -62,21 +61,21 @@ __device__ __forceinline__ void axis_pass(float2* s, int B, int bs, int es, int 
         for (int i = 1; i < R; ++i) v[i] = twmul<DIR>(v[i], wN[j * i]);
       }
 #pragma unroll
-      for (int i = 0; i < R; ++i) base[(N2 * i + j) * es] = v[i];
+      for (int i = 0; i < R; ++i) base[i * st] = v[i];
     } else {           // j = k1; elements at N2 k1 + n2
 #pragma unroll
-      for (int i = 0; i < R; ++i) v[i] = base[(N2 * j + i) * es];
+      for (int i = 0; i < R; ++i) v[i] = base[i * st];
       Dft<R, DIR>::run(v, nullptr);
 #pragma unroll
-      for (int i = 0; i < R; ++i) base[(N2 * j + i) * es] = v[i];
+      for (int i = 0; i < R; ++i) base[i * st] = v[i];
     }
   }
 }
 
 template <int DIR, int STEP>
-__device__ void axis_dispatch(float2* s, int B, int bs, int es, int N1, int N2, const float2* wN, int N) {
+__device__ __forceinline__ void axis_dispatch(float2* s, FastDiv dB, int bs, int es, int N1, int N2, const float2* wN) {
   with_radix(STEP == 0 ? N1 : N2, [&](auto rc) {
-    axis_pass<decltype(rc)::value, DIR, STEP>(s, B, bs, es, N1, N2, wN, N);
+    axis_pass<decltype(rc)::value, DIR, STEP>(s, dB, bs, es, N1, N2, wN);
   });
 }
 
@@ -92,6 +91,9 @@ struct FftDcArgs {
   int nx, ny, nz, nq;
   int y1, y2, z1, z2;        // ny = y1 y2, nz = z1 z2
   int pitch;                 // odd row pitch of the shared plane
+  FastDiv dny, dnz;
+  float unc_scale;           // run-time sizes, != 0: elements outside the block grid of zsrc are multiplied by
+                             // this as they are loaded (the prox leaves them raw)
   const int* zero_ra;        // optional: per-block kept counts of this iteration's prox; blocks
                              // with 0 were left unwritten and are zero-filled on load
   BlockSource zsrc;          // block grid and shift of that prox (when zero_ra is set)
@@ -164,23 +166,24 @@ __device__ __forceinline__ void z_pass_hbm(float2* s, float2* g, const float2* w
 struct GeoRt {
   static constexpr bool kHbmPasses = false;
   int ny, nz, y1, y2, z1, z2, P;
+  FastDiv dny, dnz;
   __device__ void forward(float2* s, const float2* tw, const FftTab& T) const {
-    axis_dispatch<1, 0>(s, nz, P, 1, y1, y2, tw + T.off_y, ny);
+    axis_dispatch<1, 0>(s, dnz, P, 1, y1, y2, tw + T.off_y);
     __syncthreads();
-    axis_dispatch<1, 1>(s, nz, P, 1, y1, y2, tw + T.off_y, ny);
+    axis_dispatch<1, 1>(s, dnz, P, 1, y1, y2, tw + T.off_y);
     __syncthreads();
-    axis_dispatch<1, 0>(s, ny, 1, P, z1, z2, tw + T.off_z, nz);
+    axis_dispatch<1, 0>(s, dny, 1, P, z1, z2, tw + T.off_z);
     __syncthreads();
-    axis_dispatch<1, 1>(s, ny, 1, P, z1, z2, tw + T.off_z, nz);
+    axis_dispatch<1, 1>(s, dny, 1, P, z1, z2, tw + T.off_z);
   }
   __device__ void inverse(float2* s, const float2* tw, const FftTab& T) const {
-    axis_dispatch<-1, 1>(s, ny, 1, P, z1, z2, tw + T.off_z, nz);
+    axis_dispatch<-1, 1>(s, dny, 1, P, z1, z2, tw + T.off_z);
     __syncthreads();
-    axis_dispatch<-1, 0>(s, ny, 1, P, z1, z2, tw + T.off_z, nz);
+    axis_dispatch<-1, 0>(s, dny, 1, P, z1, z2, tw + T.off_z);
     __syncthreads();
-    axis_dispatch<-1, 1>(s, nz, P, 1, y1, y2, tw + T.off_y, ny);
+    axis_dispatch<-1, 1>(s, dnz, P, 1, y1, y2, tw + T.off_y);
     __syncthreads();
-    axis_dispatch<-1, 0>(s, nz, P, 1, y1, y2, tw + T.off_y, ny);
+    axis_dispatch<-1, 0>(s, dnz, P, 1, y1, y2, tw + T.off_y);
   }
 };
 
@@ -232,9 +235,10 @@ __device__ __forceinline__ void fft_dc_body(const FftDcArgs& a, const Geo& geo) 
                                                         32 * sizeof(double) + sizeof(float2) * (size_t)P * nz +
                                                         align16b(sizeof(int) * (size_t)(ny + nz + 4)));
   const bool zf = a.zero_ra != nullptr;
+  const bool unc = !Geo::kHbmPasses && a.unc_scale != 0.f;
   const int tid = threadIdx.x;
   for (int i = tid; i < T.total; i += blockDim.x) tw[i] = a.twiddle[i];
-  if (zf) {
+  if (zf || unc) {
     if (tid == 0) block_shift(a.zsrc, zsh);
     __syncthreads();
     const BlockSource& zs = a.zsrc;
@@ -261,18 +265,20 @@ __device__ __forceinline__ void fft_dc_body(const FftDcArgs& a, const Geo& geo) 
   };
   const long long nyz = (long long)ny * nz;
   const long long planes = (long long)a.nx * a.nq;
-  const int dz = (int)blockDim.x / ny, dy = (int)blockDim.x - dz * ny;   // per-stride (z, y) step
   double err = 0.0;
   for (long long pl = blockIdx.x; pl < planes; pl += gridDim.x) {
     const int q = (int)(pl / a.nx), ix = (int)(pl - (long long)q * a.nx);
     float2* g = a.u + pl * nyz;
     __syncthreads();   // previous plane stored, twiddles visible
-    if (zf) {          // flags of the blocks of this plane's x slab
+    int gxi = 0;
+    if (zf || unc) {
       const BlockSource& zs = a.zsrc;
       int r = (ix - zsh[0]) % a.nx;
       if (r < 0) r += a.nx;
-      const int gxi = r < zs.gx * zs.bx ? r / zs.bx : -1;
-      const int nslab = zs.gy * zs.gz;
+      gxi = r < zs.gx * zs.bx ? r / zs.bx : -1;
+    }
+    if (zf) {          // flags of the blocks of this plane's x slab
+      const int nslab = a.zsrc.gy * a.zsrc.gz;
       for (int t = tid; t < nslab; t += blockDim.x)
         zfl[t] = gxi >= 0 && a.zero_ra[t + (long long)nslab * gxi] == 0;
       __syncthreads();
@@ -281,20 +287,27 @@ __device__ __forceinline__ void fft_dc_body(const FftDcArgs& a, const Geo& geo) 
       // forward: z axis (its first pass loads the plane from HBM), then y axis
       geo.forward_hbm(s, g, tw, T, zero_at);
     } else {
-      {   // asynchronous 8-byte copies: every element in flight at once, no register staging
-        int z = tid / ny, y = tid - (tid / ny) * ny;
-        for (int e = tid; e < ny * nz; e += blockDim.x) {
-          const unsigned dst = (unsigned)__cvta_generic_to_shared(s + z * P + y);
-          if (zero_at(y, z))
-            s[z * P + y] = make_float2(0.f, 0.f);
-          else
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(g + e) : "memory");
-          y += dy;
-          z += dz;
-          if (y >= ny) { y -= ny; ++z; }
+      // asynchronous 8-byte copies: every element in flight at once, no register staging; elements of
+      // blocks left unwritten become zero, those outside the block grid are scaled
+      for (int e = tid; e < ny * nz; e += blockDim.x) {
+        const int z = (int)geo.dny.div(e), y = e - z * ny;
+        float2* d = s + z * P + y;
+        if (zf || unc) {
+          const int by = zgy[y], bz = zgz[z];
+          if (by < 0 || bz < 0 || gxi < 0) {
+            if (unc) {
+              *d = cscale(g[e], a.unc_scale);
+              continue;
+            }
+          } else if (zf && zfl[by + a.zsrc.gy * bz]) {
+            *d = make_float2(0.f, 0.f);
+            continue;
+          }
         }
-        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(d);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(g + e) : "memory");
       }
+      asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
       __syncthreads();
       // forward: y axis (rows, element stride 1, batch stride P), then z axis (columns)
       geo.forward(s, tw, T);
@@ -324,12 +337,9 @@ __device__ __forceinline__ void fft_dc_body(const FftDcArgs& a, const Geo& geo) 
       // inverse: z axis then y axis, each mirrored (step 1 then step 0)
       geo.inverse(s, tw, T);
       __syncthreads();
-      int z = tid / ny, y = tid - (tid / ny) * ny;
       for (int e = tid; e < ny * nz; e += blockDim.x) {
-        g[e] = s[z * P + y];
-        y += dy;
-        z += dz;
-        if (y >= ny) { y -= ny; ++z; }
+        const int z = (int)geo.dny.div(e);
+        g[e] = s[z * P + e - z * ny];
       }
     }
   }
@@ -345,9 +355,14 @@ __device__ __forceinline__ void fft_dc_body(const FftDcArgs& a, const Geo& geo) 
   }
 }
 
-__global__ void __launch_bounds__(kFftThreads, 1) fft_dc_kernel(FftDcArgs a) {
+// Run-time sizes.  Every instance keeps 24 warps per SM at 85 registers; small planes run them as several
+// small CTAs, whose barriers hold back fewer warps (75 x 52 planes, 90 x 33 of them: 264 us with one CTA
+// of 512 threads per SM, 169 us now).
+template <int NT, int PER_SM>
+__global__ void __launch_bounds__(NT, PER_SM) fft_dc_kernel(FftDcArgs a) {
   GeoRt geo;
   geo.ny = a.ny; geo.nz = a.nz; geo.y1 = a.y1; geo.y2 = a.y2; geo.z1 = a.z1; geo.z2 = a.z2; geo.P = a.pitch;
+  geo.dny = a.dny; geo.dnz = a.dnz;
   fft_dc_body(a, geo);
 }
 
@@ -402,8 +417,12 @@ FftKernelChoice choose_fft(int ny, int nz) {
   else if (ny == 96 && nz == 48) c = {fft_dc_fixed_kernel<12, 8, 8, 6, 192>, 192, 12, 8, 8, 6};
   else if (ny == 64 && nz == 64) c = {fft_dc_fixed_kernel<8, 8, 8, 8, 256>, 256, 8, 8, 8, 8};
   else {
-    c.kern = fft_dc_kernel;
-    c.nt = kFftThreads;
+    // CTAs per SM that the plane's shared memory allows
+    const size_t per = (228 * 1024) / (fft_dc_smem(ny, nz, ny | 1) + 1024);
+    if (per >= 6) c = {fft_dc_kernel<128, 6>, 128};
+    else if (per >= 3) c = {fft_dc_kernel<256, 3>, 256};
+    else if (per == 2) c = {fft_dc_kernel<384, 2>, 384};
+    else c = {fft_dc_kernel<768, 1>, 768};
     radix_split(ny, c.y1, c.y2);
     radix_split(nz, c.z1, c.z2);
   }
@@ -411,6 +430,11 @@ FftKernelChoice choose_fft(int ny, int nz) {
 }
 
 }  // namespace
+
+// Whether the plane's kernel scales the elements outside the block grid itself.
+bool fft_dc_scales_uncovered(int ny, int nz) {
+  return !((ny == 192 && nz == 96) || (ny == 96 && nz == 48) || (ny == 64 && nz == 64));
+}
 
 int fft_dc_grid(int ny, int nz) {
   int dev = 0, nsm = 0, smem_sm = 0, regs_sm = 0;
@@ -424,16 +448,23 @@ int fft_dc_grid(int ny, int nz) {
   const int by_smem = smem_sm / (int)(fft_dc_smem(ny, nz, ny | 1) + 1024);
   const int regs_warp = ((fa.numRegs * 32 + 255) / 256) * 256;
   const int by_regs = regs_sm / std::max(1, regs_warp * (c.nt / 32));
-  const int per = std::max(1, std::min(4, std::min(by_smem, by_regs)));
+  const int per = std::max(1, std::min(6, std::min(by_smem, by_regs)));
   return nsm * per;
 }
 
 int launch_fft_dc(float2* u, const float2* yhat, const int* pos, const long long* off, const float2* twiddle,
                   const Geom& g, double* partials, int grid, const int* zero_ra, const BlockSource* zsrc,
-                  cudaStream_t s) {
+                  float unc_scale, cudaStream_t s) {
   FftDcArgs a;
   a.zero_ra = nullptr;
   a.zsrc = BlockSource{};
+  a.unc_scale = 0.f;
+  if (unc_scale != 0.f && zsrc) {
+    a.unc_scale = unc_scale;
+    a.zsrc = *zsrc;
+  }
+  a.dny = FastDiv(g.ny);
+  a.dnz = FastDiv(g.nz);
   if (zero_ra && zsrc && zsrc->kind == 1 && (long long)zsrc->gy * zsrc->gz <= kZeroFlagMax) {
     a.zero_ra = zero_ra;
     a.zsrc = *zsrc;

@@ -80,7 +80,8 @@ std::vector<float2> fft_dc_twiddles(int ny, int nz);
 int fft_dc_grid(int ny, int nz);
 int launch_fft_dc(float2* u, const float2* yhat, const int* pos, const long long* off, const float2* twiddle,
                   const Geom& g, double* partials, int grid, const int* zero_ra, const BlockSource* zsrc,
-                  cudaStream_t s);
+                  float unc_scale, cudaStream_t s);
+bool fft_dc_scales_uncovered(int ny, int nz);
 // planes that do not fit shared memory (fft_rows.cu)
 bool fft_rows_supported(int ny, int nz);
 bool fft_rows_expand_supported(int ny, int nq, int srank);
