@@ -245,6 +245,8 @@ static int prox_pass(llr_ctx* c, cudaStream_t s, const int* explicit_shift, bool
     op.defer_zero = (!standalone && !block_stat && !explicit_shift && defer_zero_blocks(c)) ? 1 : 0;
     op.vwide = c->d_vwide;
     op.vwide_ctas = c->vwide_ctas;
+    op.rot_log = c->d_rot_log;
+    op.rot_ctas = c->rot_ctas;
     if (c->obj_mode == 2 && !standalone && !block_stat && !explicit_shift) {
       LLR_CUDA_TRY(cudaMemsetAsync(c->d_blk_nuc, 0, sizeof(double) * (size_t)std::max<long long>(1, c->nblocks), s));
       op.blk_nuc = c->d_blk_nuc;
@@ -421,6 +423,9 @@ int llr_ctx_create(const llr_config* cfg, llr_ctx** out) {
   if (cfg->subspace_rank == 0 && (c->g.nq > 64 || prox_needs_wide_fallback(c->m, c->g.nq))) {
     c->vwide_ctas = wide_jacobi_ctas();
     if ((st = dalloc(&c->d_vwide, (size_t)c->vwide_ctas * (size_t)wide_v_stride()))) return fail(st);
+    c->rot_ctas = (int)std::min<long long>(std::max<long long>(1, c->nblocks), (long long)kJacobiPerSm * c->vwide_ctas);
+    if (c->g.nq > 64 && (st = dalloc(&c->d_rot_log, (size_t)c->rot_ctas * (size_t)jacobi_log_stride(c->g.nq))))
+      return fail(st);
   }
   {
     int per[3], P = 1;
@@ -440,7 +445,7 @@ int llr_ctx_create(const llr_config* cfg, llr_ctx** out) {
   }
   e = cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
   if (e != cudaSuccess) return fail(cuda_error(e, "cudaMemsetAsync", __FILE__, __LINE__));
-  if (cfg->subspace_rank == 0 && c->g.nq <= 64 &&
+  if (cfg->subspace_rank == 0 && c->g.nq <= kProxMaxN &&
       ((st = dalloc(&c->d_gram, (size_t)std::max<long long>(1, c->nblocks) * (size_t)prox_gram_stride(c->g.nq))) ||
        (st = dalloc(&c->d_blk_ra, (size_t)std::max<long long>(1, c->nblocks) + 1))))
     return fail(st);
@@ -500,7 +505,7 @@ int llr_ctx_destroy(llr_ctx* c) {
   dfree(c->d_x); dfree(c->d_work); dfree(c->d_yhat); dfree(c->d_samp_pos); dfree(c->d_samp_off);
   dfree(c->d_ph_ksp); dfree(c->d_ph_img); dfree(c->d_S); dfree(c->d_partials); dfree(c->d_hist); dfree(c->d_iter);
   dfree(c->d_obj); dfree(c->d_blk_nuc);
-  dfree(c->d_block_stat); dfree(c->d_fb); dfree(c->d_gram); dfree(c->d_blk_ra); dfree(c->d_fft_tw); dfree(c->d_rows_tw); dfree(c->d_rows_ptr); dfree(c->d_err); dfree(c->d_vwide); dfree(c->d_wavelet_work); dfree(c->d_fft_work);
+  dfree(c->d_block_stat); dfree(c->d_fb); dfree(c->d_gram); dfree(c->d_blk_ra); dfree(c->d_fft_tw); dfree(c->d_rows_tw); dfree(c->d_rows_ptr); dfree(c->d_err); dfree(c->d_vwide); dfree(c->d_rot_log); dfree(c->d_wavelet_work); dfree(c->d_fft_work);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   scratch_trim();
   delete c;
@@ -1075,6 +1080,7 @@ int llr_ctx_device_bytes(const llr_ctx* c, size_t* bytes) {
   b += c->fft_work_bytes + c->wavelet_work_elems * sizeof(float2);
   if (c->d_gram) b += (size_t)std::max<long long>(1, c->nblocks) * (size_t)prox_gram_stride(c->g.nq) * sizeof(float2);
   if (c->d_rows_ptr) b += (size_t)c->g.nq * (c->g.nz + 1) * sizeof(int);
+  if (c->d_rot_log) b += (size_t)c->rot_ctas * (size_t)jacobi_log_stride(c->g.nq) * sizeof(float);
   if (c->d_vwide) b += (size_t)c->vwide_ctas * (size_t)wide_v_stride() * sizeof(float2);
   *bytes = b;
   return LLR_OK;

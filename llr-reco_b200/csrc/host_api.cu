@@ -393,6 +393,11 @@ static int batch_prox(int m, int n, int mode, int rank, float lam, int batch, ll
   // fallback list + count, then the per-block kept counts + queue counter
   LLR_CUDA_TRY(scratch_alloc((void**)&fb, sizeof(int) * (2 * (size_t)batch + 2), s));
   cudaError_t e = scratch_alloc((void**)&gram, sizeof(float2) * (size_t)batch * (size_t)prox_gram_stride(n), s);
+  if (e == cudaErrorMemoryAllocation && n > 64) {   // the wide Jacobi kernel needs no Gram scratch
+    cudaGetLastError();
+    gram = nullptr;
+    e = cudaSuccess;
+  }
   if (e != cudaSuccess) {
     cudaFreeAsync(fb, s);
     return cuda_error(e, "scratch_alloc", __FILE__, __LINE__);
@@ -410,15 +415,25 @@ static int batch_prox(int m, int n, int mode, int rank, float lam, int batch, ll
     e = scratch_alloc((void**)&vwide, sizeof(float2) * (size_t)op.vwide_ctas * (size_t)wide_v_stride(), s);
     if (e != cudaSuccess) {
       cudaFreeAsync(fb, s);
-      cudaFreeAsync(gram, s);
+      if (gram) cudaFreeAsync(gram, s);
       return cuda_error(e, "scratch_alloc", __FILE__, __LINE__);
     }
     op.vwide = vwide;
   }
+  float* rot_log = nullptr;
+  if (gram && n > 64 && n <= kProxMaxN) {   // without the log every block takes the wide kernel
+    op.rot_ctas = (int)std::min<long long>(batch, (long long)kJacobiPerSm * wide_jacobi_ctas());
+    if (scratch_alloc((void**)&rot_log, sizeof(float) * (size_t)op.rot_ctas * (size_t)jacobi_log_stride(n), s) != cudaSuccess) {
+      cudaGetLastError();
+      rot_log = nullptr;
+    }
+    op.rot_log = rot_log;
+  }
   int st = launch_llr_prox(src, op, s);
   if (vwide) cudaFreeAsync(vwide, s);
+  if (rot_log) cudaFreeAsync(rot_log, s);
   e = cudaFreeAsync(fb, s);
-  cudaError_t e2 = cudaFreeAsync(gram, s);
+  cudaError_t e2 = gram ? cudaFreeAsync(gram, s) : cudaSuccess;
   if (st == LLR_OK && e != cudaSuccess) st = cuda_error(e, "cudaFreeAsync", __FILE__, __LINE__);
   if (st == LLR_OK && e2 != cudaSuccess) st = cuda_error(e2, "cudaFreeAsync", __FILE__, __LINE__);
   return st;

@@ -9,6 +9,9 @@
 // computes D^T D directly.
 // Precision: 3xTF32 -- x = hi + lo with hi = tf32(x), and P accumulates hi*hi + hi*lo + lo*hi
 // in FP32, which keeps FP32-level accuracy (the lo*lo term is below FP32 rounding).
+// Wider matrices (64 < n <= 128, NPMAX = 128): Re C and Im C are two operand tiles of 128 columns, and the
+// accumulator pair R = Re^T Re + Im^T Im, Q = Re^T Im (256 TMEM columns) gives Re G = R and
+// Im G[i][j] = Q[i][j] - Q[j][i].  One CTA of 16 warps per SM (the two chunk buffers take 128 KB).
 // Rows stream in 32-row chunks, double-buffered, with the loads of the chunk two positions
 // ahead (possibly of the CTA's next block) in flight: while the tensor core consumes one chunk
 // the 8 warps gather, phase-correct and split the next one.  One elected thread issues the
@@ -24,10 +27,9 @@ namespace llr {
 
 namespace {
 
-constexpr int kTcWarps = 8;
-constexpr int kTcThreads = 32 * kTcWarps;
 constexpr int kKC = 32;                    // rows (K) per staged chunk
-constexpr int kQT = (64 + kTcWarps - 1) / kTcWarps;   // volumes per warp per chunk (kTcWarps x kQT >= n)
+constexpr int kQT = 8;                     // volumes per warp per chunk (warps x kQT >= n)
+constexpr int tc_warps(int npmax) { return npmax / kQT; }
 constexpr int kOpBytes = 128 * kKC * 4;    // one operand plane (hi or lo) of one chunk
 // Row table of one block: planar offset of every row and either the row's phase (uniform
 // over the volumes) or its coordinates (per-volume phase).  The kernel keeps kRowBufs tables:
@@ -55,7 +57,12 @@ struct TcHdr {
 constexpr uint32_t kIdesc = umma_idesc_tf32(128, 128);
 
 template <int NPMAX>
-__global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource src, ProxOp op, TcLayout L) {
+__global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
+    llr_gram_tc_kernel(BlockSource src, ProxOp op, TcLayout L) {
+  constexpr bool WIDE = NPMAX > 64;
+  constexpr int kTcWarps = tc_warps(NPMAX), kTcThreads = 32 * kTcWarps;
+  constexpr int kPlanes = WIDE ? 2 : 1;            // operand tiles per precision part (Re, Im)
+  constexpr uint32_t kTmemCols = WIDE ? 256u : 128u;
   extern __shared__ __align__(1024) unsigned char smem[];
   TcHdr* hdr = reinterpret_cast<TcHdr*>(smem + L.off_hdr);
   int* row_off = reinterpret_cast<int*>(smem + L.off_row);        // [nbuf][m]
@@ -68,7 +75,7 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hdr->tmem)),
-                 "r"(128u));
+                 "r"(kTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
@@ -133,11 +140,12 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
   // one chunk: wait for its operand buffer, convert `pre` into it, refill `pre` two chunks
   // ahead, hand the buffer to the tensor core
   int gpar = 0;
-  // operand offsets of this thread's elements: row q = warp + kTcWarps t (and n + q), column
-  // lane; adding 8 to a row leaves its swizzle phase and moves it one 1 KB atom on, so
+  // operand offsets of this thread's elements: row q = warp + kTcWarps t (and n + q, or the Im tile's
+  // row q), column lane; adding 8 to a row leaves its swizzle phase and moves it one 1 KB atom on, so
   // op_offset(q + 8 t, lane) = op_offset(q, lane) + 1024 t
-  static_assert(kTcWarps == 8, "the 1 KB step per t assumes rows 8 apart");
-  const int oq0 = op_offset(warp, lane), oi0 = op_offset(n + warp, lane);
+  static_assert(kTcWarps % 8 == 0, "the step per t assumes rows a multiple of 8 apart");
+  constexpr int kStepT = 1024 * (kTcWarps / 8);
+  const int oq0 = op_offset(warp, lane), oi0 = WIDE ? kOpBytes + oq0 : op_offset(n + warp, lane);
   auto step = [&](float2 (&pre)[kQT], long long blk, int j, int c) -> bool {
     const int b = gpar;
     if (used[b]) {  // the MMAs that read this buffer two chunks ago must be done
@@ -145,8 +153,8 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
       phase[b] ^= 1u;
       if (__syncthreads_or(!ok)) return false;
     }
-    unsigned char* hi = ops + (size_t)b * 2 * kOpBytes;
-    unsigned char* lo = hi + kOpBytes;
+    unsigned char* hi = ops + (size_t)b * 2 * kPlanes * kOpBytes;
+    unsigned char* lo = hi + kPlanes * kOpBytes;
     const int r = c * kKC + lane;
     const TcRowAux* ra = row_aux + (size_t)(j % nbuf) * m;
     const bool ph_row = src.kind == 1 && r < m;
@@ -165,7 +173,7 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
         x = cscale(cmul_bc(x, p), src.load_scale);
       }
       const uint32_t a = tf32_rna(x.x), bb = tf32_rna(x.y);
-      const int oq = oq0 + 1024 * t, oi = oi0 + 1024 * t;
+      const int oq = oq0 + kStepT * t, oi = oi0 + kStepT * t;
       *reinterpret_cast<uint32_t*>(hi + oq) = a;
       *reinterpret_cast<uint32_t*>(hi + oi) = bb;
       *reinterpret_cast<uint32_t*>(lo + oq) = __float_as_uint(x.x - __uint_as_float(a));
@@ -185,9 +193,20 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
       for (int s = 0; s < kKC / 8; ++s) {
         const uint64_t dh = umma_desc_sw128(ah + s * 32);
         const uint64_t dl = umma_desc_sw128(al + s * 32);
-        umma_tf32(tmem, dh, dh, kIdesc, (c > 0 || s > 0) ? 1u : 0u);
+        const uint32_t acc = (c > 0 || s > 0) ? 1u : 0u;
+        umma_tf32(tmem, dh, dh, kIdesc, acc);
         umma_tf32(tmem, dh, dl, kIdesc, 1u);
         umma_tf32(tmem, dl, dh, kIdesc, 1u);
+        if (WIDE) {
+          const uint64_t ih = umma_desc_sw128(ah + kOpBytes + s * 32);
+          const uint64_t il = umma_desc_sw128(al + kOpBytes + s * 32);
+          umma_tf32(tmem, ih, ih, kIdesc, 1u);
+          umma_tf32(tmem, ih, il, kIdesc, 1u);
+          umma_tf32(tmem, il, ih, kIdesc, 1u);
+          umma_tf32(tmem + 128, dh, ih, kIdesc, acc);
+          umma_tf32(tmem + 128, dh, il, kIdesc, 1u);
+          umma_tf32(tmem + 128, dl, ih, kIdesc, 1u);
+        }
       }
       umma_commit(smem_u32(&hdr->mbar[b]));
       if (c == nchunks - 1) umma_commit(smem_u32(&hdr->mbar[2]));
@@ -197,8 +216,8 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
     return true;
   };
 
-  // operand planes start zeroed: rows 2n..127 (M padding) are never written by the gather
-  for (int i = tid; i < 4 * kOpBytes / 16; i += kTcThreads)
+  // operand planes start zeroed: the padding rows (M up to 128) are never written by the gather
+  for (int i = tid; i < 4 * kPlanes * kOpBytes / 16; i += kTcThreads)
     reinterpret_cast<float4*>(ops)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   long long blk = blockIdx.x;
   if (blk < src.nblocks) {
@@ -237,12 +256,16 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
     }
     asm volatile("tcgen05.fence::after_thread_sync;");
     float* Ps = reinterpret_cast<float*>(ops);
-    const int ldp = 2 * n + 1;
+    // narrow: P (2n x 2n), odd pitch; wide: R then Q (n x n each, odd pitch)
+    const int cols = WIDE ? n : 2 * n, ldp = cols | 1;
     // warp w reads TMEM lanes 32 (w mod 4) .. + 31 (its quadrant); the warps sharing a quadrant
     // split the 32-column chunks
     const int quad = warp & 3;
     const int a = 32 * quad + lane;          // accumulator row held by this thread
-    for (int cc = 32 * (warp >> 2); cc < 2 * n; cc += 32 * (kTcWarps / 4)) {
+    for (int c2 = 32 * (warp >> 2); c2 < (int)kTmemCols; c2 += 32 * (kTcWarps / 4)) {
+      const int cc = WIDE ? c2 & 127 : c2;          // column within R, Q or P
+      if (cc >= cols) continue;                     // warp-uniform
+      float* Pd = Ps + (WIDE && c2 >= 128 ? (size_t)n * ldp : 0);
       uint32_t r[32];
       asm volatile(
           "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -251,12 +274,12 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
             "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
             "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
             "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-          : "r"(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)cc));
+          : "r"(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)c2));
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (a < 2 * n) {
+      if (a < cols) {
 #pragma unroll
         for (int jj = 0; jj < 32; ++jj)
-          if (cc + jj < 2 * n) Ps[a * ldp + cc + jj] = __uint_as_float(r[jj]);
+          if (cc + jj < cols) Pd[a * ldp + cc + jj] = __uint_as_float(r[jj]);
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -274,8 +297,14 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
           const int s = min(s0 + 32 * u, len - 1);
           row[u] = s <= i ? i : i2;
           col[u] = s <= i ? s : s - i - 1;
-          re[u] = Ps[row[u] * ldp + col[u]] + Ps[(n + row[u]) * ldp + n + col[u]];
-          im[u] = Ps[row[u] * ldp + n + col[u]] - Ps[(n + row[u]) * ldp + col[u]];
+          if (WIDE) {
+            const float* Q = Ps + (size_t)n * ldp;
+            re[u] = Ps[row[u] * ldp + col[u]];
+            im[u] = Q[row[u] * ldp + col[u]] - Q[col[u] * ldp + row[u]];
+          } else {
+            re[u] = Ps[row[u] * ldp + col[u]] + Ps[(n + row[u]) * ldp + n + col[u]];
+            im[u] = Ps[row[u] * ldp + n + col[u]] - Ps[(n + row[u]) * ldp + col[u]];
+          }
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u)
@@ -283,10 +312,10 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
       }
     }
     __syncthreads();
-    // the staging overwrote the padding rows 2n..127 of the operand planes: zero them again
-    for (int i = tid; i < 4 * (128 - 2 * n) * 8; i += kTcThreads) {   // 8 x 16 B per 128-B row
-      const int plane = i / ((128 - 2 * n) * 8), rem = i - plane * ((128 - 2 * n) * 8);
-      const int mn = 2 * n + (rem >> 3), c16 = rem & 7;
+    // the staging overwrote the padding rows of the operand planes: zero them again
+    for (int i = tid; i < 4 * kPlanes * (128 - cols) * 8; i += kTcThreads) {   // 8 x 16 B per 128-B row
+      const int plane = i / ((128 - cols) * 8), rem = i - plane * ((128 - cols) * 8);
+      const int mn = cols + (rem >> 3), c16 = rem & 7;
       *reinterpret_cast<float4*>(ops + (size_t)plane * kOpBytes + (mn >> 3) * 1024 + (mn & 7) * 128 + c16 * 16) =
           make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -301,7 +330,7 @@ __global__ void __launch_bounds__(kTcThreads, 3) llr_gram_tc_kernel(BlockSource 
   mbar_wait(smem_u32(&hdr->mbar[2]), phase[2]);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128u));
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
 template <int NPMAX>
@@ -314,7 +343,8 @@ TcLayout make_tc_layout(int m, int n) {
   L.off_aux = off; off = align16(off + sizeof(TcRowAux) * (size_t)m * L.nbuf);
   off = (off + 1023) & ~size_t(1023);
   L.off_op = off;
-  const size_t opb = std::max<size_t>(4 * (size_t)kOpBytes, sizeof(float) * (size_t)(2 * n) * (2 * n + 1));
+  const size_t stage = NPMAX > 64 ? 2 * (size_t)n * (n | 1) : (size_t)(2 * n) * (2 * n + 1);
+  const size_t opb = std::max<size_t>((NPMAX > 64 ? 8 : 4) * (size_t)kOpBytes, sizeof(float) * stage);
   L.op_bytes = (int)opb;
   off += opb;
   L.total = off;
@@ -324,15 +354,18 @@ TcLayout make_tc_layout(int m, int n) {
 }  // namespace
 
 bool llr_gram_tc_supported(int m, int n) {
-  if (n < 1 || 2 * n > 128 || m < 1 || 8 * n > 4 * kTcThreads) return false;
-  return make_tc_layout<64>(m, n).total <= 227 * 1024;
+  if (n < 1 || n > 128 || m < 1) return false;
+  return (n <= 64 ? make_tc_layout<64>(m, n) : make_tc_layout<128>(m, n)).total <= 227 * 1024;
 }
 
-int launch_llr_gram_tc(const BlockSource& src, const ProxOp& op, cudaStream_t stream) {
-  if (2 * op.n > 128) return set_error(LLR_ERR_UNSUPPORTED, "tensor-core Gram needs 2n <= 128 (n = %d)", op.n);
-  TcLayout L = make_tc_layout<64>(op.m, op.n);
+namespace {
+
+template <int NPMAX>
+int launch_gram_instance(const BlockSource& src, const ProxOp& op, cudaStream_t stream) {
+  constexpr int kTcThreads = 32 * tc_warps(NPMAX);
+  TcLayout L = make_tc_layout<NPMAX>(op.m, op.n);
   if (L.total > 227 * 1024) return set_error(LLR_ERR_UNSUPPORTED, "tensor-core Gram needs %zu B smem", L.total);
-  auto kern = llr_gram_tc_kernel<64>;
+  auto kern = llr_gram_tc_kernel<NPMAX>;
   LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
   LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   int dev = 0, nsm = 0, smem_sm = 0, regs_sm = 0;
@@ -344,13 +377,13 @@ int launch_llr_gram_tc(const BlockSource& src, const ProxOp& op, cudaStream_t st
   LLR_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));
   // Residency from the kernel's own resources. The occupancy query reports one CTA per SM for
   // this kernel although three fit, so the count is derived here: shared memory (the driver
-  // reserves 1 KB per CTA), registers (allocated per warp in units of 256) and TMEM (128 of
+  // reserves 1 KB per CTA), registers (allocated per warp in units of 256) and TMEM (128 or 256 of
   // the SM's 512 columns per CTA). The kernel strides over blocks, so a grid larger than
   // what is resident is still correct, only slower.
   const int regs_warp = ((fa.numRegs * 32 + 255) / 256) * 256;
   const int by_regs = regs_warp > 0 ? regs_sm / (regs_warp * (kTcThreads / 32)) : 4;
   const int by_smem = smem_sm / (int)(L.total + fa.sharedSizeBytes + 1024);
-  int occ = std::min(std::min(by_regs, by_smem), 4);
+  int occ = std::min(std::min(by_regs, by_smem), NPMAX > 64 ? 2 : 4);
   if (occ < 1) return set_error(LLR_ERR_UNSUPPORTED, "tensor-core Gram kernel cannot be resident");
   const long long grid = std::min<long long>(src.nblocks, (long long)nsm * occ);
   if (grid < 1) return LLR_OK;
@@ -358,6 +391,13 @@ int launch_llr_gram_tc(const BlockSource& src, const ProxOp& op, cudaStream_t st
   kern<<<(unsigned)grid, kTcThreads, L.total, stream>>>(src, op, L);
   LLR_CUDA_TRY(cudaGetLastError());
   return LLR_OK;
+}
+
+}  // namespace
+
+int launch_llr_gram_tc(const BlockSource& src, const ProxOp& op, cudaStream_t stream) {
+  if (op.n > 128) return set_error(LLR_ERR_UNSUPPORTED, "tensor-core Gram needs n <= 128 (n = %d)", op.n);
+  return op.n <= 64 ? launch_gram_instance<64>(src, op, stream) : launch_gram_instance<128>(src, op, stream);
 }
 
 }  // namespace llr

@@ -54,6 +54,8 @@ struct ProxOp {
                        // FFT that follows in the same iteration zero-fills them as it loads
   float2* vwide = nullptr;  // 64 < n <= 128: per-CTA eigenvector scratch of the wide Jacobi kernel,
   int vwide_ctas = 0;       // vwide_ctas * wide_v_stride() float2
+  float* rot_log = nullptr;    // 64 < n <= 128, split path: rot_ctas * jacobi_log_stride(n) floats
+  int rot_ctas = 0;
   double* blk_nuc = nullptr;   // soft threshold: per block sum over its singular values s of
                                // (s - lambda)+ in FP64, the nuclear norm of the block's prox output
                                // (the regulariser term of the objective); blocks left at 0 keep none
@@ -62,8 +64,16 @@ struct ProxOp {
 // Widest Casorati column count of the prox kernels, and the per-CTA eigenvector scratch the
 // wide (64 < n <= 128) Jacobi kernel needs, in float2.
 constexpr int kProxMaxN = 128;
+constexpr int kJacobiLogSweeps = 12;   // sweeps the rotation log holds (a block of 106 columns converges in 7 to 9)
 __host__ __device__ inline long long wide_v_stride() { return (long long)kProxMaxN * (kProxMaxN + 1); }
 int wide_jacobi_ctas();   // CTAs of the wide Jacobi kernel on the current device
+// Rotation log of the split path's Jacobi kernel (64 < n <= 128), in floats per CTA; it runs at most
+// kJacobiPerSm wide_jacobi_ctas() CTAs.
+constexpr int kJacobiPerSm = 4;
+__host__ __device__ inline long long jacobi_log_stride(int n) {
+  const int n2 = (n + 1) & ~1;
+  return 3ll * kJacobiLogSweeps * (n2 - 1) * (n2 / 2);
+}
 
 // Kept eigenvectors per block that the warp eigen kernel hands to the apply kernel.
 constexpr int kFacCols = 8;
@@ -94,7 +104,8 @@ int launch_fft_rows(int mode, float2* u, const float2* coef, const float2* S, in
                     double* partials, int* np, cudaStream_t s);
 int launch_diff_norm(const float2* a, const float2* b, long long n, double* part_d, double* part_b, int nblocks,
                      cudaStream_t s);
-int launch_llr_eig_warp(const ProxOp& op, long long nblocks, cudaStream_t stream);
+int launch_llr_eig_warp(const ProxOp& op, long long nblocks, cudaStream_t stream);   // n <= 64
+int launch_llr_eig_jacobi(const ProxOp& op, long long nblocks, cudaStream_t stream);   // 64 < n <= 128
 
 int launch_llr_prox(const BlockSource& src, const ProxOp& op, cudaStream_t stream);
 bool llr_prox_supported(int m, int n);
@@ -198,8 +209,10 @@ struct llr_ctx {
   int* d_blk_ra;            // per-block kept count of the split prox path + queue counter
   int* d_err;               // device error flag of the prox kernels
   int ph_uniform;           // all volumes share the image-domain phase tables
+  float* d_rot_log;         // rotation log of the split path for 64 < nq <= 128
   float2* d_vwide;          // eigenvector scratch of the wide (64 < nq <= 128) Jacobi kernel
   int vwide_ctas;
+  int rot_ctas;
   std::vector<int> phase_off;   // overlapping blocks: 3 offsets per phase (empty: non-overlapping)
   float2* d_wavelet_work;
   size_t wavelet_work_elems;

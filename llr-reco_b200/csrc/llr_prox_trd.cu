@@ -918,7 +918,8 @@ __global__ void __launch_bounds__(kApplyThreads, 3) llr_apply_kernel(BlockSource
   const int m = op.m, n = op.n, tid = threadIdx.x;
   const long long qstride = src.kind == 1 ? src.g.V : (long long)m;
   // soft threshold: gains from ||C v||^2 (FP64 sum) when the block's rows fit two per thread
-  const bool refine = op.mode != LLR_PROX_HARD_RANK && m <= 2 * (int)blockDim.x;
+  // (64 < n: the Jacobi kernel's own gains, as the wide kernel applies them)
+  const bool refine = op.mode != LLR_PROX_HARD_RANK && m <= 2 * (int)blockDim.x && n <= 64;
   if (tid == 0) block_shift(src, sh_s);
   __syncthreads();
   const int sh[3] = {sh_s[0], sh_s[1], sh_s[2]};
@@ -952,7 +953,7 @@ __global__ void __launch_bounds__(kApplyThreads, 3) llr_apply_kernel(BlockSource
       if (tid < kFacCols) g[tid] = F[n * kFacCols + tid].x;
     }
     __syncthreads();
-    if (ra > 0 && !refine && op.blk_nuc && op.mode != LLR_PROX_HARD_RANK && tid == 0) {
+    if (ra > 0 && !refine && n <= 64 && op.blk_nuc && op.mode != LLR_PROX_HARD_RANK && tid == 0) {
       // unrefined gains g = 1 - lambda / s: s - lambda = lambda g / (1 - g)
       double t = 0.0;
       for (int a = 0; a < ra; ++a)
@@ -1215,13 +1216,28 @@ bool llr_prox_supported(int m, int n) {
 int launch_llr_prox(const BlockSource& src, const ProxOp& op, cudaStream_t stream) {
   if (op.n < 1 || op.m < 1) return set_error(LLR_ERR_INVALID, "empty Casorati matrix %dx%d", op.m, op.n);
   if (src.nblocks == 0) return LLR_OK;
-  if (op.n > 64) {   // wide matrices (64 < n <= 128): the wide Jacobi kernel over every block
+  if (op.n > 64) {   // wide matrices (64 < n <= 128)
     if (op.n > kProxMaxN)
       return set_error(LLR_ERR_UNSUPPORTED, "Casorati column count %d > %d is not supported", op.n, kProxMaxN);
     if (!op.vwide)
       return set_error(LLR_ERR_UNSUPPORTED, "Casorati column count %d > 64 needs the wide-kernel scratch of a "
                                             "context or of an allocating entry point", op.n);
-    return launch_prox_wide(src, op, stream);
+    // Tensor-core Gram, Jacobi eigen kernel and apply, then the wide Jacobi kernel over the blocks handed back.  It
+    // takes every block for the block statistics, the Jacobi solver, the FP32 Gram and callers without scratch.
+    const bool split = op.gram && op.blk_ra && op.rot_log && op.fb_list && !op.block_stat && op.eig_solver == 0 &&
+                       op.gram_mode == 0 && llr_gram_tc_supported(op.m, op.n);
+    if (!split) {
+      if (op.fb_count && !op.block_stat) LLR_CUDA_TRY(cudaMemsetAsync(op.fb_count, 0, sizeof(int), stream));
+      return launch_prox_wide(src, op, stream);
+    }
+    LLR_CUDA_TRY(cudaMemsetAsync(op.fb_count, 0, sizeof(int), stream));
+    LLR_TRY(launch_llr_gram_tc(src, op, stream));
+    LLR_TRY(launch_llr_eig_jacobi(op, src.nblocks, stream));
+    LLR_TRY(launch_apply(src, op, stream));
+    BlockSource fb = src;
+    fb.blk_list = op.fb_list;
+    fb.blk_count = op.fb_count;
+    return launch_prox_wide(fb, op, stream);
   }
   if (op.eig_solver == 1) return launch_llr_prox_jacobi(src, op, stream);   // every block by Jacobi
   if (op.block_stat) {   // largest Gram eigenvalue per block (sigma_max): fused kernel, chunked Gram, any m

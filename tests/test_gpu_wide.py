@@ -1,0 +1,47 @@
+"""Casorati matrices of 65 to 128 columns: the split path (tensor-core Gram, Jacobi eigen kernel with a rotation
+log, apply kernel, wide kernel over the blocks handed back) against the FP64 oracle."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import crandn, rel_err
+from oracle import llr_oracle as O
+
+from llr_b200 import DeviceBuffer, _lib as L
+
+pytestmark = pytest.mark.gpu
+
+
+def _low_rank_mats(rng, m, n, k, batch, noise):
+    """k components between 1 and 0.3 over noise, the last matrix noise alone."""
+    out = noise * crandn(rng, (m, n, batch), np.complex128)
+    for b in range(batch - 1):
+        u = np.linalg.qr(crandn(rng, (m, k), np.complex128))[0]
+        v = np.linalg.qr(crandn(rng, (n, k), np.complex128))[0]
+        out[:, :, b] += (u * np.linspace(1.0, 0.3, k)) @ v.conj().T
+    return np.asfortranarray(out.astype(np.complex64))
+
+
+@pytest.mark.parametrize("m,n,k,batch", [(65, 65, 1, 3), (512, 106, 4, 7), (130, 128, 8, 5), (33, 127, 3, 4),
+                                         (512, 107, 12, 2), (64, 80, 2, 700)])
+@pytest.mark.parametrize("mode", ["soft", "hard"])
+def test_wide_batch_matches_oracle(gpu, m, n, k, batch, mode):
+    """Column counts at both ends and odd, more rows or fewer than columns, kept counts up to and beyond what a
+    block's factor holds (8; 12 takes the wide kernel), blocks that are zero, more blocks than CTAs.  FP32 Gram and
+    rotations: relative 5e-5, the prox tolerance."""
+    rng = np.random.default_rng(m + n)
+    x = _low_rank_mats(rng, m, n, k, batch, 1e-3)
+    d = DeviceBuffer.from_array(x)
+    if mode == "soft":
+        L.check(L.lib.llr_soft_threshold_batch_dev(m, n, 0.1, batch, d.ptr, None))
+        exp = O.low_rank_soft(x.astype(np.complex128), 0.1)
+    else:
+        L.check(L.lib.llr_low_rank_batch_dev(m, n, k, batch, d.ptr, None))
+        exp = O.low_rank_hard(x.astype(np.complex128), k)
+    got = d.download(np.empty_like(x, order="F"))
+    d.close()
+    cut = batch - 1 if mode == "hard" else batch      # the noise matrix has no gap for a rank cut
+    assert rel_err(got[..., :cut], exp[..., :cut]) < 5e-5
+    if mode == "soft":
+        assert not got[..., -1].any()
