@@ -2,7 +2,7 @@
 // layers, out = in + net(in)) with hand-written forward, backward-data and backward-weight
 // kernels, mean-squared-error loss and Adam.  BF16 weights feed the convolutions with FP32
 // accumulation on the tensor cores: forward and backward-data as tcgen05 kind::f16 MMAs with
-// the activations split into three BF16 planes, the weight gradient as 3xTF32 MMAs; the
+// the activations split into three BF16 planes, the weight gradient with both factors split; the
 // optimizer keeps FP32 master weights.
 //
 // Activations are channels-last FP32, voxel v = x + nx (y + ny z) (the reference image order,
@@ -71,12 +71,6 @@ __host__ __device__ __forceinline__ uint16_t f32_to_bf16(float f) {
 // ---------------------------------------------------------------------------------------
 // Geometry shared by the tensor-core conv kernels.
 // ---------------------------------------------------------------------------------------
-constexpr int kCvThreads = 256;
-constexpr int kCvTX = 8, kCvTY = 4, kCvTZ = 4;                  // weight-gradient tile: 128 voxels
-constexpr int kCvHX = kCvTX + 2, kCvHY = kCvTY + 2, kCvHZ = kCvTZ + 2;
-constexpr int kCvHV = kCvHX * kCvHY * kCvHZ;
-constexpr int kCvPlane = 128 * 128;                              // one 128 x 32 TF32 operand plane (bytes)
-
 __host__ __device__ constexpr int cv_np(int cout) { return cout <= 16 ? 16 : 32; }
 
 // ---------------------------------------------------------------------------------------
@@ -378,161 +372,206 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
 }
 
 // ---------------------------------------------------------------------------------------
-// Weight gradient on the tensor cores: D[(tap, ci)][co] = sum_v x[v + d(tap)][ci] dy[v][co]
-// as MT = ceil(27 CIN / 128) GEMMs of M = 128 rows (tap, ci), N = COUT (padded to 16 / 32),
-// K = voxels, accumulated in tensor memory over every tile the CTA visits (MT x N columns).
-// Per 128-voxel tile the input halo and the tile's dy are staged once; dy goes to TF32 hi / lo
-// B planes (N rows x 32 voxels per K chunk), and for each (K chunk, M tile) the tap-shifted
-// input rows are written as hi / lo A planes (double-buffered) and multiplied with 3xTF32
-// (hi hi + hi lo + lo hi).  At the end each CTA writes its partial sums (and the bias
-// gradient, summed in FP32 from the staged dy); a fixed-order reduction adds the CTAs.
+// Weight gradient on the tensor cores: dW[tap][ci][co] = sum_v x[v + d(tap)][ci] dy[v][co], a GEMM whose K
+// dimension is the voxels, tcgen05 kind::f16 with both operands MN-major: in shared memory 16 bytes are eight
+// channels of one voxel, eight voxels along x are 128 contiguous bytes, which is the forward kernel's halo
+// layout read the other way round.
+//
+// A CTA owns tiles of 128 voxels, 8 (x) x 16 (y) x 1 (z).  A = the input halo: its three z slices are stored
+// one behind the other in 8-channel chunks of equal stride, so the 128 rows of one MMA are the taps dz = 0..2
+// of all input channels (rows past them are not used), and the tap (dx, dy) is a start-address offset of
+// dx + 10 dy voxels: nine accumulators of COUT columns, one per (dx, dy), stay in tensor memory over
+// every tile of the CTA.  B = the tile's dy.  No operand is copied per tap.
+// FP32 accuracy: x and dy are split into three BF16 planes each (about 24 significant bits), and the six
+// products of order down to 2^-16 are summed: b1 b1, b1 b2, b2 b1, b2 b2, b1 b3, b3 b1 (two more change
+// nothing).  What is left is the truncation of the FP32 sums in tensor memory, which grows with the
+// number of tiles per CTA; see the launch.
+// Bound: shared-memory reads of the A operand (4 KB per 128 x 32 x 16 MMA, 432 MMAs per tile).  The same GEMM in
+// 3xTF32 with a K-major copy of the operand per tap and 32 voxels (TF32 operands cannot be MN-major in
+// this layout) spent its time on those copies: 3.95 ms per 32 -> 32 layer at 96^3, now 1.2 ms.
+//
+// Warps 0-7 convert, load the next tile's FP32 data with cp.async while the MMAs run, and sum the bias
+// gradient; warp 8 issues the MMAs.  At the end each CTA writes its partial sums; a fixed-order reduction
+// adds the CTAs (deterministic).
 // ---------------------------------------------------------------------------------------
+constexpr int kWgSV = kFwHX * kFwHY;                               // voxels of one halo slice
+
 template <int CIN, int COUT>
 struct WgLayout {
   static constexpr int NP = cv_np(COUT);
-  static constexpr int HP = CIN | 1;
-  static constexpr int MT = (27 * CIN + 127) / 128;
-  static constexpr int TCOLS = MT * NP <= 32 ? 32 : MT * NP <= 64 ? 64 : MT * NP <= 128 ? 128 : 256;
+  static constexpr int KC = (CIN + 15) / 16 * 2;                   // 8-channel chunks per slice
+  static constexpr int RC = 2 * KC;                                // 4-channel chunks of the FP32 halo
+  static constexpr int NC = NP / 8;                                // 8-channel chunks of dy
+  static constexpr int SROWS = 8 * KC;                             // accumulator rows per slice
+  static constexpr uint32_t TCOLS = 9 * NP <= 256 ? 256 : 512;
+  static constexpr size_t PA = (size_t)3 * KC * kWgSV * 16;        // bytes of one BF16 plane of x
+  static constexpr size_t PB = (size_t)NC * 128 * 16;              // bytes of one BF16 plane of dy
   static constexpr size_t off_hdr = 0;
-  static constexpr size_t off_b = 1024;                              // 4 K chunks x (hi, lo) x NP x 128 B
-  static constexpr size_t off_a = off_b + (size_t)8 * NP * 128;       // 2 buffers x (hi, lo)
-  static constexpr size_t off_halo = off_a + (size_t)4 * kCvPlane;
-  static constexpr size_t off_dy = off_halo + sizeof(float) * (size_t)kCvHV * HP;
+  static constexpr size_t off_a = 1024;
+  static constexpr size_t off_b = off_a + 3 * PA;
+  static constexpr size_t off_raw = off_b + 3 * PB;                // FP32 halo, chunk r at r NV 16
+  static constexpr size_t off_dy = off_raw + (size_t)RC * kFwNV * 16;   // FP32 dy [128][COUT]
   static constexpr size_t total = off_dy + sizeof(float) * 128 * COUT;
+  // the unused rows of the last plane's A operand (16 chunks) read past the planes, inside the buffer
+  static_assert(off_a + 2 * PA + (size_t)16 * kWgSV * 16 <= total, "A operand rows");
+  static_assert(3 * SROWS <= 128, "three slices of channels fill the M dimension");
 };
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kCvThreads, 1) conv3d_wgrad_tc_kernel(const float* __restrict__ x,
+__global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const float* __restrict__ x,
                                                                         const float* __restrict__ dy,
                                                                         float* __restrict__ part, CvGeo G, int* err) {
   using Lay = WgLayout<CIN, COUT>;
-  constexpr int NP = Lay::NP, HP = Lay::HP, MT = Lay::MT, ROWS = 27 * CIN;
-  constexpr uint32_t idesc = umma_idesc_tf32(128, NP);
+  constexpr int NP = Lay::NP, KC = Lay::KC, RC = Lay::RC, NC = Lay::NC, ROWS = 27 * CIN;
+  constexpr uint32_t idesc = umma_idesc_bf16(128, NP) | (1u << 15) | (1u << 16);   // A and B MN-major
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned long long* mbar = reinterpret_cast<unsigned long long*>(smem + Lay::off_hdr);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Lay::off_hdr + 32);
-  unsigned char* bsm = smem + Lay::off_b;
-  unsigned char* asm_ = smem + Lay::off_a;
-  float* halo = reinterpret_cast<float*>(smem + Lay::off_halo);
-  float* sdy = reinterpret_cast<float*>(smem + Lay::off_dy);
+  unsigned long long* mb = reinterpret_cast<unsigned long long*>(smem + Lay::off_hdr);
+  unsigned long long* conv_full = mb;        // workers -> MMA warp: the tile's planes are written
+  unsigned long long* mma_done = mb + 1;     // MMA warp -> workers: the tile's planes are read
+  unsigned long long* drain = mb + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Lay::off_hdr + 128);
+  unsigned char* apl = smem + Lay::off_a;
+  unsigned char* bpl = smem + Lay::off_b;
+  unsigned char* raw = smem + Lay::off_raw;
+  float* rdy = reinterpret_cast<float*>(smem + Lay::off_dy);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"((uint32_t)Lay::TCOLS));
+                 "r"(Lay::TCOLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    for (int b = 0; b < 3; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[b])));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(conv_full)), "r"((uint32_t)kFwWorkers));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mma_done)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(drain)));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
-  for (int i = tid; i < (int)((Lay::off_halo - Lay::off_b) / 16); i += kCvThreads)
-    reinterpret_cast<float4*>(bsm)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
-  uint32_t phase[3] = {0u, 0u, 0u};
-  bool used[2] = {false, false};
-  bool failed = false, first = true;
-  int gpar = 0;
+  const long long n = (long long)blockIdx.x < G.ntiles ? (G.ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+  bool failed = false;
   float dbacc = 0.f;
-  for (long long tile = blockIdx.x; tile < G.ntiles && !failed; tile += gridDim.x) {
-    const int ox = (int)(tile % G.tx) * kCvTX;
-    const long long rt = tile / G.tx;
-    const int oy = (int)(rt % G.ty) * kCvTY, oz = (int)(rt / G.ty) * kCvTZ;
-    for (int i = tid; i < kCvHV * CIN; i += kCvThreads) {
-      const int hv = i / CIN, c = i - hv * CIN;
-      const int hx = hv % kCvHX, hy = (hv / kCvHX) % kCvHY, hz = hv / (kCvHX * kCvHY);
-      const int gx = ox + hx - 1, gy = oy + hy - 1, gz = oz + hz - 1;
-      float v = 0.f;
-      if (gx >= 0 && gx < G.nx && gy >= 0 && gy < G.ny && gz >= 0 && gz < G.nz)
-        v = x[((long long)gx + (long long)G.nx * (gy + (long long)G.ny * gz)) * CIN + c];
-      halo[hv * HP + c] = v;
-    }
-    for (int i = tid; i < 128 * COUT; i += kCvThreads) {   // dy of the tile's voxels -> B planes (row co, column voxel)
-      const int a = i / COUT, c = i - a * COUT;
-      const int gx = ox + (a & 7), gy = oy + ((a >> 3) & 3), gz = oz + (a >> 5);
-      float v = 0.f;
-      if (gx < G.nx && gy < G.ny && gz < G.nz) v = dy[((long long)gx + (long long)G.nx * (gy + (long long)G.ny * gz)) * COUT + c];
-      sdy[i] = v;
-      const int kc = a >> 5, kv = a & 31;
-      unsigned char* bh = bsm + (size_t)kc * 2 * NP * 128;
-      const uint32_t h = tf32_rna(v);
-      const int o = op_offset(c, kv);
-      *reinterpret_cast<uint32_t*>(bh + o) = h;
-      *reinterpret_cast<float*>(bh + NP * 128 + o) = v - __uint_as_float(h);
-    }
-    __syncthreads();
-    if (tid < COUT)
-      for (int a = 0; a < 128; ++a) dbacc += sdy[a * COUT + tid];
-    for (int kc = 0; kc < 4 && !failed; ++kc) {
-      for (int mt = 0; mt < MT; ++mt) {
-        const int b = gpar;
-        if (used[b]) {
-          const bool ok = mbar_wait(smem_u32(&mbar[b]), phase[b]);
-          phase[b] ^= 1u;
-          if (__syncthreads_or(!ok)) { failed = true; break; }
-        }
-        unsigned char* hi = asm_ + (size_t)b * 2 * kCvPlane;
-        unsigned char* lo = hi + kCvPlane;
-        for (int e = tid; e < 128 * 32; e += kCvThreads) {   // row r = (tap, ci), column kv = voxel 32 kc + kv
-          const int rl = e >> 5, kv = e & 31;
-          const int r = mt * 128 + rl;
-          float v = 0.f;
-          if (r < ROWS) {
-            const int tap = r / CIN, ci = r - tap * CIN;
-            const int dx = tap % 3, dyy = (tap / 3) % 3, dz = tap / 9;
-            const int a = 32 * kc + kv;
-            const int lx = a & 7, ly = (a >> 3) & 3, lz = a >> 5;
-            v = halo[((lx + dx) + kCvHX * ((ly + dyy) + kCvHY * (lz + dz))) * HP + ci];
-          }
-          const uint32_t h = tf32_rna(v);
-          const int o = op_offset(rl, kv);
-          *reinterpret_cast<uint32_t*>(hi + o) = h;
-          *reinterpret_cast<float*>(lo + o) = v - __uint_as_float(h);
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t ah = smem_u32(hi), al = smem_u32(lo);
-          const uint32_t bh = smem_u32(bsm + (size_t)kc * 2 * NP * 128), bl = bh + NP * 128;
-          const uint32_t d = tmem + (uint32_t)(mt * NP);
-#pragma unroll
-          for (int st = 0; st < 4; ++st) {
-            const uint64_t dah = umma_desc_sw128(ah + st * 32), dal = umma_desc_sw128(al + st * 32);
-            const uint64_t dbh = umma_desc_sw128(bh + st * 32), dbl = umma_desc_sw128(bl + st * 32);
-            umma_tf32(d, dah, dbh, idesc, (first && kc == 0 && st == 0) ? 0u : 1u);
-            umma_tf32(d, dah, dbl, idesc, 1u);
-            umma_tf32(d, dal, dbh, idesc, 1u);
-          }
-          umma_commit(smem_u32(&mbar[b]));
-          if (kc == 3 && mt == MT - 1) umma_commit(smem_u32(&mbar[2]));
-        }
-        used[b] = true;
-        gpar ^= 1;
+
+  if (warp < 8) {
+    constexpr int VW = CIN % 4 == 0 ? 4 : 1, PER = 4 * RC / VW;
+    constexpr int DW = COUT % 4 == 0 ? 4 : 1;
+    auto load_raw = [&](long long t) {
+      const int ox = (int)(t % G.tx) * kFwTX;
+      const long long rt = t / G.tx;
+      const int oy = (int)(rt % G.ty) * kFwTY, oz = (int)(rt / G.ty);
+      for (int i = tid; i < kFwNV * PER; i += kFwWorkers) {
+        const int h = i / PER, c = (i - h * PER) * VW;
+        const int hx = h % kFwHX, hy = (h / kFwHX) % kFwHY, hz = h / (kFwHX * kFwHY);
+        const int gx = ox + hx - 1, gy = oy + hy - 1, gz = oz + hz - 1;
+        const bool in = c < CIN && gx >= 0 && gx < G.nx && gy >= 0 && gy < G.ny && gz >= 0 && gz < G.nz;
+        const float* src = in ? x + ((long long)gx + (long long)G.nx * (gy + (long long)G.ny * gz)) * CIN + c : x;
+        const uint32_t dst = smem_u32(raw + ((size_t)(c >> 2) * kFwNV + h) * 16 + (c & 3) * 4);
+        if constexpr (VW == 4)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+        else
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
       }
+      for (int i = tid; i < 128 * COUT / DW; i += kFwWorkers) {
+        const int a = i / (COUT / DW), c = (i - a * (COUT / DW)) * DW;
+        const int gx = ox + (a & 7), gy = oy + (a >> 3);
+        const bool in = gx < G.nx && gy < G.ny;
+        const float* src = in ? dy + ((long long)gx + (long long)G.nx * (gy + (long long)G.ny * oz)) * COUT + c : dy;
+        const uint32_t dst = smem_u32(rdy + a * COUT + c);
+        if constexpr (DW == 4)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+        else
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto put = [&](unsigned char* o, size_t plane, const float* v) {   // eight values -> three planes
+      uint4 q1, q2, q3;
+      split3_bf16(v[0], v[1], q1.x, q2.x, q3.x);
+      split3_bf16(v[2], v[3], q1.y, q2.y, q3.y);
+      split3_bf16(v[4], v[5], q1.z, q2.z, q3.z);
+      split3_bf16(v[6], v[7], q1.w, q2.w, q3.w);
+      *reinterpret_cast<uint4*>(o) = q1;
+      *reinterpret_cast<uint4*>(o + plane) = q2;
+      *reinterpret_cast<uint4*>(o + 2 * plane) = q3;
+    };
+    auto convert = [&]() {
+      for (int i = tid; i < KC * kFwNV; i += kFwWorkers) {   // chunk c of halo voxel h = slice hz, voxel hs
+        const int c = i / kFwNV, h = i - c * kFwNV, hz = h / kWgSV, hs = h - hz * kWgSV;
+        const float4 v0 = *reinterpret_cast<const float4*>(raw + ((size_t)(2 * c) * kFwNV + h) * 16);
+        const float4 v1 = *reinterpret_cast<const float4*>(raw + ((size_t)(2 * c + 1) * kFwNV + h) * 16);
+        const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        put(apl + ((size_t)(hz * KC + c) * kWgSV + hs) * 16, Lay::PA, v);
+      }
+      for (int i = tid; i < NC * 128; i += kFwWorkers) {
+        const int c = i >> 7, a = i & 127;
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = 8 * c + k < COUT ? rdy[a * COUT + 8 * c + k] : 0.f;
+        put(bpl + ((size_t)c * 128 + a) * 16, Lay::PB, v);
+      }
+    };
+    if (n > 0) load_raw(blockIdx.x);
+    for (long long i = 0; i < n; ++i) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (lane < COUT)
+#pragma unroll 4
+        for (int a = 16 * warp; a < 16 * warp + 16; ++a) dbacc += rdy[a * COUT + lane];
+      if (i > 0) {   // the MMAs of tile i - 1 no longer read the planes
+        const bool ok = mbar_wait(smem_u32(mma_done), (uint32_t)((i - 1) & 1));
+        if (workers_any(!ok)) { failed = true; break; }
+      }
+      convert();
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mbar_arrive(smem_u32(conv_full));
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // every worker is done with the staging buffers
+      if (i + 1 < n) load_raw((long long)blockIdx.x + (i + 1) * gridDim.x);
     }
-    if (failed) break;
-    first = false;
-    {   // the next tile overwrites the B planes and the halo: this tile's MMAs must be done
-      const bool ok = mbar_wait(smem_u32(&mbar[2]), phase[2]);
-      phase[2] ^= 1u;
-      for (int bb = 0; bb < 2; ++bb)
-        if (used[bb]) {
-          mbar_wait(smem_u32(&mbar[bb]), phase[bb]);
-          phase[bb] ^= 1u;
-          used[bb] = false;
-        }
-      if (__syncthreads_or(!ok)) { failed = true; break; }
+    if (!failed && n > 0) {
+      const bool ok = mbar_wait(smem_u32(mma_done), (uint32_t)((n - 1) & 1));
+      if (workers_any(!ok)) failed = true;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (lane == 0) {
+    // MN-major without swizzle: LBO = step between groups of 8 voxels (K), SBO = step between 8-channel chunks
+    const uint64_t a0 = umma_desc_kmajor(smem_u32(apl), kFwHX * 16, kWgSV * 16);
+    const uint64_t b0 = umma_desc_kmajor(smem_u32(bpl), 128, 128 * 16);
+    constexpr int PX[6] = {0, 0, 1, 1, 0, 2}, PY[6] = {0, 1, 0, 1, 2, 0};   // planes of x and dy
+    for (long long i = 0; i < n; ++i) {
+      if (!mbar_wait(smem_u32(conv_full), (uint32_t)(i & 1))) { failed = true; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+      for (int ks = 0; ks < 8; ++ks) {           // rows y = 2 ks, 2 ks + 1 of the tile
+        const uint64_t bs = b0 + (uint64_t)(16 * ks);
+#pragma unroll 1
+        for (int dyt = 0; dyt < 3; ++dyt)
+#pragma unroll
+          for (int dx = 0; dx < 3; ++dx) {
+            const uint64_t as = a0 + (uint64_t)(kFwHX * (2 * ks + dyt) + dx);
+            const uint32_t d = tmem + (uint32_t)((3 * dyt + dx) * NP);
+#pragma unroll
+            for (int p = 0; p < 6; ++p)
+              umma_bf16(d, as + (uint64_t)((PX[p] * Lay::PA) >> 4), bs + (uint64_t)((PY[p] * Lay::PB) >> 4), idesc,
+                        (i > 0 || ks > 0 || p > 0) ? 1u : 0u);
+          }
+      }
+      umma_commit(smem_u32(mma_done));
     }
   }
+  // bias gradient: the warps' sums in a fixed order (the staging buffer is free)
+  __syncthreads();
+  if (warp < 8 && lane < COUT) rdy[warp * COUT + lane] = dbacc;
+  const bool any_failed = __syncthreads_or(failed);
   float* P = part + (long long)blockIdx.x * (ROWS * COUT + COUT);
-  if (!failed) {
+  if (!any_failed && n > 0) {
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (warp < 4) {
-      for (int mt = 0; mt < MT; ++mt) {
+      const int row = 32 * warp + lane, dz = row / Lay::SROWS, ci = row - dz * Lay::SROWS;
+      for (int g = 0; g < 9; ++g) {
         uint32_t r[NP];
-        const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(mt * NP);
+        const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(g * NP);
         if constexpr (NP == 32) {
           asm volatile(
               "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -552,22 +591,26 @@ __global__ void __launch_bounds__(kCvThreads, 1) conv3d_wgrad_tc_kernel(const fl
               : "r"(taddr));
         }
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const int row = mt * 128 + 32 * warp + lane;
-        if (row < ROWS) {
+        if (dz < 3 && ci < CIN) {
 #pragma unroll
-          for (int c = 0; c < COUT; ++c) P[(long long)row * COUT + c] = first ? 0.f : __uint_as_float(r[c]);
+          for (int c = 0; c < COUT; ++c) P[((long long)(g + 9 * dz) * CIN + ci) * COUT + c] = __uint_as_float(r[c]);
         }
       }
     }
-    if (tid < COUT) P[ROWS * COUT + tid] = dbacc;
+    if (tid < COUT) {
+      float s = 0.f;
+      for (int w = 0; w < 8; ++w) s += rdy[w * COUT + tid];
+      P[ROWS * COUT + tid] = s;
+    }
   }
-  if (failed && tid == 0 && err) atomicExch(err, 1);
-  if (tid == 0) umma_commit(smem_u32(&mbar[2]));
-  mbar_wait(smem_u32(&mbar[2]), phase[2]);
+  if (failed && err) atomicExch(err, 1);
+  // nothing may still write an accumulator when tensor memory is released
+  if (warp == 8 && lane == 0) umma_commit(smem_u32(drain));
+  mbar_wait(smem_u32(drain), 0u);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)Lay::TCOLS));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Lay::TCOLS));
 }
 
 // out[i] = sum over `nb` partial blocks (fixed order), i < n
@@ -745,6 +788,9 @@ int wgrad_inst(const float* x, const float* dy, float* part, long long part_cap,
                cudaStream_t s) {
   const size_t smem = WgLayout<CIN, COUT>::total;
   static_assert(WgLayout<CIN, COUT>::total <= 227 * 1024, "wgrad operands exceed shared memory");
+  if ((CIN % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) != 0) ||
+      (COUT % 4 == 0 && (reinterpret_cast<uintptr_t>(dy) & 15) != 0))
+    return set_error(LLR_ERR_INVALID, "conv3d weight gradient needs 16-byte aligned activations");
   auto k = conv3d_wgrad_tc_kernel<CIN, COUT>;
   LLR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int dev = 0, nsm = 0;
@@ -752,13 +798,18 @@ int wgrad_inst(const float* x, const float* dy, float* part, long long part_cap,
   LLR_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   CvGeo G;
   G.nx = dims[0]; G.ny = dims[1]; G.nz = dims[2];
-  G.tx = (G.nx + kCvTX - 1) / kCvTX;
-  G.ty = (G.ny + kCvTY - 1) / kCvTY;
-  G.ntiles = (long long)G.tx * G.ty * ((G.nz + kCvTZ - 1) / kCvTZ);
+  G.tx = (G.nx + kFwTX - 1) / kFwTX;
+  G.ty = (G.ny + kFwTY - 1) / kFwTY;
+  G.ntiles = (long long)G.tx * G.ty * G.nz;
   const long long per = 27LL * CIN * COUT + COUT;
-  const int grid = (int)std::max<long long>(1, std::min<long long>(std::min<long long>(G.ntiles, nsm), part_cap / per));
+  // The tensor core truncates its running sums: each gradient comes out a few 1e-5 short, in proportion to
+  // the tiles a CTA adds up.  104 CTAs keep the gradients of 1.2 M voxels within 2e-5 of those of the 3xTF32
+  // kernel, which truncated more often (finer K steps): 96^3 differs by 1.3e-5, by 2.0e-5 with one CTA per SM
+  // (2.8 ms of a 12.9 ms gradient faster).
+  const int grid = (int)std::max<long long>(
+      1, std::min<long long>(std::min<long long>(G.ntiles, std::min(nsm, 104)), part_cap / per));
   note_launch();
-  k<<<grid, kCvThreads, smem, s>>>(x, dy, part, G, err);
+  k<<<grid, kFwThreads, smem, s>>>(x, dy, part, G, err);
   LLR_CUDA_TRY(cudaGetLastError());
   note_launch();
   reduce_partials_kernel<<<grid_1d(per), 256, 0, s>>>(part, grid, per, out);
