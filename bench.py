@@ -342,7 +342,7 @@ def run_b200(args, dist: Dist) -> None:
     value = dist.world * args.steps / (t_max / 1e3)
 
     # roofline of the dominant stage: the LLR proximal step (llr_gram_tc_kernel: gather + 3xTF32
-    # tcgen05 Gram; llr_eig_team_kernel: eigen decomposition; llr_apply_kernel: apply + scatter).
+    # tcgen05 Gram; llr_eig_warp_kernel: eigen decomposition; llr_apply_kernel: apply + scatter).
     # Algorithmic bytes = the operator's minimum, one read and one write of every complex64
     # element of the iterate (16 B per voxel-volume element).
     names = ["llr_prox", "wavelet", "fft_fwd", "dc", "fft_inv"]
@@ -353,7 +353,7 @@ def run_b200(args, dist: Dist) -> None:
     prof = profiled_traffic("llr_prox", args.config)
     it_bytes = 16.0 * E * 3 + 24.0 * E / c["accel"]
     prox_label = ("LLR prox stage: llr_subspace_kernel (X <- LR(X S) S^H)" if "srank" in c else
-                  "LLR prox stage: llr_gram_tc_kernel + llr_eig_team_kernel + llr_apply_kernel")
+                  "LLR prox stage: llr_gram_tc_kernel + llr_eig_warp_kernel + llr_apply_kernel")
     roofline = {"bound": "hbm", "kernel": prox_label,
                 "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "peak_source": peaks["source"],
                 "unit": "GB/s", "frac": round(achieved / peaks["hbm_gbs"], 4),
@@ -531,7 +531,7 @@ def main(argv=None):
                     help="write profiles/<--traffic-name>_<--config>.json from `ncu -i REP --page raw --csv` output "
                          "and exit")
     ap.add_argument("--traffic-name", default="llr_prox")
-    ap.add_argument("--traffic-kernels", default="llr_gram_tc|llr_eig|llr_apply")
+    ap.add_argument("--traffic-kernels", default="llr_gram_tc|llr_eig_warp|llr_apply")
     ap.add_argument("--traffic-scale", type=float, default=1.0)
     ap.add_argument("--traffic-captured-on", default=None)
     ap.add_argument("--cnn-timing", action="store_true", help="time the warm-start network and exit")

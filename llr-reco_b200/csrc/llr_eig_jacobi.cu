@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(kJacThreads, 4) llr_eig_jacobi_kernel(ProxOp o
   const int n = op.n, n2 = (n + 1) & ~1, half = n2 >> 1, M = n2 - 1;
   auto row = [&](int i) { return (i * (2 * n2 - 1 - i)) >> 1; };
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int P = n * (n + 1) / 2;
   const bool soft = op.mode != LLR_PROX_HARD_RANK;
   const float thr = op.lambda * op.lambda;
   float* log = op.rot_log + (long long)blockIdx.x * jacobi_log_stride(n);   // (t, e) per pair and step

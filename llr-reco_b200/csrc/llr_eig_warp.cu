@@ -1,4 +1,4 @@
-// Eigen stage of the split LLR prox path for n <= 48 columns, one warp per Casorati block (llr_eig_team.cu: wider).
+// Eigen stage of the split LLR prox path, one warp per Casorati block.
 //
 // Input: the packed lower Gram matrix G = C^H C of every block (written by the Gram kernel).
 // Output, in place of G: the block's kept eigenvectors V_a (n x r_a, q-major, r_a <= kFacCols)
@@ -22,12 +22,6 @@
 // Blocks keeping more than kFacCols components, or whose eigenvectors fail the residual
 // check, get r_a = -1 and go to the Jacobi kernel; hard rank >= n leaves the block as is
 // (r_a = -2).
-//
-// Bound: latency of the Householder steps (a chain of n of them, each with two reductions) and their shared-memory
-// reads.  Complex multiply-adds are two packed FMAs on vector entries stored twice per component: no
-// component shuffles, half of the FMA issue slots (blocks of 33 columns: 172 -> 140 us; 16 columns: 56.3 -> 52.3).
-// Above 48 columns one warp's shared memory per block leaves too few warps per SM; two share a block there
-// (61 columns: 719 us here, 627 there).
 #include <cstdio>
 #include <algorithm>
 
@@ -48,7 +42,8 @@ struct WarpEig {
   float2 A[NPMAX * (NPMAX + 1) / 2];   // packed lower triangle; later Householder vectors
   union {
     struct {
-      float4 ud[NPMAX];                // (u.x, u.x, u.y, u.y): Householder vector / Cholesky column
+      float2 u[NPMAX];                 // Householder vector / Cholesky column
+      float2 w[NPMAX];                 // p - K u
       float2 e[NPMAX];                 // complex sub-diagonal of T
       float e2[NPMAX];                 // |e|^2 for the Sturm counts
       float spare[NPMAX];
@@ -60,10 +55,7 @@ struct WarpEig {
   float ae[NPMAX];
   float tau[NPMAX];
   float lam[kFacCols];
-  union {
-    float4 wd[NPMAX];                  // p - K u, stored as ud
-    float Y[kFacCols * NPMAX];         // eigenvectors of T', column a at Y[a * NPMAX]
-  };
+  float Y[kFacCols * NPMAX];           // eigenvectors of T', column a at Y[a * NPMAX]
 };
 
 __device__ __forceinline__ int pk(int i, int j) { return (i * (i + 1)) / 2 + j; }
@@ -77,20 +69,22 @@ __device__ __forceinline__ float wmax(float v) {
   return v;
 }
 
-__device__ __forceinline__ float4 dup2(float2 v) { return make_float4(v.x, v.x, v.y, v.y); }
-__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
-__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
-
-// Rows of the trailing L x L matrix owned by a lane: `lane` and, above 32 columns, 32 + lane.  The steps walk
-// the columns in order, so the vector entries are broadcast reads; they are kept twice per component
-// (ud, wd), which makes a complex multiply-add two packed FMAs without shuffling components:
-// a u = a u.x + i (a u.y), with the two sums kept apart and i applied once at the end.
+// Rows of the trailing L x L matrix owned by a lane: i1 = lane and i2 = L - 1 - lane, so
+// that every lane holds L + 1 lower-triangle elements (the middle row of an odd L once).
+struct RowPair {
+  int i1, i2, n1, tot;
+  __device__ __forceinline__ RowPair(int L, int lane) {
+    i1 = lane < (L + 1) / 2 ? lane : -1;
+    i2 = lane < L / 2 ? L - 1 - lane : -1;
+    n1 = i1 + 1;
+    tot = n1 + (i2 >= 0 ? i2 + 1 : 0);
+  }
+};
 
 // True when thr I - G is positive definite, i.e. every eigenvalue of G is below thr:
 // unpivoted Cholesky stopping at the first non-positive pivot.  Overwrites A.
 template <int NPMAX>
 __device__ bool warp_below(WarpEig<NPMAX>* W, int n, float thr) {
-  constexpr int H = NPMAX > 32 ? 2 : 1;
   const int lane = threadIdx.x & 31;
   float2* A = W->A;
   const int P = n * (n + 1) / 2;
@@ -104,36 +98,20 @@ __device__ bool warp_below(WarpEig<NPMAX>* W, int n, float thr) {
     const float s = 1.f / sqrtf(dk);
     const int o = k + 1, L = n - o;
     if (L == 0) break;
-    float2 l[H];
-#pragma unroll
-    for (int h = 0; h < H; ++h) {
-      const int i = min(lane + 32 * h, L - 1);
-      l[h] = cscale(A[pk(o + i, k)], s);
-      if (lane + 32 * h < L) W->ud[lane + 32 * h] = dup2(l[h]);
-    }
+    const RowPair rp(L, lane);
+    float2 l1 = make_float2(0.f, 0.f), l2 = l1;
+    if (rp.i1 >= 0) { l1 = cscale(A[pk(o + rp.i1, k)], s); W->u[rp.i1] = l1; }
+    if (rp.i2 >= 0) { l2 = cscale(A[pk(o + rp.i2, k)], s); W->u[rp.i2] = l2; }
     __syncwarp();
-    // A[i][j] -= l_i conj(l_j): l conj(m) = l m.x + (l.y, -l.x) m.y
-#pragma unroll
-    for (int h = 0; h < H; ++h) {
-      if (32 * h >= L) break;
-      const int row = lane + 32 * h, i = min(row, L - 1);
-      const bool own = row < L;
-      const float2 nl = make_float2(-l[h].x, -l[h].y), nls = make_float2(-l[h].y, l[h].x);
-      float2* a = A + pk(o + i, o);
-#pragma unroll 8
-      for (int j = 0; j < 32 * h; ++j) {
-        const float4 m = W->ud[j];
-        const float2 v = ffma2(nls, hi2(m), ffma2(nl, lo2(m), a[j]));
-        if (own) a[j] = v;
-      }
-      const int je = min(32 * h + 32, L);
-#pragma unroll 4
-      for (int j = 32 * h; j < je; ++j) {
-        const float4 m = W->ud[j];
-        const bool on = own && j <= row;
-        const float2 v = ffma2(nls, hi2(m), ffma2(nl, lo2(m), a[on ? j : 0]));
-        if (on) a[j] = v;
-      }
+    const int rb1 = rp.i1 >= 0 ? pk(o + rp.i1, o) : 0, rb2 = rp.i2 >= 0 ? pk(o + rp.i2, o) : 0;
+    const float2 nl1 = make_float2(-l1.x, -l1.y), nl2 = make_float2(-l2.x, -l2.y);
+    float2 cl = nl1;
+    int jo = 0, ib = rb1;
+    for (int t = 0; t < rp.tot; ++t) {
+      if (t == rp.n1) { cl = nl2; jo = rp.n1; ib = rb2 - rp.n1; }
+      float2 a = A[ib + t];
+      cfma_cb(a, cl, W->u[t - jo]);
+      A[ib + t] = a;
     }
     __syncwarp();
   }
@@ -144,21 +122,16 @@ __device__ bool warp_below(WarpEig<NPMAX>* W, int n, float thr) {
 // column k keeps u_k below the diagonal for the back-transformation.
 template <int NPMAX>
 __device__ void warp_tridiag(WarpEig<NPMAX>* W, int n) {
-  constexpr int H = NPMAX > 32 ? 2 : 1;
   const int lane = threadIdx.x & 31;
   float2* A = W->A;
   const float2 z = make_float2(0.f, 0.f);
   for (int k = 0; k + 2 < n; ++k) {
     const int o = k + 1, L = n - o;
-    float2 x[H];
-    float loc = 0.f;
-#pragma unroll
-    for (int h = 0; h < H; ++h) {
-      x[h] = lane + 32 * h < L ? A[pk(o + lane + 32 * h, k)] : z;
-      loc += cabs2(x[h]);
-    }
-    const float s2 = wsum(loc);
-    const float2 x0 = make_float2(__shfl_sync(0xffffffffu, x[0].x, 0), __shfl_sync(0xffffffffu, x[0].y, 0));
+    const RowPair rp(L, lane);
+    float2 x1 = rp.i1 >= 0 ? A[pk(o + rp.i1, k)] : z;
+    float2 x2 = rp.i2 >= 0 ? A[pk(o + rp.i2, k)] : z;
+    const float s2 = wsum(cabs2(x1) + cabs2(x2));
+    const float2 x0 = make_float2(__shfl_sync(0xffffffffu, x1.x, 0), __shfl_sync(0xffffffffu, x1.y, 0));
     const float xn = sqrtf(s2), aa = sqrtf(cabs2(x0));
     const float phx = aa > 0.f ? x0.x / aa : 1.f, phy = aa > 0.f ? x0.y / aa : 0.f;
     const float2 u0 = make_float2(x0.x + phx * xn, x0.y + phy * xn);
@@ -168,96 +141,76 @@ __device__ void warp_tridiag(WarpEig<NPMAX>* W, int n) {
       W->tau[k] = t;
       W->e[k] = make_float2(-phx * xn, -phy * xn);
       A[pk(o, k)] = u0;
-      x[0] = u0;
     }
+    if (rp.i1 == 0) x1 = u0;
     if (t == 0.f) {   // warp-uniform: no reflection at this step
       __syncwarp();
       continue;
     }
-#pragma unroll
-    for (int h = 0; h < H; ++h)
-      if (lane + 32 * h < L) W->ud[lane + 32 * h] = dup2(x[h]);
+    if (rp.i1 >= 0) W->u[rp.i1] = x1;
+    if (rp.i2 >= 0) W->u[rp.i2] = x2;
     __syncwarp();
-    // p = t A22 u: columns left of the 32 rows of a half from the rows themselves, columns right of them from
-    // the rows below (conjugated), the 32 in between by comparison.  Lanes without a row repeat the
-    // last one and drop the result.
-    float2 p[H];
-    float dploc = 0.f;
+    // p = t A22 u, reading A22[i][j] = conj(A22[j][i]) above the diagonal.  Lanes without a
+    // row read row 0 (a valid element) and drop the result; four columns are in flight at once.
+    const int r1 = max(rp.i1, 0), r2 = max(rp.i2, 0);
+    const int rb1 = pk(o + r1, o), rb2 = pk(o + r2, o);
+    float2 p1 = z, p2 = z, q1 = z, q2 = z;
+    for (int j0 = 0; j0 < L; j0 += 4) {
+      float2 a1[4], a2[4], uj[4];
 #pragma unroll
-    for (int h = 0; h < H; ++h) {
-      p[h] = z;
-      if (32 * h >= L) continue;
-      const int i = min(lane + 32 * h, L - 1);
-      float2 c1 = z, c2 = z, c3 = z, c4 = z;
-      const float2* a = A + pk(o + i, o);
-#pragma unroll 8
-      for (int j = 0; j < 32 * h; ++j) {
-        const float4 u = W->ud[j];
-        const float2 v = a[j];
-        c1 = ffma2(v, lo2(u), c1);
-        c2 = ffma2(v, hi2(u), c2);
+      for (int e = 0; e < 4; ++e) {
+        const int j = min(j0 + e, L - 1);
+        const int cb = pk(o + j, o);              // trailing row j
+        uj[e] = W->u[j];
+        a1[e] = A[j <= r1 ? rb1 + j : cb + r1];
+        a2[e] = A[j <= r2 ? rb2 + j : cb + r2];
       }
-      const int je = min(32 * h + 32, L);
-      const float2* b = A + pk(o + 32 * h, o) + i;   // A22[j][i]
-      int step = o + 32 * h + 1;
-#pragma unroll 8
-      for (int j = 32 * h; j < je; ++j) {
-        const float4 u = W->ud[j];
-        const bool low = j <= i;
-        float2 v = *(low ? a + j : b);
-        if (!low) v.y = -v.y;
-        c1 = ffma2(v, lo2(u), c1);
-        c2 = ffma2(v, hi2(u), c2);
-        b += step++;
-      }
-      if (h + 1 < H) {
-#pragma unroll 8
-        for (int j = je; j < L; ++j) {
-          const float4 u = W->ud[j];
-          const float2 v = *b;
-          c3 = ffma2(v, lo2(u), c3);
-          c4 = ffma2(v, hi2(u), c4);
-          b += step++;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int j = j0 + e;
+        if (j < L) {                              // warp-uniform
+          float2 b1 = a1[e], b2 = a2[e];
+          if (j > r1) b1.y = -b1.y;
+          if (j > r2) b2.y = -b2.y;
+          if (e & 1) { cfma(q1, b1, uj[e]); cfma(q2, b2, uj[e]); }
+          else { cfma(p1, b1, uj[e]); cfma(p2, b2, uj[e]); }
         }
       }
-      const float2 q = make_float2((c1.x - c2.y) + (c3.x + c4.y), (c1.y + c2.x) + (c4.x - c3.y));
-      if (lane + 32 * h < L) p[h] = cscale(q, t);
-      dploc += x[h].x * p[h].x + x[h].y * p[h].y;
     }
-    const float dp = wsum(dploc);
+    p1 = rp.i1 >= 0 ? cscale(cadd(p1, q1), t) : z;
+    p2 = rp.i2 >= 0 ? cscale(cadd(p2, q2), t) : z;
+    const float dp = wsum(x1.x * p1.x + x1.y * p1.y + x2.x * p2.x + x2.y * p2.y);
     const float K = 0.5f * t * dp;
-    float2 w[H];
-#pragma unroll
-    for (int h = 0; h < H; ++h) {
-      w[h] = csub(p[h], cscale(x[h], K));
-      if (lane + 32 * h < L) W->wd[lane + 32 * h] = dup2(w[h]);
-    }
+    const float2 w1 = csub(p1, cscale(x1, K)), w2 = csub(p2, cscale(x2, K));
+    if (rp.i1 >= 0) W->w[rp.i1] = w1;
+    if (rp.i2 >= 0) W->w[rp.i2] = w2;
     __syncwarp();
-    // A22 -= u w^H + w u^H on the lower triangle
+    // A22 -= u w^H + w u^H on the lower triangle of the lane's rows: element s of the lane is
+    // row i1 column s for s < n1, else row i2 column s - n1; every element has one owner lane,
+    // so the four loads of a group can all go out before its stores.
+    const float2 nu1 = make_float2(-x1.x, -x1.y), nu2 = make_float2(-x2.x, -x2.y);
+    const float2 nw1 = make_float2(-w1.x, -w1.y), nw2 = make_float2(-w2.x, -w2.y);
+    const int smax = max(rp.tot - 1, 0);
+    for (int s0 = 0; s0 <= L; s0 += 4) {
+      float2 a[4], wj[4], uj[4];
+      int id[4];
 #pragma unroll
-    for (int h = 0; h < H; ++h) {
-      if (32 * h >= L) continue;
-      const int row = lane + 32 * h, i = min(row, L - 1);
-      const bool own = row < L;
-      const float2 nu = make_float2(-x[h].x, -x[h].y), nus = make_float2(-x[h].y, x[h].x);
-      const float2 nw = make_float2(-w[h].x, -w[h].y), nws = make_float2(-w[h].y, w[h].x);
-      float2* a = A + pk(o + i, o);
-#pragma unroll 4
-      for (int j = 0; j < 32 * h; ++j) {
-        const float4 wj = W->wd[j], uj = W->ud[j];
-        float2 v = ffma2(nus, hi2(wj), ffma2(nu, lo2(wj), a[j]));
-        v = ffma2(nws, hi2(uj), ffma2(nw, lo2(uj), v));
-        if (own) a[j] = v;
+      for (int e = 0; e < 4; ++e) {
+        const int sc = min(s0 + e, smax);
+        const bool f = sc < rp.n1;
+        const int j = f ? sc : sc - rp.n1;
+        id[e] = f ? rb1 + sc : rb2 + j;
+        a[e] = A[id[e]];
+        wj[e] = W->w[j];
+        uj[e] = W->u[j];
       }
-      const int je = min(32 * h + 32, L);
-#pragma unroll 4
-      for (int j = 32 * h; j < je; ++j) {
-        const float4 wj = W->wd[j], uj = W->ud[j];
-        const bool on = own && j <= row;
-        float2 v = a[on ? j : 0];
-        v = ffma2(nus, hi2(wj), ffma2(nu, lo2(wj), v));
-        v = ffma2(nws, hi2(uj), ffma2(nw, lo2(uj), v));
-        if (on) a[j] = v;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const bool f = s0 + e < rp.n1;
+        float2 r = a[e];
+        cfma_cb(r, f ? nu1 : nu2, wj[e]);
+        cfma_cb(r, f ? nw1 : nw2, uj[e]);
+        if (s0 + e < rp.tot) A[id[e]] = r;
       }
     }
     __syncwarp();
@@ -513,7 +466,7 @@ __device__ void warp_backtransform(WarpEig<NPMAX>* W, int n, int ra, float2* fac
 }
 
 template <int NPMAX>
-__global__ void __launch_bounds__(32 * kEigWarps, NPMAX > 32 ? 7 : 8) llr_eig_warp_kernel(ProxOp op, long long nblocks) {
+__global__ void __launch_bounds__(32 * kEigWarps, 5) llr_eig_warp_kernel(ProxOp op, long long nblocks) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   WarpEig<NPMAX>* W = reinterpret_cast<WarpEig<NPMAX>*>(smem) + wib;
@@ -633,8 +586,8 @@ int launch_llr_eig_warp(const ProxOp& op, long long nblocks, cudaStream_t stream
   if (nblocks == 0) return LLR_OK;
   if (op.n <= 16) return launch_eig_warp_instance<16>(op, nblocks, stream);
   if (op.n <= 32) return launch_eig_warp_instance<32>(op, nblocks, stream);
-  if (op.n <= 48) return launch_eig_warp_instance<48>(op, nblocks, stream);
-  return set_error(LLR_ERR_UNSUPPORTED, "Casorati column count %d > 48 needs the team kernel", op.n);
+  if (op.n <= 64) return launch_eig_warp_instance<64>(op, nblocks, stream);
+  return set_error(LLR_ERR_UNSUPPORTED, "Casorati column count %d > 64 is not supported", op.n);
 }
 
 }  // namespace llr

@@ -104,8 +104,7 @@ int launch_fft_rows(int mode, float2* u, const float2* coef, const float2* S, in
                     double* partials, int* np, cudaStream_t s);
 int launch_diff_norm(const float2* a, const float2* b, long long n, double* part_d, double* part_b, int nblocks,
                      cudaStream_t s);
-int launch_llr_eig_warp(const ProxOp& op, long long nblocks, cudaStream_t stream);   // n <= 48
-int launch_llr_eig_team(const ProxOp& op, long long nblocks, cudaStream_t stream);   // 48 < n <= 64
+int launch_llr_eig_warp(const ProxOp& op, long long nblocks, cudaStream_t stream);   // n <= 64
 int launch_llr_eig_jacobi(const ProxOp& op, long long nblocks, cudaStream_t stream);   // 64 < n <= 128
 
 int launch_llr_prox(const BlockSource& src, const ProxOp& op, cudaStream_t stream);

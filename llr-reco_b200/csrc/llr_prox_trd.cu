@@ -1184,7 +1184,7 @@ int launch_split_instance(const BlockSource& src, const ProxOp& op, cudaStream_t
     kern<<<(unsigned)grid, kLlrThreads, L.total, stream>>>(src, op, L);
     LLR_CUDA_TRY(cudaGetLastError());
   }
-  LLR_TRY(op.n <= 48 ? launch_llr_eig_warp(op, src.nblocks, stream) : launch_llr_eig_team(op, src.nblocks, stream));
+  LLR_TRY(launch_llr_eig_warp(op, src.nblocks, stream));
   return launch_apply(src, op, stream);
 }
 

@@ -183,30 +183,6 @@ def test_soft_threshold_eigen_branches(gpu, n):
     assert rel_err(got, exp) < 5e-5
 
 
-@pytest.mark.parametrize("n", [2, 16, 17, 32, 33, 48, 49, 63, 64])
-@pytest.mark.parametrize("mode", ["soft", "hard"])
-def test_eigen_kernel_column_edges(gpu, n, mode):
-    """Both sides of each eigen-kernel size: blocks whose kept count runs from none to beyond what a factor holds,
-    a block near the threshold, a zero block.  FP32 Gram and reflections: relative 5e-5, the prox tolerance."""
-    rng, m = np.random.default_rng(n), max(2 * n, 40)
-    spectra = [np.linspace(1.0, 0.3, min(k, n)) for k in (1, 2, 3, 5, 8, 12)] + [np.array([0.02, 0.01][:n]), np.array([1.0, 0.097][:n])]
-    spectra = [np.pad(s, (0, n - len(s))) for s in spectra + [np.zeros(0)]]
-    x = np.asfortranarray(_spectrum_blocks(rng, m, n, spectra).astype(np.complex64))
-    d = DeviceBuffer.from_array(x)
-    if mode == "soft":
-        L.check(L.lib.llr_soft_threshold_batch_dev(m, n, 0.1, x.shape[2], d.ptr, None))
-        exp = O.low_rank_soft(x.astype(np.complex128), 0.1)
-    else:
-        L.check(L.lib.llr_low_rank_batch_dev(m, n, 2, x.shape[2], d.ptr, None))
-        exp = O.low_rank_hard(x.astype(np.complex128), 2)
-    got = d.download(np.empty_like(x, order="F"))
-    d.close()
-    assert rel_err(got, exp) < 5e-5
-    assert not got[..., -1].any()
-    if mode == "soft":
-        assert not got[..., 6].any()
-
-
 def test_zero_and_rank_deficient_blocks(gpu):
     m, n, batch = 64, 8, 3
     A = np.zeros((m, n, batch), dtype=np.complex64)
