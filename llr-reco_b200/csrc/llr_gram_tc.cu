@@ -12,11 +12,23 @@
 // Wider matrices (64 < n <= 128, NPMAX = 128): Re C and Im C are two operand tiles of 128 columns, and the
 // accumulator pair R = Re^T Re + Im^T Im, Q = Re^T Im (256 TMEM columns) gives Re G = R and
 // Im G[i][j] = Q[i][j] - Q[j][i].  One CTA of 16 warps per SM (the two chunk buffers take 128 KB).
-// Rows stream in 32-row chunks, double-buffered, with the loads of the chunk two positions
-// ahead (possibly of the CTA's next block) in flight: while the tensor core consumes one chunk
-// the 8 warps gather, phase-correct and split the next one.  One elected thread issues the
+// Narrow matrices: up to 32, 16 and 8 columns the 128 tile rows hold S = 2, 4 and 8 row chunks side by side
+// (2n <= 128 / S columns of D each), so a step covers 32 S rows; the S diagonal blocks of the accumulator
+// are the chunks' own sums (the blocks off the diagonal are never read) and the epilogue adds them.
+// With one chunk per step a step of 16 columns had two loads per thread in flight and took 2 us of latency.
+// Rows stream in steps of S 32-row chunks, double-buffered, with the loads of the chunk two positions
+// ahead (possibly of the CTA's next block) in flight: while the tensor core consumes one step's chunks
+// the 8 warps gather, phase-correct and split the next ones.  One elected thread issues the
 // MMAs and commits them to an mbarrier; every wait is bounded and reports a timeout through
 // op.err instead of hanging.
+// Tile rows beyond 2n hold whatever was there: row i and column j of the accumulator depend on tile rows i and j
+// alone, and only those below 2n are read.
+// Bound at 61 columns: the gather (48-byte runs of 6^3 blocks; 154 us of 290 remain without it) on top of the split's
+// instruction issue and the shared memory that MMAs and stores share; MMA count hardly matters (one of three
+// products less: 284 us).  32-bit block coordinates, the source's kind and phases as template arguments, one
+// barrier per step, no re-zeroing: 192 x 192 x 96 x 61, 6^3 blocks 1244 -> 1181 us, 2048 contiguous blocks of
+// 216 x 61 105 -> 90 us, 512 x 106 stride 4 2167 -> 1666 us.  Chunks side by side: 512 blocks of 512 x 17
+// 65.2 -> 44.3 us, 32 blocks of 512 x 9 29.9 -> 20.4 us.
 #include <cstdio>
 #include <algorithm>
 
@@ -42,7 +54,7 @@ union TcRowAux {
 struct TcLayout {
   size_t off_hdr, off_row, off_aux, off_op, total;
   int op_bytes;        // bytes of the operand / P-staging region
-  int nbuf;            // row tables: 2 (3 when a block is a single chunk)
+  int nbuf;            // row tables: 2 (3 when a block is a single step)
 };
 
 struct TcHdr {
@@ -56,12 +68,16 @@ struct TcHdr {
 // Instruction descriptor: TF32 x TF32 -> F32, both K-major, M = 128, N = 128.
 constexpr uint32_t kIdesc = umma_idesc_tf32(128, 128);
 
-template <int NPMAX>
+// S: row chunks side by side in the tile; PH: 0 contiguous matrices, 1 planar volumes with one phase per row,
+// 2 with a phase per row and volume.
+template <int NPMAX, int S, int PH>
 __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
     llr_gram_tc_kernel(BlockSource src, ProxOp op, TcLayout L) {
   constexpr bool WIDE = NPMAX > 64;
   constexpr int kTcWarps = tc_warps(NPMAX), kTcThreads = 32 * kTcWarps;
   constexpr int kPlanes = WIDE ? 2 : 1;            // operand tiles per precision part (Re, Im)
+  constexpr int kT = kQT / S;                      // volumes per warp
+  static_assert(!WIDE || S == 1, "two operand tiles leave no room for chunks side by side");
   constexpr uint32_t kTmemCols = WIDE ? 256u : 128u;
   extern __shared__ __align__(1024) unsigned char smem[];
   TcHdr* hdr = reinterpret_cast<TcHdr*>(smem + L.off_hdr);
@@ -69,8 +85,8 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
   TcRowAux* row_aux = reinterpret_cast<TcRowAux*>(smem + L.off_aux);   // [nbuf][m]
   unsigned char* ops = smem + L.off_op;   // [buf][hi, lo] planes; reused as P staging
   const int m = op.m, n = op.n, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const long long qstride = src.kind == 1 ? src.g.V : (long long)m;
-  const int nchunks = (m + kKC - 1) / kKC;
+  const long long qstride = PH != 0 ? src.g.V : (long long)m;
+  const int nsteps = (m + kKC * S - 1) / (kKC * S);
   const int nbuf = L.nbuf, la = nbuf - 1;   // row-table lookahead in blocks
 
   if (warp == 0) {
@@ -102,87 +118,84 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
   // loads are in flight while the tensor core and the epilogue run.
   float2 preA[kQT], preB[kQT];
   auto build_rows = [&](long long b, int buf) {
+    if (PH == 0) return;
     int* ro = row_off + (size_t)buf * m;
     TcRowAux* ra = row_aux + (size_t)buf * m;
     for (int r = tid; r < m; r += kTcThreads) {
-      if (src.kind == 1) {
-        int ix, iy, iz;
-        block_row_coord(src, b, sh, r, ix, iy, iz);
-        ro[r] = (int)planar_index(src.g, ix, iy, iz, 0);
-        TcRowAux a;
-        if (src.ph_uniform) a.ph = phase_at(src.ph, src.g, 0, ix, iy, iz);
-        else a.c = make_int2(ix, iy | (iz << 16));
-        ra[r] = a;
-      } else {
-        ro[r] = r;
+      int ix, iy, iz;
+      block_row_coord(src, b, sh, r, ix, iy, iz);
+      ro[r] = (int)planar_index(src.g, ix, iy, iz, 0);
+      TcRowAux a;
+      if (PH == 1) a.ph = phase_at(src.ph, src.g, 0, ix, iy, iz);
+      else a.c = make_int2(ix, iy | (iz << 16));
+      ra[r] = a;
+    }
+  };
+  // rows past the block's end repeat its last row here and count as zero in the conversion
+  auto load_step = [&](float2 (&pre)[kQT], int c, long long b, int buf) {
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      const int r = min((c * S + s) * kKC + lane, m - 1);
+      const float2* p = src.data + (PH == 0 ? b * (long long)m * n + r : (long long)row_off[buf * m + r]) + warp * qstride;
+#pragma unroll
+      for (int t = 0; t < kT; ++t) {
+        if (warp + kTcWarps * t < n) pre[s * kT + t] = *p;      // warp-uniform
+        p += kTcWarps * qstride;
       }
     }
   };
-  auto block_base = [&](long long b) { return src.kind == 1 ? 0ll : b * (long long)m * n; };
-  auto load_chunk = [&](float2 (&pre)[kQT], int c, long long b, int buf) {
-    const int r = c * kKC + lane;
-    const int ro = r < m ? row_off[(size_t)buf * m + r] : -1;
-    const float2* rowp = src.data + block_base(b) + (ro >= 0 ? ro : 0);
-#pragma unroll
-    for (int t = 0; t < kQT; ++t) {
-      const int q = warp + kTcWarps * t;
-      pre[t] = (q < n && ro >= 0) ? rowp[(long long)q * qstride] : make_float2(0.f, 0.f);
-    }
-  };
-  // the chunk `ahead` positions after (block iteration j, chunk c); false past the CTA's blocks
+  // the step `ahead` positions after (block iteration j, step c); false past the CTA's blocks
   auto locate = [&](long long blk, int j, int c, int ahead, long long& b2, int& j2, int& c2) {
     c2 = c + ahead;
     j2 = j;
     b2 = blk;
-    while (c2 >= nchunks) { c2 -= nchunks; ++j2; b2 += gridDim.x; }
+    while (c2 >= nsteps) { c2 -= nsteps; ++j2; b2 += gridDim.x; }
     return b2 < src.nblocks;
   };
-  // one chunk: wait for its operand buffer, convert `pre` into it, refill `pre` two chunks
+  // one step: wait for its operand buffer, convert `pre` into it, refill `pre` two steps
   // ahead, hand the buffer to the tensor core
   int gpar = 0;
   // operand offsets of this thread's elements: row q = warp + kTcWarps t (and n + q, or the Im tile's
   // row q), column lane; adding 8 to a row leaves its swizzle phase and moves it one 1 KB atom on, so
-  // op_offset(q + 8 t, lane) = op_offset(q, lane) + 1024 t
-  static_assert(kTcWarps % 8 == 0, "the step per t assumes rows a multiple of 8 apart");
-  constexpr int kStepT = 1024 * (kTcWarps / 8);
+  // op_offset(q + 8 t, lane) = op_offset(q, lane) + 1024 t, and chunk s starts 128 / S rows on
+  static_assert(kTcWarps % 8 == 0 && (128 / S) % 8 == 0, "the step per t assumes rows a multiple of 8 apart");
+  constexpr int kStepT = 1024 * (kTcWarps / 8), kStepS = 1024 * (128 / S / 8);
   const int oq0 = op_offset(warp, lane), oi0 = WIDE ? kOpBytes + oq0 : op_offset(n + warp, lane);
-  auto step = [&](float2 (&pre)[kQT], long long blk, int j, int c) -> bool {
+  auto step = [&](float2 (&pre)[kQT], long long blk, int j, int c) {
     const int b = gpar;
-    if (used[b]) {  // the MMAs that read this buffer two chunks ago must be done
-      const bool ok = mbar_wait(smem_u32(&hdr->mbar[b]), phase[b]);
+    if (used[b] && !failed) {  // the MMAs that read this buffer two steps ago must be done
+      failed = !mbar_wait(smem_u32(&hdr->mbar[b]), phase[b]);
       phase[b] ^= 1u;
-      if (__syncthreads_or(!ok)) return false;
     }
     unsigned char* hi = ops + (size_t)b * 2 * kPlanes * kOpBytes;
     unsigned char* lo = hi + kPlanes * kOpBytes;
-    const int r = c * kKC + lane;
-    const TcRowAux* ra = row_aux + (size_t)(j % nbuf) * m;
-    const bool ph_row = src.kind == 1 && r < m;
-    float2 p = make_float2(1.f, 0.f);
-    if (ph_row && src.ph_uniform) p = ra[r].ph;
+    const TcRowAux* ra = row_aux + (j % nbuf) * m;
 #pragma unroll
-    for (int t = 0; t < kQT; ++t) {
-      const int q = warp + kTcWarps * t;
-      if (q >= n) break;                              // warp-uniform
-      float2 x = pre[t];
-      if (ph_row) {
-        if (!src.ph_uniform) {
-          const int2 cc = ra[r].c;
-          p = phase_at(src.ph, src.g, q, cc.x, cc.y & 0xffff, cc.y >> 16);
-        }
-        x = cscale(cmul_bc(x, p), src.load_scale);
+    for (int s = 0; s < S; ++s) {
+      const int r = (c * S + s) * kKC + lane;
+      const bool in = r < m;
+      const TcRowAux aux = PH == 0 ? TcRowAux{} : ra[min(r, m - 1)];
+      const float rowsc = in ? src.load_scale : 0.f;
+#pragma unroll
+      for (int t = 0; t < kT; ++t) {
+        const int q = warp + kTcWarps * t;
+        if (q >= n) break;                              // warp-uniform
+        float2 x = pre[s * kT + t];
+        if (PH == 0) x = in ? x : make_float2(0.f, 0.f);
+        if (PH == 1) x = cscale(cmul_bc(x, aux.ph), rowsc);
+        if (PH == 2) x = cscale(cmul_bc(x, phase_at(src.ph, src.g, q, aux.c.x, aux.c.y & 0xffff, aux.c.y >> 16)), rowsc);
+        const uint32_t a = tf32_rna(x.x), bb = tf32_rna(x.y);
+        const int oq = oq0 + kStepT * t + kStepS * s, oi = oi0 + kStepT * t + kStepS * s;
+        *reinterpret_cast<uint32_t*>(hi + oq) = a;
+        *reinterpret_cast<uint32_t*>(hi + oi) = bb;
+        *reinterpret_cast<uint32_t*>(lo + oq) = __float_as_uint(x.x - __uint_as_float(a));
+        *reinterpret_cast<uint32_t*>(lo + oi) = __float_as_uint(x.y - __uint_as_float(bb));
       }
-      const uint32_t a = tf32_rna(x.x), bb = tf32_rna(x.y);
-      const int oq = oq0 + kStepT * t, oi = oi0 + kStepT * t;
-      *reinterpret_cast<uint32_t*>(hi + oq) = a;
-      *reinterpret_cast<uint32_t*>(hi + oi) = bb;
-      *reinterpret_cast<uint32_t*>(lo + oq) = __float_as_uint(x.x - __uint_as_float(a));
-      *reinterpret_cast<uint32_t*>(lo + oi) = __float_as_uint(x.y - __uint_as_float(bb));
     }
     {
       long long b2;
       int j2, c2;
-      if (locate(blk, j, c, 2, b2, j2, c2)) load_chunk(pre, c2, b2, j2 % nbuf);
+      if (locate(blk, j, c, 2, b2, j2, c2)) load_step(pre, c2, b2, j2 % nbuf);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
@@ -209,16 +222,12 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
         }
       }
       umma_commit(smem_u32(&hdr->mbar[b]));
-      if (c == nchunks - 1) umma_commit(smem_u32(&hdr->mbar[2]));
+      if (c == nsteps - 1) umma_commit(smem_u32(&hdr->mbar[2]));
     }
     used[b] = true;
     gpar ^= 1;
-    return true;
   };
 
-  // operand planes start zeroed: the padding rows (M up to 128) are never written by the gather
-  for (int i = tid; i < 4 * kPlanes * kOpBytes / 16; i += kTcThreads)
-    reinterpret_cast<float4*>(ops)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   long long blk = blockIdx.x;
   if (blk < src.nblocks) {
     for (int jj = 0; jj <= la; ++jj)
@@ -226,45 +235,46 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
     __syncthreads();
     long long b2;
     int j2, c2;
-    if (locate(blk, 0, 0, 0, b2, j2, c2)) load_chunk(preA, c2, b2, j2 % nbuf);
-    if (locate(blk, 0, 0, 1, b2, j2, c2)) load_chunk(preB, c2, b2, j2 % nbuf);
+    if (locate(blk, 0, 0, 0, b2, j2, c2)) load_step(preA, c2, b2, j2 % nbuf);
+    if (locate(blk, 0, 0, 1, b2, j2, c2)) load_step(preB, c2, b2, j2 % nbuf);
   }
 
   for (int j = 0; blk < src.nblocks && !failed; blk += gridDim.x, ++j) {
-    if (j > 0) {   // the table of the block `la` ahead goes into the buffer the previous block freed
+    if (j > 0) {   // (the barrier also ends the reads of the staged accumulator) the table of the block `la` ahead goes into the buffer the previous block freed
       const long long bl = blk + (long long)la * gridDim.x;
       if (bl < src.nblocks) build_rows(bl, (j + la) % nbuf);
       __syncthreads();
     }
-    for (int c = 0; c < nchunks; ++c) {
-      const bool ok = gpar == 0 ? step(preA, blk, j, c) : step(preB, blk, j, c);
-      if (!ok) { failed = true; break; }
+    for (int c = 0; c < nsteps; ++c) {
+      if (gpar == 0) step(preA, blk, j, c);
+      else step(preB, blk, j, c);
     }
-    if (failed) break;
     // all MMAs of this block complete -> read P and stage it in the (now idle) operand area
-    {
-      const bool ok = mbar_wait(smem_u32(&hdr->mbar[2]), phase[2]);
-      phase[2] ^= 1u;
-      // the done barrier implies every chunk barrier's MMAs finished too; consume them
-      for (int bb = 0; bb < 2; ++bb)
-        if (used[bb]) {
-          mbar_wait(smem_u32(&hdr->mbar[bb]), phase[bb]);
-          phase[bb] ^= 1u;
-          used[bb] = false;
-        }
-      if (__syncthreads_or(!ok)) { failed = true; break; }
-    }
+    if (!failed) failed = !mbar_wait(smem_u32(&hdr->mbar[2]), phase[2]);
+    phase[2] ^= 1u;
+    // the done barrier implies every step barrier's MMAs finished too; consume them
+    for (int bb = 0; bb < 2; ++bb)
+      if (used[bb]) {
+        if (!failed) failed = !mbar_wait(smem_u32(&hdr->mbar[bb]), phase[bb]);
+        phase[bb] ^= 1u;
+        used[bb] = false;
+      }
+    failed = __syncthreads_or(failed);
+    if (failed) break;
     asm volatile("tcgen05.fence::after_thread_sync;");
     float* Ps = reinterpret_cast<float*>(ops);
-    // narrow: P (2n x 2n), odd pitch; wide: R then Q (n x n each, odd pitch)
+    // narrow: P (2n x 2n, its S diagonal blocks 128 / S rows apart), odd pitch; wide: R then Q (n x n each, odd pitch)
+    constexpr int W = 128 / S;
     const int cols = WIDE ? n : 2 * n, ldp = cols | 1;
     // warp w reads TMEM lanes 32 (w mod 4) .. + 31 (its quadrant); the warps sharing a quadrant
     // split the 32-column chunks
     const int quad = warp & 3;
     const int a = 32 * quad + lane;          // accumulator row held by this thread
     for (int c2 = 32 * (warp >> 2); c2 < (int)kTmemCols; c2 += 32 * (kTcWarps / 4)) {
-      const int cc = WIDE ? c2 & 127 : c2;          // column within R, Q or P
-      if (cc >= cols) continue;                     // warp-uniform
+      // column within R, Q or P's diagonal block; the tests are warp-uniform (S = 8: two blocks per 32 columns)
+      if (!WIDE && S > 1 && (S == 8 ? c2 != 32 * quad : c2 / W != 32 * quad / W)) continue;
+      const int cc = WIDE ? c2 & 127 : (S == 8 ? -(lane & 16) : c2 & (W - 1));
+      if (S < 8 && cc >= cols) continue;
       float* Pd = Ps + (WIDE && c2 >= 128 ? (size_t)n * ldp : 0);
       uint32_t r[32];
       asm volatile(
@@ -276,10 +286,10 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
             "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
           : "r"(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)c2));
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (a < cols) {
+      if ((a & (W - 1)) < cols) {
 #pragma unroll
         for (int jj = 0; jj < 32; ++jj)
-          if (cc + jj < cols) Pd[a * ldp + cc + jj] = __uint_as_float(r[jj]);
+          if (cc + jj < cols && (S < 8 || cc + jj >= 0)) Pd[a * ldp + cc + jj] = __uint_as_float(r[jj]);
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -302,24 +312,20 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
             re[u] = Ps[row[u] * ldp + col[u]];
             im[u] = Q[row[u] * ldp + col[u]] - Q[col[u] * ldp + row[u]];
           } else {
-            re[u] = Ps[row[u] * ldp + col[u]] + Ps[(n + row[u]) * ldp + n + col[u]];
-            im[u] = Ps[row[u] * ldp + n + col[u]] - Ps[(n + row[u]) * ldp + col[u]];
+            re[u] = im[u] = 0.f;
+#pragma unroll
+            for (int k = 0; k < S; ++k) {
+              const float* P = Ps + k * W * ldp;
+              re[u] += P[row[u] * ldp + col[u]] + P[(n + row[u]) * ldp + n + col[u]];
+              im[u] += P[row[u] * ldp + n + col[u]] - P[(n + row[u]) * ldp + col[u]];
+            }
           }
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u)
-          if (s0 + 32 * u < len) G[(long long)row[u] * (row[u] + 1) / 2 + col[u]] = make_float2(re[u], im[u]);
+          if (s0 + 32 * u < len) G[row[u] * (row[u] + 1) / 2 + col[u]] = make_float2(re[u], im[u]);
       }
     }
-    __syncthreads();
-    // the staging overwrote the padding rows of the operand planes: zero them again
-    for (int i = tid; i < 4 * kPlanes * (128 - cols) * 8; i += kTcThreads) {   // 8 x 16 B per 128-B row
-      const int plane = i / ((128 - cols) * 8), rem = i - plane * ((128 - cols) * 8);
-      const int mn = cols + (rem >> 3), c16 = rem & 7;
-      *reinterpret_cast<float4*>(ops + (size_t)plane * kOpBytes + (mn >> 3) * 1024 + (mn & 7) * 128 + c16 * 16) =
-          make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __syncthreads();
   }
 
   if (failed && tid == 0 && op.err) atomicExch(op.err, 1);
@@ -334,16 +340,16 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
 }
 
 template <int NPMAX>
-TcLayout make_tc_layout(int m, int n) {
+TcLayout make_tc_layout(int m, int n, int S) {
   TcLayout L;
   size_t off = 0;
   L.off_hdr = off; off = align16(off + sizeof(TcHdr));
-  L.nbuf = m <= kKC ? 3 : 2;
+  L.nbuf = m <= kKC * S ? 3 : 2;
   L.off_row = off; off = align16(off + sizeof(int) * (size_t)m * L.nbuf);
   L.off_aux = off; off = align16(off + sizeof(TcRowAux) * (size_t)m * L.nbuf);
   off = (off + 1023) & ~size_t(1023);
   L.off_op = off;
-  const size_t stage = NPMAX > 64 ? 2 * (size_t)n * (n | 1) : (size_t)(2 * n) * (2 * n + 1);
+  const size_t stage = NPMAX > 64 ? 2 * (size_t)n * (n | 1) : (size_t)(128 - 128 / S + 2 * n) * (2 * n + 1);
   const size_t opb = std::max<size_t>((NPMAX > 64 ? 8 : 4) * (size_t)kOpBytes, sizeof(float) * stage);
   L.op_bytes = (int)opb;
   off += opb;
@@ -351,21 +357,26 @@ TcLayout make_tc_layout(int m, int n) {
   return L;
 }
 
+// Chunks side by side change the order of the FP32 sums.  A soft threshold is a continuous map and carries that as
+// is; a rank cut may fall between two nearly equal singular values, where the last bits of the Gram matrix
+// turn the kept subspace (one in a few thousand blocks by 1e-3), so hard rank keeps one chunk per step.
+int chunks_side_by_side(int n, bool soft) { return !soft ? 1 : n <= 8 ? 8 : n <= 16 ? 4 : n <= 32 ? 2 : 1; }
+
 }  // namespace
 
 bool llr_gram_tc_supported(int m, int n) {
   if (n < 1 || n > 128 || m < 1) return false;
-  return (n <= 64 ? make_tc_layout<64>(m, n) : make_tc_layout<128>(m, n)).total <= 227 * 1024;
+  return (n <= 64 ? make_tc_layout<64>(m, n, 1) : make_tc_layout<128>(m, n, 1)).total <= 227 * 1024;
 }
 
 namespace {
 
-template <int NPMAX>
+template <int NPMAX, int S, int PH>
 int launch_gram_instance(const BlockSource& src, const ProxOp& op, cudaStream_t stream) {
   constexpr int kTcThreads = 32 * tc_warps(NPMAX);
-  TcLayout L = make_tc_layout<NPMAX>(op.m, op.n);
+  TcLayout L = make_tc_layout<NPMAX>(op.m, op.n, S);
   if (L.total > 227 * 1024) return set_error(LLR_ERR_UNSUPPORTED, "tensor-core Gram needs %zu B smem", L.total);
-  auto kern = llr_gram_tc_kernel<NPMAX>;
+  auto kern = llr_gram_tc_kernel<NPMAX, S, PH>;
   LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
   LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   int dev = 0, nsm = 0, smem_sm = 0, regs_sm = 0;
@@ -393,11 +404,24 @@ int launch_gram_instance(const BlockSource& src, const ProxOp& op, cudaStream_t 
   return LLR_OK;
 }
 
+template <int NPMAX, int S>
+int launch_gram_source(const BlockSource& src, const ProxOp& op, cudaStream_t stream) {
+  if (src.kind != 1) return launch_gram_instance<NPMAX, S, 0>(src, op, stream);
+  return src.ph_uniform ? launch_gram_instance<NPMAX, S, 1>(src, op, stream)
+                        : launch_gram_instance<NPMAX, S, 2>(src, op, stream);
+}
+
 }  // namespace
 
 int launch_llr_gram_tc(const BlockSource& src, const ProxOp& op, cudaStream_t stream) {
   if (op.n > 128) return set_error(LLR_ERR_UNSUPPORTED, "tensor-core Gram needs n <= 128 (n = %d)", op.n);
-  return op.n <= 64 ? launch_gram_instance<64>(src, op, stream) : launch_gram_instance<128>(src, op, stream);
+  if (op.n > 64) return launch_gram_source<128, 1>(src, op, stream);
+  switch (chunks_side_by_side(op.n, op.mode != LLR_PROX_HARD_RANK)) {
+    case 8: return launch_gram_source<64, 8>(src, op, stream);
+    case 4: return launch_gram_source<64, 4>(src, op, stream);
+    case 2: return launch_gram_source<64, 2>(src, op, stream);
+    default: return launch_gram_source<64, 1>(src, op, stream);
+  }
 }
 
 }  // namespace llr

@@ -46,14 +46,10 @@ __device__ __forceinline__ void block_shift(const BlockSource& s, int* sh) {
 // block + shift (block.rs:122-133); every coordinate wraps modulo the volume (block.rs:20-22).
 __device__ __forceinline__ void block_row_coord(const BlockSource& s, long long blk, const int* sh, int r,
                                                 int& ix, int& iy, int& iz) {
-  int gyi = (int)(blk % s.gy);
-  long long t = blk / s.gy;
-  int gzi = (int)(t % s.gz);
-  int gxi = (int)(t / s.gz);
-  int ry = r % s.by;
-  int t2 = r / s.by;
-  int rz = t2 % s.bz;
-  int rx = t2 / s.bz;
+  // fewer blocks than voxels, and planar offsets are 32-bit: unsigned divisions
+  const unsigned b = (unsigned)blk, t = b / (unsigned)s.gy, ur = (unsigned)r, t2 = ur / (unsigned)s.by;
+  const int gyi = (int)(b - t * s.gy), gxi = (int)(t / (unsigned)s.gz), gzi = (int)(t - gxi * (unsigned)s.gz);
+  const int ry = (int)(ur - t2 * s.by), rx = (int)(t2 / (unsigned)s.bz), rz = (int)(t2 - rx * (unsigned)s.bz);
   ix = gxi * s.bx + sh[0] + rx; if (ix >= s.g.nx) ix -= s.g.nx; if (ix >= s.g.nx) ix %= s.g.nx;
   iy = gyi * s.by + sh[1] + ry; if (iy >= s.g.ny) iy -= s.g.ny; if (iy >= s.g.ny) iy %= s.g.ny;
   iz = gzi * s.bz + sh[2] + rz; if (iz >= s.g.nz) iz -= s.g.nz; if (iz >= s.g.nz) iz %= s.g.nz;

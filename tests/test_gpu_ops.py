@@ -183,6 +183,23 @@ def test_soft_threshold_eigen_branches(gpu, n):
     assert rel_err(got, exp) < 5e-5
 
 
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("m", [5, 32, 33, 64, 129, 256, 257, 512])
+def test_gram_row_and_column_edges(gpu, m, n):
+    """Column counts on both sides of each number of row chunks a Gram step takes (8, 4, 2, 1), rows at the ends of chunks
+    and of steps, blocks of one step and of many, more blocks than CTAs.  The soft threshold in FP32: relative
+    5e-5, the prox tolerance."""
+    rng, batch = np.random.default_rng(m + 1000 * n), 5 if m * n > 4096 else 700
+    k = min(3, m, n)
+    u, v = crandn(rng, (m, k, batch)), crandn(rng, (n, k, batch))
+    x = np.asfortranarray((np.einsum("mkb,nkb->mnb", u, v) + 0.01 * crandn(rng, (m, n, batch))).astype(np.complex64))
+    d = DeviceBuffer.from_array(x)
+    L.check(L.lib.llr_soft_threshold_batch_dev(m, n, 0.5, batch, d.ptr, None))
+    got = d.download(np.empty_like(x, order="F"))
+    d.close()
+    assert rel_err(got, O.low_rank_soft(x.astype(np.complex128), 0.5)) < 5e-5
+
+
 def test_zero_and_rank_deficient_blocks(gpu):
     m, n, batch = 64, 8, 3
     A = np.zeros((m, n, batch), dtype=np.complex64)
