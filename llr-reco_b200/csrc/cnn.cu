@@ -19,6 +19,7 @@
 #include <cstring>
 #include <vector>
 #include <algorithm>
+#include <climits>
 
 #include <cuda_bf16.h>
 
@@ -369,6 +370,324 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+}
+
+// ---------------------------------------------------------------------------------------
+// conv3d of the network's inference: the GEMM and the operand split of conv3d_tc_kernel, summed in another order.
+// The gradients keep that kernel: tensor memory truncates its FP32 sums, what that leaves in the activations depends
+// on the order, and sums over a million voxels show it (3e-5 of a gradient between the two orders, either of
+// them 6e-5 from 64 bits; an inference pass: 1.2e-6).
+//
+// A CTA walks columns of 8 (x) x 16 (y) voxels along z, one input plane at a time.  The plane's halo
+// (10 x 18 voxels, all channels) is written once into shared memory in the unswizzled K-major
+// operand layout: channel chunk c (8 BF16 = 16 B) of halo voxel h at byte c * CS + 16 h.  The operand of
+// the in-plane tap (dx, dy) is the same array read from voxel dx + 10 dy on: 8 consecutive x form one
+// core matrix (128 contiguous bytes), the 16 rows y step by 10 voxels (SBO = 160 B) and the K chunks by CS
+// (LBO).  An input plane z contributes to the output planes z - 1, z, z + 1 through the taps dz = 2, 1, 0: their
+// accumulators are consecutive column groups of a ring in tensor memory, and the weights of the three taps
+// are consecutive rows of B, so one MMA of N = 3 COUT serves all three with one read of A (fewer groups at the ends
+// of a column, two MMAs where the ring wraps).  A group is zeroed when its plane has been read back, so every
+// MMA accumulates.
+//
+// Pipeline: the next plane's FP32 halo is copied with cp.async (zero fill outside the volume and for
+// padding channels) while the current plane's MMAs run on one of two operand buffers; finished output planes are
+// read back (tcgen05.ld, bias, ReLU, residual, store) beside the next plane's MMAs.  Every
+// mbarrier wait is bounded; one that runs out sets the error flag and the CTA stops.
+//
+// Bound: shared-memory reads of A (4 KB per MMA at rows of 160-byte pitch).  One z plane per tile with one tap per MMA
+// (N = COUT, a 540-voxel halo converted for 128 outputs) took 1548 us per 32 -> 32 layer at 192 x 192 x 96; here
+// 896 us (the 8-layer network: 11.8 -> 6.5 ms).
+// ---------------------------------------------------------------------------------------
+constexpr int kCvTX = 8, kCvTY = 16;                               // 128 voxels of one z plane
+constexpr int kCvHX = kCvTX + 2, kCvHY = kCvTY + 2;
+constexpr int kCvNV = kCvHX * kCvHY;                               // 180 halo voxels of a plane
+constexpr int kCvCS = kCvNV * 16;                                  // bytes of one 8-channel chunk of a BF16 part
+
+template <int CIN, int COUT>
+struct CrLayout {
+  static constexpr int NP = cv_np(COUT);                           // accumulator columns of one output plane
+  static constexpr int KC = (CIN + 15) / 16 * 2;                   // 8-channel chunks, K padded to 16
+  static constexpr int KS = KC / 2;                                // K steps of 16 channels per tap
+  static constexpr int RC = 2 * KC;                                // 4-channel chunks of the FP32 halo
+  static constexpr int NPL = 3;                                    // BF16 parts per activation
+  static constexpr int SLOTS = 512 / NP;                           // ring of output planes: all of tensor memory
+  static constexpr int WT = KC * 3 * NP * 16;                      // bytes of one in-plane tap's weights
+  static constexpr size_t PB = (size_t)KC * kCvCS;                 // bytes of one BF16 part
+  static constexpr size_t off_hdr = 0;                             // mbarriers, TMEM address
+  static constexpr size_t off_pl = 1024;                           // two buffers of NPL parts
+  static constexpr size_t off_w = off_pl + 2 * NPL * PB;           // 9 in-plane taps of weights
+  static constexpr size_t off_raw = off_w + (size_t)9 * WT;        // FP32 halo staging, chunk r at r NV 16
+  static constexpr size_t total = off_raw + (size_t)RC * kCvNV * 16;
+};
+
+// Work items: runs of `run` output planes of one column, item = column + ncols * run index.
+struct CvRuns {
+  int nx, ny, nz, tx, run;
+  long long ncols, nitems;
+};
+
+// Position in a CTA's stream of input planes (items blockIdx.x, + gridDim.x, ...; planes zi = first .. last of each).
+struct CvPos {
+  long long item;
+  int cx, cy, z0, nout, zi, last;
+  int slot0;                                                       // ring slot of the item's first output plane
+  __device__ __forceinline__ void open(const CvRuns& G) {
+    if (item >= G.nitems) return;
+    const int col = (int)(item % G.ncols);
+    cx = col % G.tx * kCvTX;
+    cy = col / G.tx * kCvTY;
+    z0 = (int)(item / G.ncols) * G.run;
+    nout = min(G.run, G.nz - z0);
+    zi = max(z0 - 1, 0);
+    last = min(z0 + nout, G.nz - 1);
+  }
+  __device__ __forceinline__ bool valid(const CvRuns& G) const { return item < G.nitems; }
+  __device__ __forceinline__ void next(const CvRuns& G, int slots) {
+    if (zi < last) { ++zi; return; }
+    slot0 = (slot0 + nout) % slots;
+    item += gridDim.x;
+    open(G);
+  }
+};
+
+// Zeroes HC columns of this warp's 32 TMEM lanes (asynchronous: tcgen05.wait::st)
+template <int HC>
+__device__ __forceinline__ void tmem_zero(uint32_t taddr) {
+  static_assert(HC == 16 || HC == 8, "column count");
+  if constexpr (HC == 16)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+                 "r"(0u) : "memory");
+  else
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr), "r"(0u) : "memory");
+}
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* __restrict__ x,
+                                                                  const uint16_t* __restrict__ wb,
+                                                                  const float* __restrict__ bias,
+                                                                  const float* __restrict__ add, float* __restrict__ y,
+                                                                  CvRuns G, int relu, int* err) {
+  using Lay = CrLayout<CIN, COUT>;
+  constexpr int NP = Lay::NP, KC = Lay::KC, KS = Lay::KS, RC = Lay::RC, NPL = Lay::NPL, SLOTS = Lay::SLOTS;
+  static_assert(NPL == 3, "the operand split writes three parts");
+  // Live ring slots when plane i + 1 is multiplied: its three output planes and the (at most two) that plane i finished;
+  // older ones were read before the workers announced plane i + 1.
+  static_assert(SLOTS >= 6, "ring of output planes");
+  extern __shared__ __align__(1024) unsigned char smem[];
+  // mbarriers per operand buffer: full (workers -> MMA warp: the plane's parts are written), done (its MMAs are)
+  unsigned long long* mb = reinterpret_cast<unsigned long long*>(smem + Lay::off_hdr);
+  unsigned long long* full = mb;
+  unsigned long long* done = mb + 2;
+  unsigned long long* drain = mb + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Lay::off_hdr + 128);
+  unsigned char* pl = smem + Lay::off_pl;
+  unsigned char* wsm = smem + Lay::off_w;
+  unsigned char* raw = smem + Lay::off_raw;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    for (int b = 0; b < 5; ++b)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&mb[b])), "r"(b < 2 ? (uint32_t)kFwWorkers : 1u));
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  // weights W[tap][ci][co] (BF16), tap = dx + 3 dy + 9 dz -> in-plane tap block, chunk ci / 8, row (2 - dz) NP + co,
+  // element ci % 8; padding rows (co >= COUT) and columns (ci >= CIN) stay zero
+  for (int i = tid; i < 9 * Lay::WT / 16; i += kFwThreads) reinterpret_cast<uint4*>(wsm)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+  for (int i = tid; i < 27 * CIN * COUT; i += kFwThreads) {
+    const int tap = i / (CIN * COUT), r = i - tap * (CIN * COUT), ci = r / COUT, co = r - ci * COUT;
+    const int dz = tap / 9, t9 = tap - 9 * dz;
+    *reinterpret_cast<uint16_t*>(wsm + t9 * Lay::WT + (ci >> 3) * 3 * NP * 16 + ((2 - dz) * NP + co) * 16 + (ci & 7) * 2) = wb[i];
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = *tmem_slot;
+  bool failed = false;
+  CvPos first;
+  first.item = blockIdx.x;
+  first.slot0 = 0;
+  first.open(G);
+
+  if (warp < 8) {
+    // FP32 halo of plane p into the staging buffer (4-channel chunk r of halo voxel h at
+    // (r NV + h) 16 bytes), zero outside the volume and for channels >= CIN
+    constexpr int VW = CIN % 4 == 0 ? 4 : 1, PER = 4 * RC / VW;
+    auto load_raw = [&](const CvPos& p) {
+      for (int i = tid; i < kCvNV * PER; i += kFwWorkers) {
+        const int h = i / PER, c = (i - h * PER) * VW;
+        const int hy = h / kCvHX, hx = h - hy * kCvHX;
+        const int gx = p.cx - 1 + hx, gy = p.cy - 1 + hy;
+        const bool in = c < CIN && gx >= 0 && gx < G.nx && gy >= 0 && gy < G.ny;
+        const float* src = in ? x + ((long long)gx + (long long)G.nx * (gy + (long long)G.ny * p.zi)) * CIN + c : x;
+        const uint32_t dst = smem_u32(raw + ((size_t)(c >> 2) * kCvNV + h) * 16 + (c & 3) * 4);
+        if constexpr (VW == 4)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+        else
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the staging buffer -> the three BF16 parts in operand buffer b (item = 8 channels of one voxel)
+    auto convert = [&](int b) {
+      for (int i = tid; i < KC * kCvNV; i += kFwWorkers) {
+        const int c = i / kCvNV, h = i - c * kCvNV;
+        const float4 v0 = *reinterpret_cast<const float4*>(raw + ((size_t)(2 * c) * kCvNV + h) * 16);
+        const float4 v1 = *reinterpret_cast<const float4*>(raw + ((size_t)(2 * c + 1) * kCvNV + h) * 16);
+        uint4 q1, q2, q3;
+        split3_bf16(v0.x, v0.y, q1.x, q2.x, q3.x);
+        split3_bf16(v0.z, v0.w, q1.y, q2.y, q3.y);
+        split3_bf16(v1.x, v1.y, q1.z, q2.z, q3.z);
+        split3_bf16(v1.z, v1.w, q1.w, q2.w, q3.w);
+        unsigned char* o = pl + (size_t)b * NPL * Lay::PB + (size_t)c * kCvCS + (size_t)h * 16;
+        *reinterpret_cast<uint4*>(o) = q1;
+        *reinterpret_cast<uint4*>(o + Lay::PB) = q2;
+        *reinterpret_cast<uint4*>(o + 2 * Lay::PB) = q3;
+      }
+    };
+    // output planes that input plane p (the i-th of the stream) finished -> y: warp w reads TMEM lanes
+    // 32 (w & 3) .. + 31 (tile rows) and the column half w >> 2; false when the wait for the MMAs ran out
+    constexpr int HC = NP / 2;
+    const int q = warp & 3, hs = warp >> 2;
+    float bz[HC];
+#pragma unroll
+    for (int j = 0; j < HC; ++j) bz[j] = (bias && hs * HC + j < COUT) ? bias[hs * HC + j] : 0.f;
+    auto epilogue = [&](const CvPos& p, long long i) -> bool {
+      const bool ok = mbar_wait(smem_u32(&done[i & 1]), (uint32_t)((i >> 1) & 1));
+      if (workers_any(!ok)) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const int a = 32 * q + lane;
+      const int gx = p.cx + (a & 7), gy = p.cy + (a >> 3);
+      const int hi = p.zi == p.last ? p.nout - 1 : p.zi - 1 - p.z0;
+      for (int o = max(p.zi - 1 - p.z0, 0); o <= hi; ++o) {
+        uint32_t r[HC];
+        const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)((p.slot0 + o) % SLOTS * NP + hs * HC);
+        if constexpr (HC == 16) {
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+              : "r"(taddr));
+        } else {
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                       : "r"(taddr));
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        tmem_zero<HC>(taddr);                              // for the slot's next output plane
+        if (gx < G.nx && gy < G.ny) {
+          const long long v = (long long)gx + (long long)G.nx * (gy + (long long)G.ny * (p.z0 + o));
+          float f[HC];
+#pragma unroll
+          for (int k = 0; k < HC; ++k) {
+            float val = __uint_as_float(r[k]) + bz[k];
+            if (relu) val = fmaxf(val, 0.f);
+            f[k] = val;
+          }
+          if constexpr (COUT == 2 * HC && HC % 4 == 0) {   // whole 16-byte groups of this voxel's channels
+            float4* yp = reinterpret_cast<float4*>(y + v * COUT + hs * HC);
+            const float4* ap = add ? reinterpret_cast<const float4*>(add + v * COUT + hs * HC) : nullptr;
+#pragma unroll
+            for (int k = 0; k < HC / 4; ++k) {
+              float4 w4 = make_float4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
+              if (ap) {
+                const float4 a4 = ap[k];
+                w4.x += a4.x; w4.y += a4.y; w4.z += a4.z; w4.w += a4.w;
+              }
+              yp[k] = w4;
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < HC; ++k) {
+              const int c = hs * HC + k;
+              if (c < COUT) y[v * COUT + c] = f[k] + (add ? add[v * COUT + c] : 0.f);
+            }
+          }
+        }
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      return true;
+    };
+
+    // every slot starts from zero: warp w clears its lanes of one half of the columns
+    for (int c = 0; c < 256; c += 16) tmem_zero<16>(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(256 * hs + c));
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;");
+
+    CvPos ld = first, ep = first;
+    if (ld.valid(G)) load_raw(ld);
+    long long i = 0;
+    while (ld.valid(G) && !failed) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      // buffer i & 1: the MMAs of plane i - 2 were waited for by the epilogue of the last turn
+      convert((int)(i & 1));
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mbar_arrive(smem_u32(&full[i & 1]));
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // every worker is done with the staging buffer
+      ld.next(G, SLOTS);
+      if (ld.valid(G)) load_raw(ld);
+      if (i > 0) {
+        if (!epilogue(ep, i - 1)) failed = true;
+        ep.next(G, SLOTS);
+      }
+      ++i;
+    }
+    if (!failed && i > 0 && !epilogue(ep, i - 1)) failed = true;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (lane == 0) {
+    const uint64_t a0 = umma_desc_kmajor(smem_u32(pl), kCvCS, kCvHX * 16);
+    const uint64_t b0 = umma_desc_kmajor(smem_u32(wsm), 3 * NP * 16, 128);
+    constexpr uint32_t idesc[3] = {umma_idesc_bf16(128, NP), umma_idesc_bf16(128, 2 * NP), umma_idesc_bf16(128, 3 * NP)};
+    long long i = 0;
+    for (CvPos p = first; p.valid(G); p.next(G, SLOTS), ++i) {
+      // the plane before has to be complete too: its MMAs write overlapping column groups at another base or width,
+      // and only MMAs on the same accumulator and shape are ordered among themselves
+      if (!mbar_wait(smem_u32(&full[i & 1]), (uint32_t)((i >> 1) & 1)) ||
+          (i > 0 && !mbar_wait(smem_u32(&done[(i - 1) & 1]), (uint32_t)(((i - 1) >> 1) & 1)))) { failed = true; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      // output planes lo .. hi of the item; plane o takes B rows from (o - (zi - 1 - z0)) NP on
+      const int rel = p.zi - 1 - p.z0, lo = max(rel, 0), hi = min(p.nout - 1, rel + 2);
+      const int slot = (p.slot0 + lo) % SLOTS, cnt = hi - lo + 1;
+      const int n0 = min(cnt, SLOTS - slot), n1 = cnt - n0;      // before and after the ring's wrap
+      const uint32_t d0 = tmem + (uint32_t)(slot * NP);
+      const uint64_t bj = b0 + (uint64_t)((lo - rel) * NP);       // rows are 16 bytes, addresses count 16 bytes
+      const uint32_t id0 = n0 == 3 ? idesc[2] : n0 == 2 ? idesc[1] : idesc[0], id1 = n1 == 2 ? idesc[1] : idesc[0];
+      const uint64_t ab = a0 + (uint64_t)(((i & 1) * NPL * Lay::PB) >> 4);
+#pragma unroll 1
+      for (int s = 0; s < KS; ++s) {
+        const uint64_t as = ab + (uint64_t)((s * 2 * kCvCS) >> 4), bs = bj + (uint64_t)((s * 2 * 3 * NP * 16) >> 4);
+#pragma unroll 1
+        for (int dy = 0; dy < 3; ++dy) {
+#pragma unroll
+          for (int dx = 0; dx < 3; ++dx) {
+            const uint64_t db = bs + (uint64_t)(((3 * dy + dx) * Lay::WT) >> 4);
+#pragma unroll
+            for (int k = 0; k < NPL; ++k) {
+              const uint64_t da = as + (uint64_t)((k * Lay::PB) >> 4) + (uint64_t)(kCvHX * dy + dx);
+              umma_bf16(d0, da, db, id0, 1u);
+              if (n1 > 0) umma_bf16(tmem, da, db + (uint64_t)(n0 * NP), id1, 1u);
+            }
+          }
+        }
+      }
+      umma_commit(smem_u32(&done[i & 1]));
+    }
+  }
+  if (failed && err) atomicExch(err, 1);
+  __syncthreads();
+  // nothing may still write an accumulator when tensor memory is released
+  if (warp == 8 && lane == 0) umma_commit(smem_u32(drain));
+  mbar_wait(smem_u32(drain), 0u);
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -775,8 +1094,43 @@ int conv_inst(const float* x, const uint16_t* w, const float* b, const float* ad
   return LLR_OK;
 }
 
+template <int CIN, int COUT>
+int conv_run_inst(const float* x, const uint16_t* w, const float* b, const float* add, float* y, const int* dims, int relu,
+              int* err, cudaStream_t s) {
+  const size_t smem = CrLayout<CIN, COUT>::total;
+  static_assert(CrLayout<CIN, COUT>::total <= 227 * 1024, "conv operands exceed shared memory");
+  if (CIN % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) != 0)
+    return set_error(LLR_ERR_INVALID, "conv3d input must be 16-byte aligned for %d channels", CIN);
+  auto k = conv3d_run_kernel<CIN, COUT>;
+  LLR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int dev = 0, nsm = 0;
+  LLR_CUDA_TRY(cudaGetDevice(&dev));
+  LLR_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  CvRuns G;
+  G.nx = dims[0]; G.ny = dims[1]; G.nz = dims[2];
+  G.tx = (G.nx + kCvTX - 1) / kCvTX;
+  G.ncols = (long long)G.tx * ((G.ny + kCvTY - 1) / kCvTY);
+  // run length: the fewest input planes on the busiest CTA (a run reads one plane more at either end)
+  long long best = LLONG_MAX;
+  for (int runs = 1; runs <= G.nz; ++runs) {
+    const int len = (G.nz + runs - 1) / runs, used = (G.nz + len - 1) / len;
+    const long long planes = (G.ncols * used + nsm - 1) / nsm * (len + (used > 1 ? 2 : 0));
+    if (planes < best) { best = planes; G.run = len; G.nitems = G.ncols * used; }
+  }
+  const long long grid = std::min<long long>(G.nitems, nsm);
+  note_launch();
+  k<<<(unsigned)grid, kFwThreads, smem, s>>>(x, w, b, add, y, G, relu, err);
+  LLR_CUDA_TRY(cudaGetLastError());
+  return LLR_OK;
+}
+
 int conv(int cin, int cout, const float* x, const uint16_t* w, const float* b, const float* add, float* y,
-         const int* dims, int relu, int* err, cudaStream_t s) {
+         const int* dims, int relu, bool grad, int* err, cudaStream_t s) {
+  if (!grad) {   // nothing but the output is kept: see conv3d_run_kernel
+    if (cin == 14 && cout == 32) return conv_run_inst<14, 32>(x, w, b, add, y, dims, relu, err, s);
+    if (cin == 32 && cout == 32) return conv_run_inst<32, 32>(x, w, b, add, y, dims, relu, err, s);
+    if (cin == 32 && cout == 14) return conv_run_inst<32, 14>(x, w, b, add, y, dims, relu, err, s);
+  }
   if (cin == 14 && cout == 32) return conv_inst<14, 32>(x, w, b, add, y, dims, relu, err, s);
   if (cin == 32 && cout == 32) return conv_inst<32, 32>(x, w, b, add, y, dims, relu, err, s);
   if (cin == 32 && cout == 14) return conv_inst<32, 14>(x, w, b, add, y, dims, relu, err, s);
@@ -864,13 +1218,13 @@ int ensure_workspace(llr_cnn* n, long long vox) {
 }
 
 // forward through every layer; act[l] keeps each layer's input (act[0] = in)
-int forward(llr_cnn* n, const float* in, float* out, const int* dims, cudaStream_t s) {
+int forward(llr_cnn* n, const float* in, float* out, const int* dims, bool grad, cudaStream_t s) {
   n->act[0] = const_cast<float*>(in);
   for (int l = 0; l < n->n_layers; ++l) {
     const bool last = l + 1 == n->n_layers;
     float* y = last ? out : n->act[l + 1];
     LLR_TRY(conv(n->cin[l], n->cout[l], n->act[l], n->d_wb + wtab_off(n, l), n->d_master + n->b_off[l],
-                 last ? in : nullptr, y, dims, last ? 0 : 1, n->d_err, s));
+                 last ? in : nullptr, y, dims, last ? 0 : 1, grad, n->d_err, s));
   }
   return LLR_OK;
 }
@@ -1002,7 +1356,7 @@ int llr_cnn_forward_dev(llr_cnn* n, const float* d_in, float* d_out, const int32
   LLR_TRY(check_dims(dims));
   LLR_CUDA_TRY(cudaSetDevice(n->device));
   LLR_TRY(ensure_workspace(n, (long long)dims[0] * dims[1] * dims[2]));
-  return forward(n, d_in, d_out, dims, (cudaStream_t)stream);
+  return forward(n, d_in, d_out, dims, false, (cudaStream_t)stream);
 }
 
 int llr_cnn_loss_grad_dev(llr_cnn* n, const float* d_in, const float* d_target, const int32_t* dims, double* loss,
@@ -1013,7 +1367,7 @@ int llr_cnn_loss_grad_dev(llr_cnn* n, const float* d_in, const float* d_target, 
   cudaStream_t s = (cudaStream_t)stream;
   const long long vox = (long long)dims[0] * dims[1] * dims[2];
   LLR_TRY(ensure_workspace(n, vox));
-  LLR_TRY(forward(n, d_in, n->d_out, dims, s));
+  LLR_TRY(forward(n, d_in, n->d_out, dims, true, s));
   const long long nout = vox * n->cout.back();
   const int lg = std::min(n->loss_cap, grid_1d(nout));
   note_launch();
@@ -1027,7 +1381,7 @@ int llr_cnn_loss_grad_dev(llr_cnn* n, const float* d_in, const float* d_target, 
                   n->d_err, s));
     if (l == 0) break;
     // dL/d act[l] = conv(g, W') masked by the ReLU that produced act[l]
-    LLR_TRY(conv(n->cout[l], n->cin[l], g, n->d_wt + wtab_off(n, l), nullptr, nullptr, gn, dims, 0, n->d_err, s));
+    LLR_TRY(conv(n->cout[l], n->cin[l], g, n->d_wt + wtab_off(n, l), nullptr, nullptr, gn, dims, 0, true, n->d_err, s));
     const long long na = vox * n->cin[l];
     note_launch();
     relu_mask_kernel<<<grid_1d(na), 256, 0, s>>>(gn, n->act[l], na);

@@ -30,6 +30,30 @@ def test_forward_matches_oracle(gpu):
     assert rel_err(got - x, exp - x) < 1e-4
 
 
+@pytest.mark.parametrize("dims", [(1, 16, 8), (2, 17, 9), (3, 1, 1), (40, 205, 101), (97, 33, 7)])
+def test_forward_runs_and_edges(gpu, dims):
+    """One plane and two, a single voxel per plane, columns cut by the volume's edge, several runs per CTA with more
+    output planes than tensor memory holds at once.  Large volumes are checked on crops (the network reaches
+    8 voxels).  BF16 weights are exact on both sides, activations carry 24 bits: 1e-4 of the residual, as
+    above, and the rounding of the sum with the input, which a thin volume's small residual lets show."""
+    rng = np.random.default_rng(8)
+    x = rng.standard_normal(dims + (14,)).astype(np.float32)
+    with _net(seed=3) as net:
+        p = net.params
+        w0, b0 = CO.layer_slices(CH)[0][-1]                     # a last layer as large as the others: residual of order x
+        p[w0:b0] = rng.standard_normal(b0 - w0) * np.sqrt(2 / (27 * CH[-2]))
+        net.params = p
+        got = net.forward(x)
+    ny, nx = dims[1:]
+    for y0, x0 in {(0, 0), (ny // 2, nx // 2), (max(ny - 4, 0), max(nx - 4, 0))}:
+        y1, x1 = min(y0 + 4, ny), min(x0 + 4, nx)
+        ya, xa = max(y0 - 8, 0), max(x0 - 8, 0)
+        exp, _ = CO.forward(p, CH, x[:, ya:y1 + 8, xa:x1 + 8].astype(np.float64))
+        exp = exp[:, y0 - ya:y1 - ya, x0 - xa:x1 - xa]
+        res = np.linalg.norm(exp - x[:, y0:y1, x0:x1])
+        assert np.linalg.norm(got[:, y0:y1, x0:x1] - exp) <= 1e-4 * res + 2.0 ** -24 * np.linalg.norm(exp)
+
+
 @pytest.mark.parametrize("dims", [(4, 9, 10), (9, 8, 17)])
 def test_gradients_match_oracle(gpu, dims):
     """dL/dW and dL/db of every layer for L = mean |out - target|^2."""
