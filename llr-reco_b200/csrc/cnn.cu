@@ -331,15 +331,16 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
     }
     if (!failed && n > 0 && !epilogue(n - 1)) failed = true;
     asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if (lane == 0) {
+  } else {   // the whole warp, one lane issuing
+    const uint32_t leader = elect_one();
     const uint64_t a0 = umma_desc_kmajor(smem_u32(pl), kFwCS, kFwHX * 16);
     const uint64_t b0 = umma_desc_kmajor(smem_u32(wsm), NP * 16, 128);
     for (long long i = 0; i < n && !failed; ++i) {
       const uint32_t acc = (uint32_t)(i & 1);
-      if (i >= 2 && !mbar_wait(smem_u32(&acc_empty[acc]), (uint32_t)(((i - 2) >> 1) & 1))) { failed = true; break; }
+      if (i >= 2 && !mbar_wait_warp(smem_u32(&acc_empty[acc]), (uint32_t)(((i - 2) >> 1) & 1))) { failed = true; break; }
       const uint32_t d = tmem + acc * NP;
       for (int s = 0; s < KS; ++s) {
-        if (!mbar_wait(smem_u32(&conv_full[s]), (uint32_t)(i & 1))) { failed = true; break; }
+        if (!mbar_wait_warp(smem_u32(&conv_full[s]), (uint32_t)(i & 1))) { failed = true; break; }
         asm volatile("tcgen05.fence::after_thread_sync;");
         // descriptor start addresses advance in 16-byte units
         const uint64_t as = a0 + (uint64_t)((s * 2 * kFwCS) >> 4), bs = b0 + (uint64_t)((s * 2 * NP * 16) >> 4);
@@ -352,14 +353,14 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
 #pragma unroll
             for (int p = 0; p < NPL; ++p) {
               const uint64_t da = as + (uint64_t)((p * Lay::PB) >> 4) + vrow + dx;
-              umma_bf16(d, da, db, idesc, (s > 0 || dzy > 0 || dx > 0 || p > 0) ? 1u : 0u);
+              umma_bf16_by(leader, d, da, db, idesc, (s > 0 || dzy > 0 || dx > 0 || p > 0) ? 1u : 0u);
             }
           }
         }
-        umma_commit(smem_u32(&mma_done[s]));
+        umma_commit_by(leader, smem_u32(&mma_done[s]));
       }
       if (failed) break;
-      umma_commit(smem_u32(&acc_full[acc]));
+      umma_commit_by(leader, smem_u32(&acc_full[acc]));
     }
   }
   if (failed && err) atomicExch(err, 1);
@@ -641,7 +642,8 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
     }
     if (!failed && i > 0 && !epilogue(ep, i - 1)) failed = true;
     asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if (lane == 0) {
+  } else {   // the whole warp, one lane issuing
+    const uint32_t leader = elect_one();
     const uint64_t a0 = umma_desc_kmajor(smem_u32(pl), kCvCS, kCvHX * 16);
     const uint64_t b0 = umma_desc_kmajor(smem_u32(wsm), 3 * NP * 16, 128);
     constexpr uint32_t idesc[3] = {umma_idesc_bf16(128, NP), umma_idesc_bf16(128, 2 * NP), umma_idesc_bf16(128, 3 * NP)};
@@ -649,8 +651,8 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
     for (CvPos p = first; p.valid(G); p.next(G, SLOTS), ++i) {
       // the plane before has to be complete too: its MMAs write overlapping column groups at another base or width,
       // and only MMAs on the same accumulator and shape are ordered among themselves
-      if (!mbar_wait(smem_u32(&full[i & 1]), (uint32_t)((i >> 1) & 1)) ||
-          (i > 0 && !mbar_wait(smem_u32(&done[(i - 1) & 1]), (uint32_t)(((i - 1) >> 1) & 1)))) { failed = true; break; }
+      if (!mbar_wait_warp(smem_u32(&full[i & 1]), (uint32_t)((i >> 1) & 1)) ||
+          (i > 0 && !mbar_wait_warp(smem_u32(&done[(i - 1) & 1]), (uint32_t)(((i - 1) >> 1) & 1)))) { failed = true; break; }
       asm volatile("tcgen05.fence::after_thread_sync;");
       // output planes lo .. hi of the item; plane o takes B rows from (o - (zi - 1 - z0)) NP on
       const int rel = p.zi - 1 - p.z0, lo = max(rel, 0), hi = min(p.nout - 1, rel + 2);
@@ -671,13 +673,13 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
 #pragma unroll
             for (int k = 0; k < NPL; ++k) {
               const uint64_t da = as + (uint64_t)((k * Lay::PB) >> 4) + (uint64_t)(kCvHX * dy + dx);
-              umma_bf16(d0, da, db, id0, 1u);
-              if (n1 > 0) umma_bf16(tmem, da, db + (uint64_t)(n0 * NP), id1, 1u);
+              umma_bf16_by(leader, d0, da, db, id0, 1u);
+              if (n1 > 0) umma_bf16_by(leader, tmem, da, db + (uint64_t)(n0 * NP), id1, 1u);
             }
           }
         }
       }
-      umma_commit(smem_u32(&done[i & 1]));
+      umma_commit_by(leader, smem_u32(&done[i & 1]));
     }
   }
   if (failed && err) atomicExch(err, 1);
@@ -853,13 +855,14 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const fl
       if (workers_any(!ok)) failed = true;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if (lane == 0) {
+  } else {   // the whole warp, one lane issuing
+    const uint32_t leader = elect_one();
     // MN-major without swizzle: LBO = step between groups of 8 voxels (K), SBO = step between 8-channel chunks
     const uint64_t a0 = umma_desc_kmajor(smem_u32(apl), kFwHX * 16, kWgSV * 16);
     const uint64_t b0 = umma_desc_kmajor(smem_u32(bpl), 128, 128 * 16);
     constexpr int PX[6] = {0, 0, 1, 1, 0, 2}, PY[6] = {0, 1, 0, 1, 2, 0};   // planes of x and dy
     for (long long i = 0; i < n; ++i) {
-      if (!mbar_wait(smem_u32(conv_full), (uint32_t)(i & 1))) { failed = true; break; }
+      if (!mbar_wait_warp(smem_u32(conv_full), (uint32_t)(i & 1))) { failed = true; break; }
       asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll 1
       for (int ks = 0; ks < 8; ++ks) {           // rows y = 2 ks, 2 ks + 1 of the tile
@@ -872,11 +875,11 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const fl
             const uint32_t d = tmem + (uint32_t)((3 * dyt + dx) * NP);
 #pragma unroll
             for (int p = 0; p < 6; ++p)
-              umma_bf16(d, as + (uint64_t)((PX[p] * Lay::PA) >> 4), bs + (uint64_t)((PY[p] * Lay::PB) >> 4), idesc,
+              umma_bf16_by(leader, d, as + (uint64_t)((PX[p] * Lay::PA) >> 4), bs + (uint64_t)((PY[p] * Lay::PB) >> 4), idesc,
                         (i > 0 || ks > 0 || p > 0) ? 1u : 0u);
           }
       }
-      umma_commit(smem_u32(mma_done));
+      umma_commit_by(leader, smem_u32(mma_done));
     }
   }
   // bias gradient: the warps' sums in a fixed order (the staging buffer is free)

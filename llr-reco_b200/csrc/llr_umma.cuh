@@ -49,6 +49,23 @@ __device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t a, uint64_t b, ui
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
 }
 
+// One lane of a converged warp (the same one every time).  A warp that issues MMAs runs its loops whole, with only the
+// instruction itself predicated on this lane: descriptors then stay in uniform registers.  Under `if (lane == 0)`
+// each MMA first moved its operands there, 115 cycles an MMA whatever its width.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
+}
+
+__device__ __forceinline__ void umma_bf16_by(uint32_t leader, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader));
+}
+
 // Instruction descriptor: TF32 x TF32 -> F32, both operands K-major, M x N.
 __host__ __device__ constexpr uint32_t umma_idesc_tf32(uint32_t M, uint32_t N) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
@@ -65,6 +82,13 @@ __device__ __forceinline__ void umma_commit(uint32_t mbar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
 
+__device__ __forceinline__ void umma_commit_by(uint32_t leader, uint32_t mbar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(mbar), "r"(leader)
+      : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try(uint32_t mbar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -78,6 +102,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
   for (unsigned long long i = 0; i < kUmmaWaitLimit; ++i)
     if (mbar_try(mbar, parity)) return true;
   return false;
+}
+
+// The same for a converged warp: one answer for all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t mbar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(mbar, parity));
 }
 
 // TF32 part of x rounded to nearest (ties away from zero) on the 10-bit mantissa: add half a
