@@ -333,8 +333,8 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {   // the whole warp, one lane issuing
     const uint32_t leader = elect_one();
-    const uint64_t a0 = umma_desc_kmajor(smem_u32(pl), kFwCS, kFwHX * 16);
-    const uint64_t b0 = umma_desc_kmajor(smem_u32(wsm), NP * 16, 128);
+    const uint64_t da0 = umma_desc_kmajor(smem_u32(pl), kFwCS, kFwHX * 16), db0 = umma_desc_kmajor(smem_u32(wsm), NP * 16, 128);
+    const uint32_t a0 = (uint32_t)da0, ah = (uint32_t)(da0 >> 32), b0 = (uint32_t)db0, bh = (uint32_t)(db0 >> 32);
     for (long long i = 0; i < n && !failed; ++i) {
       const uint32_t acc = (uint32_t)(i & 1);
       if (i >= 2 && !mbar_wait_warp(smem_u32(&acc_empty[acc]), (uint32_t)(((i - 2) >> 1) & 1))) { failed = true; break; }
@@ -343,17 +343,17 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
         if (!mbar_wait_warp(smem_u32(&conv_full[s]), (uint32_t)(i & 1))) { failed = true; break; }
         asm volatile("tcgen05.fence::after_thread_sync;");
         // descriptor start addresses advance in 16-byte units
-        const uint64_t as = a0 + (uint64_t)((s * 2 * kFwCS) >> 4), bs = b0 + (uint64_t)((s * 2 * NP * 16) >> 4);
+        const uint32_t as = a0 + (uint32_t)((s * 2 * kFwCS) >> 4), bs = b0 + (uint32_t)((s * 2 * NP * 16) >> 4);
 #pragma unroll 1
         for (int dzy = 0; dzy < 9; ++dzy) {   // dy + 3 dz
           const uint32_t vrow = (uint32_t)(kFwHX * (dzy % 3 + kFwHY * (dzy / 3)));
 #pragma unroll
           for (int dx = 0; dx < 3; ++dx) {
-            const uint64_t db = bs + (uint64_t)(((3 * dzy + dx) * Lay::WT) >> 4);
+            const uint32_t db = bs + (uint32_t)(((3 * dzy + dx) * Lay::WT) >> 4);
 #pragma unroll
             for (int p = 0; p < NPL; ++p) {
-              const uint64_t da = as + (uint64_t)((p * Lay::PB) >> 4) + vrow + dx;
-              umma_bf16_by(leader, d, da, db, idesc, (s > 0 || dzy > 0 || dx > 0 || p > 0) ? 1u : 0u);
+              const uint32_t da = as + vrow + (uint32_t)(((p * Lay::PB) >> 4) + dx);
+              umma_bf16_by(leader, d, da, ah, db, bh, idesc, (s > 0 || dzy > 0 || dx > 0 || p > 0) ? 1u : 0u);
             }
           }
         }
@@ -395,9 +395,10 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
 // read back (tcgen05.ld, bias, ReLU, residual, store) beside the next plane's MMAs.  Every
 // mbarrier wait is bounded; one that runs out sets the error flag and the CTA stops.
 //
-// Bound: shared-memory reads of A (4 KB per MMA at rows of 160-byte pitch).  One z plane per tile with one tap per MMA
-// (N = COUT, a 540-voxel halo converted for 128 outputs) took 1548 us per 32 -> 32 layer at 192 x 192 x 96; here
-// 896 us (the 8-layer network: 11.8 -> 6.5 ms).
+// Bound: the MMAs' issue (one thread, 54 per plane) and their operand reads; with one tap and one z plane per tile (N = COUT, a
+// 540-voxel halo converted for 128 outputs) a 32 -> 32 layer at 192 x 192 x 96 took 1548 us, this way 896, with
+// the MMAs issued by a converged warp 638, with 32-bit descriptor arithmetic and unrolled taps 531 (the 8-layer
+// network: 11.8 -> 4.4 ms).
 // ---------------------------------------------------------------------------------------
 constexpr int kCvTX = 8, kCvTY = 16;                               // 128 voxels of one z plane
 constexpr int kCvHX = kCvTX + 2, kCvHY = kCvTY + 2;
@@ -644,8 +645,8 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {   // the whole warp, one lane issuing
     const uint32_t leader = elect_one();
-    const uint64_t a0 = umma_desc_kmajor(smem_u32(pl), kCvCS, kCvHX * 16);
-    const uint64_t b0 = umma_desc_kmajor(smem_u32(wsm), 3 * NP * 16, 128);
+    const uint64_t da0 = umma_desc_kmajor(smem_u32(pl), kCvCS, kCvHX * 16), db0 = umma_desc_kmajor(smem_u32(wsm), 3 * NP * 16, 128);
+    const uint32_t a0 = (uint32_t)da0, ah = (uint32_t)(da0 >> 32), b0 = (uint32_t)db0, bh = (uint32_t)(db0 >> 32);
     constexpr uint32_t idesc[3] = {umma_idesc_bf16(128, NP), umma_idesc_bf16(128, 2 * NP), umma_idesc_bf16(128, 3 * NP)};
     long long i = 0;
     for (CvPos p = first; p.valid(G); p.next(G, SLOTS), ++i) {
@@ -659,22 +660,22 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
       const int slot = (p.slot0 + lo) % SLOTS, cnt = hi - lo + 1;
       const int n0 = min(cnt, SLOTS - slot), n1 = cnt - n0;      // before and after the ring's wrap
       const uint32_t d0 = tmem + (uint32_t)(slot * NP);
-      const uint64_t bj = b0 + (uint64_t)((lo - rel) * NP);       // rows are 16 bytes, addresses count 16 bytes
+      const uint32_t bj = b0 + (uint32_t)((lo - rel) * NP);       // rows are 16 bytes, addresses count 16 bytes
       const uint32_t id0 = n0 == 3 ? idesc[2] : n0 == 2 ? idesc[1] : idesc[0], id1 = n1 == 2 ? idesc[1] : idesc[0];
-      const uint64_t ab = a0 + (uint64_t)(((i & 1) * NPL * Lay::PB) >> 4);
+      const uint32_t ab = a0 + (uint32_t)(((i & 1) * NPL * Lay::PB) >> 4);
 #pragma unroll 1
       for (int s = 0; s < KS; ++s) {
-        const uint64_t as = ab + (uint64_t)((s * 2 * kCvCS) >> 4), bs = bj + (uint64_t)((s * 2 * 3 * NP * 16) >> 4);
-#pragma unroll 1
+        const uint32_t as = ab + (uint32_t)((s * 2 * kCvCS) >> 4), bs = bj + (uint32_t)((s * 2 * 3 * NP * 16) >> 4);
+#pragma unroll
         for (int dy = 0; dy < 3; ++dy) {
 #pragma unroll
           for (int dx = 0; dx < 3; ++dx) {
-            const uint64_t db = bs + (uint64_t)(((3 * dy + dx) * Lay::WT) >> 4);
+            const uint32_t db = bs + (uint32_t)(((3 * dy + dx) * Lay::WT) >> 4);
 #pragma unroll
             for (int k = 0; k < NPL; ++k) {
-              const uint64_t da = as + (uint64_t)((k * Lay::PB) >> 4) + (uint64_t)(kCvHX * dy + dx);
-              umma_bf16_by(leader, d0, da, db, id0, 1u);
-              if (n1 > 0) umma_bf16_by(leader, tmem, da, db + (uint64_t)(n0 * NP), id1, 1u);
+              const uint32_t da = as + (uint32_t)(((k * Lay::PB) >> 4) + kCvHX * dy + dx);
+              umma_bf16_by(leader, d0, da, ah, db, bh, id0, 1u);
+              if (n1 > 0) umma_bf16_by(leader, tmem, da, ah, db + (uint32_t)(n0 * NP), bh, id1, 1u);
             }
           }
         }
@@ -707,9 +708,9 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
 // products of order down to 2^-16 are summed: b1 b1, b1 b2, b2 b1, b2 b2, b1 b3, b3 b1 (two more change
 // nothing).  What is left is the truncation of the FP32 sums in tensor memory, which grows with the
 // number of tiles per CTA; see the launch.
-// Bound: shared-memory reads of the A operand (4 KB per 128 x 32 x 16 MMA, 432 MMAs per tile).  The same GEMM in
-// 3xTF32 with a K-major copy of the operand per tap and 32 voxels (TF32 operands cannot be MN-major in
-// this layout) spent its time on those copies: 3.95 ms per 32 -> 32 layer at 96^3, now 1.2 ms.
+// Bound: the MMAs, 432 of 128 x 32 x 16 per tile.  The same GEMM in 3xTF32 with a K-major copy of the operand per tap
+// and 32 voxels (TF32 operands cannot be MN-major in this layout) spent its time on those copies: 3.95 ms per 32 -> 32
+// layer at 96^3, 1.16 ms this way, 0.82 ms with the MMAs issued by a converged warp.
 //
 // Warps 0-7 convert, load the next tile's FP32 data with cp.async while the MMAs run, and sum the bias
 // gradient; warp 8 issues the MMAs.  At the end each CTA writes its partial sums; a fixed-order reduction
@@ -858,24 +859,24 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const fl
   } else {   // the whole warp, one lane issuing
     const uint32_t leader = elect_one();
     // MN-major without swizzle: LBO = step between groups of 8 voxels (K), SBO = step between 8-channel chunks
-    const uint64_t a0 = umma_desc_kmajor(smem_u32(apl), kFwHX * 16, kWgSV * 16);
-    const uint64_t b0 = umma_desc_kmajor(smem_u32(bpl), 128, 128 * 16);
+    const uint64_t da0 = umma_desc_kmajor(smem_u32(apl), kFwHX * 16, kWgSV * 16), db0 = umma_desc_kmajor(smem_u32(bpl), 128, 128 * 16);
+    const uint32_t a0 = (uint32_t)da0, ah = (uint32_t)(da0 >> 32), b0 = (uint32_t)db0, bh = (uint32_t)(db0 >> 32);
     constexpr int PX[6] = {0, 0, 1, 1, 0, 2}, PY[6] = {0, 1, 0, 1, 2, 0};   // planes of x and dy
     for (long long i = 0; i < n; ++i) {
       if (!mbar_wait_warp(smem_u32(conv_full), (uint32_t)(i & 1))) { failed = true; break; }
       asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll 1
       for (int ks = 0; ks < 8; ++ks) {           // rows y = 2 ks, 2 ks + 1 of the tile
-        const uint64_t bs = b0 + (uint64_t)(16 * ks);
+        const uint32_t bs = b0 + (uint32_t)(16 * ks);
 #pragma unroll 1
         for (int dyt = 0; dyt < 3; ++dyt)
 #pragma unroll
           for (int dx = 0; dx < 3; ++dx) {
-            const uint64_t as = a0 + (uint64_t)(kFwHX * (2 * ks + dyt) + dx);
+            const uint32_t as = a0 + (uint32_t)(kFwHX * (2 * ks + dyt) + dx);
             const uint32_t d = tmem + (uint32_t)((3 * dyt + dx) * NP);
 #pragma unroll
             for (int p = 0; p < 6; ++p)
-              umma_bf16_by(leader, d, as + (uint64_t)((PX[p] * Lay::PA) >> 4), bs + (uint64_t)((PY[p] * Lay::PB) >> 4), idesc,
+              umma_bf16_by(leader, d, as + (uint32_t)((PX[p] * Lay::PA) >> 4), ah, bs + (uint32_t)((PY[p] * Lay::PB) >> 4), bh, idesc,
                         (i > 0 || ks > 0 || p > 0) ? 1u : 0u);
           }
       }

@@ -199,30 +199,31 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0) {   // the whole warp, one lane issuing
+      const uint32_t leader = elect_one();
       asm volatile("tcgen05.fence::after_thread_sync;");
-      const uint32_t ah = smem_u32(hi), al = smem_u32(lo);
+      const uint64_t d0 = umma_desc_sw128(smem_u32(hi));
+      const uint32_t h0 = (uint32_t)d0, dw = (uint32_t)(d0 >> 32);
+      constexpr uint32_t kLo = kPlanes * kOpBytes / 16, kIm = kOpBytes / 16;   // descriptors count 16 bytes
 #pragma unroll
       for (int s = 0; s < kKC / 8; ++s) {
-        const uint64_t dh = umma_desc_sw128(ah + s * 32);
-        const uint64_t dl = umma_desc_sw128(al + s * 32);
+        const uint32_t dh = h0 + 2 * s, dl = dh + kLo;
         const uint32_t acc = (c > 0 || s > 0) ? 1u : 0u;
-        umma_tf32(tmem, dh, dh, kIdesc, acc);
-        umma_tf32(tmem, dh, dl, kIdesc, 1u);
-        umma_tf32(tmem, dl, dh, kIdesc, 1u);
+        umma_tf32_by(leader, tmem, dh, dh, dw, kIdesc, acc);
+        umma_tf32_by(leader, tmem, dh, dl, dw, kIdesc, 1u);
+        umma_tf32_by(leader, tmem, dl, dh, dw, kIdesc, 1u);
         if (WIDE) {
-          const uint64_t ih = umma_desc_sw128(ah + kOpBytes + s * 32);
-          const uint64_t il = umma_desc_sw128(al + kOpBytes + s * 32);
-          umma_tf32(tmem, ih, ih, kIdesc, 1u);
-          umma_tf32(tmem, ih, il, kIdesc, 1u);
-          umma_tf32(tmem, il, ih, kIdesc, 1u);
-          umma_tf32(tmem + 128, dh, ih, kIdesc, acc);
-          umma_tf32(tmem + 128, dh, il, kIdesc, 1u);
-          umma_tf32(tmem + 128, dl, ih, kIdesc, 1u);
+          const uint32_t ih = dh + kIm, il = dl + kIm;
+          umma_tf32_by(leader, tmem, ih, ih, dw, kIdesc, 1u);
+          umma_tf32_by(leader, tmem, ih, il, dw, kIdesc, 1u);
+          umma_tf32_by(leader, tmem, il, ih, dw, kIdesc, 1u);
+          umma_tf32_by(leader, tmem + 128, dh, ih, dw, kIdesc, acc);
+          umma_tf32_by(leader, tmem + 128, dh, il, dw, kIdesc, 1u);
+          umma_tf32_by(leader, tmem + 128, dl, ih, dw, kIdesc, 1u);
         }
       }
-      umma_commit(smem_u32(&hdr->mbar[b]));
-      if (c == nsteps - 1) umma_commit(smem_u32(&hdr->mbar[2]));
+      umma_commit_by(leader, smem_u32(&hdr->mbar[b]));
+      if (c == nsteps - 1) umma_commit_by(leader, smem_u32(&hdr->mbar[2]));
     }
     used[b] = true;
     gpar ^= 1;

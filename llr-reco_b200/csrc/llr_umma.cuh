@@ -42,13 +42,6 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(uint32_t M, uint32_t N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
-}
-
 // One lane of a converged warp (the same one every time).  A warp that issues MMAs runs its loops whole, with only the
 // instruction itself predicated on this lane: descriptors then stay in uniform registers.  Under `if (lane == 0)`
 // each MMA first moved its operands there, 115 cycles an MMA whatever its width.
@@ -58,24 +51,29 @@ __device__ __forceinline__ uint32_t elect_one() {
   return r;
 }
 
-__device__ __forceinline__ void umma_bf16_by(uint32_t leader, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+// Operands a and b: the low words of their descriptors (address and leading step), with the high words apart: offsets
+// are 32-bit adds and constants.
+__device__ __forceinline__ void umma_bf16_by(uint32_t leader, uint32_t d, uint32_t a, uint32_t a_hi, uint32_t b, uint32_t b_hi,
+                                             uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "mov.b64 da, {%1, %6};\n\tmov.b64 db, {%2, %7};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}\n" ::"r"(d),
+      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(leader), "r"(a_hi), "r"(b_hi));
+}
+
+__device__ __forceinline__ void umma_tf32_by(uint32_t leader, uint32_t d, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc,
                                              uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader));
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "mov.b64 da, {%1, %6};\n\tmov.b64 db, {%2, %6};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, p;\n\t}\n" ::"r"(d),
+      "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(leader), "r"(hi));
 }
 
 // Instruction descriptor: TF32 x TF32 -> F32, both operands K-major, M x N.
 __host__ __device__ constexpr uint32_t umma_idesc_tf32(uint32_t M, uint32_t N) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_tf32(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t mbar) {
