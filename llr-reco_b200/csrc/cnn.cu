@@ -75,7 +75,7 @@ __host__ __device__ __forceinline__ uint16_t f32_to_bf16(float f) {
 __host__ __device__ constexpr int cv_np(int cout) { return cout <= 16 ? 16 : 32; }
 
 // ---------------------------------------------------------------------------------------
-// conv3d forward (and backward-data: the same convolution with W') as an implicit GEMM on
+// conv3d forward of a gradient pass (and backward-data: the same convolution with W') as an implicit GEMM on
 // the tensor cores, tcgen05 kind::f16 with BF16 operands and FP32 accumulation in tensor
 // memory.
 //
