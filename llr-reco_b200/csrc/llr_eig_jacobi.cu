@@ -3,8 +3,8 @@
 // The decisions and the rotations of the wide Jacobi kernel (llr_prox_trd.cu): ||G||_F or the trace bound of
 // Wolkowicz and Styan (1980) proves a block zero; otherwise cyclic parallel Jacobi in round-robin order.  The packed
 // Gram matrix (tensor-core Gram kernel) is replaced by the kept eigenvectors (n x kFacCols, q-major) and gains, the
-// kept count goes to op.blk_ra, and blocks keeping more than kFacCols components, or not converged after
-// kJacobiLogSweeps sweeps, go to the wide kernel through the fallback list.
+// kept count goes to op.blk_ra, and blocks keeping more than kFacCols components, not finite, or not converged
+// after kJacobiLogSweeps sweeps, go to the wide kernel through the fallback list.
 //
 // Against that kernel, which updates the full matrix and the full eigenvector matrix in every step:
 //   * only the upper triangle is kept and updated (half the 2 x 2 blocks of a step);
@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(kJacThreads, 4) llr_eig_jacobi_kernel(ProxOp o
     int ra = 0;
     bool done = true;
     if (!soft && op.rank >= n) ra = -2;                     // every component kept: identity
+    else if (!isfinite(fro2)) ra = -1;   // no angle compares with it: the wide kernel multiplies C by W and lets NaN through
     else if (soft && op.lambda > 0.f && (fro2 <= thr * thr || ub <= (double)thr)) ra = 0;
     else done = false;
     if (!done) {

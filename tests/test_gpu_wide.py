@@ -45,3 +45,30 @@ def test_wide_batch_matches_oracle(gpu, m, n, k, batch, mode):
     assert rel_err(got[..., :cut], exp[..., :cut]) < 5e-5
     if mode == "soft":
         assert not got[..., -1].any()
+
+
+@pytest.mark.parametrize("mode", ["soft", "hard"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_wide_batch_keeps_non_finite_matrices(gpu, mode, bad):
+    """One element, and a whole matrix, that is not finite: those matrices stay so (the residual check of an
+    iteration relies on it) and the others do not change by a bit."""
+    m, n, batch = 96, 80, 6
+    x = _low_rank_mats(np.random.default_rng(3), m, n, 3, batch, 1e-3)
+    out = []
+    for hurt in (False, True):
+        y = x.copy(order="F")
+        if hurt:
+            y[5, 7, 1] = bad
+            y[:, :, 3] = bad
+        d = DeviceBuffer.from_array(y)
+        if mode == "soft":
+            L.check(L.lib.llr_soft_threshold_batch_dev(m, n, 10.0, batch, d.ptr, None))
+        else:
+            L.check(L.lib.llr_low_rank_batch_dev(m, n, 3, batch, d.ptr, None))
+        out.append(d.download(np.empty_like(x, order="F")))
+        d.close()
+    for b in range(batch):
+        if b in (1, 3):
+            assert not np.isfinite(out[1][..., b]).all()
+        else:
+            assert np.array_equal(out[0][..., b], out[1][..., b])
