@@ -76,10 +76,8 @@ __host__ __device__ constexpr uint32_t umma_idesc_tf32(uint32_t M, uint32_t N) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
-
+// Arrival on mbar when every MMA that the leader issued so far is complete; a commit from another lane would cover
+// none of them.
 __device__ __forceinline__ void umma_commit_by(uint32_t leader, uint32_t mbar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
