@@ -203,7 +203,6 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
-  const uint32_t leader = warp == 8 ? elect_one() : 0u;   // the lane that issues every MMA and commit
   // tile i of this CTA is blockIdx.x + i gridDim.x
   const long long n = (long long)blockIdx.x < G.ntiles ? (G.ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   bool failed = false;
@@ -333,6 +332,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
     if (!failed && n > 0 && !epilogue(n - 1)) failed = true;
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {   // the whole warp, one lane issuing
+    const uint32_t leader = elect_one();
     const uint64_t da0 = umma_desc_kmajor(smem_u32(pl), kFwCS, kFwHX * 16), db0 = umma_desc_kmajor(smem_u32(wsm), NP * 16, 128);
     const uint32_t a0 = (uint32_t)da0, ah = (uint32_t)(da0 >> 32), b0 = (uint32_t)db0, bh = (uint32_t)(db0 >> 32);
     for (long long i = 0; i < n && !failed; ++i) {
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
   if (failed && err) atomicExch(err, 1);
   __syncthreads();
   // nothing may still write an accumulator when tensor memory is released: a commit covers the MMAs of its own thread
-  if (warp == 8) umma_commit_by(leader, smem_u32(drain));
+  if (warp == 8) umma_commit_by(elect_one(), smem_u32(drain));
   mbar_wait(smem_u32(drain), 0u);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
@@ -510,7 +510,6 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
-  const uint32_t leader = warp == 8 ? elect_one() : 0u;   // the lane that issues every MMA and commit
   bool failed = false;
   CvPos first;
   first.item = blockIdx.x;
@@ -645,6 +644,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
     if (!failed && i > 0 && !epilogue(ep, i - 1)) failed = true;
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {   // the whole warp, one lane issuing
+    const uint32_t leader = elect_one();
     const uint64_t da0 = umma_desc_kmajor(smem_u32(pl), kCvCS, kCvHX * 16), db0 = umma_desc_kmajor(smem_u32(wsm), 3 * NP * 16, 128);
     const uint32_t a0 = (uint32_t)da0, ah = (uint32_t)(da0 >> 32), b0 = (uint32_t)db0, bh = (uint32_t)(db0 >> 32);
     constexpr uint32_t idesc[3] = {umma_idesc_bf16(128, NP), umma_idesc_bf16(128, 2 * NP), umma_idesc_bf16(128, 3 * NP)};
@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
   if (failed && err) atomicExch(err, 1);
   __syncthreads();
   // nothing may still write an accumulator when tensor memory is released: a commit covers the MMAs of its own thread
-  if (warp == 8) umma_commit_by(leader, smem_u32(drain));
+  if (warp == 8) umma_commit_by(elect_one(), smem_u32(drain));
   mbar_wait(smem_u32(drain), 0u);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
@@ -772,7 +772,6 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const fl
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
-  const uint32_t leader = warp == 8 ? elect_one() : 0u;   // the lane that issues every MMA and commit
   const long long n = (long long)blockIdx.x < G.ntiles ? (G.ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   bool failed = false;
   float dbacc = 0.f;
@@ -858,6 +857,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const fl
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {   // the whole warp, one lane issuing
+    const uint32_t leader = elect_one();
     // MN-major without swizzle: LBO = step between groups of 8 voxels (K), SBO = step between 8-channel chunks
     const uint64_t da0 = umma_desc_kmajor(smem_u32(apl), kFwHX * 16, kWgSV * 16), db0 = umma_desc_kmajor(smem_u32(bpl), 128, 128 * 16);
     const uint32_t a0 = (uint32_t)da0, ah = (uint32_t)(da0 >> 32), b0 = (uint32_t)db0, bh = (uint32_t)(db0 >> 32);
@@ -928,7 +928,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const fl
   }
   if (failed && err) atomicExch(err, 1);
   // nothing may still write an accumulator when tensor memory is released: a commit covers the MMAs of its own thread
-  if (warp == 8) umma_commit_by(leader, smem_u32(drain));
+  if (warp == 8) umma_commit_by(elect_one(), smem_u32(drain));
   mbar_wait(smem_u32(drain), 0u);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();

@@ -104,7 +104,6 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = hdr->tmem;
-  const uint32_t leader = warp == 0 ? elect_one() : 0u;   // the lane that issues every MMA and commit
   const int sh[3] = {hdr->shift[0], hdr->shift[1], hdr->shift[2]};
   uint32_t phase[3] = {0u, 0u, 0u};
   bool used[2] = {false, false};
@@ -201,6 +200,7 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (warp == 0) {   // the whole warp, one lane issuing
+      const uint32_t leader = elect_one();
       asm volatile("tcgen05.fence::after_thread_sync;");
       const uint64_t d0 = umma_desc_sw128(smem_u32(hi));
       const uint32_t h0 = (uint32_t)d0, dw = (uint32_t)(d0 >> 32);
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
 
   if (failed && tid == 0 && op.err) atomicExch(op.err, 1);
   // nothing may still write the accumulator when it is released: a commit covers the MMAs of its own thread
-  if (warp == 0) umma_commit_by(leader, smem_u32(&hdr->mbar[2]));
+  if (warp == 0) umma_commit_by(elect_one(), smem_u32(&hdr->mbar[2]));
   mbar_wait(smem_u32(&hdr->mbar[2]), phase[2]);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();

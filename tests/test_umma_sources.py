@@ -21,12 +21,12 @@ def _kernels():
 
 @pytest.mark.parametrize("file,name,body", [pytest.param(*k, id=k[1]) for k in _kernels()])
 def test_tensor_memory_is_released_behind_the_issuing_lane(file, name, body):
-    """tcgen05.commit covers the MMAs of the thread that issues it, so one lane, elected once, issues every MMA and
-    every commit, the one before the release of tensor memory included."""
-    assert body.count("elect_one()") == 1
-    assert body.index("elect_one()") < re.search(r"umma_\w+_by\(", body).start()
+    """tcgen05.commit covers the MMAs of the thread that issues it, so the elected lane (the same one at every election of
+    a whole warp) issues every MMA and every commit, the one before the release of tensor memory included."""
     assert not re.search(r"umma_(commit|bf16|tf32)\(", body)
-    last = [m.start() for m in re.finditer(r"umma_commit_by\(leader,", body)][-1]
+    assert set(re.findall(r"umma_\w+_by\((\w+)", body)) == {"leader", "elect_one"}
+    assert set(re.findall(r"leader = ([^;]+);", body)) == {"elect_one()"}
+    last = [m.start() for m in re.finditer(r"umma_commit_by\(elect_one\(\),", body)][-1]
     assert body.rindex("umma_") == last < body.index("tcgen05.dealloc")
 
 
