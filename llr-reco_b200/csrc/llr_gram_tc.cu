@@ -12,6 +12,11 @@
 // Wider matrices (64 < n <= 128, NPMAX = 128): Re C and Im C are two operand tiles of 128 columns, and the
 // accumulator pair R = Re^T Re + Im^T Im, Q = Re^T Im (256 TMEM columns) gives Re G = R and
 // Im G[i][j] = Q[i][j] - Q[j][i].  One CTA of 16 warps per SM (the two chunk buffers take 128 KB).
+// Tensor memory truncates its sums, which over a block's 512 rows left G 6.2e-6 short where FP32 FMAs are off by 4.6e-7
+// (norm of the error, 106 columns).  So each operand buffer has its own pair, a step's 32 rows start from zero, the
+// products with a low part come first, and the pair is added to FP32 sums in registers when its buffer comes
+// round again: 1.6e-7, whatever the number of rows.  It costs registers: one step of loads is in flight instead
+// of two, and 4096 blocks of 512 x 106 take 1.26 ms instead of 0.85.
 // Narrow matrices: up to 32, 16 and 8 columns the 128 tile rows hold S = 2, 4 and 8 row chunks side by side
 // (2n <= 128 / S columns of D each), so a step covers 32 S rows; the S diagonal blocks of the accumulator
 // are the chunks' own sums (the blocks off the diagonal are never read) and the epilogue adds them.
@@ -27,7 +32,7 @@
 // instruction issue and the shared memory that MMAs and stores share; MMA count hardly matters (one of three
 // products less: 284 us).  32-bit block coordinates, the source's kind and phases as template arguments, one
 // barrier per step, no re-zeroing: 192 x 192 x 96 x 61, 6^3 blocks 1244 -> 1181 us, 2048 contiguous blocks of
-// 216 x 61 105 -> 90 us, 512 x 106 stride 4 2167 -> 1666 us.  Chunks side by side: 512 blocks of 512 x 17
+// 216 x 61 105 -> 90 us.  Chunks side by side: 512 blocks of 512 x 17
 // 65.2 -> 44.3 us, 32 blocks of 512 x 9 29.9 -> 20.4 us.
 #include <cstdio>
 #include <algorithm>
@@ -78,7 +83,7 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
   constexpr int kPlanes = WIDE ? 2 : 1;            // operand tiles per precision part (Re, Im)
   constexpr int kT = kQT / S;                      // volumes per warp
   static_assert(!WIDE || S == 1, "two operand tiles leave no room for chunks side by side");
-  constexpr uint32_t kTmemCols = WIDE ? 256u : 128u;
+  constexpr uint32_t kTmemCols = WIDE ? 512u : 128u;   // WIDE: one accumulator pair per operand buffer
   extern __shared__ __align__(1024) unsigned char smem[];
   TcHdr* hdr = reinterpret_cast<TcHdr*>(smem + L.off_hdr);
   int* row_off = reinterpret_cast<int*>(smem + L.off_row);        // [nbuf][m]
@@ -115,7 +120,8 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
   // In shared memory the 32 lanes write one 128-byte swizzled row (all banks).
   // Chunks form one stream over the CTA's blocks; two register sets alternate, and after a
   // set is converted it is refilled with the chunk two positions ahead, so two chunks of
-  // loads are in flight while the tensor core and the epilogue run.
+  // loads are in flight while the tensor core and the epilogue run.  WIDE, short of registers: one set, one step
+  // ahead.
   float2 preA[kQT], preB[kQT];
   auto build_rows = [&](long long b, int buf) {
     if (PH == 0) return;
@@ -161,11 +167,36 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
   static_assert(kTcWarps % 8 == 0 && (128 / S) % 8 == 0, "the step per t assumes rows a multiple of 8 apart");
   constexpr int kStepT = 1024 * (kTcWarps / 8), kStepS = 1024 * (128 / S / 8);
   const int oq0 = op_offset(warp, lane), oi0 = WIDE ? kOpBytes + oq0 : op_offset(n + warp, lane);
+  // WIDE: this thread's row of the block's sums, R columns 32 g .. + 31 then Q columns 32 g .. + 31 (g = warp / 4); a step's
+  // accumulators are added here in FP32
+  float sums[WIDE ? 64 : 1];
+  auto take = [&](int b) {
+    if constexpr (WIDE) {
+      if (32 * (warp >> 2) >= n) return;   // warp-uniform
+      asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        uint32_t r[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(tmem + ((uint32_t)(32 * (warp & 3)) << 16) +
+                  (uint32_t)(256 * b + 128 * (h >> 1) + 32 * (warp >> 2) + 16 * (h & 1))));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int k = 0; k < 16; ++k) sums[16 * h + k] += __uint_as_float(r[k]);
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;");
+    }
+  };
   auto step = [&](float2 (&pre)[kQT], long long blk, int j, int c) {
     const int b = gpar;
     if (used[b] && !failed) {  // the MMAs that read this buffer two steps ago must be done
       failed = !mbar_wait(smem_u32(&hdr->mbar[b]), phase[b]);
       phase[b] ^= 1u;
+      if constexpr (WIDE)
+        if (__all_sync(0xffffffffu, !failed)) take(b);
     }
     unsigned char* hi = ops + (size_t)b * 2 * kPlanes * kOpBytes;
     unsigned char* lo = hi + kPlanes * kOpBytes;
@@ -195,7 +226,7 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
     {
       long long b2;
       int j2, c2;
-      if (locate(blk, j, c, 2, b2, j2, c2)) load_step(pre, c2, b2, j2 % nbuf);
+      if (locate(blk, j, c, WIDE ? 1 : 2, b2, j2, c2)) load_step(pre, c2, b2, j2 % nbuf);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
@@ -205,21 +236,33 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
       const uint64_t d0 = umma_desc_sw128(smem_u32(hi));
       const uint32_t h0 = (uint32_t)d0, dw = (uint32_t)(d0 >> 32);
       constexpr uint32_t kLo = kPlanes * kOpBytes / 16, kIm = kOpBytes / 16;   // descriptors count 16 bytes
+      if constexpr (WIDE) {   // the products with a low part first: the small sums lose nothing to truncation
+        const uint32_t d = tmem + 256u * (uint32_t)b;
 #pragma unroll
-      for (int s = 0; s < kKC / 8; ++s) {
-        const uint32_t dh = h0 + 2 * s, dl = dh + kLo;
-        const uint32_t acc = (c > 0 || s > 0) ? 1u : 0u;
-        umma_tf32_by(leader, tmem, dh, dh, dw, kIdesc, acc);
-        umma_tf32_by(leader, tmem, dh, dl, dw, kIdesc, 1u);
-        umma_tf32_by(leader, tmem, dl, dh, dw, kIdesc, 1u);
-        if (WIDE) {
-          const uint32_t ih = dh + kIm, il = dl + kIm;
-          umma_tf32_by(leader, tmem, ih, ih, dw, kIdesc, 1u);
-          umma_tf32_by(leader, tmem, ih, il, dw, kIdesc, 1u);
-          umma_tf32_by(leader, tmem, il, ih, dw, kIdesc, 1u);
-          umma_tf32_by(leader, tmem + 128, dh, ih, dw, kIdesc, acc);
-          umma_tf32_by(leader, tmem + 128, dh, il, dw, kIdesc, 1u);
-          umma_tf32_by(leader, tmem + 128, dl, ih, dw, kIdesc, 1u);
+        for (int s = 0; s < kKC / 8; ++s) {
+          const uint32_t dh = h0 + 2 * s, dl = dh + kLo, ih = dh + kIm, il = dl + kIm;
+          umma_tf32_by(leader, d, dh, dl, dw, kIdesc, s > 0 ? 1u : 0u);
+          umma_tf32_by(leader, d, dl, dh, dw, kIdesc, 1u);
+          umma_tf32_by(leader, d, ih, il, dw, kIdesc, 1u);
+          umma_tf32_by(leader, d, il, ih, dw, kIdesc, 1u);
+          umma_tf32_by(leader, d + 128, dh, il, dw, kIdesc, s > 0 ? 1u : 0u);
+          umma_tf32_by(leader, d + 128, dl, ih, dw, kIdesc, 1u);
+        }
+#pragma unroll
+        for (int s = 0; s < kKC / 8; ++s) {
+          const uint32_t dh = h0 + 2 * s, ih = dh + kIm;
+          umma_tf32_by(leader, d, dh, dh, dw, kIdesc, 1u);
+          umma_tf32_by(leader, d, ih, ih, dw, kIdesc, 1u);
+          umma_tf32_by(leader, d + 128, dh, ih, dw, kIdesc, 1u);
+        }
+      } else {
+#pragma unroll
+        for (int s = 0; s < kKC / 8; ++s) {
+          const uint32_t dh = h0 + 2 * s, dl = dh + kLo;
+          const uint32_t acc = (c > 0 || s > 0) ? 1u : 0u;
+          umma_tf32_by(leader, tmem, dh, dh, dw, kIdesc, acc);
+          umma_tf32_by(leader, tmem, dh, dl, dw, kIdesc, 1u);
+          umma_tf32_by(leader, tmem, dl, dh, dw, kIdesc, 1u);
         }
       }
       umma_commit_by(leader, smem_u32(&hdr->mbar[b]));
@@ -237,7 +280,7 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
     long long b2;
     int j2, c2;
     if (locate(blk, 0, 0, 0, b2, j2, c2)) load_step(preA, c2, b2, j2 % nbuf);
-    if (locate(blk, 0, 0, 1, b2, j2, c2)) load_step(preB, c2, b2, j2 % nbuf);
+    if (!WIDE && locate(blk, 0, 0, 1, b2, j2, c2)) load_step(preB, c2, b2, j2 % nbuf);
   }
 
   for (int j = 0; blk < src.nblocks && !failed; blk += gridDim.x, ++j) {
@@ -246,20 +289,35 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
       if (bl < src.nblocks) build_rows(bl, (j + la) % nbuf);
       __syncthreads();
     }
+    if constexpr (WIDE) {
+      gpar = 0;   // both buffers are free: a block's partial sums are added in the same order wherever it comes
+#pragma unroll
+      for (int k = 0; k < 64; ++k) sums[k] = 0.f;
+    }
     for (int c = 0; c < nsteps; ++c) {
       if (gpar == 0) step(preA, blk, j, c);
+      else if (WIDE) step(preA, blk, j, c);
       else step(preB, blk, j, c);
     }
     // all MMAs of this block complete -> read P and stage it in the (now idle) operand area
     if (!failed) failed = !mbar_wait(smem_u32(&hdr->mbar[2]), phase[2]);
     phase[2] ^= 1u;
-    // the done barrier implies every step barrier's MMAs finished too; consume them
-    for (int bb = 0; bb < 2; ++bb)
-      if (used[bb]) {
-        if (!failed) failed = !mbar_wait(smem_u32(&hdr->mbar[bb]), phase[bb]);
-        phase[bb] ^= 1u;
-        used[bb] = false;
-      }
+    // the done barrier implies every step barrier's MMAs finished too; consume them, the older step's first
+    auto consume = [&](int bb) {
+      if (!used[bb]) return;
+      if (!failed) failed = !mbar_wait(smem_u32(&hdr->mbar[bb]), phase[bb]);
+      phase[bb] ^= 1u;
+      used[bb] = false;
+      if constexpr (WIDE)
+        if (__all_sync(0xffffffffu, !failed)) take(bb);
+    };
+    if (WIDE && (nsteps & 1)) {
+      consume(1);
+      consume(0);
+    } else {
+      consume(0);
+      consume(1);
+    }
     failed = __syncthreads_or(failed);
     if (failed) break;
     asm volatile("tcgen05.fence::after_thread_sync;");
@@ -271,12 +329,21 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
     // split the 32-column chunks
     const int quad = warp & 3;
     const int a = 32 * quad + lane;          // accumulator row held by this thread
+    if constexpr (WIDE) {
+      const int cc = 32 * (warp >> 2);
+      if (a < n && cc < n) {
+#pragma unroll
+        for (int k = 0; k < 64; ++k) {
+          const int col = cc + (k & 31);
+          if (col < n) Ps[(k < 32 ? (size_t)0 : (size_t)n * ldp) + a * ldp + col] = sums[k];
+        }
+      }
+    } else
     for (int c2 = 32 * (warp >> 2); c2 < (int)kTmemCols; c2 += 32 * (kTcWarps / 4)) {
-      // column within R, Q or P's diagonal block; the tests are warp-uniform (S = 8: two blocks per 32 columns)
-      if (!WIDE && S > 1 && (S == 8 ? c2 != 32 * quad : c2 / W != 32 * quad / W)) continue;
-      const int cc = WIDE ? c2 & 127 : (S == 8 ? -(lane & 16) : c2 & (W - 1));
+      // column within P's diagonal block; the tests are warp-uniform (S = 8: two blocks per 32 columns)
+      if (S > 1 && (S == 8 ? c2 != 32 * quad : c2 / W != 32 * quad / W)) continue;
+      const int cc = S == 8 ? -(lane & 16) : c2 & (W - 1);
       if (S < 8 && cc >= cols) continue;
-      float* Pd = Ps + (WIDE && c2 >= 128 ? (size_t)n * ldp : 0);
       uint32_t r[32];
       asm volatile(
           "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -290,7 +357,7 @@ __global__ void __launch_bounds__(32 * tc_warps(NPMAX), NPMAX == 64 ? 3 : 1)
       if ((a & (W - 1)) < cols) {
 #pragma unroll
         for (int jj = 0; jj < 32; ++jj)
-          if (cc + jj < cols && (S < 8 || cc + jj >= 0)) Pd[a * ldp + cc + jj] = __uint_as_float(r[jj]);
+          if (cc + jj < cols && (S < 8 || cc + jj >= 0)) Ps[a * ldp + cc + jj] = __uint_as_float(r[jj]);
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -387,13 +454,13 @@ int launch_gram_instance(const BlockSource& src, const ProxOp& op, cudaStream_t 
   LLR_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));
   // Residency from the kernel's own resources. The occupancy query reports one CTA per SM for
   // this kernel although three fit, so the count is derived here: shared memory (the driver
-  // reserves 1 KB per CTA), registers (allocated per warp in units of 256) and TMEM (128 or 256 of
+  // reserves 1 KB per CTA), registers (allocated per warp in units of 256) and TMEM (128 or all of
   // the SM's 512 columns per CTA). The kernel strides over blocks, so a grid larger than
   // what is resident is still correct, only slower.
   const int regs_warp = ((fa.numRegs * 32 + 255) / 256) * 256;
   const int by_regs = regs_warp > 0 ? regs_sm / (regs_warp * (kTcThreads / 32)) : 4;
   const int by_smem = smem_sm / (int)(L.total + fa.sharedSizeBytes + 1024);
-  int occ = std::min(std::min(by_regs, by_smem), NPMAX > 64 ? 2 : 4);
+  int occ = std::min(std::min(by_regs, by_smem), NPMAX > 64 ? 1 : 4);
   if (occ < 1) return set_error(LLR_ERR_UNSUPPORTED, "tensor-core Gram kernel cannot be resident");
   const long long grid = std::min<long long>(src.nblocks, (long long)nsm * occ);
   if (grid < 1) return LLR_OK;

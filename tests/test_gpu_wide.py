@@ -72,3 +72,25 @@ def test_wide_batch_keeps_non_finite_matrices(gpu, mode, bad):
             assert not np.isfinite(out[1][..., b]).all()
         else:
             assert np.array_equal(out[0][..., b], out[1][..., b])
+
+
+@pytest.mark.parametrize("m,n", [(2048, 66), (512, 106), (128, 128)])
+def test_wide_gram_sums_keep_fp32_accuracy(gpu, m, n):
+    """Orthogonal columns: the Gram matrix is diagonal, no rotation acts, and the gains 1 - lambda / s show the error of
+    its sums over all m rows alone.  Six kept columns with lambda = 0.9 s (the others below lambda): a relative error e of
+    s^2 gives 4.5 e.  Sums of 32 products truncated in tensor memory (at most 2^-23 of the partial sum per eight) and m / 32
+    FP32 additions stay below 1e-6, so 5e-6; sums truncated over 2048 rows were 4e-5 short."""
+    H = np.ones((1, 1))
+    while H.shape[0] < m:
+        H = np.block([[H, H], [H, -H]])
+    amp = np.where(np.arange(n) < 6, 0.3718, 0.05)
+    x = np.asfortranarray((H[:m, :n] * amp * np.exp(0.7j))[..., None].astype(np.complex64))
+    sv = np.linalg.norm(x[:, 0, 0].astype(np.complex128))
+    lam = np.float32(0.9 * sv)
+    d = DeviceBuffer.from_array(x)
+    L.check(L.lib.llr_soft_threshold_batch_dev(m, n, float(lam), 1, d.ptr, None))
+    got = d.download(np.empty_like(x, order="F"))
+    d.close()
+    exp = x.astype(np.complex128) * (1.0 - float(lam) / sv)
+    assert rel_err(got[:, :6], exp[:, :6]) < 5e-6
+    assert np.abs(got[:, 6:]).max() < 1e-6
