@@ -703,11 +703,10 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
 // one behind the other in 8-channel chunks of equal stride, so the 128 rows of one MMA are the taps dz = 0..2
 // of all input channels (rows past them are not used), and the tap (dx, dy) is a start-address offset of
 // dx + 10 dy voxels: nine accumulators of COUT columns, one per (dx, dy), stay in tensor memory over
-// every tile of the CTA.  B = the tile's dy.  No operand is copied per tap.
+// kWgRun tiles of the CTA.  B = the tile's dy.  No operand is copied per tap.
 // FP32 accuracy: x and dy are split into three BF16 planes each (about 24 significant bits), and the six
 // products of order down to 2^-16 are summed: b1 b1, b1 b2, b2 b1, b2 b2, b1 b3, b3 b1 (two more change
-// nothing).  What is left is the truncation of the FP32 sums in tensor memory, which grows with the
-// number of tiles per CTA; see the launch.
+// nothing).  What is left is the truncation of the FP32 sums in tensor memory, bounded by kWgRun.
 // Bound: the MMAs, 432 of 128 x 32 x 16 per tile.  The same GEMM in 3xTF32 with a K-major copy of the operand per tap
 // and 32 voxels (TF32 operands cannot be MN-major in this layout) spent its time on those copies: 3.95 ms per 32 -> 32
 // layer at 96^3, 1.16 ms this way, 0.82 ms with the MMAs issued by a converged warp.
@@ -717,6 +716,11 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
 // adds the CTAs (deterministic).
 // ---------------------------------------------------------------------------------------
 constexpr int kWgSV = kFwHX * kFwHY;                               // voxels of one halo slice
+// Tensor memory truncates its running sums, each gradient a few 1e-7 short per tile that one sum runs over, so a CTA reads
+// its accumulators out every kWgRun tiles, adds them to its FP32 partial sums and starts again from zero.  With 64 tiles
+// the gradients of a 3-layer network are within 4e-5 of 64 bits at any volume (one sum per CTA: 1.6e-4 at
+// 192 x 192 x 96, 3.3e-4 at 256 x 224 x 128); a read-out costs less than a tile.
+constexpr int kWgRun = 64;
 
 template <int CIN, int COUT>
 struct WgLayout {
@@ -775,6 +779,41 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const fl
   const long long n = (long long)blockIdx.x < G.ntiles ? (G.ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   bool failed = false;
   float dbacc = 0.f;
+  float* P = part + (long long)blockIdx.x * (ROWS * COUT + COUT);
+  // accumulators -> partial sums: warps 0-3 and 4-7 read the 128 rows of groups 0-4 and 5-8
+  auto read_out = [&](bool add) {
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const int row = 32 * (warp & 3) + lane, dz = row / Lay::SROWS, ci = row - dz * Lay::SROWS;
+    for (int g = warp < 4 ? 0 : 5; g < (warp < 4 ? 5 : 9); ++g) {
+      uint32_t r[NP];
+      const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(g * NP);
+      if constexpr (NP == 32) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+              "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
+              "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
+              "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+            : "r"(taddr));
+      } else {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+              "=r"(r[15])
+            : "r"(taddr));
+      }
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (dz < 3 && ci < CIN) {
+        float* p = P + ((long long)(g + 9 * dz) * CIN + ci) * COUT;
+#pragma unroll
+        for (int c = 0; c < COUT; ++c) p[c] = __uint_as_float(r[c]) + (add ? p[c] : 0.f);
+      }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+  };
 
   if (warp < 8) {
     constexpr int VW = CIN % 4 == 0 ? 4 : 1, PER = 4 * RC / VW;
@@ -844,6 +883,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const fl
       if (i > 0) {   // the MMAs of tile i - 1 no longer read the planes
         const bool ok = mbar_wait(smem_u32(mma_done), (uint32_t)((i - 1) & 1));
         if (workers_any(!ok)) { failed = true; break; }
+        if (i % kWgRun == 0) read_out(i > kWgRun);
       }
       convert();
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -877,7 +917,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const fl
 #pragma unroll
             for (int p = 0; p < 6; ++p)
               umma_bf16_by(leader, d, as + (uint32_t)((PX[p] * Lay::PA) >> 4), ah, bs + (uint32_t)((PY[p] * Lay::PB) >> 4), bh, idesc,
-                        (i > 0 || ks > 0 || p > 0) ? 1u : 0u);
+                        (i % kWgRun > 0 || ks > 0 || p > 0) ? 1u : 0u);
           }
       }
       umma_commit_by(leader, smem_u32(mma_done));
@@ -887,39 +927,8 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_wgrad_tc_kernel(const fl
   __syncthreads();
   if (warp < 8 && lane < COUT) rdy[warp * COUT + lane] = dbacc;
   const bool any_failed = __syncthreads_or(failed);
-  float* P = part + (long long)blockIdx.x * (ROWS * COUT + COUT);
   if (!any_failed && n > 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    if (warp < 4) {
-      const int row = 32 * warp + lane, dz = row / Lay::SROWS, ci = row - dz * Lay::SROWS;
-      for (int g = 0; g < 9; ++g) {
-        uint32_t r[NP];
-        const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(g * NP);
-        if constexpr (NP == 32) {
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-              "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-                "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-                "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-              : "r"(taddr));
-        } else {
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                "=r"(r[15])
-              : "r"(taddr));
-        }
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (dz < 3 && ci < CIN) {
-#pragma unroll
-          for (int c = 0; c < COUT; ++c) P[((long long)(g + 9 * dz) * CIN + ci) * COUT + c] = __uint_as_float(r[c]);
-        }
-      }
-    }
+    if (warp < 8) read_out(n > kWgRun);
     if (tid < COUT) {
       float s = 0.f;
       for (int w = 0; w < 8; ++w) s += rdy[w * COUT + tid];
@@ -1160,12 +1169,7 @@ int wgrad_inst(const float* x, const float* dy, float* part, long long part_cap,
   G.ty = (G.ny + kFwTY - 1) / kFwTY;
   G.ntiles = (long long)G.tx * G.ty * G.nz;
   const long long per = 27LL * CIN * COUT + COUT;
-  // The tensor core truncates its running sums: each gradient comes out a few 1e-5 short, in proportion to
-  // the tiles a CTA adds up.  104 CTAs keep the gradients of 1.2 M voxels within 2e-5 of those of the 3xTF32
-  // kernel, which truncated more often (finer K steps): 96^3 differs by 1.3e-5, by 2.0e-5 with one CTA per SM
-  // (2.8 ms of a 12.9 ms gradient faster).
-  const int grid = (int)std::max<long long>(
-      1, std::min<long long>(std::min<long long>(G.ntiles, std::min(nsm, 104)), part_cap / per));
+  const int grid = (int)std::max<long long>(1, std::min<long long>(std::min<long long>(G.ntiles, nsm), part_cap / per));
   note_launch();
   k<<<grid, kFwThreads, smem, s>>>(x, dy, part, G, err);
   LLR_CUDA_TRY(cudaGetLastError());

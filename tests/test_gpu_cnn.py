@@ -176,3 +176,56 @@ def test_learned_warm_start_gain(gpu):
     for t in (1e-2, 1e-3):
         assert plain[t] is not None and learned[t] is not None, (t, plain, learned)
         assert learned[t][0] < plain[t][0], (t, learned, plain)
+
+
+@pytest.mark.parametrize("dims", [(41, 50, 40), (37, 33, 41), (75, 17, 9)])
+def test_gradients_with_several_tiles_per_cta(gpu, dims):
+    """Odd and even numbers of 8 x 16 x 1 tiles per CTA, ragged in x and y, in both passes of the convolution and in the
+    weight gradient: every layer against the oracle.  FP32 sums over up to 82 k voxels of activations whose own error is
+    4e-6 (through BF16-exact weights): relative 1e-4 for each layer's weights and biases.  Inputs, weights and biases are
+    positive: an activation that rounds across zero would switch its ReLU, which alone moves the first layer's gradient
+    by up to 1e-3 at these sizes."""
+    from llr_b200.cnn import Cnn, DeviceArray
+    rng = np.random.default_rng(dims[0])
+    ch = (14, 32, 32, 14)
+    x = rng.uniform(0.2, 1.0, dims + (14,)).astype(np.float32)
+    t = rng.standard_normal(x.shape).astype(np.float32)
+    with Cnn(ch, seed=2) as net:
+        p = rng.uniform(0.0, 0.01, net.n_params).astype(np.float32)
+        net.params = p
+        dx, dt = DeviceArray.from_numpy(x), DeviceArray.from_numpy(t)
+        net.loss_grad_dev(dx, dt)
+        got = net.grads
+        dx.close()
+        dt.close()
+    _, exp = CO.loss_and_grads(p, ch, x.astype(np.float64), t.astype(np.float64))
+    sl, total = CO.layer_slices(ch)
+    edges = [e for s in sl for e in s] + [total]
+    for a, b in zip(edges[:-1], edges[1:]):
+        assert rel_err(got[a:b], exp[a:b]) < 1e-4, (a, b)
+
+
+def test_weight_gradient_error_does_not_grow_with_the_volume(gpu):
+    """Positive activations and output gradients: every product of the weight gradient has the same sign, so what the
+    running sums lose to truncation adds up.  120000 single-voxel planes are 811 tiles per CTA.  A sum over 64 tiles, six
+    products each, loses at most 64 x 6 x 2^-23 / 2 = 2.3e-5, the activations of the layer below 1e-5 in the same way: 4e-5
+    (a sum over all the CTA's tiles was 1.6e-4 short)."""
+    from llr_b200.cnn import Cnn, DeviceArray
+    rng = np.random.default_rng(4)
+    ch, nz = (14, 32, 14), 120000
+    x = rng.uniform(0.5, 1.0, (nz, 1, 1, 14)).astype(np.float32)
+    t = np.full_like(x, -3.0)
+    with Cnn(ch, seed=2) as net:
+        p = np.zeros(net.n_params, np.float32)
+        (w0, b0), (w1, b1) = CO.layer_slices(ch)[0]
+        p[w0:b0] = rng.uniform(0.0, 0.1, b0 - w0)
+        p[w1:b1] = rng.uniform(0.0, 0.1, b1 - w1)
+        net.params = p
+        dx, dt = DeviceArray.from_numpy(x), DeviceArray.from_numpy(t)
+        net.loss_grad_dev(dx, dt)
+        got = net.grads
+        dx.close()
+        dt.close()
+    _, exp = CO.loss_and_grads(p, ch, x.astype(np.float64), t.astype(np.float64))
+    assert rel_err(got[w1:b1], exp[w1:b1]) < 4e-5
+    assert rel_err(got[w0:b0], exp[w0:b0]) < 4e-5
