@@ -3,8 +3,12 @@
 // The decisions and the rotations of the wide Jacobi kernel (llr_prox_trd.cu): ||G||_F or the trace bound of
 // Wolkowicz and Styan (1980) proves a block zero; otherwise cyclic parallel Jacobi in round-robin order.  The packed
 // Gram matrix (tensor-core Gram kernel) is replaced by the kept eigenvectors (n x kFacCols, q-major) and gains, the
-// kept count goes to op.blk_ra, and blocks keeping more than kFacCols components, not finite, or not converged
-// after kJacobiLogSweeps sweeps, go to the wide kernel through the fallback list.
+// kept count goes to op.blk_ra.  Blocks that are not finite, or not converged after kJacobiLogSweeps sweeps, go to the wide
+// kernel through the fallback list; so do blocks that keep more than kFacCols components, with W = V diag(g) V^H
+// in place of their Gram matrix, so that only the product C W is left there.  Up to kColBatch columns are formed like
+// the few of a factor; for more the rotations are undone on diag(g), which costs about what the sweeps did, whatever the
+// count.  1024 blocks of 512 x 106 keeping 12 / all: 41 ms with everything done twice, 29 / 30 ms in the wide
+// kernel alone, 16 / 20 ms this way; 16 blocks keeping all 6.3, 4.7 and 3.9 ms.
 //
 // Against that kernel, which updates the full matrix and the full eigenvector matrix in every step:
 //   * only the upper triangle is kept and updated (half the 2 x 2 blocks of a step);
@@ -21,6 +25,7 @@
 // singular values and vectors short by a few 1e-6, which every result so far carries (residuals 5e-5): its
 // more exact results differ from theirs by more than single precision explains.
 #include <algorithm>
+#include <type_traits>
 
 #include "llr_prox_common.cuh"
 
@@ -30,6 +35,7 @@ namespace {
 
 constexpr int kJacThreads = 256;
 constexpr int kJacHalf = kProxMaxN / 2;
+constexpr int kColBatch = kJacThreads / 32 * 4;   // kept columns formed one by one; above, W is
 constexpr int kJacTasks = (kJacHalf * (kJacHalf + 1) / 2 + kJacThreads - 1) / kJacThreads;   // 2 x 2 blocks per thread
 
 struct JacSmem {
@@ -46,7 +52,10 @@ struct JacSmem {
 __device__ __forceinline__ int2 jac_pair(int k, int step, int M) {
   int p, q;
   if (k == 0) { p = step; q = M; }
-  else { p = (step + k) % M; q = (step - k + M) % M; }
+  else {   // modulo M
+    p = step + k; if (p >= M) p -= M;
+    q = step - k; if (q < 0) q += M;
+  }
   return p < q ? make_int2(p, q) : make_int2(q, p);
 }
 
@@ -111,6 +120,61 @@ __global__ void __launch_bounds__(kJacThreads, 4) llr_eig_jacobi_kernel(ProxOp o
     else if (!isfinite(fro2)) ra = -1;   // no angle compares with it: the wide kernel multiplies C by W and lets NaN through
     else if (soft && op.lambda > 0.f && (fro2 <= thr * thr || ub <= (double)thr)) ra = 0;
     else done = false;
+    // one step's rotations on the packed matrix: A <- J^H A J, or undone A <- J A J^H
+    auto update = [&](auto undo) {
+#pragma unroll
+      for (int u = 0; u < kJacTasks; ++u) {
+        if (task[u] < 0) continue;
+        const int k1 = task[u] & 255, k2 = task[u] >> 8;
+        const float4 R1 = W->rot[k1], R2 = W->rot[k2];
+        const bool id1 = R1.y == 0.f, id2 = R2.y == 0.f;
+        if (id1 && id2) continue;
+        const int2 P1 = W->pairs[k1], P2 = W->pairs[k2];
+        // element (i, j) lives at (min, max), conjugated below the diagonal
+        auto at = [&](int i, int j) { return row(min(i, j)) + max(i, j); };
+        const int i11 = at(P1.x, P2.x), i12 = at(P1.x, P2.y), i21 = at(P1.y, P2.x), i22 = at(P1.y, P2.y);
+        const float2 f11 = make_float2(1.f, P1.x <= P2.x ? 1.f : -1.f), f12 = make_float2(1.f, P1.x <= P2.y ? 1.f : -1.f);
+        const float2 f21 = make_float2(1.f, P1.y <= P2.x ? 1.f : -1.f), f22 = make_float2(1.f, P1.y <= P2.y ? 1.f : -1.f);
+        float2 a11 = __fmul2_rn(A[i11], f11), a12 = __fmul2_rn(A[i12], f12);
+        float2 a21 = __fmul2_rn(A[i21], f21), a22 = __fmul2_rn(A[i22], f22);
+        // (x, y) <- (c x - s e y, s x + c e y), undone (c x + s y, e (c y - s x)); ex = (e.x, e.x), ey = (-e.y, e.y)
+        auto turn = [](float2& x, float2& y, float2 cc, float2 ss, float2 ms, float2 ex, float2 ey) {
+          if constexpr (decltype(undo)::value) {
+            const float2 d = __ffma2_rn(ms, x, __fmul2_rn(cc, y));
+            x = __ffma2_rn(ss, y, __fmul2_rn(cc, x));
+            y = __ffma2_rn(make_float2(d.y, d.x), ey, __fmul2_rn(d, ex));
+          } else {
+            const float2 ty = __ffma2_rn(make_float2(y.y, y.x), ey, __fmul2_rn(y, ex));
+            const float2 nx = __ffma2_rn(ms, ty, __fmul2_rn(cc, x));
+            y = __ffma2_rn(ss, x, __fmul2_rn(cc, ty));
+            x = nx;
+          }
+        };
+        const float sg = decltype(undo)::value ? -1.f : 1.f;
+        if (!id2) {  // columns: [x_p, x_q] J2 (undone: J2^H),  J2 = [[c, s], [-s e2*, c e2*]]
+          const float2 cc = make_float2(R2.x, R2.x), ss = make_float2(R2.y, R2.y), ms = make_float2(-R2.y, -R2.y);
+          const float2 ex = make_float2(R2.z, R2.z), ey = make_float2(sg * R2.w, -sg * R2.w);
+          turn(a11, a12, cc, ss, ms, ex, ey);
+          turn(a21, a22, cc, ss, ms, ex, ey);
+        }
+        if (!id1) {  // rows: J1^H [row_p; row_q] (undone: J1),  J1^H = [[c, -s e1], [s, c e1]]
+          const float2 cc = make_float2(R1.x, R1.x), ss = make_float2(R1.y, R1.y), ms = make_float2(-R1.y, -R1.y);
+          const float2 ex = make_float2(R1.z, R1.z), ey = make_float2(-sg * R1.w, sg * R1.w);
+          turn(a11, a21, cc, ss, ms, ex, ey);
+          turn(a12, a22, cc, ss, ms, ex, ey);
+        }
+        if (k1 == k2) {
+          A[i11] = make_float2(a11.x, 0.f);
+          A[i12] = decltype(undo)::value ? a12 : make_float2(0.f, 0.f);
+          A[i22] = make_float2(a22.x, 0.f);
+        } else {
+          A[i11] = __fmul2_rn(a11, f11);
+          A[i12] = __fmul2_rn(a12, f12);
+          A[i21] = __fmul2_rn(a21, f21);
+          A[i22] = __fmul2_rn(a22, f22);
+        }
+      }
+    };
     if (!done) {
       // Scale the matrix by a power of two (exact) so that its norm lies in [1, 2): entries that matter can
       // be squared.  The angle's quotients may be off in the last bits (its tangent only has to annihilate to
@@ -159,51 +223,7 @@ __global__ void __launch_bounds__(kJacThreads, 4) llr_eig_jacobi_kernel(ProxOp o
           }
           __syncthreads();
           if (step == 0 && tid == 0) W->flag[fs ^ 1] = 0;
-#pragma unroll
-          for (int u = 0; u < kJacTasks; ++u) {
-            if (task[u] < 0) continue;
-            const int k1 = task[u] & 255, k2 = task[u] >> 8;
-            const float4 R1 = W->rot[k1], R2 = W->rot[k2];
-            const bool id1 = R1.y == 0.f, id2 = R2.y == 0.f;
-            if (id1 && id2) continue;
-            const int2 P1 = W->pairs[k1], P2 = W->pairs[k2];
-            // element (i, j) lives at (min, max), conjugated below the diagonal
-            auto at = [&](int i, int j) { return row(min(i, j)) + max(i, j); };
-            const int i11 = at(P1.x, P2.x), i12 = at(P1.x, P2.y), i21 = at(P1.y, P2.x), i22 = at(P1.y, P2.y);
-            const float2 f11 = make_float2(1.f, P1.x <= P2.x ? 1.f : -1.f), f12 = make_float2(1.f, P1.x <= P2.y ? 1.f : -1.f);
-            const float2 f21 = make_float2(1.f, P1.y <= P2.x ? 1.f : -1.f), f22 = make_float2(1.f, P1.y <= P2.y ? 1.f : -1.f);
-            float2 a11 = __fmul2_rn(A[i11], f11), a12 = __fmul2_rn(A[i12], f12);
-            float2 a21 = __fmul2_rn(A[i21], f21), a22 = __fmul2_rn(A[i22], f22);
-            // (x, y) <- (c x - s e y, s x + c e y) with ex = (e.x, e.x), ey = (-e.y, e.y)
-            auto turn = [](float2& x, float2& y, float2 cc, float2 ss, float2 ms, float2 ex, float2 ey) {
-              const float2 ty = __ffma2_rn(make_float2(y.y, y.x), ey, __fmul2_rn(y, ex));
-              const float2 nx = __ffma2_rn(ms, ty, __fmul2_rn(cc, x));
-              y = __ffma2_rn(ss, x, __fmul2_rn(cc, ty));
-              x = nx;
-            };
-            if (!id2) {  // columns: [x_p, x_q] J2,  J2 = [[c, s], [-s e2*, c e2*]]
-              const float2 cc = make_float2(R2.x, R2.x), ss = make_float2(R2.y, R2.y), ms = make_float2(-R2.y, -R2.y);
-              const float2 ex = make_float2(R2.z, R2.z), ey = make_float2(R2.w, -R2.w);
-              turn(a11, a12, cc, ss, ms, ex, ey);
-              turn(a21, a22, cc, ss, ms, ex, ey);
-            }
-            if (!id1) {  // rows: J1^H [row_p; row_q],  J1^H = [[c, -s e1], [s, c e1]]
-              const float2 cc = make_float2(R1.x, R1.x), ss = make_float2(R1.y, R1.y), ms = make_float2(-R1.y, -R1.y);
-              const float2 ex = make_float2(R1.z, R1.z), ey = make_float2(-R1.w, R1.w);
-              turn(a11, a21, cc, ss, ms, ex, ey);
-              turn(a12, a22, cc, ss, ms, ex, ey);
-            }
-            if (k1 == k2) {
-              A[i11] = make_float2(a11.x, 0.f);
-              A[i12] = make_float2(0.f, 0.f);
-              A[i22] = make_float2(a22.x, 0.f);
-            } else {
-              A[i11] = __fmul2_rn(a11, f11);
-              A[i12] = __fmul2_rn(a12, f12);
-              A[i21] = __fmul2_rn(a21, f21);
-              A[i22] = __fmul2_rn(a22, f22);
-            }
-          }
+          update(std::false_type{});
           __syncthreads();
         }
         converged = W->flag[fs] == 0;
@@ -234,60 +254,118 @@ __global__ void __launch_bounds__(kJacThreads, 4) llr_eig_jacobi_kernel(ProxOp o
       }
       __syncthreads();
       ra = W->n_active;
-      if (!converged || ra > kFacCols) ra = -1;
-      if (ra > 0) {
-        if (warp < ra) {   // column act[warp] of J_1 ... J_steps
-          float2* v = A + warp * kProxMaxN;   // the matrix is spent
-          const int col = W->act[warp];
-          for (int i = lane; i < n2; i += 32) v[i] = make_float2(i == col ? 1.f : 0.f, 0.f);
-          __syncwarp();
-          constexpr int PF = 4;        // log entries in flight per lane and pair set
-          const int ka = lane, kb = lane + 32;
-          auto fetch = [&](int st, int k) {
-            const float* lg = log + 3 * (st * half + k);
-            return st >= 0 && k < half ? make_float3(__ldcg(lg), __ldcg(lg + 1), __ldcg(lg + 2)) : make_float3(0.f, 1.f, 0.f);
-          };
-          float3 ra4[PF], rb4[PF];
+      if (!converged) ra = -1;
+      // columns act[c0] .. act[c0 + CB - 1] of J_1 ... J_steps, each n2 entries from v on (the matrix is spent); past
+      // the last kept one zeros
+      auto columns = [&](auto cb, float2* v, int c0) {
+        constexpr int CB = decltype(cb)::value;
+#pragma unroll
+        for (int c = 0; c < CB; ++c) {
+          const int col = c0 + c < ra ? W->act[c0 + c] : -1;
+          for (int i = lane; i < n2; i += 32) v[c * n2 + i] = make_float2(i == col ? 1.f : 0.f, 0.f);
+        }
+        __syncwarp();
+        constexpr int PF = 4;        // log entries in flight per lane and pair set
+        const int ka = lane, kb = lane + 32;
+        auto fetch = [&](int st, int k) {
+          const float* lg = log + 3 * (st * half + k);
+          return st >= 0 && k < half ? make_float3(__ldcg(lg), __ldcg(lg + 1), __ldcg(lg + 2)) : make_float3(0.f, 1.f, 0.f);
+        };
+        float3 ra4[PF], rb4[PF];
+#pragma unroll
+        for (int u = 0; u < PF; ++u) {
+          ra4[u] = fetch(steps - 1 - u, ka);
+          rb4[u] = fetch(steps - 1 - u, kb);
+        }
+        auto rotate = [&](float3 r3, int k, int step) {
+          if (r3.x == 0.f) return;   // identity (also lanes past the last pair)
+          const float cs = rsqrtf(1.f + r3.x * r3.x);
+          const float4 r = make_float4(cs, r3.x * cs, r3.y, r3.z);
+          const int2 pq = jac_pair(k, step, M);
+          const float2 ec = make_float2(r.z, -r.w);
+          float2 vp[CB], vq[CB];
+#pragma unroll
+          for (int c = 0; c < CB; ++c) { vp[c] = v[c * n2 + pq.x]; vq[c] = v[c * n2 + pq.y]; }
+#pragma unroll
+          for (int c = 0; c < CB; ++c) {
+            const float2 d = make_float2(r.x * vq[c].x - r.y * vp[c].x, r.x * vq[c].y - r.y * vp[c].y);
+            v[c * n2 + pq.x] = make_float2(r.x * vp[c].x + r.y * vq[c].x, r.x * vp[c].y + r.y * vq[c].y);
+            v[c * n2 + pq.y] = cmul(ec, d);
+          }
+        };
+        int step = M - 1;
+        for (int st0 = steps - 1; st0 >= 0; st0 -= PF) {
 #pragma unroll
           for (int u = 0; u < PF; ++u) {
-            ra4[u] = fetch(steps - 1 - u, ka);
-            rb4[u] = fetch(steps - 1 - u, kb);
-          }
-          auto rotate = [&](float3 r3, int k, int step) {
-            if (r3.x == 0.f) return;   // identity (also lanes past the last pair)
-            const float c = rsqrtf(1.f + r3.x * r3.x);
-            const float4 r = make_float4(c, r3.x * c, r3.y, r3.z);
-            const int2 pq = jac_pair(k, step, M);
-            const float2 vp = v[pq.x], vq = v[pq.y];
-            const float2 ec = make_float2(r.z, -r.w);
-            const float2 d = make_float2(r.x * vq.x - r.y * vp.x, r.x * vq.y - r.y * vp.y);
-            v[pq.x] = make_float2(r.x * vp.x + r.y * vq.x, r.x * vp.y + r.y * vq.y);
-            v[pq.y] = cmul(ec, d);
-          };
-          int step = M - 1;
-          for (int st0 = steps - 1; st0 >= 0; st0 -= PF) {
-#pragma unroll
-            for (int u = 0; u < PF; ++u) {
-              const int st = st0 - u;
-              const float3 a = ra4[u], b = rb4[u];
-              ra4[u] = fetch(st - PF, ka);
-              rb4[u] = fetch(st - PF, kb);
-              if (st >= 0) {
-                rotate(a, ka, step);
-                rotate(b, kb, step);
-                __syncwarp();
-                step = step == 0 ? M - 1 : step - 1;
-              }
+            const int st = st0 - u;
+            const float3 a = ra4[u], b = rb4[u];
+            ra4[u] = fetch(st - PF, ka);
+            rb4[u] = fetch(st - PF, kb);
+            if (st >= 0) {
+              rotate(a, ka, step);
+              rotate(b, kb, step);
+              __syncwarp();
+              step = step == 0 ? M - 1 : step - 1;
             }
           }
-          for (int i = lane; i < n; i += 32) G[i * kFacCols + warp] = v[i];
-          if (lane == 0) G[n * kFacCols + warp] = make_float2(W->g[col], 0.f);
         }
+      };
+      if (ra > kColBatch) {
+        // W = J_1 ... J_steps diag(g) J_steps^H ... J_1^H: the rotations undone on the gains
+        for (int i = warp; i < n2; i += kJacThreads / 32)
+          for (int j = i + lane; j < n2; j += 32) A[row(i) + j] = make_float2(i == j && i < n ? W->g[i] : 0.f, 0.f);
+        int step = M - 1;
+        float t = 0.f, ex = 1.f, ey = 0.f;
+        auto fetch = [&](int st) {
+          if (tid >= half || st < 0) return;
+          const float* lg = log + 3 * (st * half + tid);
+          t = __ldcg(lg); ex = __ldcg(lg + 1); ey = __ldcg(lg + 2);
+        };
+        fetch(steps - 1);
+        for (int st = steps - 1; st >= 0; --st) {
+          if (tid < half) {
+            const float c = rsqrtf(1.f + t * t);
+            W->rot[tid] = make_float4(c, t * c, ex, ey);
+            W->pairs[tid] = jac_pair(tid, step, M);
+          }
+          fetch(st - 1);
+          __syncthreads();
+          update(std::true_type{});
+          __syncthreads();
+          step = step == 0 ? M - 1 : step - 1;
+        }
+        for (int i = warp; i < n; i += kJacThreads / 32)
+          for (int j = lane; j <= i; j += 32) {
+            const float2 w = A[row(j) + i];
+            G[i * (i + 1) / 2 + j] = make_float2(w.x, -w.y);
+          }
+        ra = kBlkW;
+      } else if (ra > kFacCols) {
+        // W = V diag(g) V^H from the columns themselves, four per warp
+        if (4 * warp < ra) columns(std::integral_constant<int, 4>{}, A + 4 * warp * n2, 4 * warp);
+        __syncthreads();
+        for (int i = warp; i < n; i += kJacThreads / 32)
+          for (int j = lane; j <= i; j += 32) {
+            float2 w = make_float2(0.f, 0.f);
+            for (int c = 0; c < ra; ++c) {
+              const float2 p = cmul_bc(A[c * n2 + i], A[c * n2 + j]);
+              const float gc = W->g[W->act[c]];
+              w.x = fmaf(gc, p.x, w.x);
+              w.y = fmaf(gc, p.y, w.y);
+            }
+            G[i * (i + 1) / 2 + j] = w;
+          }
+        ra = kBlkW;
+      } else if (ra > 0 && warp < ra) {
+        float2* v = A + warp * n2;
+        columns(std::integral_constant<int, 1>{}, v, warp);
+        for (int i = lane; i < n; i += 32) G[i * kFacCols + warp] = v[i];
+        if (lane == 0) G[n * kFacCols + warp] = make_float2(W->g[W->act[warp]], 0.f);
       }
     }
     if (tid == 0) {
       op.blk_ra[blk] = ra;
-      if (ra == -1) op.fb_list[atomicAdd(op.fb_count, 1)] = (int)blk;
+      if (ra == -1 || ra == kBlkW) op.fb_list[atomicAdd(op.fb_count, 1)] = (int)blk;
     }
     __syncthreads();
   }
@@ -295,8 +373,8 @@ __global__ void __launch_bounds__(kJacThreads, 4) llr_eig_jacobi_kernel(ProxOp o
 
 size_t jac_smem(int n) {
   const int n2 = (n + 1) & ~1;
-  // the packed matrix, at least the kept columns that follow it
-  return align16(sizeof(JacSmem)) + sizeof(float2) * std::max<size_t>((size_t)n2 * (n2 + 1) / 2, kFacCols * kProxMaxN);
+  // the packed matrix, or the columns that follow it (fewer from n2 = 64 on)
+  return align16(sizeof(JacSmem)) + sizeof(float2) * std::max<size_t>((size_t)n2 * (n2 + 1) / 2, (size_t)kColBatch * n2);
 }
 
 }  // namespace

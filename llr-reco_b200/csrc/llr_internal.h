@@ -77,6 +77,8 @@ __host__ __device__ inline long long jacobi_log_stride(int n) {
 
 // Kept eigenvectors per block that the warp eigen kernel hands to the apply kernel.
 constexpr int kFacCols = 8;
+// Block code in ProxOp::blk_ra (64 < n): more components kept than that, W = V diag(g) V^H in the Gram scratch.
+constexpr int kBlkW = -3;
 
 // Per-block scratch of the split prox path, in float2: the packed Gram matrix n(n+1)/2,
 // overwritten by the eigen factor (n x kFacCols eigenvectors, then kFacCols gains).

@@ -552,6 +552,28 @@ __device__ void apply_rows(const BlockSource& s, long long base, const RowTab* r
   }
 }
 
+// Offset, coordinates and (where the volumes share it) phase of every row of block `blk`.
+__device__ __forceinline__ void row_tables(const BlockSource& src, int m, long long blk, const int* sh, RowTab* rows,
+                                           float2* rowph) {
+  for (int r = threadIdx.x; r < m; r += blockDim.x) {
+    RowTab rt;
+    if (src.kind == 1) {
+      int ix, iy, iz;
+      block_row_coord(src, blk, sh, r, ix, iy, iz);
+      rt.off = (int)planar_index(src.g, ix, iy, iz, 0);
+      rt.cx = ix;
+      rt.cyz = iy | (iz << 16);
+      if (src.ph_uniform) rowph[r] = phase_at(src.ph, src.g, 0, ix, iy, iz);
+    } else {
+      rt.off = r;
+      rt.cx = 0;
+      rt.cyz = 0;
+    }
+    rt.pad = 0;
+    rows[r] = rt;
+  }
+}
+
 // Row tables of block `blk`, then its Gram matrix over staged row chunks (tile accumulators
 // in registers); every lower-or-upper element (i, j) < n is handed to sink(i, j, value).
 template <int NPMAX, int TG, class Sink>
@@ -559,24 +581,7 @@ __device__ void gram_block(const BlockSource& src, const TrdLayout& L, int m, in
                            long long base, long long qstride, const int* sh, RowTab* rows, float2* rowph,
                            float2* Cch, Sink sink) {
   const int tid = threadIdx.x;
-    // row tables
-    for (int r = tid; r < m; r += blockDim.x) {
-      RowTab rt;
-      if (src.kind == 1) {
-        int ix, iy, iz;
-        block_row_coord(src, blk, sh, r, ix, iy, iz);
-        rt.off = (int)planar_index(src.g, ix, iy, iz, 0);
-        rt.cx = ix;
-        rt.cyz = iy | (iz << 16);
-        if (src.ph_uniform) rowph[r] = phase_at(src.ph, src.g, 0, ix, iy, iz);
-      } else {
-        rt.off = r;
-        rt.cx = 0;
-        rt.cyz = 0;
-      }
-      rt.pad = 0;
-      rows[r] = rt;
-    }
+    row_tables(src, m, blk, sh, rows, rowph);
     // Gram over staged row chunks; tile accumulators stay in registers
     const int nt = (n + TG - 1) / TG;
     const int tiles = nt * nt;
@@ -925,28 +930,12 @@ __global__ void __launch_bounds__(kApplyThreads, 3) llr_apply_kernel(BlockSource
   const int sh[3] = {sh_s[0], sh_s[1], sh_s[2]};
   for (long long blk = blockIdx.x; blk < src.nblocks; blk += gridDim.x) {
     const int ra = op.blk_ra[blk];
-    // uniform over the CTA: fallback blocks (-1) belong to the Jacobi kernel; identity blocks (-2)
+    // uniform over the CTA: fallback blocks (-1, kBlkW) belong to the Jacobi kernel; identity blocks (-2)
     // stay in place unless the result goes to a separate output; zero blocks need no store when
     // deferred to the fused FFT or accumulated
-    if (ra == -1 || (ra == -2 && !src.out) || (ra == 0 && (op.defer_zero || src.accumulate))) continue;
+    if (ra == -1 || ra == kBlkW || (ra == -2 && !src.out) || (ra == 0 && (op.defer_zero || src.accumulate))) continue;
     const long long base = src.kind == 1 ? 0 : blk * (long long)m * n;
-    for (int r = tid; r < m; r += blockDim.x) {
-      RowTab rt;
-      if (src.kind == 1) {
-        int ix, iy, iz;
-        block_row_coord(src, blk, sh, r, ix, iy, iz);
-        rt.off = (int)planar_index(src.g, ix, iy, iz, 0);
-        rt.cx = ix;
-        rt.cyz = iy | (iz << 16);
-        if (src.ph_uniform) rowph[r] = phase_at(src.ph, src.g, 0, ix, iy, iz);
-      } else {
-        rt.off = r;
-        rt.cx = 0;
-        rt.cyz = 0;
-      }
-      rt.pad = 0;
-      rows[r] = rt;
-    }
+    row_tables(src, m, blk, sh, rows, rowph);
     if (ra > 0) {
       const float2* F = op.gram + blk * op.gram_stride;
       for (int i = tid; i < n * kFacCols; i += blockDim.x) Va[i] = F[i];
@@ -985,11 +974,11 @@ __global__ void __launch_bounds__(kApplyThreads, 3) llr_apply_kernel(BlockSource
 }
 
 // =======================================================================================
-// Casorati matrices with 64 < n <= 128 columns that the split path cannot finish (more kept
-// components than the warp eigen kernel holds, or a failed residual check), and every block
-// at that width for the Jacobi solver and the block statistics: Gram matrix over staged row
-// chunks into shared memory, cyclic Jacobi with the eigenvectors in a per-CTA global scratch
-// (L2-resident), W = V diag(g) V^H, C' = C W streamed over row chunks.  One CTA per SM.
+// Casorati matrices with 64 < n <= 128 columns that the split path cannot finish (not converged or not
+// finite), and every block at that width for the Jacobi solver and the block statistics: Gram matrix over
+// staged row chunks into shared memory, cyclic Jacobi with the eigenvectors in a per-CTA global scratch
+// (L2-resident), W = V diag(g) V^H, C' = C W streamed over row chunks.  One CTA per SM.  Blocks that
+// keep more components than a factor holds come with their W and only take the product.
 // =======================================================================================
 constexpr int kWideTG = 8;
 constexpr int kWideRows = 32;
@@ -1055,10 +1044,24 @@ __global__ void __launch_bounds__(kLlrThreads, 1) llr_prox_wide_kernel(BlockSour
   for (long long i = blockIdx.x; i < count; i += gridDim.x) {
     const long long blk = src.blk_list ? (long long)src.blk_list[i] : i;
     const long long base = src.kind == 1 ? 0 : blk * (long long)m * n;
-    for (int k = tid; k < ((n + 1) & ~1) * lda; k += blockDim.x) A[k] = make_float2(0.f, 0.f);
-    gram_block<NP, kWideTG>(src, W.t, m, n, blk, base, qstride, sh, rows, rowph, Cch,
-                            [&](int a, int b, float2 v) { A[a * lda + b] = v; });
-    if (!op.block_stat && op.mode != LLR_PROX_HARD_RANK && op.lambda > 0.f) {
+    // W from the eigen kernel (64 < n): only the product is left
+    const bool given = n > 64 && src.blk_list && op.blk_ra && op.blk_ra[blk] == kBlkW;
+    if (given) {
+      row_tables(src, m, blk, sh, rows, rowph);
+      const float2* G = op.gram + blk * op.gram_stride;
+      for (int a = tid >> 5; a < n; a += kLlrThreads / 32)
+        for (int b = tid & 31; b <= a; b += 32) {
+          const float2 v = G[a * (a + 1) / 2 + b];
+          A[a * lda + b] = v;
+          A[b * lda + a] = make_float2(v.x, a == b ? v.y : -v.y);
+        }
+      __syncthreads();
+    } else {
+      for (int k = tid; k < ((n + 1) & ~1) * lda; k += blockDim.x) A[k] = make_float2(0.f, 0.f);
+      gram_block<NP, kWideTG>(src, W.t, m, n, blk, base, qstride, sh, rows, rowph, Cch,
+                              [&](int a, int b, float2 v) { A[a * lda + b] = v; });
+    }
+    if (!given && !op.block_stat && op.mode != LLR_PROX_HARD_RANK && op.lambda > 0.f) {
       // ||G||_F <= lambda^2, or the trace bound lambda_max <= m + s sqrt(n - 1) (m = tr G / n,
       // s^2 = ||G||_F^2 / n - m^2; Wolkowicz & Styan 1980) <= lambda^2, puts every eigenvalue of
       // G = C^H C below the threshold: the output is zero, as the Jacobi path would make it (no kept
@@ -1085,29 +1088,32 @@ __global__ void __launch_bounds__(kLlrThreads, 1) llr_prox_wide_kernel(BlockSour
         continue;
       }
     }
-    jacobi<NP>(A, V, n, rot, pairs, misc, 20, lda);
-    if (op.block_stat) {
-      if (tid == 0) {
-        float mx = 0.f;
-        for (int k = 0; k < n; ++k) mx = fmaxf(mx, A[k * lda + k].x);
-        op.block_stat[blk] = mx;
+    bool identity = false;
+    if (!given) {
+      jacobi<NP>(A, V, n, rot, pairs, misc, 20, lda);
+      if (op.block_stat) {
+        if (tid == 0) {
+          float mx = 0.f;
+          for (int k = 0; k < n; ++k) mx = fmaxf(mx, A[k * lda + k].x);
+          op.block_stat[blk] = mx;
+        }
+        __syncthreads();
+        continue;
       }
-      __syncthreads();
-      continue;
+      singular_map(A, lda, n, op.mode, op.rank, op.lambda, ev, g, act, misc);
+      if (op.blk_nuc && op.mode != LLR_PROX_HARD_RANK && tid == 0) op.blk_nuc[blk] = nuclear_from_eigs(ev, n, op.lambda);
+      const int na = misc->n_active;
+      identity = na == n && op.mode == LLR_PROX_HARD_RANK;
+      if (identity && !src.out) {
+        __syncthreads();
+        continue;
+      }
+      if (na == 0 && src.accumulate) {
+        __syncthreads();
+        continue;
+      }
+      if (!identity) form_W(A, V, lda, n, g, act, na);
     }
-    singular_map(A, lda, n, op.mode, op.rank, op.lambda, ev, g, act, misc);
-    if (op.blk_nuc && op.mode != LLR_PROX_HARD_RANK && tid == 0) op.blk_nuc[blk] = nuclear_from_eigs(ev, n, op.lambda);
-    const int na = misc->n_active;
-    const bool identity = na == n && op.mode == LLR_PROX_HARD_RANK;
-    if (identity && !src.out) {
-      __syncthreads();
-      continue;
-    }
-    if (na == 0 && src.accumulate) {
-      __syncthreads();
-      continue;
-    }
-    if (!identity) form_W(A, V, lda, n, g, act, na);
     for (int c0 = 0; c0 < m; c0 += W.t.rc) {
       const int rc = min(W.t.rc, m - c0);
       for (int e = tid; e < rc * n; e += blockDim.x) {

@@ -8,7 +8,7 @@ import pytest
 from conftest import crandn, rel_err
 from oracle import llr_oracle as O
 
-from llr_b200 import DeviceBuffer, _lib as L
+from llr_b200 import DeviceBuffer, ReconContext, ReconParams, _lib as L
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +94,62 @@ def test_wide_gram_sums_keep_fp32_accuracy(gpu, m, n):
     exp = x.astype(np.complex128) * (1.0 - float(lam) / sv)
     assert rel_err(got[:, :6], exp[:, :6]) < 5e-6
     assert np.abs(got[:, 6:]).max() < 1e-6
+
+
+@pytest.mark.parametrize("m,n,k,batch", [(512, 106, 9, 3), (216, 80, 33, 5), (130, 128, 64, 2), (300, 65, 65, 3), (96, 71, 40, 700)])
+@pytest.mark.parametrize("mode", ["soft", "hard"])
+def test_wide_batch_keeping_more_than_a_factor_holds(gpu, mode, m, n, k, batch):
+    """Nine components, around one and two rounds of 32 columns, all of them (odd n), more blocks than CTAs: such blocks
+    get W from the eigen kernel and only the product from the wide one.  Tolerance as above."""
+    rng = np.random.default_rng(m + k)
+    x = _low_rank_mats(rng, m, n, k, batch, 1e-4)
+    d = DeviceBuffer.from_array(x)
+    if mode == "soft":
+        L.check(L.lib.llr_soft_threshold_batch_dev(m, n, 0.1, batch, d.ptr, None))
+        exp = O.low_rank_soft(x.astype(np.complex128), 0.1)
+    else:
+        L.check(L.lib.llr_low_rank_batch_dev(m, n, k, batch, d.ptr, None))
+        exp = O.low_rank_hard(x.astype(np.complex128), k)
+    got = d.download(np.empty_like(x, order="F"))
+    d.close()
+    assert rel_err(got[..., :batch - 1], exp[..., :batch - 1]) < 5e-5
+
+
+def _wide_ctx(gram_mode, lam=0.0, rank=0, stride=None, nq=70):
+    rng = np.random.default_rng(11)
+    vol = (16, 16, 16)
+    y = crandn(rng, vol + (nq,)) * (rng.random((1, 16, 16, nq)) < 0.5)
+    p = ReconParams(vol_size=vol, nq=nq, block_size=(8, 8, 8), prox_mode=0 if rank else 1, rank=max(rank, 1), lam=lam, seed=2,
+                    gram_mode=gram_mode, block_stride=stride)
+    ctx = ReconContext(p)
+    ctx.upload_kspace(np.asfortranarray(y.astype(np.complex64)))
+    ctx.init_zero_filled()
+    return ctx
+
+
+@pytest.mark.parametrize("stride", [None, (4, 8, 8)])
+def test_wide_context_with_many_kept_components(gpu, stride):
+    """Volume blocks, overlapping ones too (their results are accumulated), every component above the threshold: image,
+    residual and objective against the FP32 Gram mode, whose blocks all take the wide kernel.  Two FP32 paths of error 5e-5
+    each (prox tolerance); the objective's nuclear norms are sums of positive singular values."""
+    out = []
+    for gm in (0, 1):
+        with _wide_ctx(gm, lam=2.0, stride=stride) as ctx:
+            h = ctx.iterate(2)
+            out.append((ctx.download_image(), h, ctx.objective_history(2)))
+    assert rel_err(out[0][0], out[1][0]) < 1e-4
+    np.testing.assert_allclose(out[0][1], out[1][1], rtol=2e-4)
+    if stride is None:
+        np.testing.assert_allclose(out[0][2], out[1][2], rtol=2e-4)
+
+
+@pytest.mark.parametrize("kw", [dict(rank=12), dict(lam=2.0)])
+def test_wide_blocks_are_not_solved_twice(gpu, kw):
+    """A hard rank above eight, or a threshold that keeps more, against the FP32 Gram mode, where one kernel does all: with
+    the eigenproblem solved twice it took 1.3 times as long."""
+    ms = {}
+    for gm in (0, 1):
+        with _wide_ctx(gm, **kw) as ctx:
+            ctx.iterate(1)
+            ms[gm] = min(ctx.iterate_timed(2) for _ in range(5))
+    assert ms[0] < 1.1 * ms[1]
