@@ -423,7 +423,7 @@ int llr_ctx_create(const llr_config* cfg, llr_ctx** out) {
   if (cfg->subspace_rank == 0 && (c->g.nq > 64 || prox_needs_wide_fallback(c->m, c->g.nq))) {
     c->vwide_ctas = wide_jacobi_ctas();
     if ((st = dalloc(&c->d_vwide, (size_t)c->vwide_ctas * (size_t)wide_v_stride()))) return fail(st);
-    c->rot_ctas = (int)std::min<long long>(std::max<long long>(1, c->nblocks), (long long)kJacobiPerSm * c->vwide_ctas);
+    c->rot_ctas = (int)std::min<long long>(std::max<long long>(1, c->nblocks), jacobi_ctas(c->g.nq));
     if (c->g.nq > 64 && (st = dalloc(&c->d_rot_log, (size_t)c->rot_ctas * (size_t)jacobi_log_stride(c->g.nq))))
       return fail(st);
   }

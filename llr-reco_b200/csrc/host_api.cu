@@ -422,7 +422,11 @@ static int batch_prox(int m, int n, int mode, int rank, float lam, int batch, ll
   }
   float* rot_log = nullptr;
   if (gram && n > 64 && n <= kProxMaxN) {   // without the log every block takes the wide kernel
-    op.rot_ctas = (int)std::min<long long>(batch, (long long)kJacobiPerSm * wide_jacobi_ctas());
+    op.rot_ctas = (int)std::min<long long>(batch, jacobi_ctas(n));
+    // 474 MB at 106 columns: a call whose blocks are all zero took 4.2 ms instead of 0.4 when that was mapped each time
+    scratch_keep(sizeof(float) * (size_t)op.rot_ctas * (size_t)jacobi_log_stride(n) +
+                 sizeof(float2) * ((size_t)batch * (size_t)prox_gram_stride(n) + (size_t)op.vwide_ctas * (size_t)wide_v_stride()) +
+                 sizeof(int) * (2 * (size_t)batch + 2) + (16u << 20), s);
     if (scratch_alloc((void**)&rot_log, sizeof(float) * (size_t)op.rot_ctas * (size_t)jacobi_log_stride(n), s) != cudaSuccess) {
       cudaGetLastError();
       rot_log = nullptr;

@@ -379,6 +379,10 @@ size_t jac_smem(int n) {
 
 }  // namespace
 
+int jacobi_ctas(int n) {
+  return wide_jacobi_ctas() * (int)std::max<size_t>(1, std::min<size_t>(kJacobiPerSm, 228 * 1024 / (jac_smem(n) + 1024)));
+}
+
 int launch_llr_eig_jacobi(const ProxOp& op, long long nblocks, cudaStream_t stream) {
   if (!op.gram || !op.blk_ra || !op.fb_list || !op.fb_count || !op.rot_log || op.rot_ctas < 1)
     return set_error(LLR_ERR_INVALID, "eigen kernel needs the Gram scratch, block codes, fallback list and log");

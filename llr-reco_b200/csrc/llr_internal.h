@@ -67,9 +67,10 @@ constexpr int kProxMaxN = 128;
 constexpr int kJacobiLogSweeps = 12;   // sweeps the rotation log holds (a block of 106 columns converges in 7 to 9)
 __host__ __device__ inline long long wide_v_stride() { return (long long)kProxMaxN * (kProxMaxN + 1); }
 int wide_jacobi_ctas();   // CTAs of the wide Jacobi kernel on the current device
-// Rotation log of the split path's Jacobi kernel (64 < n <= 128), in floats per CTA; it runs at most
-// kJacobiPerSm wide_jacobi_ctas() CTAs.
+// Rotation log of the split path's Jacobi kernel (64 < n <= 128), in floats per CTA, and the CTAs that are resident at
+// once: as many as their shared memory allows, at most kJacobiPerSm per SM.
 constexpr int kJacobiPerSm = 4;
+int jacobi_ctas(int n);
 __host__ __device__ inline long long jacobi_log_stride(int n) {
   const int n2 = (n + 1) & ~1;
   return 3ll * kJacobiLogSweeps * (n2 - 1) * (n2 / 2);
@@ -153,6 +154,9 @@ int wavelet_denoise_strided(const WaveletPlan& p, float2* data, long long sx, lo
 
 // Stream-ordered scratch of one call (scratch.cu); release with cudaFreeAsync on the same stream.
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+// A call whose scratch takes `bytes` in all: the pool keeps up to that much (bounded) from now on, because mapping it again
+// on every call would cost more than the call (scratch.cu).
+void scratch_keep(size_t bytes, cudaStream_t s);
 void scratch_trim();   // unused scratch of the current device back to the driver
 cudaError_t device_alloc(void** p, size_t bytes);   // cudaMalloc, retried once without kept scratch
 

@@ -1,6 +1,7 @@
 """Casorati matrices of 65 to 128 columns: the split path (tensor-core Gram, Jacobi eigen kernel with a rotation
 log, apply kernel, wide kernel over the blocks handed back) against the FP64 oracle."""
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -153,3 +154,21 @@ def test_wide_blocks_are_not_solved_twice(gpu, kw):
             ctx.iterate(1)
             ms[gm] = min(ctx.iterate_timed(2) for _ in range(5))
     assert ms[0] < 1.1 * ms[1]
+
+
+def test_wide_scratch_is_not_mapped_on_every_call(gpu):
+    """600 blocks of 128 columns whose outputs are all zero against 100 of them: the rotation log (519 MB) outweighed what
+    the scratch pool kept and was mapped anew by every call, 85 times as long."""
+    best = {}
+    for batch in (100, 600):
+        x = _low_rank_mats(np.random.default_rng(1), 64, 128, 2, 1, 1e-3)
+        x = np.asfortranarray(np.broadcast_to(x, (64, 128, batch)))
+        d = DeviceBuffer.from_array(x)
+        for _ in range(8):
+            L.check(L.lib.llr_stream_sync(None))
+            t0 = time.perf_counter()
+            L.check(L.lib.llr_soft_threshold_batch_dev(64, 128, 100.0, batch, d.ptr, None))
+            L.check(L.lib.llr_stream_sync(None))
+            best[batch] = min(best.get(batch, 1.0), time.perf_counter() - t0)
+        d.close()
+    assert best[600] < 10 * best[100]
