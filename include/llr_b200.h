@@ -288,6 +288,9 @@ int llr_cu_dwt_denoise(llr_cf32* vol_data, const size_t vol_size[3], const float
 int llr_host_alloc(size_t bytes, void** out);
 int llr_host_free(void* p);
 int llr_device_alloc(size_t bytes, void** out);
+/* NULL: gives the scratch that the operators keep mapped on the current device between calls (256 MB at
+ * most, 768 MB after a batch of matrices of 65 to 128 columns) back to the driver; destroying a context
+ * or a network does so too. */
 int llr_device_free(void* p);
 int llr_memcpy_h2d(void* dst, const void* src, size_t bytes, void* stream);
 int llr_memcpy_d2h(void* dst, const void* src, size_t bytes, void* stream);

@@ -731,6 +731,7 @@ int llr_device_alloc(size_t bytes, void** out) {
 }
 int llr_device_free(void* p) {
   if (p) LLR_CUDA_TRY(cudaFree(p));
+  else scratch_trim();
   return LLR_OK;
 }
 int llr_memcpy_h2d(void* dst, const void* src, size_t bytes, void* stream) {

@@ -5,8 +5,9 @@
 // threshold 0), so an operator that allocated there mapped fresh pages on each call: the DTI fit's
 // 2 KB table made a 0.62 ms call take 1.0-2.9 ms.  The private pool keeps at most kKeepBytes of
 // unused memory mapped (kKeepMost once a call has asked for it, see scratch_keep); what is above it goes
-// back at the next synchronisation, all of it when a context or a network is destroyed, or when an
-// allocation of the library runs out of memory.
+// back at the next synchronisation, all of it when a context or a network is destroyed, when a caller of the
+// operators alone asks for it (llr_device_free of a null pointer), or when an allocation of the library
+// runs out of memory.
 // Allocation and free are stream-ordered, so calls on several streams and threads never share a
 // block at the same time.
 #include <mutex>
