@@ -607,61 +607,64 @@ int launch_llr_prox_subspace(const BlockSource& src, const SubspaceOp& op, cudaS
 // =======================================================================================
 namespace {
 
-// Bound: HBM, one read and one write of every element.  A CTA handles one block and a slice of its
-// volumes: the voxel offsets of a chunk of rows are computed once into shared memory (all the index
-// divisions there are), then matrix elements go by in storage order, eight in flight per thread.  With
-// three 64-bit divisions per element the kernel was issue-bound: 315 us for 4096 blocks of 216 x 61 on
-// 96 x 96 x 48 x 61 (0.43 GB moved), now about 115 us (lift, rank truncation and un-lift 1617 -> 1213 us).
-constexpr int kLiftRows = 1024;   // rows per chunk (8 KB of offsets)
+// Bound: HBM, one read and one write of every element.  A CTA takes up to kLiftRows consecutive rows of the matrices, of one
+// block or of many, and a slice of the volumes: the rows' voxel and matrix offsets are computed once into shared
+// memory (all the index divisions there are), then the elements go by volume after volume, eight in flight per thread.
+// With three 64-bit divisions per element the kernel was issue-bound: 315 us for 4096 blocks of 216 x 61 on
+// 96 x 96 x 48 x 61 (0.43 GB moved), about 100 us this way (lift, rank truncation and un-lift 1617 -> 1213 us).
+// A CTA per block in place of one per row chunk took that long for those blocks too, but 853 us for 2^3 blocks
+// of one 128^3 volume and 12.5 ms for a single 256 x 256 x 64 block of three (divisions everywhere: 37 and
+// 158 us): 36 and 79 us this way.
+constexpr int kLiftRows = 1024;   // most rows per chunk (16 KB of offsets)
 
-template <int DIR>
+// QFAST: volumes run fastest over a slice's elements, else rows.  U: unsigned where every row and block index fits.
+template <int DIR, bool QFAST, class U>
 __global__ void __launch_bounds__(256) lift_kernel(float2* __restrict__ vol, float2* __restrict__ mat, int nx, int ny,
                                                    int nz, int nq, int bx, int by, int bz, int gx, int gy, int sx,
-                                                   int sy, int sz, long long start, long long n, int qper) {
-  __shared__ long long off[kLiftRows];
+                                                   int sy, int sz, long long start, long long n, int qper, int rc) {
+  __shared__ long long off[kLiftRows], moff[kLiftRows];
   constexpr int LB = 8;
-  const long long m = (long long)bx * by * bz, V = (long long)nx * ny * nz;
+  const U m = (U)bx * by * bz;
+  const long long V = (long long)nx * ny * nz, total = (long long)m * n;
   const int q0 = blockIdx.y * qper, q1 = min(nq, q0 + qper);
-  for (long long c = blockIdx.x; c < n; c += gridDim.x) {
-    const long long blk = start + c;
-    const int gxi = (int)(blk % gx);
-    const long long t = blk / gx;
-    const int gyi = (int)(t % gy), gzi = (int)(t / gy);
-    for (long long r0 = 0; r0 < m; r0 += kLiftRows) {
-      const int rows = (int)(m - r0 < kLiftRows ? m - r0 : kLiftRows);
-      __syncthreads();
-      for (int i = threadIdx.x; i < rows; i += 256) {
-        const long long r = r0 + i;
-        const int rx = (int)(r % bx);
-        const long long t2 = r / bx;
-        const int ry = (int)(t2 % by), rz = (int)(t2 / by);
-        const int ix = (gxi * bx + sx + rx) % nx, iy = (gyi * by + sy + ry) % ny, iz = (gzi * bz + sz + rz) % nz;
-        off[i] = (long long)ix + (long long)nx * ((long long)iy + (long long)ny * iz);
-      }
-      __syncthreads();
-      // element e of the slice: row e % rows of volume q0 + e / rows, stepped without divisions
-      const int dq = 256 / rows, dr = 256 - dq * rows;
-      int q = q0 + (int)threadIdx.x / rows, r = (int)threadIdx.x % rows;
-      float2* mb = mat + c * m * nq + r0;
-      while (q < q1) {
-        float2 v[LB];
-        long long va[LB], ma[LB];
+  for (long long r0 = (long long)blockIdx.x * rc; r0 < total; r0 += (long long)gridDim.x * rc) {
+    const int rows = (int)min((long long)rc, total - r0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < rows; i += 256) {
+      const U g = (U)(r0 + i), c = g / m, r = g - c * m;
+      const U blk = (U)start + c, t = blk / (U)gx, t2 = r / (U)bx;
+      const int gxi = (int)(blk - t * gx), gzi = (int)(t / (U)gy), gyi = (int)(t - (U)gzi * gy);
+      const int rx = (int)(r - t2 * bx), rz = (int)(t2 / (U)by), ry = (int)(t2 - (U)rz * by);
+      const int ix = (gxi * bx + sx + rx) % nx, iy = (gyi * by + sy + ry) % ny, iz = (gzi * bz + sz + rz) % nz;
+      off[i] = (long long)ix + (long long)nx * ((long long)iy + (long long)ny * iz);
+      moff[i] = (long long)c * m * nq + r;
+    }
+    __syncthreads();
+    // the slice's elements, stepped without divisions
+    const int nf = QFAST ? q1 - q0 : rows, ns = QFAST ? rows : q1 - q0;
+    const int ds = 256 / nf, df = 256 - ds * nf;
+    int f = (int)threadIdx.x % nf, sl = (int)threadIdx.x / nf;
+    while (sl < ns) {
+      float2 v[LB];
+      long long va[LB], ma[LB];
 #pragma unroll
-        for (int u = 0; u < LB; ++u) {
-          va[u] = q < q1 ? off[r] + V * q : -1;
-          ma[u] = r + m * q;
-          if (va[u] >= 0) v[u] = DIR == 0 ? vol[va[u]] : mb[ma[u]];
-          r += dr;
-          q += dq;
-          if (r >= rows) { r -= rows; ++q; }
+      for (int u = 0; u < LB; ++u) {
+        const int r = QFAST ? sl : f, q = q0 + (QFAST ? f : sl);
+        va[u] = sl < ns ? off[r] + V * q : -1;
+        if (va[u] >= 0) {
+          ma[u] = moff[r] + (long long)m * q;
+          v[u] = DIR == 0 ? vol[va[u]] : mat[ma[u]];
         }
-#pragma unroll
-        for (int u = 0; u < LB; ++u)
-          if (va[u] >= 0) {
-            if (DIR == 0) mb[ma[u]] = v[u];
-            else vol[va[u]] = v[u];
-          }
+        f += df;
+        sl += ds;
+        if (f >= nf) { f -= nf; ++sl; }
       }
+#pragma unroll
+      for (int u = 0; u < LB; ++u)
+        if (va[u] >= 0) {
+          if (DIR == 0) mat[ma[u]] = v[u];
+          else vol[va[u]] = v[u];
+        }
     }
   }
 }
@@ -675,14 +678,26 @@ int launch_lift(const float2* vol, float2* mat, const int* vs, int nq, const int
   const long long tot = (long long)bs[0] * bs[1] * bs[2] * nq * n;
   if (tot == 0) return LLR_OK;
   if (tot < 0) return set_error(LLR_ERR_INVALID, "negative block count");
-  // at least sixteen CTAs per SM where the block count alone does not give them: the volumes are split
-  const long long want = n < 148 * 16 ? std::min<long long>(nq, (148 * 16 + n - 1) / n) : 1;
+  // rows per chunk: with few volumes a thread needs 1024 for four loads in flight (one 128^3 volume 36 us, 42 with 512),
+  // with more 512 (64^3 x 16 29 us, 38 with 1024); 256 where the call is too small for two CTAs per SM
+  const long long rows = (long long)bs[0] * bs[1] * bs[2] * n;
+  const int rc = rows * nq < 148ll * 2 * 512 ? 256 : nq < 4 ? kLiftRows : 512;
+  const long long chunks = (rows + rc - 1) / rc;
+  // at least sixteen CTAs per SM where the rows alone do not give them: the volumes are split
+  const long long want = chunks < 148 * 16 ? std::min<long long>(nq, (148 * 16 + chunks - 1) / chunks) : 1;
   const int qper = (int)((nq + want - 1) / want);
-  dim3 grid((unsigned)std::min<long long>(n, 1ll << 30), (unsigned)((nq + qper - 1) / qper));
+  dim3 grid((unsigned)std::min<long long>(chunks, 1ll << 30), (unsigned)((nq + qper - 1) / qper));
+  const bool narrow = rows < (1ll << 31) && start >= 0 && start + n < (1ll << 31);
+  // where a matrix has only one to three rows, a column's stores are single elements: 96^3 x 61 in 1^3 blocks took
+  // 846 us with rows fastest, 309 with volumes fastest
+  const bool qfast = (long long)bs[0] * bs[1] * bs[2] < 4;
+  using u64 = unsigned long long;
+  auto kern = dir == 1 ? (narrow ? lift_kernel<1, false, unsigned> : lift_kernel<1, false, u64>)
+              : qfast  ? (narrow ? lift_kernel<0, true, unsigned> : lift_kernel<0, true, u64>)
+                       : (narrow ? lift_kernel<0, false, unsigned> : lift_kernel<0, false, u64>);
   note_launch();
-  (dir == 0 ? lift_kernel<0> : lift_kernel<1>)<<<grid, 256, 0, s>>>(const_cast<float2*>(vol), mat, vs[0], vs[1], vs[2],
-                                                                    nq, bs[0], bs[1], bs[2], g[0], g[1], sh[0], sh[1],
-                                                                    sh[2], start, n, qper);
+  kern<<<grid, 256, 0, s>>>(const_cast<float2*>(vol), mat, vs[0], vs[1], vs[2], nq, bs[0], bs[1], bs[2], g[0], g[1], sh[0],
+                            sh[1], sh[2], start, n, qper, rc);
   LLR_CUDA_TRY(cudaGetLastError());
   return LLR_OK;
 }

@@ -492,3 +492,57 @@ def test_subspace_construction_matches_oracle(gpu):
     P, Pe = S.astype(np.complex128) @ S.conj().T.astype(np.complex128), Se @ Se.conj().T
     assert np.linalg.norm(P - Pe) < 1e-6
     np.testing.assert_allclose(S.real, Se.real, atol=1e-6)   # same sign convention
+
+
+def _lift_us(vs, nq, bs, reps=8):
+    import time
+    n = int(np.prod([v // b for v, b in zip(vs, bs)]))
+    m = int(np.prod(bs))
+    vol, mat = DeviceBuffer(8 * int(np.prod(vs)) * nq), DeviceBuffer(8 * m * nq * n)
+    best = {}
+    for _ in range(reps):
+        for k, f in (("lift", L.lib.llr_lift_data_set_dev), ("un_lift", L.lib.llr_un_lift_data_set_dev)):
+            L.check(L.lib.llr_stream_sync(None))
+            t0 = time.perf_counter()
+            L.check(f(vol.ptr, nq, mat.ptr, L.i32x3(vs), L.i32x3(bs), L.i32x3((1, 0, 2)), 0, n, None))
+            L.check(L.lib.llr_stream_sync(None))
+            best[k] = min(best.get(k, 1.0), time.perf_counter() - t0)
+    vol.close()
+    mat.close()
+    return best
+
+
+@pytest.mark.parametrize("vs,nq,bs", [((128, 128, 128), 1, (2, 2, 2)), ((256, 256, 64), 3, (256, 256, 64))])
+def test_lift_time_does_not_depend_on_the_block_size(gpu, vs, nq, bs):
+    """Tiny blocks, and one block of the whole volume, against 8^3 blocks of the same volume (as many bytes): a CTA per block
+    made them 20 and 200 times as long."""
+    ref, got = _lift_us(vs, nq, (8, 8, 8)), _lift_us(vs, nq, bs)
+    for k in ref:
+        assert got[k] < 4 * ref[k], (k, got[k], ref[k])
+
+
+@pytest.mark.parametrize("vs,nq,bs,start,n", [((10, 9, 7), 5, (2, 1, 3), 3, 61), ((13, 11, 9), 3, (1, 1, 1), 0, 1287),
+                                              ((31, 17, 11), 2, (31, 17, 11), 0, 1), ((24, 18, 12), 7, (5, 7, 3), 2, 9),
+                                              ((16, 16, 33), 1, (8, 8, 8), 0, 16)])
+def test_lift_row_chunks_match_oracle(gpu, vs, nq, bs, start, n):
+    """Chunks of 512 rows that span many blocks, end inside one, or are part of one; a range of blocks; odd sizes.
+    Exact copies both ways, and what no block covers stays."""
+    rng = np.random.default_rng(sum(vs))
+    x = crandn(rng, vs + (nq,))
+    sh = tuple(int(v) for v in rng.integers(0, vs))
+    m = int(np.prod(bs))
+    exp = O.lift_data_set(x, bs, sh, start, n)
+    vol, mat = DeviceBuffer.from_array(np.asfortranarray(x)), DeviceBuffer(8 * m * nq * n)
+    args = (L.i32x3(vs), L.i32x3(bs), L.i32x3(sh), start, n, None)
+    L.check(L.lib.llr_lift_data_set_dev(vol.ptr, nq, mat.ptr, *args))
+    got = mat.download(np.empty((m, nq, n), np.complex64, order="F"))
+    assert np.array_equal(got, exp)
+    y = np.asfortranarray(crandn(rng, (m, nq, n)))
+    mat.upload(y)
+    L.check(L.lib.llr_un_lift_data_set_dev(vol.ptr, nq, mat.ptr, *args))
+    back = vol.download(np.empty(vs + (nq,), np.complex64, order="F"))
+    ref = np.asfortranarray(x.copy())
+    O.un_lift_data_set(ref, y, bs, sh, start, n)
+    assert np.array_equal(back, ref)
+    vol.close()
+    mat.close()
