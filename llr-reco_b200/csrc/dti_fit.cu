@@ -97,6 +97,25 @@ __device__ __forceinline__ void add_samples(const float2 (&z)[2][QB], const floa
       r[h][u] = z[h][u].x * z[h][u].x + z[h][u].y * z[h][u].y;
       fast = fast && r[h][u] >= lo2[h];
     }
+  if (!fast) {   // nothing out of range but zeros: their terms are added here, and an infinity in their place adds ln 1
+    fast = true;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int u = 0; u < QB; ++u) fast = fast && (r[h][u] >= lo2[h] || r[h][u] == 0.f);
+    if (fast) {
+      const float ln_tiny = 2.f * logf(FLT_MIN);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < QB; ++u)
+          if (r[h][u] == 0.f) {
+            r[h][u] = INFINITY;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) dt[h][k] = fmaf(w[8 * u + k], ln_tiny, dt[h][k]);
+          }
+    }
+  }
   if (fast) {
 #pragma unroll
     for (int h = 0; h < 2; ++h)
@@ -129,7 +148,9 @@ __device__ __forceinline__ void add_samples(const float2 (&z)[2][QB], const floa
 // per thread before the first logarithm, and a row of the weights (two shared loads) serves both voxels.
 // Calls at that size: 625 us with a square root, a division and a logf per sample, one load at a time and
 // IEEE rotations; 485 us with ln_normal and the one-division rotations; 433 us with one range check per
-// batch instead of per sample; 409 us at four CTAs per SM (64 registers) instead of three.
+// batch instead of per sample; 409 us at four CTAs per SM (64 registers) instead of three.  Half of the volume masked
+// to zero: 1290 us with the ratios formed one by one, 500 to 550 us with the zeros' terms added apart (two forms
+// unrolled side by side took 500 too but 412 to 460 us without zeros).
 __global__ void __launch_bounds__(256, 4) dti_fit_kernel(const float2* __restrict__ dwi, const float2* __restrict__ b0,
                                                       long long V, int nq, int nb0, const float* __restrict__ pinv,
                                                       float* __restrict__ out) {

@@ -96,3 +96,59 @@ def test_dti_fit_edges_and_extreme_scales(gpu, V, nq, scale):
     exp = O.dti_fit(dwi.astype(np.complex128), b0.astype(np.complex128), b, g)
     for k in ("b0av", "e1", "e2", "e3", "md", "rd"):
         assert rel_err(got[k], exp[k]) < 1e-4, k
+
+
+def _masked(V, nq, nb0, rng):
+    """Background of exact zeros in runs of 24 voxels, and single zero samples inside."""
+    g = rng.standard_normal((nq, 3))
+    g /= np.linalg.norm(g, axis=1, keepdims=True)
+    s0 = rng.uniform(0.5, 1.0, (V, 1)) * np.ones((1, nb0))
+    dwi = s0[:, :1] * np.exp(-1000.0 * rng.uniform(0.2e-3, 2e-3, (V, nq))) * np.exp(1j * rng.uniform(0, 6, (V, nq)))
+    out = (np.arange(V) // 24) % 2 == 0
+    dwi[out] = 0
+    s0[out] = 0
+    dwi[rng.random((V, nq)) < 0.01] = 0
+    return dwi.astype(np.complex64), s0.astype(np.complex64), np.full(nq, 1000.0), g
+
+
+def test_dti_fit_zero_samples_match_oracle(gpu):
+    """Exact zeros clamp to the smallest normal number, in voxels with signal and in the background, where b0 is zero
+    too.  The logarithm of that number is exact to a few roundings: the phantom test's 1e-4."""
+    rng = np.random.default_rng(6)
+    dwi, b0, b, g = _masked(1500, 19, 2, rng)
+    got = _fit(dwi, b0, b, g)
+    exp = O.dti_fit(dwi.astype(np.complex128), b0.astype(np.complex128), b, g)
+    for k in ("b0av", "e1", "e2", "e3", "md", "rd"):
+        assert rel_err(got[k], exp[k]) < 1e-4, k
+
+
+def test_dti_fit_masked_volume_is_not_slower(gpu):
+    """A volume that is half background of exact zeros against one without any: each batch with a zero formed its ratios
+    one by one, 3.3 times as long."""
+    import time
+    from llr_b200 import DeviceBuffer, _lib as L
+    rng = np.random.default_rng(7)
+    V, nq = 1 << 20, 48
+    _, _, b, g = _masked(8, nq, 1, rng)
+    bb, gg = np.ascontiguousarray(b, np.float32), np.ascontiguousarray(g, np.float32)
+    x = np.full((V, nq), 0.5, np.complex64, order="F")
+    s0 = np.ones((V, 1), np.complex64, order="F")
+    out = DeviceBuffer(4 * 7 * V)
+    us = []
+    for mask in (False, True):
+        if mask:
+            x[(np.arange(V) // 96) % 2 == 0] = 0
+            s0[(np.arange(V) // 96) % 2 == 0] = 0
+        dx, db = DeviceBuffer.from_array(x), DeviceBuffer.from_array(s0)
+        best = 1.0
+        for _ in range(10):
+            L.check(L.lib.llr_stream_sync(None))
+            t0 = time.perf_counter()
+            L.check(L.lib.llr_dti_fit_dev(dx.ptr, nq, db.ptr, 1, V, L.fptr(bb), L.fptr(gg), out.ptr, None))
+            L.check(L.lib.llr_stream_sync(None))
+            best = min(best, time.perf_counter() - t0)
+        us.append(best)
+        dx.close()
+        db.close()
+    out.close()
+    assert us[1] < 1.5 * us[0]
