@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256, 4) dti_fit_kernel(const float2* __restric
       s0c[h] = fmaxf(s0[h], FLT_MIN);
       const bool in_range = s0c[h] >= 1e-15f && s0c[h] <= 1e15f;
       inv2[h] = in_range ? 1.f / (s0c[h] * s0c[h]) : 0.f;
-      lo2[h] = in_range ? fmaxf(1e-30f * (s0c[h] * s0c[h]), FLT_MIN) : INFINITY;
+      lo2[h] = in_range ? fmaxf(1e-30f * (s0c[h] * s0c[h]), FLT_MIN) : NAN;   // no sample compares with it, infinite ones included
 #pragma unroll
       for (int j = 0; j < 6; ++j) dt[h][j] = 0.f;
     }

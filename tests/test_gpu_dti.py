@@ -152,3 +152,17 @@ def test_dti_fit_masked_volume_is_not_slower(gpu):
         db.close()
     out.close()
     assert us[1] < 1.5 * us[0]
+
+
+def test_dti_fit_infinite_reference(gpu):
+    """With an infinite b0 every ratio clamps to the smallest normal number, finite / infinite and infinite / infinite
+    alike (the maximum of NaN and a number is the number), so the maps are those of zero samples."""
+    rng = np.random.default_rng(9)
+    _, _, b, g = _masked(8, 16, 1, rng)
+    V = 1024
+    b0 = np.full((V, 1), np.inf, np.complex64)
+    got = [_fit(np.full((V, 16), v, np.complex64), b0, b, g) for v in (0.0, 1.0, np.inf)]
+    for k in ("e1", "e2", "e3", "md"):
+        assert np.isfinite(got[0][k]).all()
+        np.testing.assert_allclose(got[1][k], got[0][k], rtol=1e-4, atol=1e-6 * np.abs(got[0]["e1"]).max())
+        np.testing.assert_allclose(got[2][k], got[0][k], rtol=1e-4, atol=1e-6 * np.abs(got[0]["e1"]).max())
