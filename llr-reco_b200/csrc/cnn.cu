@@ -1091,7 +1091,7 @@ int conv_inst(const float* x, const uint16_t* w, const float* b, const float* ad
   if (CIN % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) != 0)
     return set_error(LLR_ERR_INVALID, "conv3d input must be 16-byte aligned for %d channels", CIN);
   auto k = conv3d_tc_kernel<CIN, COUT>;
-  LLR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LLR_CUDA_TRY(allow_smem(k));
   int dev = 0, nsm = 0;
   LLR_CUDA_TRY(cudaGetDevice(&dev));
   LLR_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -1115,7 +1115,7 @@ int conv_run_inst(const float* x, const uint16_t* w, const float* b, const float
   if (CIN % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) != 0)
     return set_error(LLR_ERR_INVALID, "conv3d input must be 16-byte aligned for %d channels", CIN);
   auto k = conv3d_run_kernel<CIN, COUT>;
-  LLR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LLR_CUDA_TRY(allow_smem(k));
   int dev = 0, nsm = 0;
   LLR_CUDA_TRY(cudaGetDevice(&dev));
   LLR_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -1159,7 +1159,7 @@ int wgrad_inst(const float* x, const float* dy, float* part, long long part_cap,
       (COUT % 4 == 0 && (reinterpret_cast<uintptr_t>(dy) & 15) != 0))
     return set_error(LLR_ERR_INVALID, "conv3d weight gradient needs 16-byte aligned activations");
   auto k = conv3d_wgrad_tc_kernel<CIN, COUT>;
-  LLR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LLR_CUDA_TRY(allow_smem(k));
   int dev = 0, nsm = 0;
   LLR_CUDA_TRY(cudaGetDevice(&dev));
   LLR_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));

@@ -289,7 +289,7 @@ int llr_dti_fit_dev(const llr_cf32* d_dwi, int32_t nq, const llr_cf32* d_b0, int
   cudaError_t e = cudaMemcpyAsync(d_pinv, pinv.data(), sizeof(float) * pinv.size(), cudaMemcpyHostToDevice, s);
   const size_t smem = sizeof(float) * 8 * (size_t)nq;
   if (e == cudaSuccess && smem > 48 * 1024)
-    e = cudaFuncSetAttribute(dti_fit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(dti_fit_kernel);
   if (e == cudaSuccess) {
     const long long blocks = std::min<long long>((n_vox + 511) / 512, 148LL * 32);
     note_launch();

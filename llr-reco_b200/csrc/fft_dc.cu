@@ -477,7 +477,7 @@ int launch_fft_dc(float2* u, const float2* yhat, const int* pos, const long long
   a.y1 = c.y1; a.y2 = c.y2; a.z1 = c.z1; a.z2 = c.z2;
   a.pitch = g.ny | 1;
   const size_t smem = fft_dc_smem(g.ny, g.nz, a.pitch);
-  LLR_CUDA_TRY(cudaFuncSetAttribute(c.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LLR_CUDA_TRY(allow_smem(c.kern));
   LLR_CUDA_TRY(cudaFuncSetAttribute(c.kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   if (grid < 1) return set_error(LLR_ERR_INVALID, "fused FFT: empty grid");
   note_launch();

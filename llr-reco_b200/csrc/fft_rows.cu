@@ -332,7 +332,7 @@ int resident_grid(K kern, int threads, size_t sm, long long items, int* grid) {
   int dev = 0, nsm = 0, occ = 0;
   LLR_CUDA_TRY(cudaGetDevice(&dev));
   LLR_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  LLR_CUDA_TRY(allow_smem(kern));
   LLR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, sm));
   if (occ < 1) return set_error(LLR_ERR_UNSUPPORTED, "row / column FFT kernel needs %zu B of shared memory", sm);
   *grid = (int)std::max<long long>(1, std::min<long long>(items, (long long)nsm * occ));

@@ -390,7 +390,7 @@ int launch_llr_eig_jacobi(const ProxOp& op, long long nblocks, cudaStream_t stre
   if (nblocks == 0) return LLR_OK;
   auto kern = llr_eig_jacobi_kernel;
   const size_t smem = jac_smem(op.n);
-  LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LLR_CUDA_TRY(allow_smem(kern));
   LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   LLR_CUDA_TRY(cudaMemsetAsync(op.blk_ra + nblocks, 0, sizeof(int), stream));
   note_launch();

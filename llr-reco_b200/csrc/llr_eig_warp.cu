@@ -561,7 +561,7 @@ template <int NPMAX>
 int launch_eig_warp_instance(const ProxOp& op, long long nblocks, cudaStream_t stream) {
   const size_t smem = sizeof(WarpEig<NPMAX>) * kEigWarps;
   auto kern = llr_eig_warp_kernel<NPMAX>;
-  LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LLR_CUDA_TRY(allow_smem(kern));
   LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   int dev = 0, nsm = 0, occ = 0;
   LLR_CUDA_TRY(cudaGetDevice(&dev));

@@ -443,7 +443,7 @@ int launch_gram_instance(const BlockSource& src, const ProxOp& op, cudaStream_t 
   TcLayout L = make_tc_layout<NPMAX>(op.m, op.n, S);
   if (L.total > 227 * 1024) return set_error(LLR_ERR_UNSUPPORTED, "tensor-core Gram needs %zu B smem", L.total);
   auto kern = llr_gram_tc_kernel<NPMAX, S, PH>;
-  LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+  LLR_CUDA_TRY(allow_smem(kern));
   LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   int dev = 0, nsm = 0, smem_sm = 0, regs_sm = 0;
   LLR_CUDA_TRY(cudaGetDevice(&dev));

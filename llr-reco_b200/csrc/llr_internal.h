@@ -11,6 +11,18 @@ namespace llr {
 
 constexpr int kLlrThreads = 256;
 
+// Lets a kernel take all the dynamic shared memory a CTA can have.  The limit belongs to the function, not to the launch: a
+// caller that set it to its own size would make another thread's larger launch of the same kernel fail.
+template <class K>
+inline cudaError_t allow_smem(K* kern) {
+  cudaFuncAttributes fa;
+  const cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+  if (e != cudaSuccess) return e;
+  const int most = 227 * 1024 - (int)fa.sharedSizeBytes;
+  if (fa.maxDynamicSharedSizeBytes >= most) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 // Where the Casorati matrices of one prox launch come from and go to.
 struct BlockSource {
   int kind;            // 0: contiguous (m, n, batch) matrices; 1: planar volume blocks

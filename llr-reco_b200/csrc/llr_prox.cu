@@ -107,7 +107,7 @@ int launch_jacobi_instance(const BlockSource& src, const ProxOp& op, cudaStream_
     return set_error(LLR_ERR_UNSUPPORTED, "Casorati %dx%d needs %zu B of shared memory (max 232448)", op.m, op.n,
                      L.total);
   auto kern = llr_prox_jacobi_kernel<NPMAX, TG>;
-  LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+  LLR_CUDA_TRY(allow_smem(kern));
     LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   int dev = 0, nsm = 0, occ = 0;
   LLR_CUDA_TRY(cudaGetDevice(&dev));
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(32 * kCoefWarps, 5) llr_coef_warp_kernel(Block
 
 int launch_coef_warp(const BlockSource& src, const SubspaceOp& op, cudaStream_t stream) {
   const size_t sm = sizeof(CoefWarp) * kCoefWarps + sizeof(unsigned short) * 4 * (size_t)op.m;
-  LLR_CUDA_TRY(cudaFuncSetAttribute(llr_coef_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  LLR_CUDA_TRY(allow_smem(llr_coef_warp_kernel));
   int occ = 0;
   LLR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, llr_coef_warp_kernel, 32 * kCoefWarps, sm));
   if (occ < 1) return set_error(LLR_ERR_UNSUPPORTED, "coefficient kernel cannot be resident (smem %zu B)", sm);
@@ -524,7 +524,7 @@ template <int KM>
 int launch_subspace_project(const BlockSource& src, const SubspaceOp& op, cudaStream_t stream) {
   const size_t sm = sizeof(float4) * (size_t)op.nq * KM;
   auto kern = src.ph_uniform ? subspace_project_kernel<KM, true> : subspace_project_kernel<KM, false>;
-  if (sm > 48 * 1024) LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (sm > 48 * 1024) LLR_CUDA_TRY(allow_smem(kern));
   int occ = 0;
   LLR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, sm));
   if (occ < 1) return set_error(LLR_ERR_UNSUPPORTED, "subspace projection needs %zu B smem", sm);
@@ -587,7 +587,7 @@ int launch_llr_prox_subspace(const BlockSource& src, const SubspaceOp& op, cudaS
   // per-thread coefficient registers sized to the rank class (fewer registers, more CTAs per SM)
   auto kern = op.coef_out ? llr_coef_low_rank_kernel<16>
                           : (op.srank <= 8 ? llr_subspace_kernel<16, 8> : llr_subspace_kernel<16, 16>);
-  LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+  LLR_CUDA_TRY(allow_smem(kern));
     LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   int dev = 0, nsm = 0, occ = 0;
   LLR_CUDA_TRY(cudaGetDevice(&dev));

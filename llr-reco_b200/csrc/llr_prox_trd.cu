@@ -771,7 +771,7 @@ int launch_trd_instance(const BlockSource& src, const ProxOp& op, cudaStream_t s
   if (L.total > 227 * 1024)
     return set_error(LLR_ERR_UNSUPPORTED, "Casorati %dx%d needs %zu B of shared memory", op.m, op.n, L.total);
   auto kern = llr_prox_trd_kernel<NPMAX, TG>;
-  LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+  LLR_CUDA_TRY(allow_smem(kern));
     LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   int dev = 0, nsm = 0, occ = 0;
   LLR_CUDA_TRY(cudaGetDevice(&dev));
@@ -1142,7 +1142,7 @@ int launch_prox_wide(const BlockSource& src, const ProxOp& op, cudaStream_t stre
   const WideLayout W = make_wide_layout(op.m, op.n);
   if (W.total > 227 * 1024)
     return set_error(LLR_ERR_UNSUPPORTED, "Casorati %dx%d needs %zu B of shared memory", op.m, op.n, W.total);
-  LLR_CUDA_TRY(cudaFuncSetAttribute(llr_prox_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W.total));
+  LLR_CUDA_TRY(allow_smem(llr_prox_wide_kernel));
   const long long grid = std::min<long long>(src.blk_list ? op.vwide_ctas : src.nblocks, op.vwide_ctas);
   if (grid < 1) return LLR_OK;
   note_launch();
@@ -1154,7 +1154,7 @@ int launch_prox_wide(const BlockSource& src, const ProxOp& op, cudaStream_t stre
 int launch_apply(const BlockSource& src, const ProxOp& op, cudaStream_t stream) {
   const ApplyLayout L = make_apply_layout(op.m, op.n);
   if (L.total > 227 * 1024) return set_error(LLR_ERR_UNSUPPORTED, "apply kernel needs %zu B smem", L.total);
-  LLR_CUDA_TRY(cudaFuncSetAttribute(llr_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+  LLR_CUDA_TRY(allow_smem(llr_apply_kernel));
   // shared memory for up to eight resident CTAs (the thread limit; registers allow three); the
   // rest of the SM's memory stays L1
   const int carve = (int)std::min<size_t>(100, (8 * (L.total + 1024) * 100) / (228 * 1024) + 1);
@@ -1181,7 +1181,7 @@ int launch_split_instance(const BlockSource& src, const ProxOp& op, cudaStream_t
     L.off_C = L.off_A;
     L.total = align16(L.off_C + std::max(chunk, scr));
     auto kern = llr_gram_kernel<NPMAX, TG>;
-    LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+    LLR_CUDA_TRY(allow_smem(kern));
     LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     LLR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kLlrThreads, L.total));
     if (occ < 1) return set_error(LLR_ERR_UNSUPPORTED, "Gram kernel cannot be resident (smem %zu B)", L.total);

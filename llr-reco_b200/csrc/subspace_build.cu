@@ -237,7 +237,7 @@ int llr_dti_subspace(const float* b_vals, const float* b_vecs, int32_t nq, int32
   if (e == cudaSuccess) e = cudaMemcpy(d_bg, bg.data(), sizeof(double) * bg.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
     const size_t smem = sizeof(double) * (4 * (size_t)nq + (size_t)kSimBatch * (nq + 1));
-    e = cudaFuncSetAttribute(gram_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(gram_partial_kernel);
     if (e == cudaSuccess) {
       note_launch();
       gram_partial_kernel<<<nparts, kSimThreads, smem>>>(d_bg, nq, n_signals, seed, (double)lam_lo, (double)lam_hi,
@@ -253,7 +253,7 @@ int llr_dti_subspace(const float* b_vals, const float* b_vecs, int32_t nq, int32
   if (e == cudaSuccess) {
     const int n2 = (nq + 1) & ~1;
     const size_t smem = sizeof(double) * (2 * (size_t)n2 * (n2 + 1) + n2) + sizeof(int) * n2;
-    e = cudaFuncSetAttribute(jacobi_sym_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(jacobi_sym_kernel);
     if (e == cudaSuccess) {
       note_launch();
       jacobi_sym_kernel<<<1, 256, smem>>>(d_gram, nq, d_ev, d_vec, 30);

@@ -401,7 +401,7 @@ int launch_analysis(const View& in, const View& out, const Taps& t, int nvol, fl
   if ((long long)nvol * nchunk > 65535) return set_error(LLR_ERR_UNSUPPORTED, "too many wavelet volumes");
   auto kern = wave_analysis_kernel<F>;
   const size_t sm = AnaShape<F>::smem;
-  LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  LLR_CUDA_TRY(allow_smem(kern));
   dim3 grid((cy + kWT - 1) / kWT, (cz + kWT - 1) / kWT, nvol * nchunk);
   note_launch();
   kern<<<grid, kWaveThreads, sm, s>>>(in, out, t, kchunk, nchunk, alpha, keep_corner);
@@ -419,7 +419,7 @@ int launch_synthesis(const View& in, const View& out, const Taps& t, int nvol, c
   if ((long long)nvol * nchunk > 65535) return set_error(LLR_ERR_UNSUPPORTED, "too many wavelet volumes");
   auto kern = wave_synthesis_kernel<F>;
   const size_t sm = SynShape<F>::smem;
-  LLR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  LLR_CUDA_TRY(allow_smem(kern));
   dim3 grid((ny + kWS - 1) / kWS, (nz + kWS - 1) / kWS, nvol * nchunk);
   note_launch();
   kern<<<grid, kWaveThreads, sm, s>>>(in, out, t, schunk, nchunk, xf);
