@@ -97,6 +97,42 @@ void dfree(void* p) {
   if (p) cudaFree(p);
 }
 
+// The split path of 65 to 128 volumes (Gram matrix and code per block, rotation log) needs (n + 1) / (2 m) of an image and
+// the log; the wide kernel needs none of it.  It is taken when at most half of the free memory goes into it, and given up
+// when a later allocation of the context finds no memory.
+void drop_wide_split(llr_ctx* c) {
+  drop_graph(c);
+  dfree(c->d_gram); dfree(c->d_blk_ra); dfree(c->d_rot_log);
+  c->d_gram = nullptr; c->d_blk_ra = nullptr; c->d_rot_log = nullptr;
+}
+
+template <class T>
+int ctx_alloc(llr_ctx* c, T** p, size_t n) {
+  int st = dalloc(p, n);
+  if (st == LLR_ERR_NOMEM && c->g.nq > 64 && c->d_gram) {
+    cudaGetLastError();
+    drop_wide_split(c);
+    st = dalloc(p, n);
+  }
+  return st;
+}
+
+void take_wide_split(llr_ctx* c) {
+  const llr_config& cfg = c->cfg;
+  if (cfg.subspace_rank > 0 || c->g.nq <= 64 || c->g.nq > kProxMaxN || cfg.eig_solver != 0 || cfg.gram_mode != 0 ||
+      !llr_gram_tc_supported(c->m, c->g.nq))
+    return;
+  const size_t nb = (size_t)std::max<long long>(1, c->nblocks), log = (size_t)c->rot_ctas * (size_t)jacobi_log_stride(c->g.nq);
+  const size_t gram = nb * (size_t)prox_gram_stride(c->g.nq);
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return; }
+  if (sizeof(float2) * gram + sizeof(float) * log + sizeof(int) * (nb + 1) > free_b / 2) return;
+  if (dalloc(&c->d_gram, gram) != LLR_OK || dalloc(&c->d_blk_ra, nb + 1) != LLR_OK || dalloc(&c->d_rot_log, log) != LLR_OK) {
+    cudaGetLastError();
+    drop_wide_split(c);
+  }
+}
+
 int make_plan(llr_ctx* c) {
   if (c->have_plan) {
     cufftDestroy(c->plan_fwd);
@@ -120,7 +156,8 @@ int make_plan(llr_ctx* c) {
   if (ws > c->fft_work_bytes) {
     dfree(c->d_fft_work);
     c->d_fft_work = nullptr;
-    LLR_CUDA_TRY(device_alloc(&c->d_fft_work, ws));
+    c->fft_work_bytes = 0;
+    LLR_TRY(ctx_alloc(c, (char**)&c->d_fft_work, ws));
     c->fft_work_bytes = ws;
   }
   r = cufftSetWorkArea(c->plan_fwd, c->d_fft_work);
@@ -424,8 +461,6 @@ int llr_ctx_create(const llr_config* cfg, llr_ctx** out) {
     c->vwide_ctas = wide_jacobi_ctas();
     if ((st = dalloc(&c->d_vwide, (size_t)c->vwide_ctas * (size_t)wide_v_stride()))) return fail(st);
     c->rot_ctas = (int)std::min<long long>(std::max<long long>(1, c->nblocks), jacobi_ctas(c->g.nq));
-    if (c->g.nq > 64 && (st = dalloc(&c->d_rot_log, (size_t)c->rot_ctas * (size_t)jacobi_log_stride(c->g.nq))))
-      return fail(st);
   }
   {
     int per[3], P = 1;
@@ -445,7 +480,7 @@ int llr_ctx_create(const llr_config* cfg, llr_ctx** out) {
   }
   e = cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
   if (e != cudaSuccess) return fail(cuda_error(e, "cudaMemsetAsync", __FILE__, __LINE__));
-  if (cfg->subspace_rank == 0 && c->g.nq <= kProxMaxN &&
+  if (cfg->subspace_rank == 0 && c->g.nq <= 64 &&
       ((st = dalloc(&c->d_gram, (size_t)std::max<long long>(1, c->nblocks) * (size_t)prox_gram_stride(c->g.nq))) ||
        (st = dalloc(&c->d_blk_ra, (size_t)std::max<long long>(1, c->nblocks) + 1))))
     return fail(st);
@@ -491,6 +526,7 @@ int llr_ctx_create(const llr_config* cfg, llr_ctx** out) {
   const bool plain = cfg->subspace_rank == 0 && !c->wavelet_on && c->phase_off.empty();
   c->obj_mode = !plain ? 0 : (cfg->prox_mode == LLR_PROX_SOFT_THRESH ? 2 : 1);
   if ((st = upload_tables(c))) return fail(st);
+  take_wide_split(c);
   c->h_iter = 0;
   *out = c;
   return LLR_OK;
@@ -554,7 +590,7 @@ static int upload_kspace_device(llr_ctx* c) {
   // per-line non-zero counts
   const long long nlines = g.nyz * g.nq;
   int* d_cnt = nullptr;
-  LLR_TRY(dalloc(&d_cnt, (size_t)nlines));
+  LLR_TRY(ctx_alloc(c, &d_cnt, (size_t)nlines));
   int st = launch_line_nnz(c->d_work, nlines, g.nx, d_cnt, s);
   std::vector<int> cnt((size_t)nlines);
   if (st == LLR_OK) {
@@ -594,14 +630,14 @@ static int upload_kspace_device(llr_ctx* c) {
     }
     c->h_samp_off[g.nq] = (long long)pos.size();
     c->n_samp_lines = (long long)pos.size();
-    LLR_TRY(dalloc(&c->d_samp_pos, pos.size()));
-    LLR_TRY(dalloc(&c->d_samp_off, (size_t)g.nq + 1));
+    LLR_TRY(ctx_alloc(c, &c->d_samp_pos, pos.size()));
+    LLR_TRY(ctx_alloc(c, &c->d_samp_off, (size_t)g.nq + 1));
     LLR_CUDA_TRY(cudaMemcpyAsync(c->d_samp_pos, pos.data(), sizeof(int) * pos.size(), cudaMemcpyHostToDevice, s));
     LLR_CUDA_TRY(cudaMemcpyAsync(c->d_samp_off, c->h_samp_off.data(), sizeof(long long) * (g.nq + 1),
                                  cudaMemcpyHostToDevice, s));
     if (c->rows_fft) {
       const std::vector<int> rp = fft_rows_ptr(pos, c->h_samp_off, g.ny, g.nz);
-      LLR_TRY(dalloc(&c->d_rows_ptr, rp.size()));
+      LLR_TRY(ctx_alloc(c, &c->d_rows_ptr, rp.size()));
       LLR_CUDA_TRY(cudaMemcpyAsync(c->d_rows_ptr, rp.data(), sizeof(int) * rp.size(), cudaMemcpyHostToDevice, s));
       LLR_CUDA_TRY(cudaStreamSynchronize(s));   // the host copy goes out of scope
     }
@@ -617,12 +653,12 @@ static int upload_kspace_device(llr_ctx* c) {
     LLR_TRY(launch_phase_x(c->d_work, g, g.nq, c->d_ph_ksp, -1, (float)(1.0 / std::sqrt((double)g.nx)), s));
     PhaseTab none{nullptr, nullptr, nullptr};
     LLR_TRY(launch_ref_to_planar(c->d_work, c->d_x, g, 1.f, none, 0, s));
-    LLR_TRY(dalloc(&c->d_yhat, (size_t)std::max<long long>(1, c->n_samp_lines * g.nx)));
+    LLR_TRY(ctx_alloc(c, &c->d_yhat, (size_t)std::max<long long>(1, c->n_samp_lines * g.nx)));
     LLR_TRY(launch_gather_lines(c->d_x, c->d_yhat, c->d_samp_pos, c->d_samp_off, g, ctx_phase(c, c->d_ph_img, false),
                                 (float)std::sqrt((double)g.nyz), s));
     c->load_scale = (float)(1.0 / (double)g.nyz);
   } else {
-    LLR_TRY(dalloc(&c->d_yhat, (size_t)E));
+    LLR_TRY(ctx_alloc(c, &c->d_yhat, (size_t)E));
     PhaseTab none{nullptr, nullptr, nullptr};
     LLR_TRY(launch_ref_to_planar(c->d_work, c->d_yhat, g, 1.f, none, 0, s));
     LLR_TRY(launch_prep_full(c->d_yhat, g, ph_img_full, (float)std::sqrt((double)g.V), s));

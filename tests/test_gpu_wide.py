@@ -172,3 +172,24 @@ def test_wide_scratch_is_not_mapped_on_every_call(gpu):
             best[batch] = min(best.get(batch, 1.0), time.perf_counter() - t0)
         d.close()
     assert best[600] < 10 * best[100]
+
+
+def test_wide_context_without_room_for_the_split_path(gpu):
+    """128 volumes in blocks of one voxel: a Gram matrix per block would be 197 GB.  The context is created without it, as
+    before there was a split path, and holds the image buffers, the tables and the wide kernel's scratch only."""
+    p = ReconParams(vol_size=(144, 144, 144), nq=128, block_size=(1, 1, 1), prox_mode=1, lam=0.1)
+    with ReconContext(p) as ctx:
+        assert ctx.device_bytes() < 8 << 30
+    y = np.zeros((4, 4, 4, 80), np.complex64, order="F")
+    with ReconContext(ReconParams(vol_size=(4, 4, 4), nq=80, block_size=(2, 2, 2), prox_mode=1, lam=0.1)) as ctx:
+        ctx.upload_kspace(y)      # the next allocations do not see the failed one
+        ctx.init_zero_filled()
+        ctx.iterate(1)
+
+
+@pytest.mark.parametrize("kw", [dict(eig_solver=1), dict(gram_mode=1)])
+def test_wide_context_takes_no_scratch_that_it_cannot_use(gpu, kw):
+    """The Jacobi solver and the FP32 Gram mode run the wide kernel: no Gram matrices, no rotation log."""
+    p = dict(vol_size=(16, 16, 16), nq=100, block_size=(4, 4, 4), prox_mode=1, lam=0.1)
+    with ReconContext(ReconParams(**p)) as a, ReconContext(ReconParams(**p, **kw)) as b:
+        assert a.device_bytes() - b.device_bytes() >= 64 * 5050 * 8
