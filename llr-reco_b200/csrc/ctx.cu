@@ -490,7 +490,8 @@ int llr_ctx_create(const llr_config* cfg, llr_ctx** out) {
   if (e == cudaSuccess) e = cudaMemsetAsync(c->d_x, 0, sizeof(float2) * E, c->stream);
   if (e != cudaSuccess) return fail(cuda_error(e, "cudaMemsetAsync", __FILE__, __LINE__));
   if (cfg->subspace_rank > 0 && (st = dalloc(&c->d_S, (size_t)c->g.nq * cfg->subspace_rank))) return fail(st);
-  if (cfg->fft_mode == 0 && fft_dc_supported(c->g.ny, c->g.nz)) {   // fused FFT + DC twiddles (FP64-computed)
+  const bool plane_fits = cfg->fft_mode == 0 && fft_dc_supported(c->g.ny, c->g.nz);
+  if (plane_fits && fft_dc_preferred(c->g.ny, c->g.nz, (long long)c->g.nx * c->g.nq)) {   // fused FFT + DC twiddles (FP64-computed)
     const std::vector<float2> tw = fft_dc_twiddles(c->g.ny, c->g.nz);
     c->fft_grid = fft_dc_grid(c->g.ny, c->g.nz);
     if (c->fft_grid > 0) {
@@ -499,7 +500,7 @@ int llr_ctx_create(const llr_config* cfg, llr_ctx** out) {
       if (e != cudaSuccess) return fail(cuda_error(e, "cudaMemcpy", __FILE__, __LINE__));
     }
   }
-  if (cfg->fft_mode == 0 && !c->d_fft_tw && fft_rows_supported(c->g.ny, c->g.nz)) {
+  if (cfg->fft_mode == 0 && !plane_fits && fft_rows_supported(c->g.ny, c->g.nz)) {
     const std::vector<float2> tw = fft_rows_twiddles(c->g.ny, c->g.nz);
     if ((st = dalloc(&c->d_rows_tw, tw.size()))) return fail(st);
     e = cudaMemcpy(c->d_rows_tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice);

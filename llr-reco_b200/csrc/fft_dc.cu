@@ -452,6 +452,14 @@ int fft_dc_grid(int ny, int nz) {
   return nsm * per;
 }
 
+// Planes of a few hundred samples leave a CTA more barriers than work; with several of them per CTA, cuFFT's batched kernels
+// and the DC pass are faster.  Forward, DC and inverse, fused / cuFFT: 12000 planes of 5 x 5 79 / 37 us, 11 x 13
+// 113 / 58, 16 x 16 105 / 73, 25 x 20 137 / 107, 25 x 25 154 / 145 us; 7680 of 35 x 30 139 / 161.  With up to two planes
+// per CTA the launches count: 1920 planes of 16 x 16 34 / 35 us, 640 of 11 x 13 27 / 31.
+bool fft_dc_preferred(int ny, int nz, long long planes) {
+  return (long long)ny * nz >= 768 || planes <= 2ll * fft_dc_grid(ny, nz);
+}
+
 int launch_fft_dc(float2* u, const float2* yhat, const int* pos, const long long* off, const float2* twiddle,
                   const Geom& g, double* partials, int grid, const int* zero_ra, const BlockSource* zsrc,
                   float unc_scale, cudaStream_t s) {

@@ -101,6 +101,7 @@ inline long long prox_gram_stride(int n) {
 }
 
 bool fft_dc_supported(int ny, int nz);
+bool fft_dc_preferred(int ny, int nz, long long planes);   // to cuFFT, where supported
 std::vector<float2> fft_dc_twiddles(int ny, int nz);
 int fft_dc_grid(int ny, int nz);
 int launch_fft_dc(float2* u, const float2* yhat, const int* pos, const long long* off, const float2* twiddle,
