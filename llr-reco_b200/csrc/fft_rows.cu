@@ -346,10 +346,11 @@ bool fft_rows_supported(int ny, int nz) {
   return radix_split(ny, a, b) && radix_split(nz, a, b);
 }
 
-// The expanding row pass keeps srank rows, S and the exchange buffer in shared memory.
+// The expanding row pass keeps srank rows, S and the exchange buffer in shared memory.  More than 64 volumes are
+// refused by launch_subspace_expand, whatever the plane.
 bool fft_rows_expand_supported(int ny, int nq, int srank) {
   int a, b;
-  return radix_split(ny, a, b) && row_smem(a, b, nq, srank) <= 200 * 1024;
+  return nq <= 64 && radix_split(ny, a, b) && row_smem(a, b, nq, srank) <= 200 * 1024;
 }
 
 // W_ny^j then W_nz^j, FP64-computed.

@@ -80,3 +80,20 @@ def test_kspace_expansion_matches_oracle(gpu, vol, bs, nq, srank, corr):
     ox, oh = O.recon(y.astype(np.complex128), ocfg, 2, x0=x0)
     assert rel_err(out[0][0], ox) < 2e-4
     np.testing.assert_allclose(out[0][1], oh, rtol=2e-4)
+
+
+@pytest.mark.parametrize("ny,nz", [(16, 12), (256, 128)])
+def test_coefficient_volumes_of_more_than_64_stay_refused(gpu, ny, nz):
+    """The coefficient wavelet takes at most 64 volumes, on planes of either path."""
+    rng = np.random.default_rng(3)
+    vol, nq, srank = (8, ny, nz), 66, 4
+    p = ReconParams(vol_size=vol, nq=nq, block_size=(4, 4, 4), lam=0.1, subspace_rank=srank, wavelet_space=1,
+                    prox_mode=L.LLR_PROX_SOFT_THRESH)
+    p.wavelet_alpha, p.wavelet_moments, p.wavelet_levels = 0.003, 2, 1
+    with ReconContext(p) as ctx:
+        ctx.upload_kspace(_lines(rng, vol, nq))
+        ctx.upload_subspace(np.asfortranarray(np.linalg.qr(crandn(rng, (nq, srank)))[0].astype(np.complex64)))
+        ctx.init_zero_filled()
+        with pytest.raises(L.LlrError) as err:
+            ctx.iterate(1)
+    assert err.value.status == L.LLR_ERR_UNSUPPORTED
