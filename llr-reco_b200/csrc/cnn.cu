@@ -376,8 +376,8 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
 // ---------------------------------------------------------------------------------------
 // conv3d of the network's inference: the GEMM and the operand split of conv3d_tc_kernel, summed in another order.
 // The gradients keep that kernel: tensor memory truncates its FP32 sums, what that leaves in the activations depends
-// on the order, and sums over a million voxels show it (3e-5 of a gradient between the two orders, either of
-// them 6e-5 from 64 bits; an inference pass: 1.2e-6).
+// on the order, and sums over a million voxels show it (3e-5 of a gradient between the two orders; an inference
+// pass: 1.2e-6, either order 4.2e-6 from 64 bits).
 //
 // A CTA walks columns of 8 (x) x 16 (y) voxels along z, one input plane at a time.  The plane's halo
 // (10 x 18 voxels, all channels) is written once into shared memory in the unswizzled K-major
@@ -709,7 +709,8 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
 // nothing).  What is left is the truncation of the FP32 sums in tensor memory, bounded by kWgRun.
 // Bound: the MMAs, 432 of 128 x 32 x 16 per tile.  The same GEMM in 3xTF32 with a K-major copy of the operand per tap
 // and 32 voxels (TF32 operands cannot be MN-major in this layout) spent its time on those copies: 3.95 ms per 32 -> 32
-// layer at 96^3, 1.16 ms this way, 0.82 ms with the MMAs issued by a converged warp.
+// layer at 96^3, 1.16 ms this way, 0.82 ms with the MMAs issued by a converged warp, 0.60 ms on every SM
+// instead of 104.
 //
 // Warps 0-7 convert, load the next tile's FP32 data with cp.async while the MMAs run, and sum the bias
 // gradient; warp 8 issues the MMAs.  At the end each CTA writes its partial sums; a fixed-order reduction

@@ -363,13 +363,12 @@ static int finalize_iteration(llr_ctx* c, int np, cudaStream_t s) {
 }
 
 // Forward 2-D DFT, DC with residual, inverse 2-D DFT in one kernel; residual finalized.
-static int fused_dc_pass(llr_ctx* c, cudaStream_t s, double* out) {
+static int fused_dc_pass(llr_ctx* c, cudaStream_t s) {
   const bool zf = defer_zero_blocks(c);
   const BlockSource zsrc = make_source(c, nullptr, 1.f);
   LLR_TRY(launch_fft_dc(c->d_x, c->d_yhat, c->d_samp_pos, c->d_samp_off, c->d_fft_tw, c->g, c->d_partials,
                         c->fft_grid, zf ? c->d_blk_ra : nullptr, &zsrc, uncovered_in_fft(c) ? c->load_scale : 0.f, s));
-  if (!out) return finalize_iteration(c, c->fft_grid, s);
-  return launch_finalize(c->d_partials, c->fft_grid, (double)c->load_scale, nullptr, 0, nullptr, 0, out, s);
+  return finalize_iteration(c, c->fft_grid, s);
 }
 
 // The same through the row and column kernels, for planes that do not fit shared memory.
@@ -394,7 +393,7 @@ static int rows_dc_pass(llr_ctx* c, cudaStream_t s) {
 int ctx_enqueue_iteration(llr_ctx* c, cudaStream_t s) {
   LLR_TRY(prox_pass(c, s, nullptr, false, nullptr));
   if (c->wavelet_on) LLR_TRY(wavelet_pass(c, s, 1.f, true));
-  if (c->fused_fft) return fused_dc_pass(c, s, nullptr);
+  if (c->fused_fft) return fused_dc_pass(c, s);
   if (c->rows_fft) return rows_dc_pass(c, s);
   LLR_TRY(exec_fft(c, c->d_x, CUFFT_FORWARD, s));
   LLR_TRY(dc_pass(c, s, 0));
@@ -803,7 +802,7 @@ static int capture_stage(llr_ctx* c, int stage, cudaGraphExec_t* out) {
     case 0: st = prox_pass(c, s, nullptr, false, nullptr); break;
     case 1: if (c->wavelet_on) st = wavelet_pass(c, s, 1.f, true); break;
     case 2:
-      st = c->fused_fft ? fused_dc_pass(c, s, nullptr)
+      st = c->fused_fft ? fused_dc_pass(c, s)
            : c->rows_fft ? rows_dc_pass(c, s) : exec_fft(c, c->d_x, CUFFT_FORWARD, s);
       break;
     case 3:

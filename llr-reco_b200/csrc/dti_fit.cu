@@ -5,7 +5,7 @@
 // 3 x 3 tensor (e1 >= e2 >= e3), and MD = mean, RD = (e2 + e3) / 2,
 // FA = sqrt(3/2) sqrt(sum (e_i - MD)^2) / sqrt(sum e_i^2) (NaN for a zero tensor, as there).
 //
-// One thread per voxel: the least-squares solve is the same pseudo-inverse for every voxel
+// Two voxels per thread: the least-squares solve is the same pseudo-inverse for every voxel
 // (A has full column rank for six or more non-coplanar directions), formed once on the host in
 // FP64 from the normal equations and applied from shared memory; the symmetric 3 x 3 eigen
 // problem is a few cyclic Jacobi sweeps in registers.
@@ -148,9 +148,9 @@ __device__ __forceinline__ void add_samples(const float2 (&z)[2][QB], const floa
 // per thread before the first logarithm, and a row of the weights (two shared loads) serves both voxels.
 // Calls at that size: 625 us with a square root, a division and a logf per sample, one load at a time and
 // IEEE rotations; 485 us with ln_normal and the one-division rotations; 433 us with one range check per
-// batch instead of per sample; 409 us at four CTAs per SM (64 registers) instead of three.  Half of the volume masked
-// to zero: 1290 us with the ratios formed one by one, 500 to 550 us with the zeros' terms added apart (two forms
-// unrolled side by side took 500 too but 412 to 460 us without zeros).
+// batch instead of per sample; 404 us at four CTAs per SM (64 registers) instead of three.  Half of the volume masked
+// to zero: 1290 us with the ratios formed one by one, 500 to 550 us with the zeros' terms added apart, which
+// costs a volume without zeros 3 % (416 us, in turn with the 404).
 __global__ void __launch_bounds__(256, 4) dti_fit_kernel(const float2* __restrict__ dwi, const float2* __restrict__ b0,
                                                       long long V, int nq, int nb0, const float* __restrict__ pinv,
                                                       float* __restrict__ out) {

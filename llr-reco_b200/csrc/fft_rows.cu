@@ -10,7 +10,13 @@
 // line of length n = n1 n2 is two register DFTs and one exchange); natural order in HBM throughout.
 // cuFFT's four kernels plus the scattered DC pass moved 64 + 8 bytes per element and rewrote single 8-byte
 // samples; here it is 48.  At 128 x 256 x 256 x 61, rank 7, per iteration: expand 0.97 + cuFFT 2 x 2.53 + DC
-// 1.45 ms before, coefficient columns 0.21 + expanding rows 2.36 + columns 1.65 ms now.
+// 1.45 ms before, coefficient columns 0.21 + expanding rows 2.33 + columns 1.65 ms now.
+//
+// Every plane whose extents factor comes here: data consistency with both transforms, 64 x 16 planes, cuFFT / here:
+// 256 x 256 1.15 / 0.75 ms, 240 x 240 1.47 / 0.80, 224 x 224 1.44 / 0.68, 192 x 192 0.75 / 0.51, 176 x 176 0.63 / 0.49, 169 x 196
+// 0.66 / 0.54, 130 x 256 0.68 / 0.58, 117 x 256 0.62 / 0.55; one plane of 256 x 256 32.5 / 31.4 us.  Length 256 alone
+// has its sizes at compile time (the usual matrix size beyond shared memory): 11 ns per 1000 samples, other
+// lengths 13 to 14.
 //
 // With a temporal subspace whose volumes share their phase, X = C S^H and the transforms commute: the forward
 // transform runs on the srank coefficient volumes, and the row pass expands each k-space row of every

@@ -21,9 +21,9 @@
 // rotations), then the two barriers per step.  4096 blocks of 512 x 106, 1857 of them through the sweeps:
 // 67.6 ms in the wide kernel (Gram and apply included), 14.5 ms here with two CTAs of 512 threads per SM, 12.9 ms
 // with four of 256.
-// A Householder path in its place took 2.5 ms, but a rotation's c^2 + s^2 = 1 + O(eps) makes the Jacobi kernels'
-// singular values and vectors short by a few 1e-6, which every result so far carries (residuals 5e-5): its
-// more exact results differ from theirs by more than single precision explains.
+// A Householder path in its place took 2.5 ms.  A rotation's c^2 + s^2 = 1 + O(eps) makes the Jacobi kernels' singular
+// values and vectors short by a few 1e-6 (residuals 5e-5), so its results differ from these by that much, towards
+// 64 bits; it is not built.
 #include <algorithm>
 #include <type_traits>
 
@@ -67,7 +67,6 @@ __global__ void __launch_bounds__(kJacThreads, 4) llr_eig_jacobi_kernel(ProxOp o
   const int n = op.n, n2 = (n + 1) & ~1, half = n2 >> 1, M = n2 - 1;
   auto row = [&](int i) { return (i * (2 * n2 - 1 - i)) >> 1; };
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int P = n * (n + 1) / 2;
   const bool soft = op.mode != LLR_PROX_HARD_RANK;
   const float thr = op.lambda * op.lambda;
   float* log = op.rot_log + (long long)blockIdx.x * jacobi_log_stride(n);   // (t, e) per pair and step
