@@ -376,8 +376,11 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
 // ---------------------------------------------------------------------------------------
 // conv3d of the network's inference: the GEMM and the operand split of conv3d_tc_kernel, summed in another order.
 // The gradients keep that kernel: tensor memory truncates its FP32 sums, what that leaves in the activations depends
-// on the order, and sums over a million voxels show it (3e-5 of a gradient between the two orders; an inference
-// pass: 1.2e-6, either order 4.2e-6 from 64 bits).
+// on the order, and sums over a million voxels show it (3e-5 of a gradient between two orders).
+// The high BF16 parts and the two low ones are summed apart, in two rings of tensor memory, and added in FP32: a third of
+// the additions at full size.  The 8-layer network is 0.8e-6 from 64 bits (one ring for all: 4.3e-6 at 192 x 192 x 96,
+// 5 to 20 % above conv3d_tc_kernel on volumes of 16 to 48 planes; that kernel 4.2e-6 to 5.3e-6); 4.57 ms instead of 4.48
+// there.
 //
 // A CTA walks columns of 8 (x) x 16 (y) voxels along z, one input plane at a time.  The plane's halo
 // (10 x 18 voxels, all channels) is written once into shared memory in the unswizzled K-major
@@ -398,12 +401,13 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_tc_kernel(const float* _
 // Bound: the MMAs' issue (one thread, 54 per plane) and their operand reads; with one tap and one z plane per tile (N = COUT, a
 // 540-voxel halo converted for 128 outputs) a 32 -> 32 layer at 192 x 192 x 96 took 1548 us, this way 896, with
 // the MMAs issued by a converged warp 638, with 32-bit descriptor arithmetic and unrolled taps 531 (the 8-layer
-// network: 11.8 -> 4.4 ms).
+// network: 11.8 -> 4.5 ms).
 // ---------------------------------------------------------------------------------------
 constexpr int kCvTX = 8, kCvTY = 16;                               // 128 voxels of one z plane
 constexpr int kCvHX = kCvTX + 2, kCvHY = kCvTY + 2;
 constexpr int kCvNV = kCvHX * kCvHY;                               // 180 halo voxels of a plane
 constexpr int kCvCS = kCvNV * 16;                                  // bytes of one 8-channel chunk of a BF16 part
+constexpr int kCvLow = 256;                                        // first tensor-memory column of the low parts' ring
 
 template <int CIN, int COUT>
 struct CrLayout {
@@ -412,7 +416,7 @@ struct CrLayout {
   static constexpr int KS = KC / 2;                                // K steps of 16 channels per tap
   static constexpr int RC = 2 * KC;                                // 4-channel chunks of the FP32 halo
   static constexpr int NPL = 3;                                    // BF16 parts per activation
-  static constexpr int SLOTS = 512 / NP;                           // ring of output planes: all of tensor memory
+  static constexpr int SLOTS = kCvLow / NP;                        // ring of output planes: half of tensor memory
   static constexpr int WT = KC * 3 * NP * 16;                      // bytes of one in-plane tap's weights
   static constexpr size_t PB = (size_t)KC * kCvCS;                 // bytes of one BF16 part
   static constexpr size_t off_hdr = 0;                             // mbarriers, TMEM address
@@ -461,6 +465,33 @@ __device__ __forceinline__ void tmem_zero(uint32_t taddr) {
                  "r"(0u) : "memory");
   else
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr), "r"(0u) : "memory");
+}
+
+// HC columns of this warp's 32 TMEM lanes at two places, complete on return
+template <int HC>
+__device__ __forceinline__ void tmem_load2(uint32_t (&hi)[HC], uint32_t (&lo)[HC], uint32_t thi, uint32_t tlo) {
+  if constexpr (HC == 16) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(hi[0]), "=r"(hi[1]), "=r"(hi[2]), "=r"(hi[3]), "=r"(hi[4]), "=r"(hi[5]), "=r"(hi[6]), "=r"(hi[7]),
+                   "=r"(hi[8]), "=r"(hi[9]), "=r"(hi[10]), "=r"(hi[11]), "=r"(hi[12]), "=r"(hi[13]), "=r"(hi[14]), "=r"(hi[15])
+                 : "r"(thi));
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
+                 : "=r"(lo[0]), "=r"(lo[1]), "=r"(lo[2]), "=r"(lo[3]), "=r"(lo[4]), "=r"(lo[5]), "=r"(lo[6]), "=r"(lo[7]),
+                   "=r"(lo[8]), "=r"(lo[9]), "=r"(lo[10]), "=r"(lo[11]), "=r"(lo[12]), "=r"(lo[13]), "=r"(lo[14]), "=r"(lo[15]),
+                   "+r"(hi[0]), "+r"(hi[1]), "+r"(hi[2]), "+r"(hi[3]), "+r"(hi[4]), "+r"(hi[5]), "+r"(hi[6]), "+r"(hi[7]),
+                   "+r"(hi[8]), "+r"(hi[9]), "+r"(hi[10]), "+r"(hi[11]), "+r"(hi[12]), "+r"(hi[13]), "+r"(hi[14]), "+r"(hi[15])
+                 : "r"(tlo)
+                 : "memory");
+  } else {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(hi[0]), "=r"(hi[1]), "=r"(hi[2]), "=r"(hi[3]), "=r"(hi[4]), "=r"(hi[5]), "=r"(hi[6]), "=r"(hi[7])
+                 : "r"(thi));
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
+                 : "=r"(lo[0]), "=r"(lo[1]), "=r"(lo[2]), "=r"(lo[3]), "=r"(lo[4]), "=r"(lo[5]), "=r"(lo[6]), "=r"(lo[7]),
+                   "+r"(hi[0]), "+r"(hi[1]), "+r"(hi[2]), "+r"(hi[3]), "+r"(hi[4]), "+r"(hi[5]), "+r"(hi[6]), "+r"(hi[7])
+                 : "r"(tlo)
+                 : "memory");
+  }
 }
 
 template <int CIN, int COUT>
@@ -567,27 +598,17 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
       const int gx = p.cx + (a & 7), gy = p.cy + (a >> 3);
       const int hi = p.zi == p.last ? p.nout - 1 : p.zi - 1 - p.z0;
       for (int o = max(p.zi - 1 - p.z0, 0); o <= hi; ++o) {
-        uint32_t r[HC];
+        uint32_t r[2][HC];                                 // sums of the high and of the low parts
         const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)((p.slot0 + o) % SLOTS * NP + hs * HC);
-        if constexpr (HC == 16) {
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-              : "r"(taddr));
-        } else {
-          asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                       : "r"(taddr));
-        }
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        tmem_zero<HC>(taddr);                              // for the slot's next output plane
+        tmem_load2<HC>(r[0], r[1], taddr, taddr + kCvLow);
+#pragma unroll
+        for (int l = 0; l < 2; ++l) tmem_zero<HC>(taddr + l * kCvLow);   // for the slot's next output plane
         if (gx < G.nx && gy < G.ny) {
           const long long v = (long long)gx + (long long)G.nx * (gy + (long long)G.ny * (p.z0 + o));
           float f[HC];
 #pragma unroll
           for (int k = 0; k < HC; ++k) {
-            float val = __uint_as_float(r[k]) + bz[k];
+            float val = __uint_as_float(r[0][k]) + __uint_as_float(r[1][k]) + bz[k];
             if (relu) val = fmaxf(val, 0.f);
             f[k] = val;
           }
@@ -673,9 +694,9 @@ __global__ void __launch_bounds__(kFwThreads, 1) conv3d_run_kernel(const float* 
             const uint32_t db = bs + (uint32_t)(((3 * dy + dx) * Lay::WT) >> 4);
 #pragma unroll
             for (int k = 0; k < NPL; ++k) {
-              const uint32_t da = as + (uint32_t)(((k * Lay::PB) >> 4) + kCvHX * dy + dx);
-              umma_bf16_by(leader, d0, da, ah, db, bh, id0, 1u);
-              if (n1 > 0) umma_bf16_by(leader, tmem, da, ah, db + (uint32_t)(n0 * NP), bh, id1, 1u);
+              const uint32_t da = as + (uint32_t)(((k * Lay::PB) >> 4) + kCvHX * dy + dx), low = k > 0 ? kCvLow : 0;
+              umma_bf16_by(leader, d0 + low, da, ah, db, bh, id0, 1u);
+              if (n1 > 0) umma_bf16_by(leader, tmem + low, da, ah, db + (uint32_t)(n0 * NP), bh, id1, 1u);
             }
           }
         }

@@ -54,6 +54,26 @@ def test_forward_runs_and_edges(gpu, dims):
         assert np.linalg.norm(got[:, y0:y1, x0:x1] - exp) <= 1e-4 * res + 2.0 ** -24 * np.linalg.norm(exp)
 
 
+@pytest.mark.parametrize("dims", [(1, 17, 9), (2, 5, 8), (3, 16, 16), (11, 18, 11)])
+def test_forward_sums_of_one_sign(gpu, dims):
+    """Positive activations and weights: every addition in tensor memory truncates in the same direction.  The high BF16
+    parts take 27 additions in the first layer and 54 in the three others, a unit of 2^-23 of a sum that grows steadily
+    at most and half of that on average: 189 x 2^-23 / 2 / 2 = 5.6e-6; the low parts' own sums lose 2^-8 of that.  7e-6
+    (with one sum for all parts, three times as many additions: 1.2e-5)."""
+    from llr_b200.cnn import Cnn
+    rng = np.random.default_rng(11)
+    ch = (14, 32, 32, 32, 14)
+    x = rng.uniform(0.5, 1.0, dims + (14,)).astype(np.float32)
+    with Cnn(ch, seed=2) as net:
+        p = np.zeros(net.n_params, np.float32)
+        for w0, b0 in CO.layer_slices(ch)[0]:
+            p[w0:b0] = rng.uniform(0.0, 0.1, b0 - w0)
+        net.params = p
+        got = net.forward(x)
+    exp, _ = CO.forward(p, ch, x.astype(np.float64))
+    assert rel_err(got, exp) < 7e-6
+
+
 @pytest.mark.parametrize("dims", [(4, 9, 10), (9, 8, 17)])
 def test_gradients_match_oracle(gpu, dims):
     """dL/dW and dL/db of every layer for L = mean |out - target|^2."""
