@@ -115,9 +115,9 @@ __global__ void __launch_bounds__(kJacThreads, 4) llr_eig_jacobi_kernel(ProxOp o
     const double ub = mu + sqrt(fmax((double)fro2 / n - mu * mu, 0.0)) * sqrt((double)(n - 1));
     int ra = 0;
     bool done = true;
-    if (!soft && op.rank >= n) ra = -2;                     // every component kept: identity
+    if (soft ? op.lambda <= 0.f : op.rank >= n) ra = -2;    // every component kept: identity
     else if (!isfinite(fro2)) ra = -1;   // no angle compares with it: the wide kernel multiplies C by W and lets NaN through
-    else if (soft && op.lambda > 0.f && (fro2 <= thr * thr || ub <= (double)thr)) ra = 0;
+    else if (soft && (fro2 <= thr * thr || ub <= (double)thr)) ra = 0;
     else done = false;
     // one step's rotations on the packed matrix: A <- J^H A J, or undone A <- J A J^H
     auto update = [&](auto undo) {

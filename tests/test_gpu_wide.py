@@ -193,3 +193,33 @@ def test_wide_context_takes_no_scratch_that_it_cannot_use(gpu, kw):
     p = dict(vol_size=(16, 16, 16), nq=100, block_size=(4, 4, 4), prox_mode=1, lam=0.1)
     with ReconContext(ReconParams(**p)) as a, ReconContext(ReconParams(**p, **kw)) as b:
         assert a.device_bytes() - b.device_bytes() >= 64 * 5050 * 8
+
+
+@pytest.mark.parametrize("n", [64, 65, 128])
+def test_zero_threshold_is_the_identity(gpu, n):
+    """A soft threshold of zero keeps every component: the matrices come back bit for bit, rank-deficient and not finite
+    ones too, on both sides of the kernels' limit."""
+    m, batch = 72, 5
+    x = _low_rank_mats(np.random.default_rng(n), m, n, 5, batch, 0.0)
+    x[0, 1, 2] = np.nan
+    d = DeviceBuffer.from_array(x)
+    L.check(L.lib.llr_soft_threshold_batch_dev(m, n, 0.0, batch, d.ptr, None))
+    got = d.download(np.empty_like(x, order="F"))
+    d.close()
+    np.testing.assert_array_equal(got, x)
+
+
+def test_zero_threshold_with_overlapping_blocks(gpu):
+    """The mean over the tilings of an identity is the image itself, to the rounding of the scaled sum of eight."""
+    rng = np.random.default_rng(4)
+    vol, nq = (8, 16, 8), 66
+    y = crandn(rng, vol + (nq,)) * (rng.random((1,) + vol[1:] + (nq,)) < 0.5)
+    p = ReconParams(vol_size=vol, nq=nq, block_size=(4, 4, 4), block_stride=(2, 2, 2), lam=0.0, seed=1,
+                    prox_mode=L.LLR_PROX_SOFT_THRESH)
+    with ReconContext(p) as ctx:
+        ctx.upload_kspace(np.asfortranarray(y.astype(np.complex64)))
+        ctx.init_zero_filled()
+        x0 = ctx.download_image()
+        ctx.iterate(1)
+        x1 = ctx.download_image()
+    assert rel_err(x1, x0) < 2e-6
