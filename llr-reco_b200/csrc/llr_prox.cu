@@ -612,14 +612,15 @@ namespace {
 // memory (all the index divisions there are), then the elements go by volume after volume, eight in flight per thread.
 // With three 64-bit divisions per element the kernel was issue-bound: 315 us for 4096 blocks of 216 x 61 on
 // 96 x 96 x 48 x 61 (0.43 GB moved), about 100 us this way (lift, rank truncation and un-lift 1617 -> 1213 us).
-// A CTA per block in place of one per row chunk took that long for those blocks too, but 853 us for 2^3 blocks
-// of one 128^3 volume and 12.5 ms for a single 256 x 256 x 64 block of three (divisions everywhere: 37 and
-// 158 us): 36 and 79 us this way.
+// A CTA per block in place of one per row chunk took, both ways, 1.80 ms for 2^3 blocks of one 128^3 volume and 23.9 ms for a
+// single 256 x 256 x 64 block of three: 53 and 119 us this way.  One address per element is kept for the second half of a
+// batch, so four CTAs fit an SM (both addresses took 80 registers, three CTAs); over 36 shapes of blocks of one to 32^3
+// voxels and 1 to 61 volumes nothing is slower than with a CTA per block, 4^3 to 8^3 blocks 1.0 to 1.7 times as fast.
 constexpr int kLiftRows = 1024;   // most rows per chunk (16 KB of offsets)
 
 // QFAST: volumes run fastest over a slice's elements, else rows.  U: unsigned where every row and block index fits.
 template <int DIR, bool QFAST, class U>
-__global__ void __launch_bounds__(256) lift_kernel(float2* __restrict__ vol, float2* __restrict__ mat, int nx, int ny,
+__global__ void __launch_bounds__(256, 4) lift_kernel(float2* __restrict__ vol, float2* __restrict__ mat, int nx, int ny,
                                                    int nz, int nq, int bx, int by, int bz, int gx, int gy, int sx,
                                                    int sy, int sz, long long start, long long n, int qper, int rc) {
   __shared__ long long off[kLiftRows], moff[kLiftRows];
@@ -646,14 +647,15 @@ __global__ void __launch_bounds__(256) lift_kernel(float2* __restrict__ vol, flo
     int f = (int)threadIdx.x % nf, sl = (int)threadIdx.x / nf;
     while (sl < ns) {
       float2 v[LB];
-      long long va[LB], ma[LB];
+      long long to[LB];
 #pragma unroll
       for (int u = 0; u < LB; ++u) {
-        const int r = QFAST ? sl : f, q = q0 + (QFAST ? f : sl);
-        va[u] = sl < ns ? off[r] + V * q : -1;
-        if (va[u] >= 0) {
-          ma[u] = moff[r] + (long long)m * q;
-          v[u] = DIR == 0 ? vol[va[u]] : mat[ma[u]];
+        to[u] = -1;
+        if (sl < ns) {
+          const int r = QFAST ? sl : f, q = q0 + (QFAST ? f : sl);
+          const long long va = off[r] + V * q, ma = moff[r] + (long long)m * q;
+          v[u] = DIR == 0 ? vol[va] : mat[ma];
+          to[u] = DIR == 0 ? ma : va;
         }
         f += df;
         sl += ds;
@@ -661,10 +663,7 @@ __global__ void __launch_bounds__(256) lift_kernel(float2* __restrict__ vol, flo
       }
 #pragma unroll
       for (int u = 0; u < LB; ++u)
-        if (va[u] >= 0) {
-          if (DIR == 0) mat[ma[u]] = v[u];
-          else vol[va[u]] = v[u];
-        }
+        if (to[u] >= 0) (DIR == 0 ? mat : vol)[to[u]] = v[u];
     }
   }
 }
@@ -678,14 +677,21 @@ int launch_lift(const float2* vol, float2* mat, const int* vs, int nq, const int
   const long long tot = (long long)bs[0] * bs[1] * bs[2] * nq * n;
   if (tot == 0) return LLR_OK;
   if (tot < 0) return set_error(LLR_ERR_INVALID, "negative block count");
-  // rows per chunk: with few volumes a thread needs 1024 for four loads in flight (one 128^3 volume 36 us, 42 with 512),
-  // with more 512 (64^3 x 16 29 us, 38 with 1024); 256 where the call is too small for two CTAs per SM
+  // Rows per chunk: 512, with few volumes 1024, so that a thread has loads in flight; shorter chunks where the split of the
+  // volumes below would leave a chunk's offsets fewer than eight volumes to serve (55 x 119 x 17 x 25 in 5 x 6 x 8 blocks, both
+  // ways: 53 us with 512 rows and two volumes, 33 with 128 and seven).  The volumes are split for eight CTAs per SM where the
+  // chunks alone do not give them: one wave; for sixteen above 64 MB, where a second wave evens out the end (96 x 96 x 48 x 61
+  // in 6^3 blocks 229 us, 238 with eight; 48 x 48 x 24 x 20 in 8^3 blocks 25 us, 33 with sixteen).
   const long long rows = (long long)bs[0] * bs[1] * bs[2] * n;
-  const int rc = rows * nq < 148ll * 2 * 512 ? 256 : nq < 4 ? kLiftRows : 512;
-  const long long chunks = (rows + rc - 1) / rc;
-  // at least sixteen CTAs per SM where the rows alone do not give them: the volumes are split
-  const long long want = chunks < 148 * 16 ? std::min<long long>(nq, (148 * 16 + chunks - 1) / chunks) : 1;
-  const int qper = (int)((nq + want - 1) / want);
+  const long long ctas = 148 * (rows * nq > 8000000 ? 16 : 8);
+  int rc = nq < 4 ? kLiftRows : 512, qper;
+  long long chunks;
+  for (;; rc /= 2) {
+    chunks = (rows + rc - 1) / rc;
+    const long long want = chunks < ctas ? std::min<long long>(nq, (ctas + chunks - 1) / chunks) : 1;
+    qper = (int)((nq + want - 1) / want);
+    if (rc <= 128 || qper >= std::min(nq, 8)) break;
+  }
   dim3 grid((unsigned)std::min<long long>(chunks, 1ll << 30), (unsigned)((nq + qper - 1) / qper));
   const bool narrow = rows < (1ll << 31) && start >= 0 && start + n < (1ll << 31);
   // where a matrix has only one to three rows, a column's stores are single elements: 96^3 x 61 in 1^3 blocks took
